@@ -3,20 +3,24 @@
 // diagonal aligned to the bottom-right corner, grouped-query attention: H query heads share
 // Hk key/value heads, dropout on the probabilities from a Philox counter indexed by position).
 //
-// One CTA owns a 128-row query tile of one (batch, head). Roles:
-//   warp 0      TMA producer: Q once, then K_j / V_j tiles through a 2-stage ring
-//   warp 1      tcgen05 issuer: S_j = Q K_j^T and O_j = P_j V_j, accumulators in TMEM
-//   warps 2..9  softmax, two warps per scheduler: query row r is shared by two threads (warps 2..5 take key columns
-//               0..63 of every tile, warps 6..9 columns 64..127; a warp reaches the TMEM lanes of its own quarter
-//               only, so the split is by columns). Each reads its half of the S row with tcgen05.ld, the two exchange
-//               their row maxima through shared memory (one bounded rendezvous per tile), keep identical running
-//               maxima and their own partial sums, and write their half of P_j (bf16) to shared memory in the
-//               128-byte-swizzled K-major layout the second MMA consumes. One softmax warp per scheduler issued
-//               only a third of the cycles (a single warp cannot hide the MUFU and TMEM-load latencies); two do.
-// O accumulates in TMEM across all key tiles (the PV product runs with accumulate on); the exponent
-// reference trails the true running maximum by up to 2^8, so O is only rescaled in TMEM
-// (tcgen05.ld / st) on the rare tiles where a row maximum jumps. S is double-buffered in TMEM so the
-// tensor core computes tile j+1 while the softmax warps work on tile j.
+// One CTA runs two independent softmax streams of 128 query rows against the same tensor core, so that the products of one
+// stream hide behind the exponentials of the other. Roles:
+//   warp 0      TMA producer: the query tile(s) once, then K / V tiles through a ring in the order the products use them
+//   warp 1      tcgen05 issuer: S_t = Q_t K^T, then O_t += P_t V with P_t read from TMEM (it lies over the S_t it came from)
+//   warps 2..5  softmax of stream 0, warps 6..9 of stream 1: one thread owns one whole query row (a TMEM lane), so row
+//               maxima and sums need no exchange, and P goes back to TMEM without touching shared memory
+// The streams are two neighbouring query tiles (SPLIT = false: every K / V tile is loaded once for 256 rows), or, when that
+// would leave SMs without a CTA, the even and the odd key tiles of ONE query tile whose two results are merged at the end
+// (SPLIT = true: twice the CTAs, half the chain).
+//
+// What bounds it: the exponentials (16 per clock and SM: 1024 clocks for a 128 x 128 tile) and the two products of a D = 128
+// tile (1024 clocks) alike. Measured on a B200, forward alone, against the one-stream kernel this replaced (P through shared
+// memory, two threads a row that met at a barrier on every tile): batch 4, 32 heads, 2048 x 2048, D = 128, causal
+// 283 -> 187 us; batch 1, 32 / 8 heads, 8192 x 8192, D = 128, causal 847 -> 468 us; batch 32, 16 heads, 512 x 512, D = 64
+// 143 -> 88 us.
+// The exponent reference trails the true running maximum by up to 2^8, so O is only rescaled in TMEM (tcgen05.ld / st) on
+// the rare tiles where a row maximum jumps. tcgen05 products of one thread run in issue order, hence: S_t of the next tile
+// is issued right behind the P_t V that reads the same columns, and a finished S_t means that the P V before it is finished.
 //
 // Reference counterparts: oneflow/user/kernels/scaled_dot_product_attention_kernel.cu (flash
 // attention library call), fused_attention_kernels.cu :710 (CUTLASS fMHA, no sm_100 path) and the
@@ -37,36 +41,32 @@ struct FmhaFwdParams {
   int causal_off;       // Sk - Sq: query row r sees key columns <= r + causal_off
   DropoutCfg drop;
   float scale_log2e;    // softmax scale * log2(e)
+  int n_qt;             // query tiles (SPLIT) or pairs of query tiles of one head
+  int chunk;            // heads (of B * H) that are walked together, longest tiles first
   int* status;
 };
 
 template <int D>
 struct FmhaFwdCfg {
   static constexpr int BM = 128, BN = 128;
-  static constexpr int Q_BYTES = BM * D * 2;
+  static constexpr int Q_BYTES = BM * D * 2;            // one query tile
   static constexpr int KV_BYTES = BN * D * 2;
-  static constexpr int P_BYTES = BM * BN * 2;
-  static constexpr int BAR_BYTES = 128;                 // 14 mbarriers, the TMEM slot, the abort flag
-  static constexpr int XCHG_BYTES = 2 * 2 * 128 * 4;    // row maxima of the two column halves, one buffer per tile parity
+  static constexpr int SLOTS = D == 128 ? 5 : 8;        // K / V ring
+  static constexpr int BAR_BYTES = 256;                 // mbarriers, the TMEM slot, the abort flag
+  static constexpr int XCHG_BYTES = 2 * 128 * 8;        // SPLIT: row maximum and sum of both streams
   // At D = 128 the tiles take 224 KiB of the 227 KiB a CTA may have: the dynamic shared memory is declared 1024-byte
   // aligned (the kernel has no static shared memory, so it starts the CTA's window) instead of being aligned by hand
   // with a kilobyte of slack; the kernel checks the alignment and reports a status instead of running if it is not there.
-  static constexpr int SMEM_BYTES = Q_BYTES + 4 * KV_BYTES + 2 * P_BYTES + BAR_BYTES + XCHG_BYTES;
+  static constexpr int SMEM_BYTES = 2 * Q_BYTES + SLOTS * KV_BYTES + BAR_BYTES + XCHG_BYTES;
 };
 
-// ex2.approx: one MUFU op (inputs here are <= ~8, -inf gives 0)
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-template <int D, bool DROP>
+template <int D, bool DROP, bool SPLIT>
 __global__ void __launch_bounds__(320, 1)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, FmhaFwdParams p) {
   using Cfg = FmhaFwdCfg<D>;
   constexpr int BM = 128, BN = 128, DCH = D / 64;  // 64-element chunks along the head dimension
+  constexpr int SLOTS = Cfg::SLOTS;
   constexpr uint32_t IDESC_S = make_idesc_bf16(BM, BN, 0, 0);
   constexpr uint32_t IDESC_O = make_idesc_bf16(BM, D, 0, 1);
   constexpr int CH_BYTES = 128 * 128;  // one [128 rows x 64 elements] swizzled chunk
@@ -77,45 +77,57 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, (int)kStatusBounds);
     return;
   }
-  uint8_t* sQ = smem;
-  uint8_t* sK = sQ + Cfg::Q_BYTES;            // 2 stages
-  uint8_t* sV = sK + 2 * Cfg::KV_BYTES;       // 2 stages
-  uint8_t* sP = sV + 2 * Cfg::KV_BYTES;       // 2 buffers
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + 2 * Cfg::P_BYTES);
-  uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;     // [2]
-  uint64_t* v_full = bars + 3;     // [2]
-  uint64_t* kv_empty = bars + 5;   // [2]
-  uint64_t* s_full = bars + 7;     // [2]
-  uint64_t* p_full = bars + 9;     // [2]
-  uint64_t* pv_done = bars + 11;   // [2]
-  uint64_t* pair_bar = bars + 13;  // rendezvous of the 256 softmax threads
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint8_t* sQ = smem;                         // 2 tiles
+  uint8_t* sKV = sQ + 2 * Cfg::Q_BYTES;       // ring of K and V tiles
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + SLOTS * Cfg::KV_BYTES);
+  uint64_t* q_full = bars;               // [2]
+  uint64_t* kv_full = bars + 2;          // [SLOTS]
+  uint64_t* kv_empty = kv_full + SLOTS;  // [SLOTS]
+  uint64_t* s_full = kv_empty + SLOTS;   // [2]
+  uint64_t* p_full = s_full + 2;         // [2] 128 softmax threads of the stream
+  uint64_t* o_done = p_full + 2;         // [2]
+  uint64_t* pair_bar = o_done + 2;       // SPLIT: all 256 softmax threads, once
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pair_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* xchg = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + Cfg::BAR_BYTES);   // [2 parities][2 halves][128 rows]
+  static_assert((2 + 2 * SLOTS + 6 + 1) * 8 + 8 <= Cfg::BAR_BYTES, "barriers do not fit");
+  float2* xchg = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(bars) + Cfg::BAR_BYTES);   // [2 streams][128 rows]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Heavier (later) causal tiles first.
-  const int n_qt = (p.Sq + BM - 1) / BM;
-  const int qt = n_qt - 1 - static_cast<int>(blockIdx.x);
-  const int h = blockIdx.y, b = blockIdx.z;
+  // CTAs walk the heads in chunks whose keys and values stay in L2 together; inside a chunk the longest (last) causal tiles
+  // of all its heads come first, so that the short ones fill the tail.
+  const int in_chunk_max = p.chunk * p.n_qt;
+  const int ck = static_cast<int>(blockIdx.x) / in_chunk_max, rem = static_cast<int>(blockIdx.x) % in_chunk_max;
+  const int heads_here = min(p.chunk, p.B * p.H - ck * p.chunk);
+  const int qt = p.n_qt - 1 - rem / heads_here;
+  const int bh = ck * p.chunk + rem % heads_here;
+  const int h = bh % p.H, b = bh / p.H;
   const int hk = h / (p.H / p.Hk);
-  const int q0 = qt * BM;
+  const int q0 = qt * (SPLIT ? BM : 2 * BM);
   int kv_limit = p.Sk;
   if (p.kv_len) kv_limit = min(kv_limit, p.kv_len[b]);
-  int kv_end = kv_limit;
-  if (p.causal) kv_end = min(kv_end, q0 + BM + p.causal_off);
-  const int n_kv = kv_end > 0 ? (kv_end + BN - 1) / BN : 0;
+  // key tiles of stream t: all that its rows see, or every second one of them. Rows grow with the stream, so stream 1 never
+  // sees fewer tiles than stream 0 unless it has no rows at all.
+  int n_it[2];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int r0 = SPLIT ? q0 : q0 + t * BM;
+    int kv_end = kv_limit;
+    if (p.causal) kv_end = min(kv_end, r0 + BM + p.causal_off);
+    const int n = (kv_end > 0 && r0 < p.Sq) ? (kv_end + BN - 1) / BN : 0;
+    n_it[t] = SPLIT ? (n - t + 1) >> 1 : n;
+  }
+  const bool any = n_it[0] > 0 || n_it[1] > 0;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&v_full[s], 1);
+    for (int s = 0; s < SLOTS; ++s) {
+      mbar_init(&kv_full[s], 1);
       mbar_init(&kv_empty[s], 1);
-      mbar_init(&s_full[s], 1);
-      mbar_init(&p_full[s], 256);
-      mbar_init(&pv_done[s], 1);
+    }
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(&q_full[t], 1);
+      mbar_init(&s_full[t], 1);
+      mbar_init(&p_full[t], 128);
+      mbar_init(&o_done[t], 1);
     }
     mbar_init(pair_bar, 256);
     *abort_flag = 0;
@@ -132,222 +144,305 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tS = tmem_base;            // S[0], S[1] at +0, +128
-  const uint32_t tO = tmem_base + 256;      // running O accumulator, D columns
+  const uint32_t tS = tmem_base;            // S[0], S[1] at +0, +128; P[t] takes the first 64 columns of S[t]
+  const uint32_t tO = tmem_base + 256;      // O[0], O[1] at +0, +128, D columns each
 
   if (warp == 0) {
-    if (elect_one() && n_kv > 0) {
-      mbar_arrive_expect_tx(q_full, Cfg::Q_BYTES);
+    if (elect_one() && any) {
+      int c = 0;                             // loads issued so far: load c uses slot c % SLOTS
+      auto load_kv = [&](const CUtensorMap* m, int tile) -> bool {
+        const int s = c % SLOTS;
+        if (!mbar_wait(&kv_empty[s], ((c / SLOTS) & 1) ^ 1, abort_flag)) return false;
+        mbar_arrive_expect_tx(&kv_full[s], Cfg::KV_BYTES);
 #pragma unroll
-      for (int c = 0; c < DCH; ++c) tma_load_4d(sQ + c * CH_BYTES, &tmQ, q_full, c * 64, h, q0, b);
-      for (int j = 0; j < n_kv; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait(&kv_empty[s], ((j >> 1) & 1) ^ 1, abort_flag)) break;
-        mbar_arrive_expect_tx(&k_full[s], Cfg::KV_BYTES);
+        for (int d = 0; d < DCH; ++d) tma_load_4d(sKV + s * Cfg::KV_BYTES + d * CH_BYTES, m, &kv_full[s], d * 64, hk, tile * BN, b);
+        ++c;
+        return true;
+      };
+      auto load_q = [&](int t) {
+        mbar_arrive_expect_tx(&q_full[t], Cfg::Q_BYTES);
 #pragma unroll
-        for (int c = 0; c < DCH; ++c) tma_load_4d(sK + s * Cfg::KV_BYTES + c * CH_BYTES, &tmK, &k_full[s], c * 64, hk, j * BN, b);
-        mbar_arrive_expect_tx(&v_full[s], Cfg::KV_BYTES);
-#pragma unroll
-        for (int c = 0; c < DCH; ++c) tma_load_4d(sV + s * Cfg::KV_BYTES + c * CH_BYTES, &tmV, &v_full[s], c * 64, hk, j * BN, b);
+        for (int d = 0; d < DCH; ++d) tma_load_4d(sQ + t * Cfg::Q_BYTES + d * CH_BYTES, &tmQ, &q_full[t], d * 64, h, q0 + t * BM, b);
+      };
+      if (n_it[0] > 0) load_q(0);   // only what a product will wait for: no copy may be in flight when the CTA leaves
+      bool ok = load_kv(&tmK, 0);
+      if constexpr (SPLIT) {
+        const int n = n_it[0] + n_it[1];
+        if (n > 1) ok = ok && load_kv(&tmK, 1);
+        for (int g = 0; g < n && ok; ++g) {
+          ok = load_kv(&tmV, g);
+          if (ok && g + 2 < n) ok = load_kv(&tmK, g + 2);
+        }
+      } else {
+        if (n_it[1] > 0) load_q(1);
+        const int n = max(n_it[0], n_it[1]);
+        for (int i = 0; i < n && ok; ++i) {
+          ok = load_kv(&tmV, i);
+          if (ok && i + 1 < n) ok = load_kv(&tmK, i + 1);
+        }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (elect_one() && n_kv > 0) {
-      bool ok = mbar_wait(q_full, 0, abort_flag);
-      const uint32_t q_base = smem_u32(sQ);
-      auto issue_s = [&](int j) {
-        const int s = j & 1;
-        const uint32_t k_base = smem_u32(sK + s * Cfg::KV_BYTES);
+    if (elect_one() && any) {
+      const uint32_t kv_base = smem_u32(sKV);
+      auto slot_ready = [&](int c) -> bool { return mbar_wait(&kv_full[c % SLOTS], (c / SLOTS) & 1, abort_flag); };
+      auto issue_s = [&](int t, int c) {     // S_t = Q_t K^T with the K tile of load c
+        const uint32_t q_base = smem_u32(sQ + (SPLIT ? 0 : t) * Cfg::Q_BYTES);
+        const uint32_t k_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = (kk >> 2) * CH_BYTES + (kk & 3) * 32;
-          umma_bf16_ss(tS + s * BN, make_smem_desc_sw128(q_base + off, 16, 1024),
-                       make_smem_desc_sw128(k_base + off, 16, 1024), IDESC_S, kk != 0 ? 1u : 0u);
+          umma_bf16_ss(tS + t * BN, make_smem_desc_sw128(q_base + off, 16, 1024), make_smem_desc_sw128(k_base + off, 16, 1024),
+                       IDESC_S, kk != 0 ? 1u : 0u);
         }
-        umma_commit(&s_full[s]);
+        umma_commit(&s_full[t]);
       };
-      if (ok) ok = mbar_wait(&k_full[0], 0, abort_flag);
-      if (ok) { tc_fence_after(); issue_s(0); }
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int s = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (j + 1 < n_kv) {
-          if (!mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          issue_s(j + 1);
-        }
-        if (!mbar_wait(&p_full[s], ph, abort_flag)) { ok = false; break; }
-        if (!mbar_wait(&v_full[s], ph, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t p_base = smem_u32(sP + s * Cfg::P_BYTES);
-        const uint32_t v_base = smem_u32(sV + s * Cfg::KV_BYTES);
+      auto issue_pv = [&](int t, int c, bool first) {   // O_t (+)= P_t V with the V tile of load c
+        const uint32_t v_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES;
 #pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk) {
-          const uint64_t da = make_smem_desc_sw128(p_base + (kk >> 2) * CH_BYTES + (kk & 3) * 32, 16, 1024);
-          const uint64_t db = make_smem_desc_sw128(v_base + kk * 2048, CH_BYTES, 1024);
-          umma_bf16_ss(tO, da, db, IDESC_O, (j | kk) != 0 ? 1u : 0u);   // O accumulates in TMEM over all key tiles
+        for (int kk = 0; kk < BN / 16; ++kk)
+          umma_bf16_ts(tO + t * 128, tS + t * BN + kk * 8, make_smem_desc_sw128(v_base + kk * 2048, CH_BYTES, 1024), IDESC_O,
+                       (first && kk == 0) ? 0u : 1u);
+      };
+      auto release = [&](int c) { umma_commit(&kv_empty[c % SLOTS]); };
+      bool ok = true;
+      if constexpr (SPLIT) {
+        const int n = n_it[0] + n_it[1];
+        int c = 0;
+        ok = mbar_wait(&q_full[0], 0, abort_flag);
+        for (int t = 0; t < 2 && t < n && ok; ++t) {
+          ok = slot_ready(c);
+          if (!ok) break;
+          tc_fence_after();
+          issue_s(t, c);
+          release(c);
+          ++c;
         }
-        umma_commit(&pv_done[s]);
-        umma_commit(&kv_empty[s]);
+        for (int g = 0; g < n && ok; ++g) {
+          const int t = g & 1, i = g >> 1;
+          if (!mbar_wait(&p_full[t], i & 1, abort_flag) || !slot_ready(c)) { ok = false; break; }
+          tc_fence_after();
+          issue_pv(t, c, i == 0);
+          release(c);
+          ++c;
+          if (g + 2 < n) {
+            if (!slot_ready(c)) { ok = false; break; }
+            tc_fence_after();
+            issue_s(t, c);
+            release(c);
+            ++c;
+          } else {
+            umma_commit(&o_done[t]);
+          }
+        }
+      } else {
+        const int n = max(n_it[0], n_it[1]);
+        ok = slot_ready(0);
+        for (int t = 0; t < 2 && ok; ++t) {
+          if (n_it[t] == 0) continue;
+          ok = mbar_wait(&q_full[t], 0, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          issue_s(t, 0);
+        }
+        if (ok) release(0);
+        for (int i = 0; i < n && ok; ++i) {
+          const int cv = 2 * i + 1, ck1 = 2 * i + 2;      // loads of V_i and K_{i+1}
+          for (int t = 0; t < 2; ++t) {
+            if (i >= n_it[t]) continue;
+            if (!mbar_wait(&p_full[t], i & 1, abort_flag) || !slot_ready(cv)) { ok = false; break; }
+            tc_fence_after();
+            issue_pv(t, cv, i == 0);
+            if (t == 1 || i >= n_it[1]) release(cv);       // the last stream to use the tile
+            if (i + 1 < n_it[t]) {
+              if (!slot_ready(ck1)) { ok = false; break; }
+              tc_fence_after();
+              issue_s(t, ck1);
+              if (t == 1 || i + 1 >= n_it[1]) release(ck1);
+            } else {
+              umma_commit(&o_done[t]);
+            }
+          }
+        }
       }
     }
     __syncwarp();
-  } else if (n_kv > 0) {
+  } else {
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;        // which 64 key columns of every tile this thread takes
+    const int t = (warp - 2) >> 2;           // stream
     const int r = quad * 32 + lane;          // row inside the tile == TMEM lane
-    const int row_g = q0 + r;
+    const int row0 = SPLIT ? q0 : q0 + t * BM;
+    const int row_g = row0 + r;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
+    const uint32_t tSt = tS + lane_addr + t * BN, tOt = tO + lane_addr + t * 128;
+    const int n = n_it[t];
     // m_ref is the exponent reference actually used for P and l; it trails the true running maximum by at
     // most kLazy (log2 units) so that the TMEM-resident O only has to be rescaled when the maximum jumps.
-    // Both threads of a row carry the same m_ref (they see the same joint maxima); l_run is this half's sum.
     constexpr float kLazy = 8.0f;
     float m_ref = -INFINITY, l_run = 0.f;
     bool ok = true;
-    uint32_t pair_parity = 0;
-    auto pair_sync = [&]() {   // bounded: a thread that gave up elsewhere can never leave the others stuck here
-      mbar_arrive(pair_bar);
-      const bool w = mbar_wait(pair_bar, pair_parity, abort_flag);
-      pair_parity ^= 1;
-      return w;
-    };
-    for (int j = 0; j < n_kv; ++j) {
-      const int s = j & 1;
-      const uint32_t ph = (j >> 1) & 1;
-      if (!mbar_wait(&s_full[s], ph, abort_flag)) { ok = false; break; }
+    const uint64_t scale2 = pack_f32x2(__float_as_uint(p.scale_log2e), __float_as_uint(p.scale_log2e));
+    const int col_max = p.causal ? min(row_g + p.causal_off, kv_limit - 1) : kv_limit - 1;  // last visible column
+    for (int i = 0; i < n; ++i) {
+      const int col_base = (SPLIT ? 2 * i + t : i) * BN;
+      if (!mbar_wait(&s_full[t], i & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      const int col_base = j * BN + half * 64;
-      const bool need_mask = (p.causal && j * BN + BN - 1 > q0 + p.causal_off) || (j * BN + BN > kv_limit);
-      const int col_max = p.causal ? min(row_g + p.causal_off, kv_limit - 1) : kv_limit - 1;  // last visible column
-      uint32_t sv[2][32];
+      const bool need_mask = (p.causal && col_base + BN - 1 > row0 + p.causal_off) || (col_base + BN > kv_limit);
+      uint32_t sv[4][32];
       __syncwarp();
 #pragma unroll
-      for (int c = 0; c < 2; ++c) tmem_ld_32x32(tS + lane_addr + s * BN + half * 64 + c * 32, sv[c]);
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(tSt + c * 32, sv[c]);
       tmem_wait_ld();
-      // eight independent max chains: a dependent chain of 64 cannot be hidden
-      float mxs[8] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY, -INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (need_mask) {
+        const int lim = col_max - col_base;
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          // the scores stay unscaled here: the scale is positive, so the maximum commutes with it, and the exponent below
-          // applies it inside one fused multiply-add (one instruction per element less)
-          float e = __uint_as_float(sv[c][i]);
-          if (need_mask && col_base + c * 32 + i > col_max) { e = -INFINITY; sv[c][i] = __float_as_uint(e); }
-          mxs[i & 7] = fmaxf(mxs[i & 7], e);
-        }
+          for (int e = 0; e < 32; ++e)
+            if (c * 32 + e > lim) sv[c][e] = 0xFF800000u;   // -inf
+      }
+      // the scores stay unscaled here: the scale is positive, so the maximum commutes with it, and the exponent below
+      // applies it inside one fused multiply-add. Eight chains: a dependent chain of 128 cannot be hidden.
+      float mxs[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) mxs[e] = fmaxf(__uint_as_float(sv[0][e]), __uint_as_float(sv[0][e + 8]));
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int e = (c == 0 ? 16 : 0); e < 32; e += 16)
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            mxs[k] = fmaxf(fmaxf(mxs[k], __uint_as_float(sv[c][e + k])), __uint_as_float(sv[c][e + 8 + k]));
       float mx = fmaxf(fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])), fmaxf(fmaxf(mxs[4], mxs[5]), fmaxf(mxs[6], mxs[7])));
       mx *= p.scale_log2e;   // -inf stays -inf
-      // joint row maximum of the two halves (buffer = tile parity: the partner may be one tile behind, never two)
-      xchg[(s * 2 + half) * 128 + r] = mx;
-      if (!pair_sync()) { ok = false; break; }
-      mx = fmaxf(mx, xchg[(s * 2 + (half ^ 1)) * 128 + r]);
-      // Rescale O (and l) only when some row of the warp moved its maximum by more than kLazy.
-      const bool jump = mx > m_ref + kLazy;
-      if (__any_sync(0xffffffffu, jump)) {
+      // Rescale O (and l) only when some row of the warp moved its maximum by more than kLazy. S of this tile is finished,
+      // so every product of the tiles before it is: O may be touched without another wait.
+      if (__any_sync(0xffffffffu, mx > m_ref + kLazy)) {
         const float m_new = fmaxf(m_ref, mx);
         const float alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m_new);  // m_new is finite here or equals m_ref
-        if (j > 0) {
-          if (!mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          // each half rescales its half of the O columns
+        if (i > 0) {
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            const int cc = half * (D / 32) + c;
+          for (int cc = 0; cc < D / 16; ++cc) {
             uint32_t o[16];
-            tmem_ld_32x16(tO + lane_addr + cc * 16, o);
+            tmem_ld_32x16(tOt + cc * 16, o);
             tmem_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x16(tO + lane_addr + cc * 16, o);
+            for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+            tmem_st_32x16(tOt + cc * 16, o);
           }
-          tmem_wait_st();
         }
         l_run *= alpha;
         m_ref = m_new;
       }
-      const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-      if (j >= 2) {  // the P buffer of parity s was last read by the PV product of tile j-2
-        if (!mbar_wait(&pv_done[s], ((j - 2) >> 1) & 1, abort_flag)) { ok = false; break; }
-      }
-      float rs[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      uint8_t* chunk = sP + s * Cfg::P_BYTES + half * CH_BYTES + r * 128;   // 64 columns = one swizzled chunk
+      const float m_neg = m_ref == -INFINITY ? 0.f : -m_ref;
+      const uint64_t m_neg2 = pack_f32x2(__float_as_uint(m_neg), __float_as_uint(m_neg));
+      uint64_t rs[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < 4; ++c) {
         uint32_t packed[16];
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
+        for (int e = 0; e < 32; e += 4) {
           float pv[4];
+          unpack_f32x2(fma_f32x2(pack_f32x2(sv[c][e], sv[c][e + 1]), scale2, m_neg2), pv[0], pv[1]);
+          unpack_f32x2(fma_f32x2(pack_f32x2(sv[c][e + 2], sv[c][e + 3]), scale2, m_neg2), pv[2], pv[3]);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) pv[e] = fast_exp2(fmaf(__uint_as_float(sv[c][i + e]), p.scale_log2e, -m_use));  // masked entries are -inf -> 0
-          rs[(i >> 2) & 7] += (pv[0] + pv[1]) + (pv[2] + pv[3]);
+          for (int k = 0; k < 4; ++k) pv[k] = fast_exp2(pv[k]);   // masked entries are -inf -> 0
+          rs[(e >> 1) & 3] = add_f32x2(rs[(e >> 1) & 3], pack_f32x2(__float_as_uint(pv[0]), __float_as_uint(pv[1])));
+          rs[((e >> 1) + 1) & 3] = add_f32x2(rs[((e >> 1) + 1) & 3], pack_f32x2(__float_as_uint(pv[2]), __float_as_uint(pv[3])));
           if constexpr (DROP) {
             // the row sum keeps every probability; only what multiplies V is dropped (1 / keep is applied at the end)
-            const uint32_t keep = dropout_keep4(p.drop, static_cast<uint32_t>(b * p.H + h), static_cast<uint32_t>(row_g),
-                                                static_cast<uint32_t>((col_base + c * 32 + i) >> 2));
+            const uint32_t keep = dropout_keep4(p.drop, static_cast<uint32_t>(bh), static_cast<uint32_t>(row_g),
+                                                static_cast<uint32_t>((col_base + c * 32 + e) >> 2));
 #pragma unroll
-            for (int e = 0; e < 4; ++e) pv[e] = (keep >> e) & 1u ? pv[e] : 0.f;
+            for (int k = 0; k < 4; ++k) pv[k] = (keep >> k) & 1u ? pv[k] : 0.f;
           }
-          packed[i >> 1] = pack_bf16x2(pv[0], pv[1]);
-          packed[(i >> 1) + 1] = pack_bf16x2(pv[2], pv[3]);
+          packed[e >> 1] = pack_bf16x2(pv[0], pv[1]);
+          packed[(e >> 1) + 1] = pack_bf16x2(pv[2], pv[3]);
         }
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const int grp = c * 4 + g;
-          *reinterpret_cast<uint4*>(chunk + ((grp ^ (r & 7)) << 4)) =
-              make_uint4(packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]);
-        }
+        tmem_st_32x16(tSt + c * 16, packed);    // the whole row of S has left TMEM above
       }
-      l_run += ((rs[0] + rs[1]) + (rs[2] + rs[3])) + ((rs[4] + rs[5]) + (rs[6] + rs[7]));
-      fence_proxy_async_smem();
+      tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(&p_full[s]);
+      mbar_arrive(&p_full[t]);
+      float lo, hi;
+      unpack_f32x2(add_f32x2(add_f32x2(rs[0], rs[1]), add_f32x2(rs[2], rs[3])), lo, hi);
+      l_run += lo + hi;
     }
-    if (ok) {
-      // The row sum is the sum of the two halves' sums. It travels through the maxima buffer of the OTHER parity than the
-      // last tile's: every thread finished reading that one before it could pass the last tile's rendezvous.
-      const int so = (n_kv - 1) & 1;
-      xchg[(((so ^ 1) * 2) + half) * 128 + r] = l_run;
-      ok = pair_sync();
-      const float l_tot = ok ? l_run + xchg[(((so ^ 1) * 2) + (half ^ 1)) * 128 + r] : 0.f;
-      if (ok) ok = mbar_wait(&pv_done[so], ((n_kv - 1) >> 1) & 1, abort_flag);
+    if (ok && n > 0) ok = mbar_wait(&o_done[t], 0, abort_flag);
+    __nv_bfloat16* orow = p.out + ((static_cast<long long>(b) * p.Sq + row_g) * p.H + h) * D;
+    float* lse = p.lse ? p.lse + (static_cast<long long>(b) * p.H + h) * p.Sq + row_g : nullptr;
+    if constexpr (SPLIT) {
+      // O = (2^(m0 - m) O_0 + 2^(m1 - m) O_1) / l: both streams' accumulators lie in the same TMEM lanes, so each stream's
+      // threads write one half of the columns of the merged row.
+      if (ok) {
+        xchg[t * 128 + r] = make_float2(m_ref, l_run);
+        tc_fence_before();
+        mbar_arrive(pair_bar);
+        ok = mbar_wait(pair_bar, 0, abort_flag);
+      }
       if (ok) {
         tc_fence_after();
+        const float2 other = xchg[(t ^ 1) * 128 + r];
+        const float m0 = t == 0 ? m_ref : other.x, m1 = t == 0 ? other.x : m_ref;
+        const float l0 = t == 0 ? l_run : other.y, l1 = t == 0 ? other.y : l_run;
+        const float m = fmaxf(m0, m1);
+        const float a0 = m0 == -INFINITY ? 0.f : exp2f(m0 - m), a1 = m1 == -INFINITY ? 0.f : exp2f(m1 - m);
+        const float l_tot = a0 * l0 + a1 * l1;
         const float inv = l_tot > 0.f ? (DROP ? p.drop.inv_keep : 1.f) / l_tot : 0.f;
-        __nv_bfloat16* orow = p.out + ((static_cast<long long>(b) * p.Sq + row_g) * p.H + h) * D;
+        const float w0 = a0 * inv, w1 = a1 * inv;
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) {
-          const int cc = half * (D / 64) + c;     // each half writes its half of the output columns
-          uint32_t v[32];
+        for (int c0 = 0; c0 < D / 64; ++c0) {
+          const int cc = t * (D / 64) + c0;
+          uint32_t u[32], v[32];
           __syncwarp();
-          tmem_ld_32x32(tO + lane_addr + cc * 32, v);
+          // an accumulator that no product wrote holds whatever TMEM held before: it must not enter the sum even with weight 0
+          if (n_it[0] > 0) tmem_ld_32x32(tO + lane_addr + cc * 32, u);
+          if (n_it[1] > 0) tmem_ld_32x32(tO + lane_addr + 128 + cc * 32, v);
           tmem_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            float f = n_it[0] > 0 ? __uint_as_float(u[e]) * w0 : 0.f;
+            if (n_it[1] > 0) f = fmaf(__uint_as_float(v[e]), w1, f);
+            u[e] = __float_as_uint(f);
+          }
           if (row_g < p.Sq) {
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-              float f[8];
+              uint32_t w4[4];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[g * 8 + i]) * inv;
-              *reinterpret_cast<uint4*>(orow + cc * 32 + g * 8) =
-                  make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
-                             pack_bf16x2(f[6], f[7]));
+              for (int e = 0; e < 4; ++e) w4[e] = pack_bf16x2(__uint_as_float(u[g * 8 + 2 * e]), __uint_as_float(u[g * 8 + 2 * e + 1]));
+              *reinterpret_cast<uint4*>(orow + cc * 32 + g * 8) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
             }
           }
         }
-        if (half == 0 && row_g < p.Sq && p.lse)
-          p.lse[(static_cast<long long>(b) * p.H + h) * p.Sq + row_g] =
-              l_tot > 0.f ? (m_ref + log2f(l_tot)) * 0.6931471805599453f : -INFINITY;
+        if (t == 0 && row_g < p.Sq && lse) *lse = l_tot > 0.f ? (m + log2f(l_tot)) * 0.6931471805599453f : -INFINITY;
       }
-    }
-  } else {
-    // No visible keys at all (kv_len == 0, or a causal tile above the shifted diagonal): the output rows are zero.
-    const int r = (warp & 3) * 32 + lane;
-    const int row_g = q0 + r;
-    if (row_g < p.Sq) {
-      __nv_bfloat16* orow = p.out + ((static_cast<long long>(b) * p.Sq + row_g) * p.H + h) * D;
-      for (int i = 0; i < D; i += 8) *reinterpret_cast<uint4*>(orow + i) = make_uint4(0, 0, 0, 0);
-      if (p.lse) p.lse[(static_cast<long long>(b) * p.H + h) * p.Sq + row_g] = -INFINITY;
+    } else if (ok && n > 0) {
+      tc_fence_after();
+      const float inv = l_run > 0.f ? (DROP ? p.drop.inv_keep : 1.f) / l_run : 0.f;
+#pragma unroll
+      for (int cc = 0; cc < D / 32; ++cc) {
+        uint32_t v[32];
+        __syncwarp();
+        tmem_ld_32x32(tOt + cc * 32, v);
+        tmem_wait_ld();
+        if (row_g < p.Sq) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[g * 8 + e]) * inv;
+            *reinterpret_cast<uint4*>(orow + cc * 32 + g * 8) =
+                make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+          }
+        }
+      }
+      if (row_g < p.Sq && lse) *lse = l_run > 0.f ? (m_ref + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
+    } else if (ok && row_g < p.Sq) {
+      // No visible keys at all (kv_len == 0, or a causal tile above the shifted diagonal): the output rows are zero.
+      for (int e = 0; e < D; e += 8) *reinterpret_cast<uint4*>(orow + e) = make_uint4(0, 0, 0, 0);
+      if (lse) *lse = -INFINITY;
     }
   }
 
@@ -362,20 +457,43 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
-template <int D, bool DROP>
-static int launch_fmha_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FmhaFwdParams& p,
-                           cudaStream_t stream) {
+template <int D, bool DROP, bool SPLIT>
+static int launch_fmha_fwd_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, FmhaFwdParams p,
+                              cudaStream_t stream) {
   using Cfg = FmhaFwdCfg<D>;
-  auto kern = fmha_fwd_kernel<D, DROP>;
+  auto kern = fmha_fwd_kernel<D, DROP, SPLIT>;
   static bool configured = false;
   if (!configured) {
     OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     configured = true;
   }
-  dim3 grid((p.Sq + 127) / 128, p.H, p.B);
-  kern<<<grid, 320, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  p.n_qt = SPLIT ? (p.Sq + 127) / 128 : (p.Sq + 255) / 256;
+  // heads walked together: as many as keep their keys and values within a third of the L2 cache (the query heads of a group
+  // share theirs), but at least one CTA for every SM
+  const long long bh = static_cast<long long>(p.B) * p.H;
+  long long chunk = (40ll << 20) / (static_cast<long long>(p.Sk) * D * 4) * (p.H / p.Hk);
+  if (chunk * p.n_qt < 148) chunk = (148 + p.n_qt - 1) / p.n_qt;
+  p.chunk = static_cast<int>(chunk < bh ? chunk : bh);
+  const long long ctas = bh * p.n_qt;
+  if (ctas > 0x7FFFFFFFll) return fail("fmha: too many query tiles");
+  kern<<<static_cast<unsigned>(ctas), 320, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
+}
+
+template <int D, bool DROP>
+static int launch_fmha_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FmhaFwdParams& p,
+                           cudaStream_t stream) {
+  // Pairs of query tiles load every key once for 256 rows, but give half the CTAs of split key tiles, each with twice the
+  // chain. Splitting pays while all its CTAs run at once (batch 1, 8 heads, 2048 keys, D = 64: 20.3 against 33.9 us), and under
+  // a causal mask also up to one wave of pairs, as the short tiles of the second wave fill in behind the long ones (16 heads,
+  // 2048 keys, D = 128: 29.3 against 37.9 us; 4 heads, 8192 keys: 67 against 125 us) once there are keys enough to split
+  // (64 heads, 512 keys: 19.1 against 16.3 us). Otherwise pairs win (16 heads, 2048 keys, D = 128, full: 38.7 against 44.5 us;
+  // 16 heads, 4096 keys, causal: 71 against 82 us).
+  const long long bh = static_cast<long long>(p.B) * p.H;
+  const long long pairs = bh * ((p.Sq + 255) / 256), tiles = bh * ((p.Sq + 127) / 128);
+  if (tiles <= 148 || (p.causal && pairs < 148 && p.Sk >= 1024)) return launch_fmha_fwd_as<D, DROP, true>(tq, tk, tv, p, stream);
+  return launch_fmha_fwd_as<D, DROP, false>(tq, tk, tv, p, stream);
 }
 
 // 4-D map over a [B, S, H, D] view with a token stride of `row_stride` elements.

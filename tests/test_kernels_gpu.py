@@ -275,6 +275,35 @@ def test_fmha_fwd_padding_and_ragged():
     close(lse, rl, 1e-2, 1e-2)
 
 
+# Forward: pairs of query tiles (at least 148 of them: many heads) and key tiles split between the two streams of a CTA (few);
+# edges of the 128-row tiles, a pair whose second tile has no rows, odd numbers of key tiles, rows that see no key, short kv_len.
+@pytest.mark.parametrize("B,H,Hk,Sq,Sk,D,causal,lens", [
+    (10, 15, 15, 100, 129, 64, False, None),     # 150 pairs, second tile empty
+    (5, 16, 4, 257, 257, 128, True, None),       # 160 pairs, one row in the last tile
+    (5, 16, 16, 300, 140, 64, True, None),       # rows above the shifted diagonal see nothing; first tile of a pair may be idle
+    (37, 4, 2, 129, 385, 64, False, (0, 1, 128, 129, 385)),
+    (2, 3, 1, 257, 300, 128, True, None),        # split: one, two and three key tiles for a row tile
+    (1, 2, 2, 1, 1, 64, False, None),
+    (1, 2, 2, 130, 640, 64, False, (513,)),
+    (2, 2, 2, 200, 100, 128, True, None),
+])
+def test_fmha_streams_and_tile_edges(B, H, Hk, Sq, Sk, D, causal, lens):
+    torch.manual_seed(15)
+    q = torch.randn(B, Sq, H, D, device=DEV, dtype=BF)
+    k, v = (torch.randn(B, Sk, Hk, D, device=DEV, dtype=BF) for _ in range(2))
+    kv_len = None if lens is None else torch.tensor([lens[i % len(lens)] for i in range(B)], dtype=torch.int32, device=DEV)
+    sc = 1 / math.sqrt(D)
+    out, lse = K.fmha_fwd(q, k, v, causal=causal, kv_len=kv_len)
+    ro, rl = K.fmha_reference(q, k, v, causal, sc, kv_len)
+    # P is rounded to bf16 (half a unit in the last place is at most 2^-8 of the value) before it multiplies v, and both results
+    # are rounded to bf16: the difference is at most 2^-8 sum p |v| + 2 * 2^-8 |o|, with 2 % for the fp32 parts
+    ab, _ = K.fmha_reference(q, k, v.abs(), causal, sc, kv_len)
+    assert bool(((out.float() - ro.float()).abs() <= 1.02 * (ab.float() / 256 + ro.float().abs() / 128) + 1e-6).all())
+    seen = torch.isfinite(rl)
+    assert torch.equal(seen, torch.isfinite(lse))
+    close(lse[seen], rl[seen], 1e-2, 1e-2)
+
+
 def test_multi_tensor_adamw_sgd_and_norm():
     torch.manual_seed(12)
     sizes = [1000, 65536 + 8, 300000, 16]
