@@ -135,7 +135,7 @@ class _Fmha(torch.autograd.Function):
         q, k, v, out, lse = ctx.saved_tensors
         p, seed, offset = ctx.drop
         dq, dk, dv = K.fmha_bwd(q, k, v, out, d_o.contiguous(), lse, causal=ctx.causal, scale=ctx.scale, dropout_p=p, seed=seed,
-                                offset=offset)
+                                offset=offset, separate=True)   # views of a packed buffer would be copied by every consumer
         return dq, dk, dv, None, None, None, None, None
 
 

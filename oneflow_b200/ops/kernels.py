@@ -554,13 +554,13 @@ def fmha_bwd_reference(q, k, v, o, d_o, lse, causal, scale, kv_len=None, dropout
     return qf.grad.to(q.dtype), kf.grad.to(q.dtype), vf.grad.to(q.dtype)
 
 
-def fmha_bwd(q, k, v, o, d_o, lse, causal=False, scale=None, kv_len=None, dqkv=None, dropout_p=0.0, seed=0, offset=0):
+def fmha_bwd(q, k, v, o, d_o, lse, causal=False, scale=None, kv_len=None, dqkv=None, dropout_p=0.0, seed=0, offset=0, separate=False):
     """Fused attention backward. Self-attention with one head count (q, k, v of one shape): returns (dq, dk, dv) as
     [B,S,H,D] views of one packed [B,S,3,H,D] buffer (``dqkv`` if given), so that the QKV projection's backward consumes a
-    single matrix. Otherwise (other key length, fewer key/value heads): three separate contiguous tensors."""
+    single matrix. Otherwise (``separate``, other key length, fewer key/value heads): three separate contiguous tensors."""
     B, Sq, H, D = q.shape
     Sk, Hk = k.shape[1], k.shape[2]
-    packed = (Sk == Sq and Hk == H)
+    packed = Sk == Sq and Hk == H and (dqkv is not None or not separate)
     scale = float(scale) if scale is not None else 1.0 / math.sqrt(D)
     if not q.is_cuda:
         if dropout_p > 0.0:
@@ -583,9 +583,8 @@ def fmha_bwd(q, k, v, o, d_o, lse, causal=False, scale=None, kv_len=None, dqkv=N
         dq_stride = dkv_stride = 3 * H * D
     else:
         dq = torch.empty((B, Sq, H, D), dtype=torch.bfloat16, device=q.device)
-        dkv = torch.empty((B, Sk, 2, Hk, D), dtype=torch.bfloat16, device=q.device)
-        dk, dv = dkv[:, :, 0], dkv[:, :, 1]
-        dq_stride, dkv_stride = H * D, 2 * Hk * D
+        dk, dv = (torch.empty((B, Sk, Hk, D), dtype=torch.bfloat16, device=q.device) for _ in range(2))
+        dq_stride, dkv_stride = H * D, Hk * D
     _lib().ofb_fmha_bwd_scratch_floats.restype = c_longlong
     n = _lib().ofb_fmha_bwd_scratch_floats(c_int(B), c_int(Sq), c_int(H), c_int(D))
     scratch = torch.empty(n, dtype=torch.float32, device=q.device)
@@ -596,7 +595,7 @@ def fmha_bwd(q, k, v, o, d_o, lse, causal=False, scale=None, kv_len=None, dqkv=N
                                  c_int(B), c_int(Sq), c_int(Sk), c_int(H), c_int(Hk), c_int(D), c_int(int(causal)), c_float(scale),
                                  c_float(dropout_p), c_ulonglong(int(seed) & (2 ** 64 - 1)), c_uint(int(offset) & 0xFFFFFFFF),
                                  stream_ptr()), "fmha_bwd")
-    _count(4)
+    _count(3)
     return dq, dk, dv
 
 

@@ -277,6 +277,7 @@ def test_fmha_fwd_padding_and_ragged():
 
 # Forward: pairs of query tiles (at least 148 of them: many heads) and key tiles split between the two streams of a CTA (few);
 # edges of the 128-row tiles, a pair whose second tile has no rows, odd numbers of key tiles, rows that see no key, short kv_len.
+# Backward: one and several key tiles, a single row, both head sizes.
 @pytest.mark.parametrize("B,H,Hk,Sq,Sk,D,causal,lens", [
     (10, 15, 15, 100, 129, 64, False, None),     # 150 pairs, second tile empty
     (5, 16, 4, 257, 257, 128, True, None),       # 160 pairs, one row in the last tile
@@ -302,6 +303,11 @@ def test_fmha_streams_and_tile_edges(B, H, Hk, Sq, Sk, D, causal, lens):
     seen = torch.isfinite(rl)
     assert torch.equal(seen, torch.isfinite(lse))
     close(lse[seen], rl[seen], 1e-2, 1e-2)
+    d_o = torch.randn_like(out)
+    got = K.fmha_bwd(q, k, v, out, d_o, lse, causal=causal, kv_len=kv_len, separate=True)
+    assert all(t.is_contiguous() for t in got)
+    for g, r in zip(got, K.fmha_bwd_reference(q, k, v, out, d_o, lse, causal, sc, kv_len)):
+        close(g, r, 3e-2, 2e-2)
 
 
 def test_multi_tensor_adamw_sgd_and_norm():
