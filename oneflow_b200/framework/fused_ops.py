@@ -822,10 +822,10 @@ class _SparseXent(torch.autograd.Function):
         pl = ctx.pl
         if pl is not None:
             dloss = GT.rebox(dloss, ctx.nd_rows)
-        dl = _loc(dloss).reshape(-1, 1).to(torch.float32)
-        # (softmax - onehot) written over the logits' own storage (they are not needed again), then the row scale
-        _, d = K.xent_grad(ll, lab, stats, vocab_start=ctx.vocab_start, inplace=True)
-        d.mul_(dl.to(d.dtype))
+        dl = _loc(dloss).reshape(-1).to(torch.float32)
+        # (softmax - onehot) * dloss written over the logits' own storage (they are not needed again). Scaling the finished
+        # gradient in a second pass took 473 of the 2670 us of a 4096 x 50304 head and loss.
+        _, d = K.xent_grad(ll, lab, stats, vocab_start=ctx.vocab_start, inplace=True, row_scale=dl)
         return (GT.wrap(d, ctx.shape, pl, ctx.nd_logits) if pl is not None else d), None, None, None, None, None
 
 

@@ -322,8 +322,9 @@ def xent_merge(parts):
     return merged
 
 
-def xent_grad(logits, labels, merged, grad_scale=1.0, vocab_start=0, ignore_index=-100, want_grad=True, inplace=False):
-    """loss[row] = log(sum) + max - target ; dlogits = (softmax - onehot) * grad_scale. Returns (loss, dlogits)."""
+def xent_grad(logits, labels, merged, grad_scale=1.0, vocab_start=0, ignore_index=-100, want_grad=True, inplace=False, row_scale=None):
+    """loss[row] = log(sum) + max - target ; dlogits = (softmax - onehot) * grad_scale, times ``row_scale[row]`` (fp32, any
+    stride: an expanded scalar does) where given. Returns (loss, dlogits)."""
     rows, cols = logits.shape
     if not logits.is_cuda:
         gm, s, tgt = merged[:, 0], merged[:, 1], merged[:, 2]
@@ -338,13 +339,18 @@ def xent_grad(logits, labels, merged, grad_scale=1.0, vocab_start=0, ignore_inde
             d[idx, lab[idx]] -= 1.0
             d = d * grad_scale
             d[ign] = 0
+            if row_scale is not None:
+                d = d * row_scale.reshape(-1, 1)
             d = d.to(logits.dtype)
         return loss, d
     loss = torch.empty(rows, dtype=torch.float32, device=logits.device)
     d = (logits if inplace else torch.empty_like(logits)) if want_grad else None
-    check(_lib().ofb_xent_grad(ptr(logits), ptr(labels), ptr(merged), ptr(loss), ptr(d), c_int(rows), c_int(cols),
-                               c_longlong(logits.stride(0)), c_int(vocab_start), c_float(grad_scale),
-                               c_longlong(ignore_index), stream_ptr()), "xent_grad")
+    if row_scale is not None and (row_scale.dtype != torch.float32 or row_scale.shape != (rows,)):
+        raise ValueError(f"xent_grad: row_scale must be fp32 [{rows}], got {row_scale.dtype} {tuple(row_scale.shape)}")
+    check(_lib().ofb_xent_grad_scaled(ptr(logits), ptr(labels), ptr(merged), ptr(loss), ptr(d), c_int(rows), c_int(cols),
+                                      c_longlong(logits.stride(0)), c_int(vocab_start), c_float(grad_scale), c_longlong(ignore_index),
+                                      ptr(row_scale), c_longlong(row_scale.stride(0) if row_scale is not None else 0), stream_ptr()),
+          "xent_grad")
     _count()
     return loss, d
 

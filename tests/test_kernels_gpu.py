@@ -249,6 +249,32 @@ def test_xent(vocab):
     close(l2, ref, 1e-3, 1e-3)
 
 
+@pytest.mark.parametrize("rows,cols,expanded", [(1, 8, False), (3, 4096, True), (5, 16384 + 8, False), (1200, 2 * 16384 - 8, True)])
+def test_xent_row_scale_and_extremes(rows, cols, expanded):
+    """Widths around the 16384 elements a block takes per step, more rows than blocks, incoming gradients per row or one value;
+    entries of -inf, the type's lowest value and a row maximum that comes last."""
+    torch.manual_seed(16)
+    logits = torch.randn(rows, cols, device=DEV, dtype=BF) * 3
+    labels = torch.randint(0, cols, (rows,), device=DEV)
+    logits[0, : cols // 2] = float("-inf")
+    labels[0] = cols - 1
+    logits[-1, -1] = 40.0
+    if rows > 2:
+        logits[1] = torch.finfo(BF).min
+        logits[1, 3] = 1.0
+        labels[1] = 3
+        labels[2] = -100
+    g = torch.rand(1 if expanded else rows, device=DEV).add(0.5).expand(rows)
+    st = K.xent_stats(logits, labels)
+    loss, d = K.xent_grad(logits, labels, st, row_scale=g)
+    lf = logits.double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(lf, labels, reduction="none", ignore_index=-100)
+    (ref * g.double()).sum().backward()
+    # fp32 sums of exponentials that are good to 2 units in the last place; the gradient is rounded to bf16 once
+    close(loss, ref, 1e-5, 1e-5)
+    close(d, lf.grad, 2.0 ** -8 * 1.05, 1e-6)
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("causal", [False, True])
 def test_fmha_fwd(D, causal):
