@@ -84,6 +84,26 @@ def test_gemm_two_sm_kernel_epilogues(shape):
     close(out32, G.gemm_reference(a.cpu(), b.cpu(), out_dtype=torch.float32), rtol=1e-3)
 
 
+def test_gelu_of_the_epilogue_against_64_bits():
+    """Every bf16 value of magnitude 2^-20 .. 12 (and the extremes) through the epilogue's GELU and its gradient, fp32 results."""
+    pos = torch.arange(0x3580, 0x4141, dtype=torch.int32).to(torch.int16).view(BF)          # 2^-20 .. 12
+    x = torch.cat([pos, -pos, torch.tensor([0.0, 1e4, -1e4, 3e38], dtype=BF)])
+    x = torch.nn.functional.pad(x, (0, -x.numel() % 128)).view(-1, 128).to(DEV)
+    eye = torch.eye(128, device=DEV, dtype=BF)
+    y = G.gemm(x.clone(), eye, act="gelu", out_dtype=torch.float32)
+    xd = x.double().requires_grad_(True)
+    ref = xd * 0.5 * torch.erfc(-xd * 0.5 ** 0.5)     # erfc keeps the relative accuracy of the negative tail
+    ref.sum().backward()
+    # relative: 1.5e-7 of the fit, 2 units in the last place each of the exponential and the reciprocal, a dozen roundings; the
+    # exponent 0.72 x^2 and its constant are rounded to 2^-24 each, which the exponential turns into 6e-8 x^2
+    assert bool(((y.double() - ref).abs() <= (1.5e-6 + 6e-8 * xd.detach() ** 2) * ref.abs() + 1e-36).all())
+    ones = torch.ones(x.shape[0], 8, device=DEV, dtype=BF)
+    one = torch.zeros(128, 8, device=DEV, dtype=BF)
+    one[:, 0] = 1
+    g = G.gemm(ones, one, aux_in=x, act="gelu", out_dtype=torch.float32)
+    assert bool(((g.double() - xd.grad).abs() <= 1e-6 * xd.grad.abs() + 5e-7).all())
+
+
 def test_gemm_default_dispatch_reaches_two_sm_kernel():
     """A problem large enough for the dispatcher's own choice of the two-SM kernel (>= 74 tiles of 256 x 256)."""
     torch.manual_seed(7)
