@@ -41,7 +41,7 @@ static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   auto kern = gemm_bf16_2cta_kernel<A_MN, B_MN>;
   static bool configured = false;
   if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Cfg::SMEM_BYTES));
+    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Cfg::SMEM8_BYTES));
     configured = true;
   }
   static int sm_count = 0;
@@ -53,7 +53,7 @@ static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   const int tiles = ((shp.M + 255) / 256) * ((shp.N + 255) / 256);
   int grid = 2 * tiles < sm_count ? 2 * tiles : (sm_count & ~1);
   if (max_ctas > 1 && grid > (max_ctas & ~1)) grid = max_ctas & ~1;
-  kern<<<grid, 192, Gemm2Cfg::SMEM_BYTES, stream>>>(tmA, tmB, shp, ep, status);
+  kern<<<grid, Gemm2Cfg::THREADS, Gemm2Cfg::SMEM8_BYTES, stream>>>(tmA, tmB, shp, ep, status);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -77,16 +77,25 @@ int gemm_dispatch(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t str
   int bn = a->bn;
   const int mode2 = gemm_mode_2cta();
   bool two = bn == 512 || (mode2 == 1 && bn == 0);
+  // Cost of the three tilings in waves: a wave of the two-SM kernel (74 pairs, 256 x 256) is one unit; measured per wave, a
+  // 128 x 128 tile of the one-SM kernel takes 0.62 of it and a 128 x 256 tile 1.08. So the two-SM kernel wins whenever its tiles
+  // fill the machine, and also where the others would need a second wave (3072 x 1024 x 16384: 48 pairs 88 us, 192 tiles of
+  // 128 x 128 114 us, 96 of 128 x 256 96 us), while few tiles belong to the small tile (2331 x 768 x 3072: 22 against 29 us).
+  const long long tiles2 = (long long)((a->M + 255) / 256) * ((a->N + 255) / 256);
+  const long long tiles256 = (long long)((a->M + 127) / 128) * ((a->N + 255) / 256);
+  const long long tiles128 = (long long)((a->M + 127) / 128) * ((a->N + 127) / 128);
+  const double cost2 = static_cast<double>((tiles2 + 73) / 74);
+  const double cost256 = 1.08 * static_cast<double>((tiles256 + 147) / 148), cost128 = 0.62 * static_cast<double>((tiles128 + 147) / 148);
+  const double cost1 = cost256 < cost128 ? cost256 : cost128;
   if (mode2 == -1 && bn == 0) {
-    // default: the two-SM kernel for problems that fill the machine with 256 x 256 tiles
-    const long long tiles2 = (long long)((a->M + 255) / 256) * ((a->N + 255) / 256);
-    two = kDefault2Cta && tiles2 >= 74 && a->N >= 256 && a->M >= 256;
+    // Below K = 256 the main loop is shorter than the epilogue, which two one-SM CTAs per SM get through faster (802816 x 256 x 64:
+    // 136 against 156 us; 50176 x 1024 x 256: 56 against 49 us).
+    two = kDefault2Cta && cost2 <= cost1 && a->N >= 256 && a->M >= 256 && a->K >= 256;
   }
   if (mode2 == 0) two = bn == 512;
-  // Few K blocks and many tiles: the epilogue is the bottleneck, so run two one-SM CTAs per SM (short ring) instead.
-  const bool short_k = a->K <= 1024 && bn == 0 && !a_mn && (long long)((a->M + 127) / 128) * ((a->N + 127) / 128) >= 2 * 148 &&
-                       std::getenv("OFB_GEMM_SHORTK_OFF") == nullptr;
-  if (short_k) two = false;
+  // Few K blocks and many tiles: the epilogue is the bottleneck, so run two one-SM CTAs per SM (short ring) instead of one with a
+  // deep ring (802816 x 256 x 64: 136 against 228 us); from K = 768 the deep ring wins (2331 x 2304 x 768: 18 against 23 us).
+  const bool short_k = !two && a->K <= 512 && bn == 0 && !a_mn && tiles128 >= 2 * 148 && std::getenv("OFB_GEMM_SHORTK_OFF") == nullptr;
   if (two) {
     if (!a_mn) {
       if (get_tensor_map(&tmA, a->A, 2, 2, a->K, a->M, 0, (uint64_t)a->lda * 2, 0, 64, 128, 0, 3)) return -1;
@@ -106,11 +115,7 @@ int gemm_dispatch(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t str
     return launch_gemm_2cta<1, 1>(tmA, tmB, shp2, ep, st2, a->max_ctas, stream);
   }
   if (short_k) bn = 128;
-  if (bn != 128 && bn != 256) {
-    // Small problems: prefer more, smaller tiles so that all SMs get work.
-    long long tiles256 = (long long)((a->M + 127) / 128) * ((a->N + 255) / 256);
-    bn = (tiles256 >= 120 && a->N >= 256) ? 256 : 128;
-  }
+  if (bn != 128 && bn != 256) bn = (cost256 < cost128 && a->N >= 256) ? 256 : 128;
   if (!a_mn) {
     if (get_tensor_map(&tmA, a->A, 2, 2, a->K, a->M, 0, (uint64_t)a->lda * 2, 0, 64, 128, 0, 3)) return -1;
   } else {

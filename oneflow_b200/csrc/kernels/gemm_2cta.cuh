@@ -6,8 +6,11 @@
 // to both CTAs with `tcgen05.commit ... multicast::cluster`. TMA loads are plain (non-multicast) tile loads
 // issued by each CTA for its own shared memory, with their byte counts landing on the leader's mbarrier.
 //
-// Roles per CTA (192 threads): warp 0 TMA producer, warp 1 MMA issuer (leader only; both allocate TMEM),
-// warps 2..5 epilogue for the CTA's own 128 accumulator rows (same fused epilogue as the one-SM kernel).
+// Roles per CTA (320 threads): warp 0 TMA producer, warp 1 MMA issuer (leader only; both allocate TMEM),
+// warps 2..9 epilogue for the CTA's own 128 accumulator rows (same fused epilogue as the one-SM kernel): two warps per
+// TMEM lane quadrant, one for each half of the 256 columns. With four warps the epilogue of a tile took longer than its
+// products up to K = 2048 or so (16384 x 3072 x 1024 + bias: 97 us with four, 77 us with eight; 16384 x 4096 x 1024 + bias, GELU
+// and pre-activations: 226 and 136 us).
 #pragma once
 #include "gemm_tcgen05.cuh"
 
@@ -23,6 +26,12 @@ struct Gemm2Cfg {
   static constexpr int B_BYTES = BNH * BK * 2;
   static constexpr int EPI_BYTES = 4 * 32 * 128;  // staging tile of each epilogue warp (gemm_epilogue.cuh)
   static constexpr int SMEM_BYTES = STAGES * (A_BYTES + B_BYTES) + EPI_BYTES + 256 + 1024;
+  // the plain product: eight epilogue warps
+  static constexpr int EPI_WARPS = 8;
+  static constexpr int EPI8_BYTES = EPI_WARPS * 32 * 128;
+  static constexpr int SMEM8_BYTES = STAGES * (A_BYTES + B_BYTES) + EPI8_BYTES + 256 + 1024;
+  static constexpr int THREADS = 64 + EPI_WARPS * 32;
+  static_assert(SMEM8_BYTES <= 232448, "shared memory");
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -81,7 +90,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 }
 
 template <int A_MN, int B_MN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Gemm2Cfg::THREADS, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmShape shp,
                       GemmEpilogue ep, int* status) {
   using Cfg = Gemm2Cfg;
@@ -94,7 +103,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * A_BYTES;
   uint8_t* epi_stage = smem + STAGES * (A_BYTES + B_BYTES);
-  uint64_t* full = reinterpret_cast<uint64_t*>(epi_stage + Gemm2Cfg::EPI_BYTES);
+  uint64_t* full = reinterpret_cast<uint64_t*>(epi_stage + Gemm2Cfg::EPI8_BYTES);
   uint64_t* empty = full + STAGES;
   uint64_t* tfull = empty + STAGES;
   uint64_t* tempty = tfull + 2;
@@ -113,7 +122,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 8);   // 4 epilogue warps of each CTA of the pair (only the leader's copy is waited on)
+      mbar_init(&tempty[a], 2 * Cfg::EPI_WARPS);   // the epilogue warps of both CTAs of the pair (only the leader's copy is waited on)
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -206,9 +215,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     __syncwarp();
   } else {
-    // ---------------------------------------------------------------- epilogue (warps 2..5, both CTAs)
+    // ---------------------------------------------------------------- epilogue (warps 2..9, both CTAs)
     const int quad = warp & 3;
-    const uint32_t stage = smem_u32(epi_stage + quad * kEpiStageBytesPerWarp);
+    const int half = (warp - 2) >> 2;
+    const uint32_t stage = smem_u32(epi_stage + (warp - 2) * kEpiStageBytesPerWarp);
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = pair; t < total_tiles; t += n_pairs) {
@@ -218,7 +228,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) break;
       tc_fence_after();
       gemm_epilogue_warp<BN>(ep, shp, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN, m0 + quad * 32, n0, lane, stage,
-                             false);
+                             false, half * (BN / 64), (half + 1) * (BN / 64));
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&tempty[acc]), 0));   // the leader owns the accumulator hand-off
