@@ -15,6 +15,7 @@ Ranks outside a tensor's placement hold an empty placeholder and skip the local 
 """
 from __future__ import annotations
 
+import functools
 import math
 from typing import Sequence
 
@@ -35,6 +36,7 @@ def _rank():
     return dist.get_rank() if dist.is_initialized() else 0
 
 
+@functools.lru_cache(maxsize=4096)
 def _contig_strides(shape):
     st, acc = [], 1
     for s in reversed(shape):
@@ -75,9 +77,7 @@ class GlobalTensor(torch.Tensor):
         shape = tuple(int(s) for s in logical_shape)
         r = torch.Tensor._make_wrapper_subclass(cls, shape, strides=_contig_strides(shape), dtype=local.dtype,
                                                 device=local.device, layout=local.layout, requires_grad=requires_grad)
-        r._local = local
-        r._placement = placement
-        r._nd_sbp = tuple(nd_sbp)
+        r.__dict__.update(_loc=local, _thunk=None, _placement=placement, _nd_sbp=tuple(nd_sbp))
         return r
 
     def __init__(self, *a, **k):

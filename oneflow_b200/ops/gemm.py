@@ -15,6 +15,7 @@ import torch
 
 from . import _native
 
+_count = None     # kernels._count, bound at the first launch (kernels imports this module's siblings)
 ACT_NONE, ACT_GELU, ACT_GELU_TANH, ACT_RELU = 0, 1, 2, 3
 _ACT_NAMES = {None: 0, "none": 0, "gelu": 1, "gelu_tanh": 2, "relu": 3}
 
@@ -106,23 +107,18 @@ def gemm(a, b, *, a_layout="mk", b_layout="nk", bias=None, act=0, residual=None,
     if out_dtype not in (torch.bfloat16, torch.float32):
         raise TypeError("gemm: output must be bfloat16 or float32")
     aux = torch.empty((M, N), dtype=torch.bfloat16, device=a.device) if want_aux else None
-    args = _native.GemmArgs()
-    args.A, args.B, args.C = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    args.bias = bias.data_ptr() if bias is not None else None
-    args.residual = residual.data_ptr() if residual is not None else None
-    args.aux_in = aux_in.data_ptr() if aux_in is not None else None
-    args.aux_out = aux.data_ptr() if aux is not None else None
-    args.lda, args.ldb, args.ldc = a.stride(0), b.stride(0), out.stride(0)
-    args.ldr = residual.stride(0) if residual is not None else 0
-    args.ld_aux = aux_in.stride(0) if aux_in is not None else (aux.stride(0) if aux is not None else 0)
-    args.M, args.N, args.K = M, N, K
-    args.a_mn_major = 0 if a_layout == "mk" else 1
-    args.b_mn_major = 0 if b_layout == "nk" else 1
-    args.act, args.out_fp32, args.accumulate = act, int(out_dtype == torch.float32), int(bool(accumulate))
-    args.bn, args.max_ctas, args.alpha = bn, max_ctas, float(alpha)
     for t, nm in ((bias, "bias"), (residual, "residual"), (aux_in, "aux_in")):
         if t is not None and (t.dtype != torch.bfloat16 or t.data_ptr() % 16 != 0):
             raise TypeError(f"gemm: {nm} must be 16-byte aligned bfloat16")
+    # positional, in the order of GemmArgs._fields_: one call instead of an attribute store per field
+    args = _native.GemmArgs(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(),
+        None if bias is None else bias.data_ptr(), None if residual is None else residual.data_ptr(),
+        None if aux_in is None else aux_in.data_ptr(), None if aux is None else aux.data_ptr(),
+        a.stride(0), b.stride(0), out.stride(0), 0 if residual is None else residual.stride(0),
+        aux_in.stride(0) if aux_in is not None else (aux.stride(0) if aux is not None else 0),
+        M, N, K, 0 if a_layout == "mk" else 1, 0 if b_layout == "nk" else 1,
+        act, out_dtype == torch.float32, bool(accumulate), bn, max_ctas, alpha)
     lib = _native.kernels()
     if _native._recorder is not None:
         for t in (a, b, out, bias, residual, aux_in, aux):
@@ -130,6 +126,8 @@ def gemm(a, b, *, a_layout="mk", b_layout="nk", bias=None, act=0, residual=None,
                 _native._recorder.saw_tensor(t)
         _native._recorder.note(flops=2.0 * M * N * K, attrs=f"act={act} a={a_layout} b={b_layout}")
     _native.check(lib.ofb_gemm_bf16(args, _native.stream_ptr()), "ofb_gemm_bf16")
-    from . import kernels as _k
-    _k._count()
+    global _count
+    if _count is None:
+        from .kernels import _count
+    _count()
     return (out, aux) if want_aux else out
