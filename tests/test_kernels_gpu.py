@@ -186,6 +186,33 @@ def test_layer_norm(cols):
     close(db, rdb, 2e-2, 5e-2)
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 8), (17, 256), (9, 264), (2500, 512), (130, 520), (1300, 1024), (7, 1032), (1, 2048), (300, 2056)])
+def test_layer_norm_narrow_rows(rows, cols):
+    """Widths on both sides of what a warp's lanes hold (256, 512, 1024, 2048), one row to more rows than warps."""
+    torch.manual_seed(17)
+    x = torch.randn(rows, cols, device=DEV, dtype=BF) * 0.5 + 3.0
+    g, b = torch.randn(cols, device=DEV, dtype=BF), torch.randn(cols, device=DEV, dtype=BF)
+    dy, add = torch.randn(rows, cols, device=DEV, dtype=BF), torch.randn(rows, cols, device=DEV, dtype=BF)
+    y, mean, rstd = K.layer_norm_fwd(x, g, b, 1e-5)
+    xd, gd, bd = (t.double().requires_grad_(True) for t in (x, g, b))
+    ref = torch.nn.functional.layer_norm(xd, (cols,), gd, bd, 1e-5)
+    ref.backward(dy.double())
+    # one rounding of the result to bf16 (2^-8); fp32 sums: 2^-24 of |x| <= 6 against a spread of 0.5, a few times over
+    close(y, ref, 2.0 ** -8 * 1.02, 2e-5)
+    close(mean, xd.mean(1), 1e-6, 1e-6)
+    dx, dg, db = K.layer_norm_bwd(dy, x, g, mean, rstd, add_to_dx=add)
+    close(dx, xd.grad + add.double(), 2.0 ** -8 * 1.02, 1e-4)
+    close(dg, gd.grad, 1e-4, 1e-4 * rows ** 0.5)
+    close(db, bd.grad, 1e-5, 1e-5 * rows ** 0.5)
+    acc_g, acc_b = torch.ones(cols, device=DEV), torch.ones(cols, device=DEV)
+    dx2, _, _ = K.layer_norm_bwd(dy, x, g, mean, rstd, dgamma=acc_g, dbeta=acc_b)
+    close(dx2, xd.grad, 2.0 ** -8 * 1.02, 1e-4)
+    close(acc_g, gd.grad + 1, 1e-4, 1e-4 * rows ** 0.5)
+    close(acc_b, bd.grad + 1, 1e-5, 1e-5 * rows ** 0.5)
+    plain, _, _ = K.layer_norm_fwd(x, None, None, 1e-5)
+    close(plain, torch.nn.functional.layer_norm(xd, (cols,)), 2.0 ** -8 * 1.02, 2e-5)
+
+
 @pytest.mark.parametrize("act", [1, 2, 3])
 def test_bias_act(act):
     torch.manual_seed(4)
