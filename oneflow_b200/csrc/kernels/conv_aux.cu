@@ -5,6 +5,8 @@
 //
 // Reference: oneflow/user/kernels/normalization_kernel.cu (cuDNN BN + fused add/relu), pool_gpu_kernel / max_pool
 // kernels, adaptive_avg_pool_gpu_kernel.cu.
+#include <type_traits>
+
 #include "../common/host_utils.h"
 #include "../common/ptx.cuh"
 #include "ofb_kernels.h"
@@ -13,8 +15,7 @@ namespace ofb {
 
 typedef __nv_bfloat16 bf16;
 
-__device__ __forceinline__ void ld8(const bf16* p, float (&v)[8]) {
-  const uint4 q = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void un8(const uint4& q, float (&v)[8]) {
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -23,6 +24,7 @@ __device__ __forceinline__ void ld8(const bf16* p, float (&v)[8]) {
     v[2 * j + 1] = f.y;
   }
 }
+__device__ __forceinline__ void ld8(const bf16* p, float (&v)[8]) { un8(*reinterpret_cast<const uint4*>(p), v); }
 __device__ __forceinline__ void st8(bf16* p, const float (&v)[8]) {
   uint4 o;
   o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]);
@@ -32,12 +34,14 @@ __device__ __forceinline__ void st8(bf16* p, const float (&v)[8]) {
 
 // ------------------------------------------------------------------------------------------------ batch norm
 // Two per-channel sums over all rows in one pass. MODE 0: (x, x^2). MODE 1: (g, g * xhat) with
-// g = dy (* [y > 0] when relu) and xhat = (x - mean) * rstd. Threads are laid out as [row lane][8-channel vector];
+// g = dy (* [y > 0] when relu: from the forward's mask, else from y) and xhat = (x - mean) * rstd; g_out receives g when a
+// residual branch wants it as its gradient. Threads are laid out as [row lane][8-channel vector], several rows in flight each;
 // a block reduces its row lanes in shared memory and adds the result to out[0..C) and out[C..2C).
 template <int MODE>
 __global__ void __launch_bounds__(256)
-bn_reduce_kernel(const bf16* __restrict__ a, const bf16* __restrict__ x, const bf16* __restrict__ y, const float* __restrict__ mean,
-                 const float* __restrict__ rstd, long long rows, int C, int relu, float* out) {
+bn_reduce_kernel(const bf16* __restrict__ a, const bf16* __restrict__ x, const bf16* __restrict__ y,
+                 const unsigned char* __restrict__ mask, const float* __restrict__ mean, const float* __restrict__ rstd, long long rows,
+                 int C, int relu, bf16* __restrict__ g_out, float* out) {
   const int vpr = C >> 3;                       // 8-channel vectors per row
   const int vec = threadIdx.x % vpr;
   const int rlane = threadIdx.x / vpr;
@@ -53,31 +57,57 @@ bn_reduce_kernel(const bf16* __restrict__ a, const bf16* __restrict__ x, const b
     }
   }
   if (rlane < rlanes) {
-    for (long long r = blockIdx.x * (long long)rlanes + rlane; r < rows; r += (long long)gridDim.x * rlanes) {
-      float v[8];
-      ld8(a + r * C + vec * 8, v);
-      if (MODE == 0) {
+    // U rows: all loads first (no branch in between: with a bounds check per row the loads were not overlapped)
+    auto rows_at = [&](long long r0, long long step, auto n) {
+      constexpr int U = decltype(n)::value;
+      uint4 qa[U], qx[MODE == 1 ? U : 1], qy[MODE == 1 ? U : 1];
+      unsigned int bits[MODE == 1 ? U : 1];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          s1[j] += v[j];
-          s2[j] += v[j] * v[j];
-        }
-      } else {
-        float xv[8];
-        ld8(x + r * C + vec * 8, xv);
-        if (relu) {
-          float yv[8];
-          ld8(y + r * C + vec * 8, yv);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = yv[j] > 0.f ? v[j] : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          s1[j] += v[j];
-          s2[j] += v[j] * (xv[j] - mu[j]) * rs[j];
+      for (int u = 0; u < U; ++u) {
+        const long long r = r0 + u * step;
+        qa[u] = *reinterpret_cast<const uint4*>(a + r * C + vec * 8);
+        if constexpr (MODE == 1) {
+          qx[u] = *reinterpret_cast<const uint4*>(x + r * C + vec * 8);
+          if (mask) bits[u] = mask[r * vpr + vec];
+          else if (relu) qy[u] = *reinterpret_cast<const uint4*>(y + r * C + vec * 8);
         }
       }
-    }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float v[8];
+        un8(qa[u], v);
+        if constexpr (MODE == 0) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            s1[j] += v[j];
+            s2[j] += v[j] * v[j];
+          }
+        } else {
+          float xv[8];
+          un8(qx[u], xv);
+          if (mask) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = (bits[u] >> j) & 1u ? v[j] : 0.f;
+          } else if (relu) {
+            float yv[8];
+            un8(qy[u], yv);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = yv[j] > 0.f ? v[j] : 0.f;
+          }
+          if (g_out) st8(g_out + (r0 + u * step) * C + vec * 8, v);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            s1[j] += v[j];
+            s2[j] += v[j] * (xv[j] - mu[j]) * rs[j];
+          }
+        }
+      }
+    };
+    constexpr int U = MODE == 0 ? 1 : 4;      // one stream: the compiler overlaps the rounds by itself (four rows by hand: 108 against 67 us)
+    const long long step = (long long)gridDim.x * rlanes;
+    long long r0 = blockIdx.x * (long long)rlanes + rlane;
+    for (; r0 + (U - 1) * step < rows; r0 += U * step) rows_at(r0, step, std::integral_constant<int, U>());
+    for (; r0 < rows; r0 += step) rows_at(r0, step, std::integral_constant<int, 1>());
   }
   __shared__ float red[256 * 16];
 #pragma unroll
@@ -137,10 +167,11 @@ __device__ __forceinline__ void load_coef8(const float* p, float (&v)[8]) {
   v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
 }
 
-// y = [relu](scale * x + shift [+ residual])
+// y = [relu](scale * x + shift [+ residual]). `mask` receives one byte per eight channels, bit j = (y of channel j > 0): what the
+// backward needs of y, at a sixteenth of its bytes.
 __global__ void __launch_bounds__(256)
 bn_apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual, const float* __restrict__ scale,
-                const float* __restrict__ shift, long long vecs, int C, int relu, bf16* __restrict__ y) {
+                const float* __restrict__ shift, long long vecs, int C, int relu, bf16* __restrict__ y, unsigned char* __restrict__ mask) {
   const int vpr = C >> 3;
   const bool fixed = (blockDim.x % vpr) == 0;
   float sc[8], sh[8];
@@ -168,14 +199,22 @@ bn_apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual, c
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j], 0.f);
     }
+    if (mask) {
+      unsigned int bits = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) bits |= (__bfloat162float(__float2bfloat16(v[j])) > 0.f ? 1u : 0u) << j;
+      mask[i] = static_cast<unsigned char>(bits);
+    }
     st8(y + i * 8, v);
   }
 }
 
-// dx = a * g + b * x + c, g = dy (* [y > 0]); d_residual = g when wanted. coef = [a | b | c], each C long.
+// dx = a * g + b * x + c, g = dy (* [y > 0], from y or from the forward's mask). coef = [a | b | c], each C long. (A residual
+// branch takes g as its gradient: then the reduction has written it and this pass reads it as dy, without y.)
 __global__ void __launch_bounds__(256)
-bn_bwd_apply_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ y, const float* __restrict__ coef,
-                    long long vecs, int C, int relu, bf16* __restrict__ dx, bf16* __restrict__ d_residual) {
+bn_bwd_apply_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ y,
+                    const unsigned char* __restrict__ mask, const float* __restrict__ coef, long long vecs, int C, int relu,
+                    bf16* __restrict__ dx) {
   const int vpr = C >> 3;
   const bool fixed = (blockDim.x % vpr) == 0;
   float ca[8], cb[8], cc[8];
@@ -195,13 +234,16 @@ bn_bwd_apply_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, con
     float g[8], xv[8];
     ld8(dy + i * 8, g);
     ld8(x + i * 8, xv);
-    if (relu) {
+    if (relu && mask) {
+      const unsigned int bits = mask[i];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] = (bits >> j) & 1u ? g[j] : 0.f;
+    } else if (relu) {
       float yv[8];
       ld8(y + i * 8, yv);
 #pragma unroll
       for (int j = 0; j < 8; ++j) g[j] = yv[j] > 0.f ? g[j] : 0.f;
     }
-    if (d_residual) st8(d_residual + i * 8, g);
     float o[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = fmaf(ca[j], g[j], fmaf(cb[j], xv[j], cc[j]));
@@ -408,21 +450,26 @@ static inline int aux_grid(long long items) {
   return static_cast<int>(b);
 }
 
-// sums [2 C] fp32 must be zero on entry. mode 0: sums of x and x^2 (pass x as `a`). mode 1: sums of g and g * xhat.
-OFB_API int ofb_bn_reduce(int mode, const void* a, const void* x, const void* y, const float* mean, const float* rstd, long long rows,
-                          int C, int relu, float* sums, void* stream) {
+// sums [2 C] fp32 must be zero on entry. mode 0: sums of x and x^2 (pass x as `a`). mode 1: sums of g and g * xhat; with relu the
+// sign of the forward's output comes from `mask` (ofb_bn_apply) or, when that is null, from y; g_out (may be null) receives g.
+OFB_API int ofb_bn_reduce(int mode, const void* a, const void* x, const void* y, const void* mask, const float* mean, const float* rstd,
+                          long long rows, int C, int relu, void* g_out, float* sums, void* stream) {
   if (C % 8 || C > 2048) return fail("bn: channels must be a multiple of 8, at most 2048");
   if (rows == 0) return 0;
   const int vpr = C / 8;
   const int rlanes = 256 / vpr;
   long long blocks = (rows + rlanes * 16 - 1) / (rlanes * 16);
-  if (blocks > 148 * 8) blocks = 148 * 8;
+  // few blocks: every one of them ends in 2 C atomic additions (12544 x 2048, mode 0: 27 us with eight blocks per SM, 20 with three)
+  const int per_sm = mode == 0 ? 3 : 2;
+  if (blocks > 148 * per_sm) blocks = 148 * per_sm;
   if (blocks < 1) blocks = 1;
   if (mode == 0)
-    bn_reduce_kernel<0><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const bf16*)a, nullptr, nullptr, nullptr, nullptr, rows, C, 0, sums);
+    bn_reduce_kernel<0><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const bf16*)a, nullptr, nullptr, nullptr, nullptr, nullptr, rows,
+                                                                         C, 0, nullptr, sums);
   else
-    bn_reduce_kernel<1><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const bf16*)a, (const bf16*)x, (const bf16*)y, mean, rstd, rows, C,
-                                                                         relu, sums);
+    bn_reduce_kernel<1><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const bf16*)a, (const bf16*)x, (const bf16*)y,
+                                                                         relu ? (const unsigned char*)mask : nullptr, mean, rstd, rows, C, relu, (bf16*)g_out,
+                                                                         sums);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -436,27 +483,27 @@ OFB_API int ofb_bn_finalize(const float* sums, long long rows, float eps, float 
   return 0;
 }
 
-// y = [relu](scale * x + shift [+ residual]) with per-channel fp32 scale / shift.
+// y = [relu](scale * x + shift [+ residual]) with per-channel fp32 scale / shift; mask [rows * C / 8] bytes or null.
 OFB_API int ofb_bn_apply(const void* x, const void* residual, const float* scale, const float* shift, long long rows, int C, int relu,
-                         void* y, void* stream) {
+                         void* y, void* mask, void* stream) {
   if (C % 8) return fail("bn: channels must be a multiple of 8");
   const long long vecs = rows * (C / 8);
   if (vecs == 0) return 0;
   bn_apply_kernel<<<aux_grid(vecs), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (const bf16*)residual, scale, shift, vecs, C, relu,
-                                                                  (bf16*)y);
+                                                                  (bf16*)y, (unsigned char*)mask);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
 // coef [3 C] is scratch written here. sums = [sum g | sum g xhat] from ofb_bn_reduce(mode 1).
-OFB_API int ofb_bn_bwd_apply(const void* dy, const void* x, const void* y, const float* mean, const float* rstd, const float* gamma,
-                             const float* sums, float* coef, long long rows, int C, int relu, void* dx, void* d_residual, void* stream) {
+OFB_API int ofb_bn_bwd_apply(const void* dy, const void* x, const void* y, const void* mask, const float* mean, const float* rstd,
+                             const float* gamma, const float* sums, float* coef, long long rows, int C, int relu, void* dx, void* stream) {
   if (C % 8) return fail("bn: channels must be a multiple of 8");
   const long long vecs = rows * (C / 8);
   if (vecs == 0) return 0;
   bn_bwd_coeffs_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(sums, mean, rstd, gamma, 1.f / rows, C, coef);
-  bn_bwd_apply_kernel<<<aux_grid(vecs), 256, 0, (cudaStream_t)stream>>>((const bf16*)dy, (const bf16*)x, (const bf16*)y, coef, vecs, C, relu,
-                                                                      (bf16*)dx, (bf16*)d_residual);
+  bn_bwd_apply_kernel<<<aux_grid(vecs), 256, 0, (cudaStream_t)stream>>>((const bf16*)dy, (const bf16*)x, (const bf16*)y,
+                                                                      (const unsigned char*)mask, coef, vecs, C, relu, (bf16*)dx);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -118,20 +118,22 @@ class _BN:
         self.relu, self.has_res = relu, residual is not None
         if not net.training:
             return N.bn_eval_fwd(x, gamma, beta, rm, rv, residual, relu, net.cfg.bn_eps)
-        y, self.mean, self.rstd = N.bn_train_fwd(x, gamma, beta, residual, relu, net.cfg.bn_eps, net.cfg.bn_momentum, rm, rv)
-        self.x, self.y = x, (y if relu else None)
+        # on the GPU the backward takes the sign of y from one bit per element instead of y itself
+        self.mask = torch.empty(x.numel() // 8, dtype=torch.uint8, device=x.device) if relu and x.is_cuda else None
+        y, self.mean, self.rstd = N.bn_train_fwd(x, gamma, beta, residual, relu, net.cfg.bn_eps, net.cfg.bn_momentum, rm, rv, self.mask)
+        self.x, self.y = x, (y if relu and self.mask is None else None)
         return y
 
     def bwd(self, dy):
         net = self.net
         gamma = net.master(self.name + ".weight")
-        dx, dres, dgamma, dbeta = N.bn_train_bwd(dy, self.x, self.y, self.mean, self.rstd, gamma, self.relu, self.has_res)
+        dx, dres, dgamma, dbeta = N.bn_train_bwd(dy, self.x, self.y, self.mean, self.rstd, gamma, self.relu, self.has_res, self.mask)
         for nm, g in ((self.name + ".weight", dgamma), (self.name + ".bias", dbeta)):
             if net.store.acc_flag(nm):
                 net.store.g[nm].add_(g)
             else:
                 net.store.g[nm].copy_(g)
-        self.x = self.y = None
+        self.x = self.y = self.mask = None
         return dx, dres
 
 

@@ -20,8 +20,9 @@ def _lib():
 
 
 # ------------------------------------------------------------------------------------------------ batch norm
-def bn_train_fwd(x, gamma, beta, residual=None, relu=False, eps=1e-5, momentum=0.1, running_mean=None, running_var=None):
-    """x [..., C] bf16; gamma / beta fp32 [C]. Returns (y, mean, rstd) with batch statistics over all leading dims."""
+def bn_train_fwd(x, gamma, beta, residual=None, relu=False, eps=1e-5, momentum=0.1, running_mean=None, running_var=None, mask=None):
+    """x [..., C] bf16; gamma / beta fp32 [C]. Returns (y, mean, rstd) with batch statistics over all leading dims. ``mask``
+    (CUDA only): uint8 [x.numel() / 8], receives one bit per element, y > 0, for ``bn_train_bwd``."""
     C = x.shape[-1]
     rows = x.numel() // C
     if not x.is_cuda:
@@ -43,11 +44,11 @@ def bn_train_fwd(x, gamma, beta, residual=None, relu=False, eps=1e-5, momentum=0
     mean, rstd, scale, shift = stats[0], stats[1], stats[2], stats[3]
     y = torch.empty_like(x)
     lib = _lib()
-    check(lib.ofb_bn_reduce(c_int(0), ptr(x), None, None, None, None, c_longlong(rows), c_int(C), c_int(0), ptr(sums), stream_ptr()),
+    check(lib.ofb_bn_reduce(c_int(0), ptr(x), None, None, None, None, None, c_longlong(rows), c_int(C), c_int(0), None, ptr(sums), stream_ptr()),
           "bn_reduce")
     check(lib.ofb_bn_finalize(ptr(sums), c_longlong(rows), c_float(eps), c_float(momentum), c_int(C), ptr(gamma), ptr(beta), ptr(mean),
                               ptr(rstd), ptr(scale), ptr(shift), ptr(running_mean), ptr(running_var), stream_ptr()), "bn_finalize")
-    check(lib.ofb_bn_apply(ptr(x), ptr(residual), ptr(scale), ptr(shift), c_longlong(rows), c_int(C), c_int(int(relu)), ptr(y),
+    check(lib.ofb_bn_apply(ptr(x), ptr(residual), ptr(scale), ptr(shift), c_longlong(rows), c_int(C), c_int(int(relu)), ptr(y), ptr(mask),
                            stream_ptr()), "bn_apply")
     K._count(3)
     return y, mean, rstd
@@ -66,13 +67,14 @@ def bn_eval_fwd(x, gamma, beta, running_mean, running_var, residual=None, relu=F
     scale = (gamma.float() * rstd).contiguous()
     shift = (beta.float() - running_mean.float() * scale).contiguous()
     check(_lib().ofb_bn_apply(ptr(x), ptr(residual), ptr(scale), ptr(shift), c_longlong(rows), c_int(C), c_int(int(relu)), ptr(y),
-                              stream_ptr()), "bn_apply")
+                              None, stream_ptr()), "bn_apply")
     K._count()
     return y
 
 
-def bn_train_bwd(dy, x, y, mean, rstd, gamma, relu=False, want_residual_grad=False):
-    """Returns (dx, d_residual or None, dgamma, dbeta); y is only read when relu."""
+def bn_train_bwd(dy, x, y, mean, rstd, gamma, relu=False, want_residual_grad=False, mask=None):
+    """Returns (dx, d_residual or None, dgamma, dbeta); y is only read when relu, and not at all when the forward's ``mask`` is
+    given (a sixteenth of its bytes in both passes)."""
     C = x.shape[-1]
     rows = x.numel() // C
     if not x.is_cuda:
@@ -89,10 +91,12 @@ def bn_train_bwd(dy, x, y, mean, rstd, gamma, relu=False, want_residual_grad=Fal
     dres = torch.empty_like(x) if want_residual_grad else None
     lib = _lib()
     dy = dy.contiguous()
-    check(lib.ofb_bn_reduce(c_int(1), ptr(dy), ptr(x), ptr(y), ptr(mean), ptr(rstd), c_longlong(rows), c_int(C), c_int(int(relu)), ptr(sums),
-                            stream_ptr()), "bn_reduce")
-    check(lib.ofb_bn_bwd_apply(ptr(dy), ptr(x), ptr(y), ptr(mean), ptr(rstd), ptr(gamma), ptr(sums), ptr(coef), c_longlong(rows), c_int(C),
-                               c_int(int(relu)), ptr(dx), ptr(dres), stream_ptr()), "bn_bwd_apply")
+    check(lib.ofb_bn_reduce(c_int(1), ptr(dy), ptr(x), ptr(y), ptr(mask), ptr(mean), ptr(rstd), c_longlong(rows), c_int(C), c_int(int(relu)),
+                            ptr(dres), ptr(sums), stream_ptr()), "bn_reduce")
+    if dres is not None:       # the reduction wrote the masked gradient: the second pass reads that and neither y nor the mask
+        dy, y, mask, relu = dres, None, None, False
+    check(lib.ofb_bn_bwd_apply(ptr(dy), ptr(x), ptr(y), ptr(mask), ptr(mean), ptr(rstd), ptr(gamma), ptr(sums), ptr(coef), c_longlong(rows),
+                               c_int(C), c_int(int(relu)), ptr(dx), stream_ptr()), "bn_bwd_apply")
     K._count(2)
     return dx, dres, sums[C:], sums[:C]
 

@@ -213,6 +213,35 @@ def test_layer_norm_narrow_rows(rows, cols):
     close(plain, torch.nn.functional.layer_norm(xd, (cols,)), 2.0 ** -8 * 1.02, 2e-5)
 
 
+@pytest.mark.parametrize("rows,C,residual", [(1, 8, False), (37, 96, True), (5003, 64, True), (4099, 64, False), (130, 2048, True)])
+def test_batch_norm_sign_mask(rows, C, residual):
+    """The backward from the forward's one-bit mask: the same masked gradient as from y (bit for bit), and right against 64 bits.
+    Channel counts that do and do not divide a block, rows around the ones a thread keeps in flight."""
+    from oneflow_b200.ops import cnn as N
+    torch.manual_seed(18)
+    x, dy = torch.randn(rows, C, device=DEV, dtype=BF), torch.randn(rows, C, device=DEV, dtype=BF)
+    res = torch.randn(rows, C, device=DEV, dtype=BF) if residual else None
+    g, b = torch.rand(C, device=DEV) + 0.5, torch.randn(C, device=DEV)
+    mask = torch.empty(rows * C // 8, device=DEV, dtype=torch.uint8)
+    y, mean, rstd = N.bn_train_fwd(x, g, b, res, True, mask=mask)
+    bits = (mask.view(-1, 1) >> torch.arange(8, device=DEV, dtype=torch.uint8)) & 1
+    assert torch.equal(bits.view(rows, C).bool(), y > 0)
+    dx, dres, dg, db = N.bn_train_bwd(dy, x, None, mean, rstd, g, True, residual, mask=mask)
+    dx2, dres2, dg2, db2 = N.bn_train_bwd(dy, x, y, mean, rstd, g, True, residual)
+    masked = torch.where(y > 0, dy, torch.zeros_like(dy))
+    if residual:
+        assert torch.equal(dres, masked) and torch.equal(dres2, masked)
+    gd = masked.double()
+    xh = (x.double() - mean.double()) * rstd.double()
+    s1, s2 = gd.sum(0), (gd * xh).sum(0)
+    ref = g.double() * rstd.double() * (gd - s1 / rows - xh * s2 / rows)
+    for d, sg, sb in ((dx, dg, db), (dx2, dg2, db2)):
+        # fp32 sums of up to 5003 terms in any order, 2^-24 each against their magnitude; dx rounded to bf16 once
+        close(sg, s2, 1e-5, 1e-5 * rows ** 0.5)
+        close(sb, s1, 1e-5, 1e-5 * rows ** 0.5)
+        close(d, ref, 2.0 ** -8 * 1.02, 1e-5 * float(rstd.max()))
+
+
 @pytest.mark.parametrize("act", [1, 2, 3])
 def test_bias_act(act):
     torch.manual_seed(4)
