@@ -242,6 +242,36 @@ def test_batch_norm_sign_mask(rows, C, residual):
         close(d, ref, 2.0 ** -8 * 1.02, 1e-5 * float(rstd.max()))
 
 
+@pytest.mark.parametrize("N,H,W,C,R,stride,pad,ldc", [(2, 224, 224, 3, 7, 2, 3, 152), (1, 9, 11, 3, 7, 2, 3, 152), (3, 5, 7, 4, 3, 1, 1, 40),
+                                                      (1, 1, 1, 1, 3, 1, 1, 16), (1, 4, 5000, 8, 3, 2, 1, 72)])
+def test_im2col_small(N, H, W, C, R, stride, pad, ldc):
+    """Odd sizes, padding columns, one pixel, and rows too wide for shared memory; copies, so bit for bit."""
+    from oneflow_b200.ops import cnn
+    x = torch.randn(N, H, W, C, device=DEV, dtype=BF)
+    got, hw = cnn.im2col_small(x, R, R, stride, pad, ldc)
+    ref, hw2 = cnn.im2col_small(x.cpu(), R, R, stride, pad, ldc)
+    assert hw == hw2 and torch.equal(got.cpu(), ref)
+
+
+@pytest.mark.parametrize("N,H,W,C", [(2, 7, 9, 8), (1, 1, 1, 16), (3, 56, 56, 24)])
+def test_pool_and_stride_index_kernels(N, H, W, C):
+    from oneflow_b200.ops import cnn
+    x = torch.randn(N, H, W, C, device=DEV, dtype=BF)
+    y, idx = cnn.maxpool3x3s2_fwd(x)
+    ry, ridx = cnn.maxpool3x3s2_fwd(x.cpu())
+    assert torch.equal(y.cpu(), ry)
+    dy = torch.randn_like(y)
+    # up to four bf16 gradients meet in fp32 and are rounded once; ties between equal pixels may choose either of them
+    d, rd = cnn.maxpool3x3s2_bwd(dy, idx, (N, H, W, C)).cpu().float(), cnn.maxpool3x3s2_bwd(dy.cpu(), ridx, (N, H, W, C)).float()
+    assert float(((d - rd).abs() > 2.0 ** -8 * rd.abs() + 1e-6).float().mean()) < 5e-3
+    s = cnn.subsample2(x)
+    assert torch.equal(s, x[:, ::2, ::2])
+    up = cnn.upsample2_zero(s, (N, H, W, C))
+    ref = torch.zeros_like(x)
+    ref[:, ::2, ::2] = s
+    assert torch.equal(up, ref)
+
+
 @pytest.mark.parametrize("act", [1, 2, 3])
 def test_bias_act(act):
     torch.manual_seed(4)
