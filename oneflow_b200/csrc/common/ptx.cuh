@@ -148,6 +148,38 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // ---------------------------------------------------------------------------------------------
+// Cluster launch control: a running CTA takes over the block index of one that has not been launched yet, so that a grid of
+// ordinary size runs as persistent CTAs in the hardware's own order. The answer (16 bytes) arrives like a bulk copy; after one
+// that says "nothing left" the CTA must not ask again.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void clc_ask(void* answer, uint64_t* bar) {
+  mbar_arrive_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(answer)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// True when the answer hands over a block index (`next`).
+__device__ __forceinline__ bool clc_take(const void* answer, int& next) {
+  uint32_t got, x;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      ".reg .b128 A;\n\t"
+      ".reg .b32 y, z, w;\n\t"
+      "ld.shared.b128 A, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 P, A;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@P clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, y, z, w}, A;\n\t"
+      "}\n"
+      : "=r"(got), "=r"(x)
+      : "r"(smem_u32(answer))
+      : "memory");
+  next = static_cast<int>(x);
+  return got != 0;
+}
+
+// ---------------------------------------------------------------------------------------------
 // tcgen05 / TMEM
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {

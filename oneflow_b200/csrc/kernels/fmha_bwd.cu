@@ -1,7 +1,7 @@
 // Fused multi-head attention backward for sm_100a (bf16, head dim 64 or 128; query length != key length,
 // grouped-query attention and Philox dropout as in the forward kernel).
 //
-// One CTA owns a 128-key tile (K_j, V_j stay resident in shared memory) of one (batch, key/value head)
+// A CTA works on one 128-key tile at a time (K_j, V_j stay resident in shared memory) of one (batch, key/value head)
 // and walks over the query tiles i that see it, for every query head of the group in turn (so dK and dV of a
 // shared key/value head accumulate in TMEM and need no second reduction). Per (i, j) pair five tcgen05 products run,
 // all fed from the same shared-memory tiles without any transposition pass. The scores are formed transposed (TMEM lane =
@@ -20,10 +20,12 @@
 // (at D = 128 dQ has no TMEM columns of its own and takes those of dP).
 // What bounds it: shared-memory bandwidth (per pair at D = 128 the products read 288 KiB of operands, staging dS and dQ and
 // the copies of Q, dO and dQ move 224 KiB: 4100 clocks, the products themselves 2560), then the fp32 reductions of dQ in L2.
+// The grid has one CTA per key tile, but a running CTA takes over the next one that has not started (cluster launch control), so
+// that barriers, TMEM and the first loads of a tile do not wait for the end of the one before; the order stays the hardware's.
 // Measured on a B200 with delta and the dQ conversion, against the kernel this replaced (one chain S -> P -> dV -> dP -> dS
-// -> dK, dQ -> drain per pair, nothing overlapped): batch 4, 32 heads, 2048 x 2048, D = 128, causal 843 -> 501 us; batch 1,
-// 32 / 8 heads, 8192 x 8192, D = 128, causal 2960 -> 1470 us; batch 32, 16 heads, 512 x 512, D = 64 349 -> 222 us (there a
-// CTA lives for four pairs, and its start and end cost as much as these).
+// -> dK, dQ -> drain per pair, nothing overlapped), and without the take-over in brackets: batch 4, 32 heads, 2048 x 2048,
+// D = 128, causal 843 -> 454 us (504); batch 1, 32 / 8 heads, 8192 x 8192, D = 128, causal 2960 -> 1445 us (1490); batch 32,
+// 16 heads, 512 x 512, D = 64 349 -> 215 us (243); batch 8, 16 heads, 500 x 1100, D = 64 179 -> 101 us (118).
 // TMEM: S/P | dP (D = 128: also dQ) | dV | dK | D = 64: dQ.
 //
 // Reference counterpart: oneflow/user/kernels/scaled_dot_product_attention_grad_kernel.cu
@@ -65,7 +67,8 @@ struct FmhaBwdCfg {
   static constexpr int SLAB_BYTES = 128 * 32 * 4;        // 32 columns of dQ in fp32, two of them in flight
   static constexpr int STAT_BYTES = 2 * 2 * 128 * 4;     // log-sum-exp and delta of two query tiles
   // no slack for aligning by hand: the dynamic shared memory starts the CTA's window (checked by the kernel)
-  static constexpr int SMEM_BYTES = (4 + DO_STAGES) * T_BYTES + DS_BYTES + 2 * SLAB_BYTES + STAT_BYTES + 256;
+  static constexpr int BAR_BYTES = 288;                  // 28 mbarriers, TMEM slot, abort flag, two answers of 16 bytes
+  static constexpr int SMEM_BYTES = (4 + DO_STAGES) * T_BYTES + DS_BYTES + 2 * SLAB_BYTES + STAT_BYTES + BAR_BYTES;
   static_assert(SMEM_BYTES <= 232448, "shared memory");
 };
 
@@ -125,28 +128,48 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* dq_full = bars + 19;
   uint64_t* dq_drained = bars + 20; // 128
   uint64_t* all_done = bars + 21;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  uint64_t* kv_empty = bars + 22;   // every product of a key tile has finished
+  uint64_t* acc_free = bars + 23;   // 256: dK and dV have left TMEM
+  uint64_t* next_full = bars + 24;  // [2] the answer that names the CTA's next key tile
+  uint64_t* next_empty = bars + 26; // [2] 16 warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
+  uint8_t* answers = reinterpret_cast<uint8_t*>(bars + 30);   // [2] 16 bytes
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // heads in chunks whose queries, gradients and dQ accumulators stay in L2 together; inside a chunk the key tiles that most
-  // query tiles see (the first ones) come first, so that the short ones fill the tail
-  const int in_chunk_max = p.chunk * p.n_kt;
-  const int ck = static_cast<int>(blockIdx.x) / in_chunk_max, rem = static_cast<int>(blockIdx.x) % in_chunk_max;
-  const int heads_here = min(p.chunk, p.B * p.Hk - ck * p.chunk);
-  const int jt = rem / heads_here;
-  const int bhk = ck * p.chunk + rem % heads_here;
-  const int hk = bhk % p.Hk, b = bhk / p.Hk;
+  // Key tile number `item`: heads in chunks whose queries, gradients and dQ accumulators stay in L2 together; inside a chunk the
+  // key tiles that most query tiles see (the first ones) come first, so that the short ones fill the tail.
   const int group = p.H / p.Hk;          // query heads per key/value head
-  const int k0 = jt * 128;
   const int n_qt = (p.Sq + 127) / 128;
-  int kv_limit = p.Sk;
-  if (p.kv_len) kv_limit = min(kv_limit, p.kv_len[b]);
-  // first query tile with a row that sees this key tile: row + causal_off >= k0
-  const int i_start = p.causal ? max(0, k0 - p.causal_off) / 128 : 0;
-  const bool tile_visible = k0 < kv_limit;
-  const int n_i = tile_visible ? max(0, n_qt - i_start) : 0;   // query tiles per head
-  const int n_iter = n_i * group;                               // iteration t: head hk*group + t / n_i, tile i_start + t % n_i
+  struct Item {
+    int hk, b, k0, kv_limit;
+    int i_start;   // first query tile with a row that sees this key tile: row + causal_off >= k0
+    int n_iter;    // pairs: query tiles i_start .. n_qt - 1 of every head of the group
+  };
+  auto item_of = [&](int item) {
+    const int in_chunk_max = p.chunk * p.n_kt;
+    const int ck = item / in_chunk_max, rem = item % in_chunk_max;
+    const int heads_here = min(p.chunk, p.B * p.Hk - ck * p.chunk);
+    const int bhk = ck * p.chunk + rem % heads_here;
+    Item it;
+    it.hk = bhk % p.Hk;
+    it.b = bhk / p.Hk;
+    it.k0 = rem / heads_here * 128;
+    it.kv_limit = p.kv_len ? min(p.Sk, p.kv_len[it.b]) : p.Sk;
+    it.i_start = p.causal ? max(0, it.k0 - p.causal_off) / 128 : 0;
+    it.n_iter = it.k0 < it.kv_limit ? max(0, n_qt - it.i_start) * group : 0;
+    return it;
+  };
+  // The CTA works through key tiles until none is left: every role walks the same sequence. `n` counts the tiles.
+  auto next_item = [&](int n, int& item) -> bool {      // called by whole warps
+    const bool ok = mbar_wait(&next_full[n & 1], (n >> 1) & 1, abort_flag);
+    int nx = 0;
+    const bool more = ok && clc_take(answers + (n & 1) * 16, nx);
+    item = nx;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&next_empty[n & 1]);
+    return more;
+  };
 
   if (threadIdx.x == 0) {
     mbar_init(k_full, 1);
@@ -167,6 +190,12 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(dq_full, 1);
     mbar_init(dq_drained, 128);
     mbar_init(all_done, 1);
+    mbar_init(kv_empty, 1);
+    mbar_init(acc_free, 256);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&next_full[s], 1);
+      mbar_init(&next_empty[s], 16);
+    }
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
@@ -189,132 +218,169 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t tdK = tmem_base + 256 + D;
   const uint32_t tdQ = kOwnDq ? tmem_base + 256 + 2 * D : tdP;
 
-  // registers: 512 threads x 128 at launch = 4 warpgroups x (48 + 144 + 160 + 160)
+  // registers: 512 threads x 128 at launch = 4 warpgroups x 128 on average; the drain warps hold D columns of dQ each
+  constexpr int kRegsControl = D == 64 ? 80 : 64, kRegsDrain = D == 64 ? 112 : 144, kRegsCompute = D == 64 ? 160 : 152;
+  static_assert(kRegsControl + kRegsDrain + 2 * kRegsCompute == 512, "a split above the launch's registers would wait for ever");
   if (warp < 4) {
-    reg_dec<48>();
-    if (warp == 0) {
-      if (elect_one() && n_iter > 0) {
-        auto load = [&](uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int head, int row) {
-          mbar_arrive_expect_tx(bar, Cfg::T_BYTES);
+    reg_dec<kRegsControl>();
+    int item = blockIdx.x;
+    int g0 = 0;        // pairs of the tiles before this one: pair t of this tile is number g0 + t, which gives slots and phases
+    int act = 0;       // tiles before this one that had any pair
+    bool ok = true;
+    for (int n = 0;; ++n) {
+      const Item it = item_of(item);
+      if (warp == 0) {
+        if (elect_one()) {
+          // Ask for the next tile a few pairs before the loads of this one end: early enough for the answer to be there, late
+          // enough that long tiles do not bind another one at their start (that cost 14 % at 512 causal tiles of 46 to 256 pairs).
+          auto ask = [&]() {      // both slots' readers of two tiles ago are done
+            if (!mbar_wait(&next_empty[n & 1], ((n >> 1) & 1) ^ 1, abort_flag)) return;
+            fence_proxy_async_smem();
+            clc_ask(answers + (n & 1) * 16, &next_full[n & 1]);
+          };
+          const int ask_at = max(0, it.n_iter - 4);
+          if (it.n_iter == 0 || !ok) ask();
+          if (it.n_iter > 0 && ok) {
+            auto load = [&](uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int head, int row) {
+              mbar_arrive_expect_tx(bar, Cfg::T_BYTES);
 #pragma unroll
-          for (int c = 0; c < DCH; ++c) tma_load_4d(dst + c * CH_BYTES, m, bar, c * 64, head, row, b);
-        };
-        load(sK, &tmK, k_full, hk, k0);
-        int h = hk * group, i = i_start;
-        for (int t = 0; t < n_iter; ++t) {
-          const int st = t & 1, sd = t % DO_ST;
-          if (!mbar_wait(&q_empty[st], ((t >> 1) & 1) ^ 1, abort_flag)) break;
-          load(sQ + st * Cfg::T_BYTES, &tmQ, &q_full[st], h, i * 128);
-          if (t == 0) load(sV, &tmV, v_full, hk, k0);
-          if (!mbar_wait(&do_empty[sd], ((t / DO_ST) & 1) ^ 1, abort_flag)) break;
-          load(sdO + sd * Cfg::T_BYTES, &tmdO, &do_full[sd], h, i * 128);
-          if (++i == n_qt) { i = i_start; ++h; }
+              for (int c = 0; c < DCH; ++c) tma_load_4d(dst + c * CH_BYTES, m, bar, c * 64, head, row, it.b);
+            };
+            int h = it.hk * group, i = it.i_start;
+            for (int t = 0; t < it.n_iter; ++t) {
+              const int g = g0 + t, st = g & 1, sd = g % DO_ST;
+              if (t == ask_at) ask();
+              if (!mbar_wait(&q_empty[st], ((g >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
+              load(sQ + st * Cfg::T_BYTES, &tmQ, &q_full[st], h, i * 128);
+              if (t == 0) {
+                if (!mbar_wait(kv_empty, (act & 1) ^ 1, abort_flag)) { ok = false; break; }
+                load(sK, &tmK, k_full, it.hk, it.k0);
+                load(sV, &tmV, v_full, it.hk, it.k0);
+              }
+              if (!mbar_wait(&do_empty[sd], ((g / DO_ST) & 1) ^ 1, abort_flag)) { ok = false; break; }
+              load(sdO + sd * Cfg::T_BYTES, &tmdO, &do_full[sd], h, i * 128);
+              if (++i == n_qt) { i = it.i_start; ++h; }
+            }
+          }
         }
-      }
-      __syncwarp();
-    } else if (warp == 1) {
-      if (elect_one() && n_iter > 0) {
-        const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV), ds_base = smem_u32(sdS);
-        auto kk_off = [](int kk) -> uint32_t { return (kk >> 2) * CH_BYTES + (kk & 3) * 32; };   // K-major step of 16
-        auto issue_s = [&](int t) {
-          const uint32_t q_base = smem_u32(sQ + (t & 1) * Cfg::T_BYTES);
+        __syncwarp();
+      } else if (warp == 1) {
+        if (elect_one() && it.n_iter > 0 && ok) {
+          const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV), ds_base = smem_u32(sdS);
+          auto kk_off = [](int kk) -> uint32_t { return (kk >> 2) * CH_BYTES + (kk & 3) * 32; };   // K-major step of 16
+          auto issue_s = [&](int g) {
+            const uint32_t q_base = smem_u32(sQ + (g & 1) * Cfg::T_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk)
-            umma_bf16_ss(tS, make_smem_desc_sw128(k_base + kk_off(kk), 16, 1024), make_smem_desc_sw128(q_base + kk_off(kk), 16, 1024),
-                         IDESC_S, kk != 0 ? 1u : 0u);
-          umma_commit(s_full);
-        };
-        auto issue_dp = [&](int t) {
-          const uint32_t do_base = smem_u32(sdO + (t % DO_ST) * Cfg::T_BYTES);
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk)
-            umma_bf16_ss(tdP, make_smem_desc_sw128(v_base + kk_off(kk), 16, 1024), make_smem_desc_sw128(do_base + kk_off(kk), 16, 1024),
-                         IDESC_S, kk != 0 ? 1u : 0u);
-          umma_commit(dp_full);
-        };
-        bool ok = mbar_wait(k_full, 0, abort_flag) && mbar_wait(&q_full[0], 0, abort_flag);
-        if (ok) { tc_fence_after(); issue_s(0); }
-        ok = ok && mbar_wait(v_full, 0, abort_flag) && mbar_wait(&do_full[0], 0, abort_flag);
-        if (ok) { tc_fence_after(); issue_dp(0); }
-        for (int t = 0; t < n_iter && ok; ++t) {
-          const uint32_t ph = t & 1;
-          const uint32_t q_base = smem_u32(sQ + (t & 1) * Cfg::T_BYTES);
-          const uint32_t do_base = smem_u32(sdO + (t % DO_ST) * Cfg::T_BYTES);
-          // dV += P^T dO_i
-          if (!mbar_wait(p_ready, ph, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_bf16_ts(tdV, tS + (kk >> 2) * 64 + (kk & 3) * 8, make_smem_desc_sw128(do_base + kk * 2048, CH_BYTES, 1024), IDESC_KV,
-                         (t | kk) != 0 ? 1u : 0u);
-          umma_commit(&do_empty[t % DO_ST]);   // dP of this pair was issued before
-          // S^T of the next pair, over the P that dV has read by then
-          if (t + 1 < n_iter) {
-            if (!mbar_wait(&q_full[(t + 1) & 1], ((t + 1) >> 1) & 1, abort_flag)) { ok = false; break; }
+            for (int kk = 0; kk < D / 16; ++kk)
+              umma_bf16_ss(tS, make_smem_desc_sw128(k_base + kk_off(kk), 16, 1024), make_smem_desc_sw128(q_base + kk_off(kk), 16, 1024),
+                           IDESC_S, kk != 0 ? 1u : 0u);
+            umma_commit(s_full);
+          };
+          // dP^T of pair g: its columns are free once dS of the pair before was read (that pair's dQ waited for it) and, at
+          // D = 128, the dQ in them was drained
+          auto issue_dp = [&](int g) -> bool {
+            if (!mbar_wait(&do_full[g % DO_ST], (g / DO_ST) & 1, abort_flag)) return false;
+            if (!kOwnDq && g > 0 && !mbar_wait(dq_drained, (g - 1) & 1, abort_flag)) return false;
             tc_fence_after();
-            issue_s(t + 1);
-          }
-          // dQ partial = dS K_j, then dK += dS^T Q_i while dQ is drained
-          if (!mbar_wait(ds_ready, ph, abort_flag)) { ok = false; break; }
-          if (kOwnDq && t > 0 && !mbar_wait(dq_drained, (t - 1) & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
+            const uint32_t do_base = smem_u32(sdO + (g % DO_ST) * Cfg::T_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_bf16_ss(tdQ, make_smem_desc_sw128(ds_base + kk * 2048, CH_BYTES, 1024),
-                         make_smem_desc_sw128(k_base + kk * 2048, CH_BYTES, 1024), IDESC_DQ, kk != 0 ? 1u : 0u);
-          umma_commit(dq_full);
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_bf16_ss(tdK, make_smem_desc_sw128(ds_base + kk_off(kk), 16, 1024),
-                         make_smem_desc_sw128(q_base + kk * 2048, CH_BYTES, 1024), IDESC_KV, (t | kk) != 0 ? 1u : 0u);
-          umma_commit(ds_free);
-          umma_commit(&q_empty[t & 1]);
-          if (t + 1 < n_iter) {
-            const int sd = (t + 1) % DO_ST;
-            if (!mbar_wait(&do_full[sd], ((t + 1) / DO_ST) & 1, abort_flag)) { ok = false; break; }
-            if (!kOwnDq && !mbar_wait(dq_drained, ph, abort_flag)) { ok = false; break; }
+            for (int kk = 0; kk < D / 16; ++kk)
+              umma_bf16_ss(tdP, make_smem_desc_sw128(v_base + kk_off(kk), 16, 1024), make_smem_desc_sw128(do_base + kk_off(kk), 16, 1024),
+                           IDESC_S, kk != 0 ? 1u : 0u);
+            umma_commit(dp_full);
+            return true;
+          };
+          ok = mbar_wait(k_full, act & 1, abort_flag) && mbar_wait(&q_full[g0 & 1], (g0 >> 1) & 1, abort_flag);
+          if (ok) { tc_fence_after(); issue_s(g0); }
+          ok = ok && mbar_wait(v_full, act & 1, abort_flag);
+          ok = ok && issue_dp(g0);
+          // the accumulators of the tile before have left TMEM
+          ok = ok && mbar_wait(acc_free, (act & 1) ^ 1, abort_flag);
+          for (int t = 0; t < it.n_iter && ok; ++t) {
+            const int g = g0 + t;
+            const uint32_t ph = g & 1;
+            const uint32_t q_base = smem_u32(sQ + (g & 1) * Cfg::T_BYTES);
+            const uint32_t do_base = smem_u32(sdO + (g % DO_ST) * Cfg::T_BYTES);
+            // dV += P^T dO_i
+            if (!mbar_wait(p_ready, ph, abort_flag)) { ok = false; break; }
             tc_fence_after();
-            issue_dp(t + 1);
-          }
-        }
-        if (ok) umma_commit(all_done);
-      }
-      __syncwarp();
-    } else if (n_iter > 0) {
-      // warp 2: log-sum-exp in log2 units, +inf where the row does not exist or saw no key (P becomes 0); warp 3: -delta
-      int h = hk * group, i = i_start;
-      for (int t = 0; t < n_iter; ++t) {
-        const int st = t & 1;
-        float val[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int row = i * 128 + lane * 4 + e;
-          const long long idx = (static_cast<long long>(b) * p.H + h) * p.Sq + row;
-          if (warp == 2) {
-            const float l = row < p.Sq ? p.lse[idx] : -INFINITY;
-            val[e] = l == -INFINITY ? INFINITY : l * 1.4426950408889634f;
-          } else {
-            val[e] = row < p.Sq ? -p.delta[idx] : 0.f;
+            for (int kk = 0; kk < 8; ++kk)
+              umma_bf16_ts(tdV, tS + (kk >> 2) * 64 + (kk & 3) * 8, make_smem_desc_sw128(do_base + kk * 2048, CH_BYTES, 1024), IDESC_KV,
+                           (t | kk) != 0 ? 1u : 0u);
+            umma_commit(&do_empty[g % DO_ST]);   // dP of this pair was issued before
+            // S^T of the next pair, over the P that dV has read by then
+            if (t + 1 < it.n_iter) {
+              if (!mbar_wait(&q_full[(g + 1) & 1], ((g + 1) >> 1) & 1, abort_flag)) { ok = false; break; }
+              tc_fence_after();
+              issue_s(g + 1);
+            }
+            // dQ partial = dS K_j, then dK += dS^T Q_i while dQ is drained
+            if (!mbar_wait(ds_ready, ph, abort_flag)) { ok = false; break; }
+            if (kOwnDq && g > 0 && !mbar_wait(dq_drained, (g - 1) & 1, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              umma_bf16_ss(tdQ, make_smem_desc_sw128(ds_base + kk * 2048, CH_BYTES, 1024),
+                           make_smem_desc_sw128(k_base + kk * 2048, CH_BYTES, 1024), IDESC_DQ, kk != 0 ? 1u : 0u);
+            umma_commit(dq_full);
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              umma_bf16_ss(tdK, make_smem_desc_sw128(ds_base + kk_off(kk), 16, 1024),
+                           make_smem_desc_sw128(q_base + kk * 2048, CH_BYTES, 1024), IDESC_KV, (t | kk) != 0 ? 1u : 0u);
+            umma_commit(ds_free);
+            umma_commit(&q_empty[g & 1]);
+            if (t + 1 < it.n_iter && !issue_dp(g + 1)) { ok = false; break; }
+          }
+          if (ok) {
+            umma_commit(all_done);
+            umma_commit(kv_empty);
           }
         }
-        if (!mbar_wait(&stat_empty[st], ((t >> 1) & 1) ^ 1, abort_flag)) break;
-        *reinterpret_cast<float4*>(sStat + (st * 2 + (warp - 2)) * 128 + lane * 4) = make_float4(val[0], val[1], val[2], val[3]);
-        mbar_arrive(&stat_full[st]);
-        if (++i == n_qt) { i = i_start; ++h; }
+        __syncwarp();
+      } else if (it.n_iter > 0 && ok) {
+        // warp 2: log-sum-exp in log2 units, +inf where the row does not exist or saw no key (P becomes 0); warp 3: -delta
+        int h = it.hk * group, i = it.i_start;
+        for (int t = 0; t < it.n_iter; ++t) {
+          const int g = g0 + t, st = g & 1;
+          float val[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int row = i * 128 + lane * 4 + e;
+            const long long idx = (static_cast<long long>(it.b) * p.H + h) * p.Sq + row;
+            if (warp == 2) {
+              const float l = row < p.Sq ? p.lse[idx] : -INFINITY;
+              val[e] = l == -INFINITY ? INFINITY : l * 1.4426950408889634f;
+            } else {
+              val[e] = row < p.Sq ? -p.delta[idx] : 0.f;
+            }
+          }
+          if (!mbar_wait(&stat_empty[st], ((g >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          *reinterpret_cast<float4*>(sStat + (st * 2 + (warp - 2)) * 128 + lane * 4) = make_float4(val[0], val[1], val[2], val[3]);
+          mbar_arrive(&stat_full[st]);
+          if (++i == n_qt) { i = it.i_start; ++h; }
+        }
+        __syncwarp();
       }
-      __syncwarp();
+      g0 += it.n_iter;
+      act += it.n_iter > 0;
+      if (!next_item(n, item)) break;
     }
   } else if (warp < 8) {
-    reg_inc<144>();
-    if (n_iter > 0) {
-      // Drain the dQ partials: TMEM -> swizzled fp32 staging slabs -> one TMA add-reduction per 32 columns into the accumulator.
-      // Every warp stages and reduces its own 32 rows, so no warp waits for another. (All 128 threads meeting around one
-      // 128-row reduction per slab: 1.78 instead of 1.47 ms for batch 1, 32 / 8 heads, 8192 x 8192, D = 128, causal.)
-      const int quad = warp & 3;
-      const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-      int h = hk * group, i = i_start;
-      for (int t = 0; t < n_iter; ++t) {
-        if (!mbar_wait(dq_full, t & 1, abort_flag)) break;
+    if constexpr (D == 64) reg_dec<kRegsDrain>();
+    else reg_inc<kRegsDrain>();
+    // Drain the dQ partials: TMEM -> swizzled fp32 staging slabs -> one TMA add-reduction per 32 columns into the accumulator.
+    // Every warp stages and reduces its own 32 rows, so no warp waits for another. (All 128 threads meeting around one
+    // 128-row reduction per slab: 1.78 instead of 1.47 ms for batch 1, 32 / 8 heads, 8192 x 8192, D = 128, causal.)
+    const int quad = warp & 3;
+    const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
+    int item = blockIdx.x, g0 = 0;
+    bool ok = true;
+    for (int n = 0;; ++n) {
+      const Item it = item_of(item);
+      int h = it.hk * group, i = it.i_start;
+      for (int t = 0; t < it.n_iter && ok; ++t) {
+        if (!mbar_wait(dq_full, (g0 + t) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         // the whole partial leaves TMEM before anything else happens: the next dP waits for these columns at D = 128
         uint32_t v[D / 32][32];
@@ -337,179 +403,194 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              tma_reduce_add_4d(&tmdQ, st, s * 32, h, i * 128 + quad * 32, b);
+              tma_reduce_add_4d(&tmdQ, st, s * 32, h, i * 128 + quad * 32, it.b);
               tma_store_commit();
             }
           }
         }
-        if (++i == n_qt) { i = i_start; ++h; }
+        if (++i == n_qt) { i = it.i_start; ++h; }
       }
-      if (lane == 0) tma_store_wait<0>();
       __syncwarp();
+      g0 += it.n_iter;
+      if (!next_item(n, item)) break;
     }
+    if (lane == 0) tma_store_wait<0>();
+    __syncwarp();
   } else {
-    reg_inc<160>();
+    reg_inc<kRegsCompute>();
     const int quad = warp & 3;
     const int half = (warp - 8) >> 2;          // which 64 query columns of every tile this thread takes
     const int r = quad * 32 + lane;            // key row of the tile == TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const int krow = k0 + r;
-    __nv_bfloat16* dk_row = p.dk + (static_cast<long long>(b) * p.Sk + krow) * p.dkv_row_stride + hk * D;
-    __nv_bfloat16* dv_row = p.dv + (static_cast<long long>(b) * p.Sk + krow) * p.dkv_row_stride + hk * D;
-    if (n_iter > 0) {
-      uint8_t* ds_row = sdS + half * CH_BYTES + r * 128;   // this half's 64 queries = one swizzled chunk
-      const uint32_t tSh = tS + lane_addr + half * 64, tdPh = tdP + lane_addr + half * 64;
-      const uint64_t scale2 = pack_f32x2(__float_as_uint(p.scale_log2e), __float_as_uint(p.scale_log2e));
-      bool ok = true;
-      int h = hk * group, i = i_start;
-      for (int t = 0; t < n_iter; ++t) {
-        const uint32_t ph = t & 1;
-        const int st = t & 1;
-        const int q0 = i * 128;
-        const float* lse = sStat + st * 256 + half * 64;
-        const float* ndelta = lse + 128;
-        const bool need_mask = (p.causal && k0 + 127 > q0 + p.causal_off) || (k0 + 128 > kv_limit);
-        // first visible query column of this thread's half
-        const int c_min = krow >= kv_limit ? 64 : (p.causal ? krow - p.causal_off - q0 - half * 64 : 0);
-        uint32_t pk[32];  // P, later dS, as packed bf16 pairs of this key row's 64 queries
-        uint32_t keep_bits[DROP ? 2 : 1];  // dropout: bit c of word w = query column 32 * w + c of this half is kept
-        if constexpr (DROP) {
-          // a Philox draw covers four neighbouring keys of one query: the four lanes that own them draw a quarter each
+    int item = blockIdx.x, g0 = 0, act = 0;
+    bool ok = true;
+    for (int n = 0;; ++n) {
+      const Item it = item_of(item);
+      const int krow = it.k0 + r;
+      __nv_bfloat16* dk_row = p.dk + (static_cast<long long>(it.b) * p.Sk + krow) * p.dkv_row_stride + it.hk * D;
+      __nv_bfloat16* dv_row = p.dv + (static_cast<long long>(it.b) * p.Sk + krow) * p.dkv_row_stride + it.hk * D;
+      if (it.n_iter > 0) {
+        uint8_t* ds_row = sdS + half * CH_BYTES + r * 128;   // this half's 64 queries = one swizzled chunk
+        const uint32_t tSh = tS + lane_addr + half * 64, tdPh = tdP + lane_addr + half * 64;
+        const uint64_t scale2 = pack_f32x2(__float_as_uint(p.scale_log2e), __float_as_uint(p.scale_log2e));
+        int h = it.hk * group, i = it.i_start;
+        for (int t = 0; t < it.n_iter && ok; ++t) {
+          const int g = g0 + t;
+          const uint32_t ph = g & 1;
+          const int st = g & 1;
+          const int q0 = i * 128;
+          const float* lse = sStat + st * 256 + half * 64;
+          const float* ndelta = lse + 128;
+          const bool need_mask = (p.causal && it.k0 + 127 > q0 + p.causal_off) || (it.k0 + 128 > it.kv_limit);
+          // first visible query column of this thread's half
+          const int c_min = krow >= it.kv_limit ? 64 : (p.causal ? krow - p.causal_off - q0 - half * 64 : 0);
+          uint32_t pk[32];  // P, later dS, as packed bf16 pairs of this key row's 64 queries
+          uint32_t keep_bits[DROP ? 2 : 1];  // dropout: bit c of word w = query column 32 * w + c of this half is kept
+          if constexpr (DROP) {
+            // a Philox draw covers four neighbouring keys of one query: the four lanes that own them draw a quarter each
 #pragma unroll
-          for (int w = 0; w < 2; ++w) {
-            uint32_t bits = 0;
+            for (int w = 0; w < 2; ++w) {
+              uint32_t bits = 0;
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              const uint32_t row = static_cast<uint32_t>(q0 + half * 64 + w * 32 + g * 4 + (lane & 3));
-              const uint32_t k4 = dropout_keep4(p.drop, static_cast<uint32_t>(b * p.H + h), row, static_cast<uint32_t>(krow >> 2));
+              for (int g4 = 0; g4 < 8; ++g4) {
+                const uint32_t row = static_cast<uint32_t>(q0 + half * 64 + w * 32 + g4 * 4 + (lane & 3));
+                const uint32_t k4 = dropout_keep4(p.drop, static_cast<uint32_t>(it.b * p.H + h), row, static_cast<uint32_t>(krow >> 2));
 #pragma unroll
-              for (int e = 0; e < 4; ++e)
-                bits |= ((__shfl_sync(0xffffffffu, k4, (lane & ~3) + e) >> (krow & 3)) & 1u) << (g * 4 + e);
-            }
-            keep_bits[w] = bits;
-          }
-        }
-        if (!mbar_wait(&stat_full[st], (t >> 1) & 1, abort_flag)) { ok = false; break; }
-        if (!mbar_wait(s_full, ph, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        {
-          uint32_t v[2][32];
-          __syncwarp();
-          tmem_ld_32x32(tSh, v[0]);
-          tmem_ld_32x32(tSh + 32, v[1]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-              const float4 l4 = *reinterpret_cast<const float4*>(lse + c * 32 + e);
-              float x[4];
-              unpack_f32x2(fma_f32x2(pack_f32x2(v[c][e], v[c][e + 1]), scale2,
-                                     pack_f32x2(__float_as_uint(-l4.x), __float_as_uint(-l4.y))), x[0], x[1]);
-              unpack_f32x2(fma_f32x2(pack_f32x2(v[c][e + 2], v[c][e + 3]), scale2,
-                                     pack_f32x2(__float_as_uint(-l4.z), __float_as_uint(-l4.w))), x[2], x[3]);
-#pragma unroll
-              for (int k = 0; k < 4; ++k) x[k] = fast_exp2(x[k]);
-              if (need_mask) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  if (c * 32 + e + k < c_min) x[k] = 0.f;
+                for (int e = 0; e < 4; ++e)
+                  bits |= ((__shfl_sync(0xffffffffu, k4, (lane & ~3) + e) >> (krow & 3)) & 1u) << (g4 * 4 + e);
               }
-              pk[c * 16 + (e >> 1)] = pack_bf16x2(x[0], x[1]);
-              pk[c * 16 + (e >> 1) + 1] = pack_bf16x2(x[2], x[3]);
+              keep_bits[w] = bits;
             }
           }
-          // Publish P^T (with dropout: only the kept probabilities, which is what multiplied V in the forward; the factor
-          // 1 / keep is applied to dV at the end). Only this thread reads these TMEM columns of S, and it has.
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            uint32_t w16[16];
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              w16[e] = pk[c * 16 + e];
-              if constexpr (DROP)
-                w16[e] &= ((keep_bits[c] >> (2 * e)) & 1u ? 0x0000FFFFu : 0u) | ((keep_bits[c] >> (2 * e + 1)) & 1u ? 0xFFFF0000u : 0u);
-            }
-            tmem_st_32x16(tSh + c * 16, w16);
-          }
-          tmem_wait_st();
-        }
-        tc_fence_before();
-        mbar_arrive(p_ready);
-        // dS = P * (dP - delta); the softmax scale is applied to the finished dK and dQ
-        if (!mbar_wait(dp_full, ph, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        {
-          uint32_t v[2][32];
-          __syncwarp();
-          tmem_ld_32x32(tdPh, v[0]);
-          tmem_ld_32x32(tdPh + 32, v[1]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-              const float4 nd = *reinterpret_cast<const float4*>(ndelta + c * 32 + e);
-              if constexpr (DROP) {   // the gradient reaches P only through the kept entries, scaled by 1 / keep
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  v[c][e + k] = (keep_bits[c] >> (e + k)) & 1u ? __float_as_uint(__uint_as_float(v[c][e + k]) * p.drop.inv_keep) : 0u;
-              }
-              const uint32_t w0 = pk[c * 16 + (e >> 1)], w1 = pk[c * 16 + (e >> 1) + 1];
-              float d[4];
-              unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[c][e], v[c][e + 1]), pack_f32x2(__float_as_uint(nd.x), __float_as_uint(nd.y))),
-                                     pack_f32x2(w0 << 16, w0 & 0xFFFF0000u)), d[0], d[1]);
-              unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[c][e + 2], v[c][e + 3]), pack_f32x2(__float_as_uint(nd.z), __float_as_uint(nd.w))),
-                                     pack_f32x2(w1 << 16, w1 & 0xFFFF0000u)), d[2], d[3]);
-              pk[c * 16 + (e >> 1)] = pack_bf16x2(d[0], d[1]);
-              pk[c * 16 + (e >> 1) + 1] = pack_bf16x2(d[2], d[3]);
-            }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&stat_empty[st]);
-        if (t > 0 && !mbar_wait(ds_free, (t - 1) & 1, abort_flag)) { ok = false; break; }
-#pragma unroll
-        for (int g = 0; g < 8; ++g)
-          *reinterpret_cast<uint4*>(ds_row + ((g ^ (r & 7)) << 4)) = make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
-        fence_proxy_async_smem();
-        tc_fence_before();
-        mbar_arrive(ds_ready);
-        if (++i == n_qt) { i = i_start; ++h; }
-      }
-      // dK, dV of this key tile: TMEM lane = key row; each half writes its half of the D columns
-      if (ok) ok = mbar_wait(all_done, 0, abort_flag);
-      if (ok) {
-        tc_fence_after();
-#pragma unroll
-        for (int which = 0; which < 2; ++which) {
-          const uint32_t src = which == 0 ? tdK : tdV;
-          __nv_bfloat16* dst = which == 0 ? dk_row : dv_row;
-          const float osc = which == 0 ? p.scale : (DROP ? p.drop.inv_keep : 1.f);
-#pragma unroll
-          for (int c0 = 0; c0 < D / 64; ++c0) {
-            const int c = half * (D / 64) + c0;
-            uint32_t v[32];
+          if (!mbar_wait(&stat_full[st], (g >> 1) & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait(s_full, ph, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          {
+            uint32_t v[2][32];
             __syncwarp();
-            tmem_ld_32x32(src + lane_addr + c * 32, v);
+            tmem_ld_32x32(tSh, v[0]);
+            tmem_ld_32x32(tSh + 32, v[1]);
             tmem_wait_ld();
-            if (krow < p.Sk) {
 #pragma unroll
-              for (int g = 0; g < 4; ++g)
-                *reinterpret_cast<uint4*>(dst + c * 32 + g * 8) = make_uint4(
-                    pack_bf16x2(__uint_as_float(v[g * 8]) * osc, __uint_as_float(v[g * 8 + 1]) * osc),
-                    pack_bf16x2(__uint_as_float(v[g * 8 + 2]) * osc, __uint_as_float(v[g * 8 + 3]) * osc),
-                    pack_bf16x2(__uint_as_float(v[g * 8 + 4]) * osc, __uint_as_float(v[g * 8 + 5]) * osc),
-                    pack_bf16x2(__uint_as_float(v[g * 8 + 6]) * osc, __uint_as_float(v[g * 8 + 7]) * osc));
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+              for (int e = 0; e < 32; e += 4) {
+                const float4 l4 = *reinterpret_cast<const float4*>(lse + c * 32 + e);
+                float x[4];
+                unpack_f32x2(fma_f32x2(pack_f32x2(v[c][e], v[c][e + 1]), scale2,
+                                       pack_f32x2(__float_as_uint(-l4.x), __float_as_uint(-l4.y))), x[0], x[1]);
+                unpack_f32x2(fma_f32x2(pack_f32x2(v[c][e + 2], v[c][e + 3]), scale2,
+                                       pack_f32x2(__float_as_uint(-l4.z), __float_as_uint(-l4.w))), x[2], x[3]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) x[k] = fast_exp2(x[k]);
+                if (need_mask) {
+#pragma unroll
+                  for (int k = 0; k < 4; ++k)
+                    if (c * 32 + e + k < c_min) x[k] = 0.f;
+                }
+                pk[c * 16 + (e >> 1)] = pack_bf16x2(x[0], x[1]);
+                pk[c * 16 + (e >> 1) + 1] = pack_bf16x2(x[2], x[3]);
+              }
+            }
+            // Publish P^T (with dropout: only the kept probabilities, which is what multiplied V in the forward; the factor
+            // 1 / keep is applied to dV at the end). Only this thread reads these TMEM columns of S, and it has.
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              uint32_t w16[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) {
+                w16[e] = pk[c * 16 + e];
+                if constexpr (DROP)
+                  w16[e] &= ((keep_bits[c] >> (2 * e)) & 1u ? 0x0000FFFFu : 0u) | ((keep_bits[c] >> (2 * e + 1)) & 1u ? 0xFFFF0000u : 0u);
+              }
+              tmem_st_32x16(tSh + c * 16, w16);
+            }
+            tmem_wait_st();
+          }
+          tc_fence_before();
+          mbar_arrive(p_ready);
+          // dS = P * (dP - delta); the softmax scale is applied to the finished dK and dQ
+          if (!mbar_wait(dp_full, ph, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          {
+            uint32_t v[2][32];
+            __syncwarp();
+            tmem_ld_32x32(tdPh, v[0]);
+            tmem_ld_32x32(tdPh + 32, v[1]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int e = 0; e < 32; e += 4) {
+                const float4 nd = *reinterpret_cast<const float4*>(ndelta + c * 32 + e);
+                if constexpr (DROP) {   // the gradient reaches P only through the kept entries, scaled by 1 / keep
+#pragma unroll
+                  for (int k = 0; k < 4; ++k)
+                    v[c][e + k] = (keep_bits[c] >> (e + k)) & 1u ? __float_as_uint(__uint_as_float(v[c][e + k]) * p.drop.inv_keep) : 0u;
+                }
+                const uint32_t w0 = pk[c * 16 + (e >> 1)], w1 = pk[c * 16 + (e >> 1) + 1];
+                float d[4];
+                unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[c][e], v[c][e + 1]), pack_f32x2(__float_as_uint(nd.x), __float_as_uint(nd.y))),
+                                       pack_f32x2(w0 << 16, w0 & 0xFFFF0000u)), d[0], d[1]);
+                unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[c][e + 2], v[c][e + 3]), pack_f32x2(__float_as_uint(nd.z), __float_as_uint(nd.w))),
+                                       pack_f32x2(w1 << 16, w1 & 0xFFFF0000u)), d[2], d[3]);
+                pk[c * 16 + (e >> 1)] = pack_bf16x2(d[0], d[1]);
+                pk[c * 16 + (e >> 1) + 1] = pack_bf16x2(d[2], d[3]);
+              }
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&stat_empty[st]);
+          if (g > 0 && !mbar_wait(ds_free, (g - 1) & 1, abort_flag)) { ok = false; break; }
+#pragma unroll
+          for (int c16 = 0; c16 < 8; ++c16)
+            *reinterpret_cast<uint4*>(ds_row + ((c16 ^ (r & 7)) << 4)) =
+                make_uint4(pk[4 * c16], pk[4 * c16 + 1], pk[4 * c16 + 2], pk[4 * c16 + 3]);
+          fence_proxy_async_smem();
+          tc_fence_before();
+          mbar_arrive(ds_ready);
+          if (++i == n_qt) { i = it.i_start; ++h; }
+        }
+        // dK, dV of this key tile: TMEM lane = key row; each half writes its half of the D columns
+        if (ok) ok = mbar_wait(all_done, act & 1, abort_flag);
+        if (ok) {
+          tc_fence_after();
+#pragma unroll
+          for (int which = 0; which < 2; ++which) {
+            const uint32_t src = which == 0 ? tdK : tdV;
+            __nv_bfloat16* dst = which == 0 ? dk_row : dv_row;
+            const float osc = which == 0 ? p.scale : (DROP ? p.drop.inv_keep : 1.f);
+#pragma unroll
+            for (int c0 = 0; c0 < D / 64; ++c0) {
+              const int c = half * (D / 64) + c0;
+              uint32_t v[32];
+              __syncwarp();
+              tmem_ld_32x32(src + lane_addr + c * 32, v);
+              tmem_wait_ld();
+              if (krow < p.Sk) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g)
+                  *reinterpret_cast<uint4*>(dst + c * 32 + g * 8) = make_uint4(
+                      pack_bf16x2(__uint_as_float(v[g * 8]) * osc, __uint_as_float(v[g * 8 + 1]) * osc),
+                      pack_bf16x2(__uint_as_float(v[g * 8 + 2]) * osc, __uint_as_float(v[g * 8 + 3]) * osc),
+                      pack_bf16x2(__uint_as_float(v[g * 8 + 4]) * osc, __uint_as_float(v[g * 8 + 5]) * osc),
+                      pack_bf16x2(__uint_as_float(v[g * 8 + 6]) * osc, __uint_as_float(v[g * 8 + 7]) * osc));
+              }
             }
           }
+          tc_fence_before();
+          mbar_arrive(acc_free);
+        }
+      } else if (krow < p.Sk) {
+        // Key tile invisible to every query (beyond kv_len, or right of the causal diagonal for all rows): zero gradients.
+        for (int i = half * (D / 2); i < (half + 1) * (D / 2); i += 8) {
+          *reinterpret_cast<uint4*>(dk_row + i) = make_uint4(0, 0, 0, 0);
+          *reinterpret_cast<uint4*>(dv_row + i) = make_uint4(0, 0, 0, 0);
         }
       }
-    } else if (krow < p.Sk) {
-      // Key tile invisible to every query (beyond kv_len, or right of the causal diagonal for all rows): zero gradients.
-      for (int i = half * (D / 2); i < (half + 1) * (D / 2); i += 8) {
-        *reinterpret_cast<uint4*>(dk_row + i) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(dv_row + i) = make_uint4(0, 0, 0, 0);
-      }
+      g0 += it.n_iter;
+      act += it.n_iter > 0;
+      __syncwarp();
+      if (!next_item(n, item)) break;
     }
   }
 
