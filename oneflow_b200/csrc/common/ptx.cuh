@@ -147,6 +147,12 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Registers per thread of a warpgroup (all four warps execute it); the shares must add up to the launch's at most.
+template <int N>
+__device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ---------------------------------------------------------------------------------------------
 // Cluster launch control: a running CTA takes over the block index of one that has not been launched yet, so that a grid of
 // ordinary size runs as persistent CTAs in the hardware's own order. The answer (16 bytes) arrives like a bulk copy; after one

@@ -80,11 +80,6 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* m, const vo
                "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z), "r"(w)
                : "memory");
 }
-template <int N>
-__device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N>
-__device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-
 template <int D, bool DROP>
 __global__ void __launch_bounds__(512, 1)
 fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,

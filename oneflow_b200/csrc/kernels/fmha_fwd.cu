@@ -7,7 +7,7 @@
 // stream hide behind the exponentials of the other. Roles:
 //   warp 0      TMA producer: the query tile(s) once, then K / V tiles through a ring in the order the products use them
 //   warp 1      tcgen05 issuer: S_t = Q_t K^T, then O_t += P_t V with P_t read from TMEM (it lies over the S_t it came from)
-//   warps 2..5  softmax of stream 0, warps 6..9 of stream 1: one thread owns one whole query row (a TMEM lane), so row
+//   warps 4..7  softmax of stream 0, warps 8..11 of stream 1: one thread owns one whole query row (a TMEM lane), so row
 //               maxima and sums need no exchange, and P goes back to TMEM without touching shared memory
 // The streams are two neighbouring query tiles (SPLIT = false: every K / V tile is loaded once for 256 rows), or, when that
 // would leave SMs without a CTA, the even and the odd key tiles of ONE query tile whose two results are merged at the end
@@ -15,9 +15,11 @@
 //
 // What bounds it: the exponentials (16 per clock and SM: 1024 clocks for a 128 x 128 tile) and the two products of a D = 128
 // tile (1024 clocks) alike. Measured on a B200, forward alone, against the one-stream kernel this replaced (P through shared
-// memory, two threads a row that met at a barrier on every tile): batch 4, 32 heads, 2048 x 2048, D = 128, causal
-// 283 -> 187 us; batch 1, 32 / 8 heads, 8192 x 8192, D = 128, causal 847 -> 468 us; batch 32, 16 heads, 512 x 512, D = 64
-// 143 -> 88 us.
+// memory, two threads a row that met at a barrier on every tile), and in brackets with one CTA per pair: batch 4, 32 heads,
+// 2048 x 2048, D = 128, causal 283 -> 163 us (187); batch 1, 32 / 8 heads, 8192 x 8192, D = 128, causal 847 -> 451 us (470);
+// batch 32, 16 heads, 512 x 512, D = 64 143 -> 73 us (88).
+// Pairs: a running CTA takes over the next item that has not started (cluster launch control), so that the first loads of an
+// item run under the end of the one before.
 // The exponent reference trails the true running maximum by up to 2^8, so O is only rescaled in TMEM (tcgen05.ld / st) on
 // the rare tiles where a row maximum jumps. tcgen05 products of one thread run in issue order, hence: S_t of the next tile
 // is issued right behind the P_t V that reads the same columns, and a finished S_t means that the P V before it is finished.
@@ -52,7 +54,7 @@ struct FmhaFwdCfg {
   static constexpr int Q_BYTES = BM * D * 2;            // one query tile
   static constexpr int KV_BYTES = BN * D * 2;
   static constexpr int SLOTS = D == 128 ? 5 : 8;        // K / V ring
-  static constexpr int BAR_BYTES = 256;                 // mbarriers, the TMEM slot, the abort flag
+  static constexpr int BAR_BYTES = 320;                 // mbarriers, the TMEM slot, the abort flag, two answers of 16 bytes
   static constexpr int XCHG_BYTES = 2 * 128 * 8;        // SPLIT: row maximum and sum of both streams
   // At D = 128 the tiles take 224 KiB of the 227 KiB a CTA may have: the dynamic shared memory is declared 1024-byte
   // aligned (the kernel has no static shared memory, so it starts the CTA's window) instead of being aligned by hand
@@ -61,7 +63,7 @@ struct FmhaFwdCfg {
 };
 
 template <int D, bool DROP, bool SPLIT>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(384, 1)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, FmhaFwdParams p) {
   using Cfg = FmhaFwdCfg<D>;
@@ -87,36 +89,61 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* p_full = s_full + 2;         // [2] 128 softmax threads of the stream
   uint64_t* o_done = p_full + 2;         // [2]
   uint64_t* pair_bar = o_done + 2;       // SPLIT: all 256 softmax threads, once
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pair_bar + 1);
+  uint64_t* q_empty = pair_bar + 1;      // every product of an item has finished
+  uint64_t* o_free = q_empty + 1;        // [2] 128 softmax threads: O has left TMEM
+  uint64_t* next_full = o_free + 2;      // [2] the answer that names the CTA's next item
+  uint64_t* next_empty = next_full + 2;  // [2] 10 warps
+  uint8_t* answers = reinterpret_cast<uint8_t*>(bars + 32);   // [2] 16 bytes
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(answers + 32);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((2 + 2 * SLOTS + 6 + 1) * 8 + 8 <= Cfg::BAR_BYTES, "barriers do not fit");
+  static_assert(2 + 2 * SLOTS + 7 + 7 <= 32 && 32 * 8 + 32 + 8 <= Cfg::BAR_BYTES, "barriers do not fit");
   float2* xchg = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(bars) + Cfg::BAR_BYTES);   // [2 streams][128 rows]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // CTAs walk the heads in chunks whose keys and values stay in L2 together; inside a chunk the longest (last) causal tiles
-  // of all its heads come first, so that the short ones fill the tail.
-  const int in_chunk_max = p.chunk * p.n_qt;
-  const int ck = static_cast<int>(blockIdx.x) / in_chunk_max, rem = static_cast<int>(blockIdx.x) % in_chunk_max;
-  const int heads_here = min(p.chunk, p.B * p.H - ck * p.chunk);
-  const int qt = p.n_qt - 1 - rem / heads_here;
-  const int bh = ck * p.chunk + rem % heads_here;
-  const int h = bh % p.H, b = bh / p.H;
-  const int hk = h / (p.H / p.Hk);
-  const int q0 = qt * (SPLIT ? BM : 2 * BM);
-  int kv_limit = p.Sk;
-  if (p.kv_len) kv_limit = min(kv_limit, p.kv_len[b]);
-  // key tiles of stream t: all that its rows see, or every second one of them. Rows grow with the stream, so stream 1 never
-  // sees fewer tiles than stream 0 unless it has no rows at all.
-  int n_it[2];
+  // Item `n` of the grid: CTAs walk the heads in chunks whose keys and values stay in L2 together; inside a chunk the longest
+  // (last) causal tiles of all its heads come first, so that the short ones fill the tail.
+  struct Item {
+    int q0, bh, h, b, hk, kv_limit;
+    int n_it[2];     // key tiles of each stream
+  };
+  auto item_of = [&](int item) {
+    const int in_chunk_max = p.chunk * p.n_qt;
+    const int ck = item / in_chunk_max, rem = item % in_chunk_max;
+    const int heads_here = min(p.chunk, p.B * p.H - ck * p.chunk);
+    Item it;
+    it.q0 = (p.n_qt - 1 - rem / heads_here) * (SPLIT ? BM : 2 * BM);
+    it.bh = ck * p.chunk + rem % heads_here;
+    it.h = it.bh % p.H;
+    it.b = it.bh / p.H;
+    it.hk = it.h / (p.H / p.Hk);
+    it.kv_limit = p.kv_len ? min(p.Sk, p.kv_len[it.b]) : p.Sk;
+    // all key tiles that a stream's rows see, or every second one of them. Rows grow with the stream, so stream 1 never sees
+    // fewer tiles than stream 0 unless it has no rows at all.
 #pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int r0 = SPLIT ? q0 : q0 + t * BM;
-    int kv_end = kv_limit;
-    if (p.causal) kv_end = min(kv_end, r0 + BM + p.causal_off);
-    const int n = (kv_end > 0 && r0 < p.Sq) ? (kv_end + BN - 1) / BN : 0;
-    n_it[t] = SPLIT ? (n - t + 1) >> 1 : n;
-  }
-  const bool any = n_it[0] > 0 || n_it[1] > 0;
+    for (int t = 0; t < 2; ++t) {
+      const int r0 = SPLIT ? it.q0 : it.q0 + t * BM;
+      int kv_end = it.kv_limit;
+      if (p.causal) kv_end = min(kv_end, r0 + BM + p.causal_off);
+      const int n = (kv_end > 0 && r0 < p.Sq) ? (kv_end + BN - 1) / BN : 0;
+      it.n_it[t] = SPLIT ? (n - t + 1) >> 1 : n;
+    }
+    return it;
+  };
+  // Pairs: the CTA works through items until none is left, every role walks the same sequence (`n` counts them). Split key tiles
+  // come in one wave or two: one item per CTA.
+  auto next_item = [&](int n, int& item) -> bool {      // called by whole warps
+    if constexpr (SPLIT) {
+      return false;
+    } else {
+      const bool ok = mbar_wait(&next_full[n & 1], (n >> 1) & 1, abort_flag);
+      int nx = 0;
+      const bool more = ok && clc_take(answers + (n & 1) * 16, nx);
+      item = nx;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&next_empty[n & 1]);
+      return more;
+    }
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < SLOTS; ++s) {
@@ -130,6 +157,12 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&o_done[t], 1);
     }
     mbar_init(pair_bar, 256);
+    mbar_init(q_empty, 1);
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(&o_free[t], 128);
+      mbar_init(&next_full[t], 1);
+      mbar_init(&next_empty[t], 10);
+    }
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
@@ -147,302 +180,363 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t tS = tmem_base;            // S[0], S[1] at +0, +128; P[t] takes the first 64 columns of S[t]
   const uint32_t tO = tmem_base + 256;      // O[0], O[1] at +0, +128, D columns each
 
-  if (warp == 0) {
-    if (elect_one() && any) {
+  // registers: 384 threads x 168 at launch = 3 warpgroups x (88 + 208 + 208); a softmax thread holds a whole row of S. (With 72
+  // for the producer and issuer their few spills cost 10 %: 181 instead of 163 us at batch 4, 32 heads, 2048 x 2048, causal.)
+  if (warp < 4) {
+    reg_dec<88>();
+    if (warp == 0) {
+      int item = blockIdx.x;
       int c = 0;                             // loads issued so far: load c uses slot c % SLOTS
-      auto load_kv = [&](const CUtensorMap* m, int tile) -> bool {
-        const int s = c % SLOTS;
-        if (!mbar_wait(&kv_empty[s], ((c / SLOTS) & 1) ^ 1, abort_flag)) return false;
-        mbar_arrive_expect_tx(&kv_full[s], Cfg::KV_BYTES);
-#pragma unroll
-        for (int d = 0; d < DCH; ++d) tma_load_4d(sKV + s * Cfg::KV_BYTES + d * CH_BYTES, m, &kv_full[s], d * 64, hk, tile * BN, b);
-        ++c;
-        return true;
-      };
-      auto load_q = [&](int t) {
-        mbar_arrive_expect_tx(&q_full[t], Cfg::Q_BYTES);
-#pragma unroll
-        for (int d = 0; d < DCH; ++d) tma_load_4d(sQ + t * Cfg::Q_BYTES + d * CH_BYTES, &tmQ, &q_full[t], d * 64, h, q0 + t * BM, b);
-      };
-      if (n_it[0] > 0) load_q(0);   // only what a product will wait for: no copy may be in flight when the CTA leaves
-      bool ok = load_kv(&tmK, 0);
-      if constexpr (SPLIT) {
-        const int n = n_it[0] + n_it[1];
-        if (n > 1) ok = ok && load_kv(&tmK, 1);
-        for (int g = 0; g < n && ok; ++g) {
-          ok = load_kv(&tmV, g);
-          if (ok && g + 2 < n) ok = load_kv(&tmK, g + 2);
-        }
-      } else {
-        if (n_it[1] > 0) load_q(1);
-        const int n = max(n_it[0], n_it[1]);
-        for (int i = 0; i < n && ok; ++i) {
-          ok = load_kv(&tmV, i);
-          if (ok && i + 1 < n) ok = load_kv(&tmK, i + 1);
-        }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (elect_one() && any) {
-      const uint32_t kv_base = smem_u32(sKV);
-      auto slot_ready = [&](int c) -> bool { return mbar_wait(&kv_full[c % SLOTS], (c / SLOTS) & 1, abort_flag); };
-      auto issue_s = [&](int t, int c) {     // S_t = Q_t K^T with the K tile of load c
-        const uint32_t q_base = smem_u32(sQ + (SPLIT ? 0 : t) * Cfg::Q_BYTES);
-        const uint32_t k_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * CH_BYTES + (kk & 3) * 32;
-          umma_bf16_ss(tS + t * BN, make_smem_desc_sw128(q_base + off, 16, 1024), make_smem_desc_sw128(k_base + off, 16, 1024),
-                       IDESC_S, kk != 0 ? 1u : 0u);
-        }
-        umma_commit(&s_full[t]);
-      };
-      auto issue_pv = [&](int t, int c, bool first) {   // O_t (+)= P_t V with the V tile of load c
-        const uint32_t v_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES;
-#pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk)
-          umma_bf16_ts(tO + t * 128, tS + t * BN + kk * 8, make_smem_desc_sw128(v_base + kk * 2048, CH_BYTES, 1024), IDESC_O,
-                       (first && kk == 0) ? 0u : 1u);
-      };
-      auto release = [&](int c) { umma_commit(&kv_empty[c % SLOTS]); };
+      int act = 0;                           // items before this one that had any key tile
       bool ok = true;
-      if constexpr (SPLIT) {
-        const int n = n_it[0] + n_it[1];
-        int c = 0;
-        ok = mbar_wait(&q_full[0], 0, abort_flag);
-        for (int t = 0; t < 2 && t < n && ok; ++t) {
-          ok = slot_ready(c);
-          if (!ok) break;
-          tc_fence_after();
-          issue_s(t, c);
-          release(c);
-          ++c;
-        }
-        for (int g = 0; g < n && ok; ++g) {
-          const int t = g & 1, i = g >> 1;
-          if (!mbar_wait(&p_full[t], i & 1, abort_flag) || !slot_ready(c)) { ok = false; break; }
-          tc_fence_after();
-          issue_pv(t, c, i == 0);
-          release(c);
-          ++c;
-          if (g + 2 < n) {
-            if (!slot_ready(c)) { ok = false; break; }
-            tc_fence_after();
-            issue_s(t, c);
-            release(c);
+      for (int n = 0;; ++n) {
+        const Item it = item_of(item);
+        const int tiles = SPLIT ? it.n_it[0] + it.n_it[1] : max(it.n_it[0], it.n_it[1]);
+        if (elect_one()) {
+          auto load_kv = [&](const CUtensorMap* m, int tile) -> bool {
+            const int s = c % SLOTS;
+            if (!mbar_wait(&kv_empty[s], ((c / SLOTS) & 1) ^ 1, abort_flag)) return false;
+            mbar_arrive_expect_tx(&kv_full[s], Cfg::KV_BYTES);
+#pragma unroll
+            for (int d = 0; d < DCH; ++d)
+              tma_load_4d(sKV + s * Cfg::KV_BYTES + d * CH_BYTES, m, &kv_full[s], d * 64, it.hk, tile * BN, it.b);
             ++c;
+            return true;
+          };
+          auto load_q = [&](int t) {      // only what a product will wait for: no copy may be in flight when the CTA leaves
+            if (it.n_it[t] == 0) return;
+            mbar_arrive_expect_tx(&q_full[t], Cfg::Q_BYTES);
+#pragma unroll
+            for (int d = 0; d < DCH; ++d)
+              tma_load_4d(sQ + t * Cfg::Q_BYTES + d * CH_BYTES, &tmQ, &q_full[t], d * 64, it.h, it.q0 + t * BM, it.b);
+          };
+          // a few tiles before the loads of this item end (see the backward kernel)
+          auto ask = [&]() {
+            if (!mbar_wait(&next_empty[n & 1], ((n >> 1) & 1) ^ 1, abort_flag)) return;
+            fence_proxy_async_smem();
+            clc_ask(answers + (n & 1) * 16, &next_full[n & 1]);
+          };
+          if constexpr (SPLIT) {
+            if (tiles > 0) {
+              load_q(0);
+              ok = load_kv(&tmK, 0);
+              if (tiles > 1) ok = ok && load_kv(&tmK, 1);
+              for (int g = 0; g < tiles && ok; ++g) {
+                ok = load_kv(&tmV, g);
+                if (ok && g + 2 < tiles) ok = load_kv(&tmK, g + 2);
+              }
+            }
           } else {
-            umma_commit(&o_done[t]);
-          }
-        }
-      } else {
-        const int n = max(n_it[0], n_it[1]);
-        ok = slot_ready(0);
-        for (int t = 0; t < 2 && ok; ++t) {
-          if (n_it[t] == 0) continue;
-          ok = mbar_wait(&q_full[t], 0, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          issue_s(t, 0);
-        }
-        if (ok) release(0);
-        for (int i = 0; i < n && ok; ++i) {
-          const int cv = 2 * i + 1, ck1 = 2 * i + 2;      // loads of V_i and K_{i+1}
-          for (int t = 0; t < 2; ++t) {
-            if (i >= n_it[t]) continue;
-            if (!mbar_wait(&p_full[t], i & 1, abort_flag) || !slot_ready(cv)) { ok = false; break; }
-            tc_fence_after();
-            issue_pv(t, cv, i == 0);
-            if (t == 1 || i >= n_it[1]) release(cv);       // the last stream to use the tile
-            if (i + 1 < n_it[t]) {
-              if (!slot_ready(ck1)) { ok = false; break; }
-              tc_fence_after();
-              issue_s(t, ck1);
-              if (t == 1 || i + 1 >= n_it[1]) release(ck1);
-            } else {
-              umma_commit(&o_done[t]);
+            const int ask_at = max(0, tiles - 4);
+            if (tiles == 0 || !ok) ask();
+            if (tiles > 0 && ok) {
+              ok = load_kv(&tmK, 0) && mbar_wait(q_empty, (act & 1) ^ 1, abort_flag);
+              if (ok) {
+                load_q(0);
+                load_q(1);
+              }
+              for (int i = 0; i < tiles; ++i) {
+                if (i == ask_at) ask();
+                ok = ok && load_kv(&tmV, i);
+                if (ok && i + 1 < tiles) ok = load_kv(&tmK, i + 1);
+              }
             }
           }
         }
+        __syncwarp();
+        act += tiles > 0;
+        if (!next_item(n, item)) break;
+      }
+    } else if (warp == 1) {
+      int item = blockIdx.x;
+      int c0 = 0;                            // loads of the items before this one
+      int act = 0;
+      int j0[2] = {0, 0}, seen[2] = {0, 0};  // key tiles and items each stream had before this item
+      bool ok = true;
+      for (int n = 0;; ++n) {
+        const Item it = item_of(item);
+        const int tiles = SPLIT ? it.n_it[0] + it.n_it[1] : max(it.n_it[0], it.n_it[1]);
+        if (elect_one() && tiles > 0 && ok) {
+          const uint32_t kv_base = smem_u32(sKV);
+          auto slot_ready = [&](int c) -> bool { return mbar_wait(&kv_full[c % SLOTS], (c / SLOTS) & 1, abort_flag); };
+          auto issue_s = [&](int t, int c) {     // S_t = Q_t K^T with the K tile of load c
+            const uint32_t q_base = smem_u32(sQ + (SPLIT ? 0 : t) * Cfg::Q_BYTES);
+            const uint32_t k_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES;
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk) {
+              const uint32_t off = (kk >> 2) * CH_BYTES + (kk & 3) * 32;
+              umma_bf16_ss(tS + t * BN, make_smem_desc_sw128(q_base + off, 16, 1024), make_smem_desc_sw128(k_base + off, 16, 1024),
+                           IDESC_S, kk != 0 ? 1u : 0u);
+            }
+            umma_commit(&s_full[t]);
+          };
+          auto issue_pv = [&](int t, int c, bool first) {   // O_t (+)= P_t V with the V tile of load c
+            const uint32_t v_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES;
+#pragma unroll
+            for (int kk = 0; kk < BN / 16; ++kk)
+              umma_bf16_ts(tO + t * 128, tS + t * BN + kk * 8, make_smem_desc_sw128(v_base + kk * 2048, CH_BYTES, 1024), IDESC_O,
+                           (first && kk == 0) ? 0u : 1u);
+          };
+          auto release = [&](int c) { umma_commit(&kv_empty[c % SLOTS]); };
+          if constexpr (SPLIT) {
+            int c = 0;
+            ok = mbar_wait(&q_full[0], 0, abort_flag);
+            for (int t = 0; t < 2 && t < tiles && ok; ++t) {
+              ok = slot_ready(c);
+              if (!ok) break;
+              tc_fence_after();
+              issue_s(t, c);
+              release(c);
+              ++c;
+            }
+            for (int g = 0; g < tiles && ok; ++g) {
+              const int t = g & 1, i = g >> 1;
+              if (!mbar_wait(&p_full[t], i & 1, abort_flag) || !slot_ready(c)) { ok = false; break; }
+              tc_fence_after();
+              issue_pv(t, c, i == 0);
+              release(c);
+              ++c;
+              if (g + 2 < tiles) {
+                if (!slot_ready(c)) { ok = false; break; }
+                tc_fence_after();
+                issue_s(t, c);
+                release(c);
+                ++c;
+              } else {
+                umma_commit(&o_done[t]);
+              }
+            }
+          } else {
+            ok = slot_ready(c0);
+            for (int t = 0; t < 2 && ok; ++t) {
+              if (it.n_it[t] == 0) continue;
+              ok = mbar_wait(&q_full[t], seen[t] & 1, abort_flag);
+              if (!ok) break;
+              tc_fence_after();
+              issue_s(t, c0);
+            }
+            if (ok) release(c0);
+            for (int i = 0; i < tiles && ok; ++i) {
+              const int cv = c0 + 2 * i + 1, ck1 = c0 + 2 * i + 2;      // loads of V_i and K_{i+1}
+              for (int t = 0; t < 2; ++t) {
+                if (i >= it.n_it[t]) continue;
+                if (!mbar_wait(&p_full[t], (j0[t] + i) & 1, abort_flag) || !slot_ready(cv)) { ok = false; break; }
+                // O of the item before has left TMEM
+                if (i == 0 && !mbar_wait(&o_free[t], (seen[t] & 1) ^ 1, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                issue_pv(t, cv, i == 0);
+                if (t == 1 || i >= it.n_it[1]) release(cv);       // the last stream to use the tile
+                if (i + 1 < it.n_it[t]) {
+                  if (!slot_ready(ck1)) { ok = false; break; }
+                  tc_fence_after();
+                  issue_s(t, ck1);
+                  if (t == 1 || i + 1 >= it.n_it[1]) release(ck1);
+                } else {
+                  umma_commit(&o_done[t]);
+                }
+              }
+            }
+            if (ok) umma_commit(q_empty);
+          }
+        }
+        __syncwarp();
+        c0 += 2 * tiles;
+        act += tiles > 0;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          j0[t] += it.n_it[t];
+          seen[t] += it.n_it[t] > 0;
+        }
+        if (!next_item(n, item)) break;
       }
     }
-    __syncwarp();
   } else {
+    reg_inc<208>();
     const int quad = warp & 3;
-    const int t = (warp - 2) >> 2;           // stream
+    const int t = (warp - 4) >> 2;           // stream
     const int r = quad * 32 + lane;          // row inside the tile == TMEM lane
-    const int row0 = SPLIT ? q0 : q0 + t * BM;
-    const int row_g = row0 + r;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t tSt = tS + lane_addr + t * BN, tOt = tO + lane_addr + t * 128;
-    const int n = n_it[t];
-    // m_ref is the exponent reference actually used for P and l; it trails the true running maximum by at
-    // most kLazy (log2 units) so that the TMEM-resident O only has to be rescaled when the maximum jumps.
-    constexpr float kLazy = 8.0f;
-    float m_ref = -INFINITY, l_run = 0.f;
+    int item = blockIdx.x;
+    int j0 = 0, seen = 0;                    // key tiles and items this stream had before this item
     bool ok = true;
-    const uint64_t scale2 = pack_f32x2(__float_as_uint(p.scale_log2e), __float_as_uint(p.scale_log2e));
-    const int col_max = p.causal ? min(row_g + p.causal_off, kv_limit - 1) : kv_limit - 1;  // last visible column
-    for (int i = 0; i < n; ++i) {
-      const int col_base = (SPLIT ? 2 * i + t : i) * BN;
-      if (!mbar_wait(&s_full[t], i & 1, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      const bool need_mask = (p.causal && col_base + BN - 1 > row0 + p.causal_off) || (col_base + BN > kv_limit);
-      uint32_t sv[4][32];
-      __syncwarp();
+    for (int n = 0;; ++n) {
+      const Item it = item_of(item);
+      const int row0 = SPLIT ? it.q0 : it.q0 + t * BM;
+      const int row_g = row0 + r;
+      const int nt = it.n_it[t];
+      // m_ref is the exponent reference actually used for P and l; it trails the true running maximum by at
+      // most kLazy (log2 units) so that the TMEM-resident O only has to be rescaled when the maximum jumps.
+      constexpr float kLazy = 8.0f;
+      float m_ref = -INFINITY, l_run = 0.f;
+      const uint64_t scale2 = pack_f32x2(__float_as_uint(p.scale_log2e), __float_as_uint(p.scale_log2e));
+      const int col_max = p.causal ? min(row_g + p.causal_off, it.kv_limit - 1) : it.kv_limit - 1;  // last visible column
+      for (int i = 0; i < nt && ok; ++i) {
+        const int col_base = (SPLIT ? 2 * i + t : i) * BN;
+        if (!mbar_wait(&s_full[t], (j0 + i) & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const bool need_mask = (p.causal && col_base + BN - 1 > row0 + p.causal_off) || (col_base + BN > it.kv_limit);
+        uint32_t sv[4][32];
+        __syncwarp();
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld_32x32(tSt + c * 32, sv[c]);
-      tmem_wait_ld();
-      if (need_mask) {
-        const int lim = col_max - col_base;
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32(tSt + c * 32, sv[c]);
+        tmem_wait_ld();
+        if (need_mask) {
+          const int lim = col_max - col_base;
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (c * 32 + e > lim) sv[c][e] = 0xFF800000u;   // -inf
+        }
+        // the scores stay unscaled here: the scale is positive, so the maximum commutes with it, and the exponent below
+        // applies it inside one fused multiply-add. Eight chains: a dependent chain of 128 cannot be hidden.
+        float mxs[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) mxs[e] = fmaxf(__uint_as_float(sv[0][e]), __uint_as_float(sv[0][e + 8]));
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (c * 32 + e > lim) sv[c][e] = 0xFF800000u;   // -inf
+          for (int e = (c == 0 ? 16 : 0); e < 32; e += 16)
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              mxs[k] = fmaxf(fmaxf(mxs[k], __uint_as_float(sv[c][e + k])), __uint_as_float(sv[c][e + 8 + k]));
+        float mx = fmaxf(fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])), fmaxf(fmaxf(mxs[4], mxs[5]), fmaxf(mxs[6], mxs[7])));
+        mx *= p.scale_log2e;   // -inf stays -inf
+        // Rescale O (and l) only when some row of the warp moved its maximum by more than kLazy. S of this tile is finished,
+        // so every product of the tiles before it is: O may be touched without another wait.
+        if (__any_sync(0xffffffffu, mx > m_ref + kLazy)) {
+          const float m_new = fmaxf(m_ref, mx);
+          const float alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m_new);  // m_new is finite here or equals m_ref
+          if (i > 0) {
+#pragma unroll
+            for (int cc = 0; cc < D / 16; ++cc) {
+              uint32_t o[16];
+              tmem_ld_32x16(tOt + cc * 16, o);
+              tmem_wait_ld();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+              tmem_st_32x16(tOt + cc * 16, o);
+            }
+          }
+          l_run *= alpha;
+          m_ref = m_new;
+        }
+        const float m_neg = m_ref == -INFINITY ? 0.f : -m_ref;
+        const uint64_t m_neg2 = pack_f32x2(__float_as_uint(m_neg), __float_as_uint(m_neg));
+        uint64_t rs[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t packed[16];
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            float pv[4];
+            unpack_f32x2(fma_f32x2(pack_f32x2(sv[c][e], sv[c][e + 1]), scale2, m_neg2), pv[0], pv[1]);
+            unpack_f32x2(fma_f32x2(pack_f32x2(sv[c][e + 2], sv[c][e + 3]), scale2, m_neg2), pv[2], pv[3]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) pv[k] = fast_exp2(pv[k]);   // masked entries are -inf -> 0
+            rs[(e >> 1) & 3] = add_f32x2(rs[(e >> 1) & 3], pack_f32x2(__float_as_uint(pv[0]), __float_as_uint(pv[1])));
+            rs[((e >> 1) + 1) & 3] = add_f32x2(rs[((e >> 1) + 1) & 3], pack_f32x2(__float_as_uint(pv[2]), __float_as_uint(pv[3])));
+            if constexpr (DROP) {
+              // the row sum keeps every probability; only what multiplies V is dropped (1 / keep is applied at the end)
+              const uint32_t keep = dropout_keep4(p.drop, static_cast<uint32_t>(it.bh), static_cast<uint32_t>(row_g),
+                                                  static_cast<uint32_t>((col_base + c * 32 + e) >> 2));
+#pragma unroll
+              for (int k = 0; k < 4; ++k) pv[k] = (keep >> k) & 1u ? pv[k] : 0.f;
+            }
+            packed[e >> 1] = pack_bf16x2(pv[0], pv[1]);
+            packed[(e >> 1) + 1] = pack_bf16x2(pv[2], pv[3]);
+          }
+          tmem_st_32x16(tSt + c * 16, packed);    // the whole row of S has left TMEM above
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(&p_full[t]);
+        float lo, hi;
+        unpack_f32x2(add_f32x2(add_f32x2(rs[0], rs[1]), add_f32x2(rs[2], rs[3])), lo, hi);
+        l_run += lo + hi;
       }
-      // the scores stay unscaled here: the scale is positive, so the maximum commutes with it, and the exponent below
-      // applies it inside one fused multiply-add. Eight chains: a dependent chain of 128 cannot be hidden.
-      float mxs[8];
+      if (ok && nt > 0) ok = mbar_wait(&o_done[t], seen & 1, abort_flag);
+      __nv_bfloat16* orow = p.out + ((static_cast<long long>(it.b) * p.Sq + row_g) * p.H + it.h) * D;
+      float* lse = p.lse ? p.lse + (static_cast<long long>(it.b) * p.H + it.h) * p.Sq + row_g : nullptr;
+      if constexpr (SPLIT) {
+        // O = (2^(m0 - m) O_0 + 2^(m1 - m) O_1) / l: both streams' accumulators lie in the same TMEM lanes, so each stream's
+        // threads write one half of the columns of the merged row.
+        if (ok) {
+          xchg[t * 128 + r] = make_float2(m_ref, l_run);
+          tc_fence_before();
+          mbar_arrive(pair_bar);
+          ok = mbar_wait(pair_bar, 0, abort_flag);
+        }
+        if (ok) {
+          tc_fence_after();
+          const float2 other = xchg[(t ^ 1) * 128 + r];
+          const float m0 = t == 0 ? m_ref : other.x, m1 = t == 0 ? other.x : m_ref;
+          const float l0 = t == 0 ? l_run : other.y, l1 = t == 0 ? other.y : l_run;
+          const float m = fmaxf(m0, m1);
+          const float a0 = m0 == -INFINITY ? 0.f : exp2f(m0 - m), a1 = m1 == -INFINITY ? 0.f : exp2f(m1 - m);
+          const float l_tot = a0 * l0 + a1 * l1;
+          const float inv = l_tot > 0.f ? (DROP ? p.drop.inv_keep : 1.f) / l_tot : 0.f;
+          const float w0 = a0 * inv, w1 = a1 * inv;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) mxs[e] = fmaxf(__uint_as_float(sv[0][e]), __uint_as_float(sv[0][e + 8]));
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int e = (c == 0 ? 16 : 0); e < 32; e += 16)
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            mxs[k] = fmaxf(fmaxf(mxs[k], __uint_as_float(sv[c][e + k])), __uint_as_float(sv[c][e + 8 + k]));
-      float mx = fmaxf(fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])), fmaxf(fmaxf(mxs[4], mxs[5]), fmaxf(mxs[6], mxs[7])));
-      mx *= p.scale_log2e;   // -inf stays -inf
-      // Rescale O (and l) only when some row of the warp moved its maximum by more than kLazy. S of this tile is finished,
-      // so every product of the tiles before it is: O may be touched without another wait.
-      if (__any_sync(0xffffffffu, mx > m_ref + kLazy)) {
-        const float m_new = fmaxf(m_ref, mx);
-        const float alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m_new);  // m_new is finite here or equals m_ref
-        if (i > 0) {
-#pragma unroll
-          for (int cc = 0; cc < D / 16; ++cc) {
-            uint32_t o[16];
-            tmem_ld_32x16(tOt + cc * 16, o);
+          for (int c0 = 0; c0 < D / 64; ++c0) {
+            const int cc = t * (D / 64) + c0;
+            uint32_t u[32], v[32];
+            __syncwarp();
+            // an accumulator that no product wrote holds whatever TMEM held before: it must not enter the sum even with weight 0
+            if (it.n_it[0] > 0) tmem_ld_32x32(tO + lane_addr + cc * 32, u);
+            if (it.n_it[1] > 0) tmem_ld_32x32(tO + lane_addr + 128 + cc * 32, v);
             tmem_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-            tmem_st_32x16(tOt + cc * 16, o);
+            for (int e = 0; e < 32; ++e) {
+              float f = it.n_it[0] > 0 ? __uint_as_float(u[e]) * w0 : 0.f;
+              if (it.n_it[1] > 0) f = fmaf(__uint_as_float(v[e]), w1, f);
+              u[e] = __float_as_uint(f);
+            }
+            if (row_g < p.Sq) {
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                uint32_t w4[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) w4[e] = pack_bf16x2(__uint_as_float(u[g * 8 + 2 * e]), __uint_as_float(u[g * 8 + 2 * e + 1]));
+                *reinterpret_cast<uint4*>(orow + cc * 32 + g * 8) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+              }
+            }
           }
+          if (t == 0 && row_g < p.Sq && lse) *lse = l_tot > 0.f ? (m + log2f(l_tot)) * 0.6931471805599453f : -INFINITY;
         }
-        l_run *= alpha;
-        m_ref = m_new;
-      }
-      const float m_neg = m_ref == -INFINITY ? 0.f : -m_ref;
-      const uint64_t m_neg2 = pack_f32x2(__float_as_uint(m_neg), __float_as_uint(m_neg));
-      uint64_t rs[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t packed[16];
-#pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          float pv[4];
-          unpack_f32x2(fma_f32x2(pack_f32x2(sv[c][e], sv[c][e + 1]), scale2, m_neg2), pv[0], pv[1]);
-          unpack_f32x2(fma_f32x2(pack_f32x2(sv[c][e + 2], sv[c][e + 3]), scale2, m_neg2), pv[2], pv[3]);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) pv[k] = fast_exp2(pv[k]);   // masked entries are -inf -> 0
-          rs[(e >> 1) & 3] = add_f32x2(rs[(e >> 1) & 3], pack_f32x2(__float_as_uint(pv[0]), __float_as_uint(pv[1])));
-          rs[((e >> 1) + 1) & 3] = add_f32x2(rs[((e >> 1) + 1) & 3], pack_f32x2(__float_as_uint(pv[2]), __float_as_uint(pv[3])));
-          if constexpr (DROP) {
-            // the row sum keeps every probability; only what multiplies V is dropped (1 / keep is applied at the end)
-            const uint32_t keep = dropout_keep4(p.drop, static_cast<uint32_t>(bh), static_cast<uint32_t>(row_g),
-                                                static_cast<uint32_t>((col_base + c * 32 + e) >> 2));
-#pragma unroll
-            for (int k = 0; k < 4; ++k) pv[k] = (keep >> k) & 1u ? pv[k] : 0.f;
-          }
-          packed[e >> 1] = pack_bf16x2(pv[0], pv[1]);
-          packed[(e >> 1) + 1] = pack_bf16x2(pv[2], pv[3]);
-        }
-        tmem_st_32x16(tSt + c * 16, packed);    // the whole row of S has left TMEM above
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(&p_full[t]);
-      float lo, hi;
-      unpack_f32x2(add_f32x2(add_f32x2(rs[0], rs[1]), add_f32x2(rs[2], rs[3])), lo, hi);
-      l_run += lo + hi;
-    }
-    if (ok && n > 0) ok = mbar_wait(&o_done[t], 0, abort_flag);
-    __nv_bfloat16* orow = p.out + ((static_cast<long long>(b) * p.Sq + row_g) * p.H + h) * D;
-    float* lse = p.lse ? p.lse + (static_cast<long long>(b) * p.H + h) * p.Sq + row_g : nullptr;
-    if constexpr (SPLIT) {
-      // O = (2^(m0 - m) O_0 + 2^(m1 - m) O_1) / l: both streams' accumulators lie in the same TMEM lanes, so each stream's
-      // threads write one half of the columns of the merged row.
-      if (ok) {
-        xchg[t * 128 + r] = make_float2(m_ref, l_run);
-        tc_fence_before();
-        mbar_arrive(pair_bar);
-        ok = mbar_wait(pair_bar, 0, abort_flag);
-      }
-      if (ok) {
+      } else if (ok && nt > 0) {
         tc_fence_after();
-        const float2 other = xchg[(t ^ 1) * 128 + r];
-        const float m0 = t == 0 ? m_ref : other.x, m1 = t == 0 ? other.x : m_ref;
-        const float l0 = t == 0 ? l_run : other.y, l1 = t == 0 ? other.y : l_run;
-        const float m = fmaxf(m0, m1);
-        const float a0 = m0 == -INFINITY ? 0.f : exp2f(m0 - m), a1 = m1 == -INFINITY ? 0.f : exp2f(m1 - m);
-        const float l_tot = a0 * l0 + a1 * l1;
-        const float inv = l_tot > 0.f ? (DROP ? p.drop.inv_keep : 1.f) / l_tot : 0.f;
-        const float w0 = a0 * inv, w1 = a1 * inv;
+        const float inv = l_run > 0.f ? (DROP ? p.drop.inv_keep : 1.f) / l_run : 0.f;
 #pragma unroll
-        for (int c0 = 0; c0 < D / 64; ++c0) {
-          const int cc = t * (D / 64) + c0;
-          uint32_t u[32], v[32];
+        for (int cc = 0; cc < D / 32; ++cc) {
+          uint32_t v[32];
           __syncwarp();
-          // an accumulator that no product wrote holds whatever TMEM held before: it must not enter the sum even with weight 0
-          if (n_it[0] > 0) tmem_ld_32x32(tO + lane_addr + cc * 32, u);
-          if (n_it[1] > 0) tmem_ld_32x32(tO + lane_addr + 128 + cc * 32, v);
+          tmem_ld_32x32(tOt + cc * 32, v);
           tmem_wait_ld();
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            float f = n_it[0] > 0 ? __uint_as_float(u[e]) * w0 : 0.f;
-            if (n_it[1] > 0) f = fmaf(__uint_as_float(v[e]), w1, f);
-            u[e] = __float_as_uint(f);
-          }
           if (row_g < p.Sq) {
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-              uint32_t w4[4];
+              float f[8];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) w4[e] = pack_bf16x2(__uint_as_float(u[g * 8 + 2 * e]), __uint_as_float(u[g * 8 + 2 * e + 1]));
-              *reinterpret_cast<uint4*>(orow + cc * 32 + g * 8) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+              for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[g * 8 + e]) * inv;
+              *reinterpret_cast<uint4*>(orow + cc * 32 + g * 8) =
+                  make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
             }
           }
         }
-        if (t == 0 && row_g < p.Sq && lse) *lse = l_tot > 0.f ? (m + log2f(l_tot)) * 0.6931471805599453f : -INFINITY;
+        tc_fence_before();
+        mbar_arrive(&o_free[t]);
+        if (row_g < p.Sq && lse) *lse = l_run > 0.f ? (m_ref + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
+      } else if (ok && row_g < p.Sq) {
+        // No visible keys at all (kv_len == 0, or a causal tile above the shifted diagonal): the output rows are zero.
+        for (int e = 0; e < D; e += 8) *reinterpret_cast<uint4*>(orow + e) = make_uint4(0, 0, 0, 0);
+        if (lse) *lse = -INFINITY;
       }
-    } else if (ok && n > 0) {
-      tc_fence_after();
-      const float inv = l_run > 0.f ? (DROP ? p.drop.inv_keep : 1.f) / l_run : 0.f;
-#pragma unroll
-      for (int cc = 0; cc < D / 32; ++cc) {
-        uint32_t v[32];
-        __syncwarp();
-        tmem_ld_32x32(tOt + cc * 32, v);
-        tmem_wait_ld();
-        if (row_g < p.Sq) {
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            float f[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[g * 8 + e]) * inv;
-            *reinterpret_cast<uint4*>(orow + cc * 32 + g * 8) =
-                make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
-          }
-        }
-      }
-      if (row_g < p.Sq && lse) *lse = l_run > 0.f ? (m_ref + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
-    } else if (ok && row_g < p.Sq) {
-      // No visible keys at all (kv_len == 0, or a causal tile above the shifted diagonal): the output rows are zero.
-      for (int e = 0; e < D; e += 8) *reinterpret_cast<uint4*>(orow + e) = make_uint4(0, 0, 0, 0);
-      if (lse) *lse = -INFINITY;
+      j0 += nt;
+      seen += nt > 0;
+      __syncwarp();
+      if (!next_item(n, item)) break;
     }
   }
 
@@ -476,7 +570,7 @@ static int launch_fmha_fwd_as(const CUtensorMap& tq, const CUtensorMap& tk, cons
   p.chunk = static_cast<int>(chunk < bh ? chunk : bh);
   const long long ctas = bh * p.n_qt;
   if (ctas > 0x7FFFFFFFll) return fail("fmha: too many query tiles");
-  kern<<<static_cast<unsigned>(ctas), 320, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  kern<<<static_cast<unsigned>(ctas), 384, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
 }
