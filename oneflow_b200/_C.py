@@ -31,7 +31,7 @@ class _BiasAct(torch.autograd.Function):
     def backward(ctx, dy):
         x, bias = ctx.saved_tensors
         dx = K.bias_act_bwd(x.contiguous(), bias, dy.contiguous(), ctx.act)
-        db = K.column_sum(dx.reshape(-1, dx.shape[-1])).to(bias.dtype) if bias is not None else None
+        db = K.column_sum(dx.reshape(-1, dx.shape[-1]), out_dtype=bias.dtype) if bias is not None else None
         return dx, db, None
 
 

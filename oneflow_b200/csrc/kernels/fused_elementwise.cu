@@ -8,6 +8,8 @@
 //   dropout mask generation        oneflow/user/kernels/random_mask_generator.cu (philox)
 #include <cuda_fp16.h>
 
+#include <cooperative_groups.h>
+
 #include "../common/host_utils.h"
 #include "../common/ptx.cuh"
 #include "ofb_kernels.h"
@@ -145,9 +147,9 @@ __global__ void cast_scale_kernel(const TIn* __restrict__ x, TOut* __restrict__ 
     y[i] = static_cast<TOut>(static_cast<float>(x[i]) * s);
 }
 
-// out[c] (+)= sum_r x[r, c]; x bf16 [rows, cols]. Grid: (cols/256 column panels, row slabs); each
+// out[c] += sum_r x[r, c] (fp32); x bf16 [rows, cols]. Grid: (cols/256 column panels, row slabs); each
 // CTA reduces its slab in registers/smem and adds the panel into out with one atomicAdd per column.
-__global__ void column_sum_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, int rows, int cols,
+__global__ void column_sum_add_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, int rows, int cols,
                                   int rows_per_cta) {
   // blockDim = (32 column-vectors, 8 row lanes); panel = 256 columns
   __shared__ float red[8][256 + 8];
@@ -172,6 +174,71 @@ __global__ void column_sum_kernel(const __nv_bfloat16* __restrict__ x, float* __
   for (int k = 0; k < 8; ++k) s += red[k][t];
   const int c = blockIdx.x * 256 + t;
   if (c < cols) atomicAdd(out + c, s);
+}
+
+// out[c] = sum_r x[r, c] as fp32 or bf16. A cluster of eight CTAs owns 64 columns and shares the rows; the first CTA adds the
+// eight partial sums over distributed shared memory and writes the result once: one launch where the kernel above needs its
+// buffer cleared and, for a bf16 gradient, its sums converted. For small matrices (2331 x 768: 3.7 us against 5.2 and two launches
+// less; 2331 x 3072 7.3 against 8.4); over large ones the slabs above use the memory better (16384 x 1024: 22.7 against 10.9 us).
+constexpr int kColSumCluster = 8;
+__global__ void __cluster_dims__(kColSumCluster, 1, 1) __launch_bounds__(256)
+column_sum_store_kernel(const __nv_bfloat16* __restrict__ x, void* __restrict__ out, int rows, int cols, int out_bf16) {
+  constexpr int VPP = 8, C = VPP * 8, RL = 256 / VPP;          // vectors per row, columns and row lanes of a CTA
+  __shared__ float red[RL][C + 1];
+  __shared__ float part[C];
+  auto cluster = cooperative_groups::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int c0 = (blockIdx.x / kColSumCluster) * C;
+  const int vec = threadIdx.x % VPP, rl = threadIdx.x / VPP;
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (c0 + vec * 8 < cols) {
+    const __nv_bfloat16* xc = x + c0 + vec * 8;
+    // every CTA takes a contiguous piece of the rows
+    const int per = (rows + kColSumCluster - 1) / kColSumCluster;
+    const long long end = min(rows, (rank + 1) * per);
+    long long r = static_cast<long long>(rank) * per + rl;
+    constexpr int U = 4;
+    for (; r + (U - 1) * RL < end; r += U * RL) {
+      uint4 q[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) q[u] = *reinterpret_cast<const uint4*>(xc + (r + u * RL) * cols);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t w[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = unpack_bf16x2(w[j]);
+          acc[2 * j] += f.x;
+          acc[2 * j + 1] += f.y;
+        }
+      }
+    }
+    for (; r < end; r += RL) {
+      float v[8];
+      load8(xc + r * cols, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += v[j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) red[rl][vec * 8 + j] = acc[j];
+  __syncthreads();
+  if (threadIdx.x < C) {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < RL; ++k) s += red[k][threadIdx.x];
+    part[threadIdx.x] = s;
+  }
+  cluster.sync();
+  const int c = c0 + threadIdx.x;
+  if (rank == 0 && threadIdx.x < C && c < cols) {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < kColSumCluster; ++k) s += cluster.map_shared_rank(part, k)[threadIdx.x];
+    if (out_bf16) reinterpret_cast<__nv_bfloat16*>(out)[c] = __float2bfloat16(s);
+    else reinterpret_cast<float*>(out)[c] = s;
+  }
+  cluster.sync();     // nobody leaves while its partial sums may still be read
 }
 
 static inline int ew_grid(long long work_items, int threads) {
@@ -264,6 +331,7 @@ OFB_API int ofb_cast_scale(const void* x, int in_dtype, void* y, int out_dtype, 
   return 0;
 }
 // out must be zeroed by the caller unless accumulating into existing values is wanted.
+// out += sums
 OFB_API int ofb_column_sum(const void* x, float* out, int rows, int cols, void* stream) {
   if (cols % 8) return fail("column_sum: cols must be a multiple of 8");
   if (rows == 0) return 0;
@@ -272,8 +340,18 @@ OFB_API int ofb_column_sum(const void* x, float* out, int rows, int cols, void* 
   if (slabs > (rows + 63) / 64) slabs = (rows + 63) / 64;
   if (slabs < 1) slabs = 1;
   const int rows_per_cta = (rows + slabs - 1) / slabs;
-  column_sum_kernel<<<dim3(panels, slabs), dim3(32, 8), 0, (cudaStream_t)stream>>>((const bf16*)x, out, rows, cols,
+  column_sum_add_kernel<<<dim3(panels, slabs), dim3(32, 8), 0, (cudaStream_t)stream>>>((const bf16*)x, out, rows, cols,
                                                                                  rows_per_cta);
+  OFB_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// out = sums, fp32 or bf16 (small matrices: see the kernel)
+OFB_API int ofb_column_sum_store(const void* x, void* out, int rows, int cols, int out_bf16, void* stream) {
+  if (cols % 8) return fail("column_sum: cols must be a multiple of 8");
+  if (cols <= 0) return 0;
+  column_sum_store_kernel<<<(unsigned)((cols + 63) / 64 * kColSumCluster), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, out, rows, cols,
+                                                                                                          out_bf16);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -652,12 +652,12 @@ layer_norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
   }
 }
 
-// Folds partial[nparts, cols] into out[cols] (fp32, optionally accumulating). Block = 32 columns x 32 part
+// Folds partial[nparts, cols] into out[cols] (fp32, optionally accumulating, or bf16). Block = 32 columns x 32 part
 // lanes: the lanes of a column stride over the parts, then a shared-memory step adds them. (With 8 lanes a column's 296 parts
 // were a chain of 37 loads: 8 us.)
 __global__ void __launch_bounds__(1024)
-fold_partials_kernel(const float* __restrict__ pa, const float* __restrict__ pb, float* __restrict__ outa,
-                     float* __restrict__ outb, int nparts, int cols, int accumulate) {
+fold_partials_kernel(const float* __restrict__ pa, const float* __restrict__ pb, void* __restrict__ outa, void* __restrict__ outb,
+                     int nparts, int cols, int accumulate, int out_bf16) {
   __shared__ float sa[32][33], sb[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -677,9 +677,14 @@ fold_partials_kernel(const float* __restrict__ pa, const float* __restrict__ pb,
   b = warp_sum(sb[tx][ty]);
   const int co = blockIdx.x * 32 + ty;
   if (tx == 0 && co < cols) {
-    if (accumulate) { a += outa[co]; b += outb[co]; }
-    outa[co] = a;
-    outb[co] = b;
+    if (out_bf16) {
+      reinterpret_cast<__nv_bfloat16*>(outa)[co] = __float2bfloat16(a);
+      reinterpret_cast<__nv_bfloat16*>(outb)[co] = __float2bfloat16(b);
+    } else {
+      float *oa = reinterpret_cast<float*>(outa), *ob = reinterpret_cast<float*>(outb);
+      oa[co] = accumulate ? oa[co] + a : a;
+      ob[co] = accumulate ? ob[co] + b : b;
+    }
   }
 }
 
@@ -730,12 +735,14 @@ OFB_API int ofb_layer_norm_fwd(const void* x, const void* gamma, const void* bet
 // Number of partial rows ofb_layer_norm_bwd writes: scratch must hold 2 * this * cols floats.
 OFB_API int ofb_layer_norm_bwd_parts(int rows) { return rows < 296 ? rows : 296; }
 
-OFB_API int ofb_layer_norm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
-                               const void* add_to_dx, void* dx, float* dgamma, float* dbeta, float* scratch,
-                               int accumulate_param_grads, int rows, int cols, void* stream) {
+// param_grads_bf16: dgamma and dbeta are bf16 (not combined with accumulation), else fp32.
+OFB_API int ofb_layer_norm_bwd_to(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
+                                  const void* add_to_dx, void* dx, void* dgamma, void* dbeta, float* scratch,
+                                  int accumulate_param_grads, int param_grads_bf16, int rows, int cols, void* stream) {
   if (cols <= 0 || cols % 8 != 0 || cols > 8 * kLnMaxVecPerThread * 1024)
     return fail("layer_norm_bwd: cols must be a positive multiple of 8 and <= 32768");
   if ((dgamma == nullptr) != (dbeta == nullptr)) return fail("layer_norm_bwd: dgamma and dbeta must be given together or not at all");
+  if (param_grads_bf16 && accumulate_param_grads) return fail("layer_norm_bwd: bf16 parameter gradients cannot be accumulated");
   if (rows <= 0) return 0;
   if (dgamma && !scratch) return fail("layer_norm_bwd: scratch required for parameter gradients");
   int nv;
@@ -780,10 +787,16 @@ OFB_API int ofb_layer_norm_bwd(const void* dy, const void* x, const void* gamma,
   }
   OFB_CUDA_OK(cudaGetLastError());
   if (dgamma) {
-    fold_partials_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(pg, pb, dgamma, dbeta, grid, cols, accumulate_param_grads);
+    fold_partials_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(pg, pb, dgamma, dbeta, grid, cols, accumulate_param_grads, param_grads_bf16);
     OFB_CUDA_OK(cudaGetLastError());
   }
   return 0;
+}
+
+OFB_API int ofb_layer_norm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
+                               const void* add_to_dx, void* dx, float* dgamma, float* dbeta, float* scratch,
+                               int accumulate_param_grads, int rows, int cols, void* stream) {
+  return ofb_layer_norm_bwd_to(dy, x, gamma, mean, rstd, add_to_dx, dx, dgamma, dbeta, scratch, accumulate_param_grads, 0, rows, cols, stream);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -872,7 +885,7 @@ OFB_API int ofb_layer_norm_bwd_noalloc(const void* dy, const void* x, const void
   }
   OFB_CUDA_OK(cudaGetLastError());
   if (dgamma) {
-    fold_partials_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(pg, pb, dgamma, dbeta, grid, cols, accumulate_param_grads);
+    fold_partials_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(pg, pb, dgamma, dbeta, grid, cols, accumulate_param_grads, 0);
     OFB_CUDA_OK(cudaGetLastError());
   }
   return 0;

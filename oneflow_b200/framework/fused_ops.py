@@ -200,12 +200,17 @@ def _wgrad(param, nd, dy2, x2):
     return _param_grad(param, nd, val, acc)
 
 
+def _grad_dtype(param, t):
+    """What the kernels write a parameter gradient as: the parameter's bf16 directly, fp32 for everything else."""
+    return torch.bfloat16 if t.is_cuda and param.dtype == torch.bfloat16 else torch.float32
+
+
 def _bgrad(param, nd, dy2):
     def acc(mg):
         K.column_sum(dy2, out=mg.view(-1))
 
     def val():
-        return K.column_sum(dy2).view(_loc(param).shape)
+        return K.column_sum(dy2, out_dtype=_grad_dtype(param, dy2)).view(_loc(param).shape)
     return _param_grad(param, nd, val, acc)
 
 
@@ -604,7 +609,8 @@ class _LayerNorm(torch.autograd.Function):
             gamma._grad_nd_sbp = beta._grad_nd_sbp = pnd
             dg = db = None
         else:
-            dx, dg, db = K.layer_norm_bwd(dy2, x2, gl, mean, rstd, add_to_dx=addend, want_param_grads=want)
+            dx, dg, db = K.layer_norm_bwd(dy2, x2, gl, mean, rstd, add_to_dx=addend, want_param_grads=want,
+                                          param_dtype=_grad_dtype(gl, dy2) if want else torch.float32)
             if want:
                 dg, db = dg.to(gl.dtype), db.to(gl.dtype)
                 if pl is not None:

@@ -27,7 +27,7 @@ class _FusedLinearAct(torch.autograd.Function):
             dy2 = K.bias_act_bwd(pre, None, dy2, ctx.act)
         dx = G.gemm(dy2, w, b_layout="kn")
         dw = G.gemm(dy2, x2, a_layout="km", b_layout="kn")
-        db = K.column_sum(dy2).to(dy.dtype) if ctx.has_bias else None
+        db = K.column_sum(dy2, out_dtype=dy.dtype) if ctx.has_bias else None
         return dx.reshape(ctx.shape), dw, db, None
 
 

@@ -67,9 +67,9 @@ def layer_norm_fwd(x, gamma, beta, eps=1e-5):
     return y, mean, rstd
 
 
-def layer_norm_bwd(dy, x, gamma, mean, rstd, add_to_dx=None, dgamma=None, dbeta=None, want_param_grads=True):
-    """Returns (dx bf16, dgamma fp32, dbeta fp32). When dgamma/dbeta buffers are given the parameter
-    gradients are accumulated into them."""
+def layer_norm_bwd(dy, x, gamma, mean, rstd, add_to_dx=None, dgamma=None, dbeta=None, want_param_grads=True, param_dtype=torch.float32):
+    """Returns (dx bf16, dgamma, dbeta). When fp32 dgamma/dbeta buffers are given the parameter gradients are accumulated into
+    them; otherwise they are returned as ``param_dtype`` (float32, or bfloat16: the fp32 sums rounded once)."""
     rows, cols = x.shape
     if (dgamma is None) != (dbeta is None):
         raise ValueError("layer_norm_bwd: dgamma and dbeta must be given together or not at all")
@@ -85,21 +85,24 @@ def layer_norm_bwd(dy, x, gamma, mean, rstd, add_to_dx=None, dgamma=None, dbeta=
         if dgamma is not None:
             dgamma += dg
             dbeta += db
-            dg, db = dgamma, dbeta
-        return dx.to(x.dtype), dg, db
+            return dx.to(x.dtype), dgamma, dbeta
+        return dx.to(x.dtype), dg.to(param_dtype), db.to(param_dtype)
     _need_bf16(dy, x, gamma, add_to_dx)
     dx = torch.empty_like(x)
     accumulate = dgamma is not None
     scratch = None
     if want_param_grads:
         if dgamma is None:
-            dgamma = torch.empty(cols, dtype=torch.float32, device=x.device)
-            dbeta = torch.empty(cols, dtype=torch.float32, device=x.device)
+            if param_dtype not in (torch.float32, torch.bfloat16):
+                raise TypeError(f"layer_norm_bwd: param_dtype must be float32 or bfloat16, got {param_dtype}")
+            dgamma = torch.empty(cols, dtype=param_dtype, device=x.device)
+            dbeta = torch.empty(cols, dtype=param_dtype, device=x.device)
         parts = _lib().ofb_layer_norm_bwd_parts(c_int(rows))
         scratch = torch.empty(2 * parts * cols, dtype=torch.float32, device=x.device)
-    check(_lib().ofb_layer_norm_bwd(ptr(dy), ptr(x), ptr(gamma), ptr(mean), ptr(rstd), ptr(add_to_dx), ptr(dx),
-                                    ptr(dgamma if want_param_grads else None), ptr(dbeta if want_param_grads else None),
-                                    ptr(scratch), c_int(int(accumulate)), c_int(rows), c_int(cols), stream_ptr()),
+    half = want_param_grads and not accumulate and param_dtype == torch.bfloat16
+    check(_lib().ofb_layer_norm_bwd_to(ptr(dy), ptr(x), ptr(gamma), ptr(mean), ptr(rstd), ptr(add_to_dx), ptr(dx),
+                                       ptr(dgamma if want_param_grads else None), ptr(dbeta if want_param_grads else None),
+                                       ptr(scratch), c_int(int(accumulate)), c_int(int(half)), c_int(rows), c_int(cols), stream_ptr()),
           "layer_norm_bwd")
     _count(2 if want_param_grads else 1)
     return dx, dgamma, dbeta
@@ -195,19 +198,28 @@ def cast_scale(x, scale=1.0, out_dtype=torch.float32, scale_by_tensor=None, out=
     return out
 
 
-def column_sum(x, out=None):
-    """fp32 sum over rows of a bf16 [rows, cols] matrix (bias gradient); accumulates into `out` if given."""
+def column_sum(x, out=None, out_dtype=torch.float32):
+    """Sum over rows of a bf16 [rows, cols] matrix (bias gradient) in fp32; accumulates into the fp32 ``out`` if given, else
+    returns ``out_dtype`` (float32 or bfloat16: the fp32 sum rounded once)."""
     rows, cols = x.shape
     if not x.is_cuda:
         r = x.float().sum(0)
         if out is not None:
             out += r
             return out
-        return r
+        return r.to(out_dtype)
     _need_bf16(x)
-    if out is None:
-        out = torch.zeros(cols, dtype=torch.float32, device=x.device)
-    check(_lib().ofb_column_sum(ptr(x), ptr(out), c_int(rows), c_int(cols), stream_ptr()), "column_sum")
+    if out is not None:
+        check(_lib().ofb_column_sum(ptr(x), ptr(out), c_int(rows), c_int(cols), stream_ptr()), "column_sum")
+        _count()
+        return out
+    if out_dtype not in (torch.float32, torch.bfloat16):
+        raise TypeError(f"column_sum: out_dtype must be float32 or bfloat16, got {out_dtype}")
+    if rows * cols > 1 << 23:      # large matrices: a cleared buffer and atomics over row slabs use the memory better
+        return column_sum(x, torch.zeros(cols, dtype=torch.float32, device=x.device)).to(out_dtype)
+    out = torch.empty(cols, dtype=out_dtype, device=x.device)
+    check(_lib().ofb_column_sum_store(ptr(x), ptr(out), c_int(rows), c_int(cols), c_int(int(out_dtype == torch.bfloat16)), stream_ptr()),
+          "column_sum")
     _count()
     return out
 

@@ -204,6 +204,8 @@ def test_layer_norm_narrow_rows(rows, cols):
     close(dx, xd.grad + add.double(), 2.0 ** -8 * 1.02, 1e-4)
     close(dg, gd.grad, 1e-4, 1e-4 * rows ** 0.5)
     close(db, bd.grad, 1e-5, 1e-5 * rows ** 0.5)
+    _, hg, hb = K.layer_norm_bwd(dy, x, g, mean, rstd, add_to_dx=add, param_dtype=BF)
+    assert torch.equal(hg, dg.to(BF)) and torch.equal(hb, db.to(BF))      # the same fp32 sums, rounded once
     acc_g, acc_b = torch.ones(cols, device=DEV), torch.ones(cols, device=DEV)
     dx2, _, _ = K.layer_norm_bwd(dy, x, g, mean, rstd, dgamma=acc_g, dbeta=acc_b)
     close(dx2, xd.grad, 2.0 ** -8 * 1.02, 1e-4)
@@ -294,6 +296,22 @@ def test_bias_mask_scale_and_dropout_mask():
     assert torch.equal(mask, mask2)
     y = K.bias_mask_scale(x, b, mask, 1 / 0.9, add)
     close(y, K.bias_mask_scale(x.cpu(), b.cpu(), mask.cpu(), 1 / 0.9, add.cpu()))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (31, 64), (256, 72), (1025, 776), (5000, 128), (3, 4096), (8200, 1024)])
+def test_column_sum_outputs(rows, cols):
+    """Rows around what a cluster takes per step (256, unrolled 1024), columns around the 64 it owns, and a matrix on the other side
+    of the size limit; all three outputs."""
+    torch.manual_seed(19)
+    x = torch.randn(rows, cols, device=DEV, dtype=BF)
+    ref = x.double().sum(0)
+    out = K.column_sum(x)
+    close(out, ref, 1e-6, 1e-6 * rows ** 0.5 * 4)       # fp32 sums in a tree of short chains
+    # one rounding to bf16 (2^-8); beside it only the order of the atomics of a large matrix
+    close(K.column_sum(x, out_dtype=BF), ref, 2.0 ** -8 * 1.01, 1e-6 * rows ** 0.5 * 4)
+    acc = torch.full((cols,), 2.0, device=DEV)
+    assert K.column_sum(x, out=acc) is acc
+    close(acc, ref + 2.0, 1e-6, 1e-6 * rows ** 0.5 * 4)
 
 
 def test_cast_scale_column_sum():
