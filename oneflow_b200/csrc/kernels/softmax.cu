@@ -219,7 +219,7 @@ xent_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __r
         for (int j = 0; j < 4; ++j) { const float2 f = unpack_bf16x2(w[j]); cm = fmaxf(cm, fmaxf(f.x, f.y)); }
       }
       if (cm > m) {
-        s *= __expf(m - cm);
+        s *= expf(m - cm);
         m = cm;
       }
       const float ref = m == -INFINITY ? 0.f : m;
@@ -233,7 +233,7 @@ xent_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __r
       s += t[0] + t[1];
     }
     const float wm = wmax(m);
-    s = wsum(wm == -INFINITY ? s : s * __expf(m - wm));
+    s = wsum(wm == -INFINITY ? s : s * expf(m - wm));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) { red_m[threadIdx.x >> 5] = wm; red_s[threadIdx.x >> 5] = s; }
     __syncthreads();
@@ -241,7 +241,7 @@ xent_stats_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __r
       const float m1 = threadIdx.x < W ? red_m[threadIdx.x] : -INFINITY;
       const float s1 = threadIdx.x < W ? red_s[threadIdx.x] : 0.f;
       const float mx = wmax(m1);
-      const float sum = wsum(s1 * __expf(m1 - mx));
+      const float sum = wsum(s1 * expf(m1 - mx));
       if (threadIdx.x == 0) {
         const long long lab = labels[row] - vocab_start;
         float tgt = 0.f;
