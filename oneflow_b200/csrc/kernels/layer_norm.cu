@@ -489,8 +489,8 @@ layer_norm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
 // ------------------------------------------------------------------------------------------------
 // Narrow rows: one warp owns a row (NV 16-byte vectors per lane, cols <= 256 NV), so a row needs ten shuffles and no barrier.
 // A CTA per row kept 4 to 8 warps waiting on two barriers for 512 to 2048 bytes of work.
-// Bound by memory. Measured on a B200, before and after: forward 16384 x 1024 18.9 -> 13.2 us (10.3 at the copy rate),
-// 2331 x 768 7.4 -> 3.3 us, 8192 x 1536 32 -> 16 us; backward with parameter gradients 16384 x 1024 56 -> 30 us, 2048 x 512
+// Bound by memory. Measured on a B200, before and after: forward 16384 x 1024 18.9 -> 14.0 us (10.3 at the copy rate),
+// 2331 x 768 7.4 -> 3.3 us, 8192 x 1536 32 -> 16 us; backward with parameter gradients 16384 x 1024 56 -> 31 us, 2048 x 512
 // 14.3 -> 7 us, 32768 x 256 90 -> 21 us.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void ln_unpack8(const uint4& q, float (&v)[8]) {
@@ -505,7 +505,6 @@ layer_norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
                            const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out,
                            float* __restrict__ rstd_out, int rows, int cols, float eps) {
   const int lane = threadIdx.x & 31, nvec = cols >> 3, stride = gridDim.x * 8;
-  const float inv_cols = 1.f / cols;
   uint4 gq[NV], bq[NV], nxt[NV];
   auto load_row = [&](int row) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<long long>(row) * cols);
@@ -532,15 +531,18 @@ layer_norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
       s += ((v[i][0] + v[i][1]) + (v[i][2] + v[i][3])) + ((v[i][4] + v[i][5]) + (v[i][6] + v[i][7]));   // absent vectors are zero
     }
     if (row + stride < rows) load_row(row + stride);   // in flight under this row's math
-    const float mean = warp_sum(s) * inv_cols;
+    const float mean = warp_sum(s) / cols;
     float q = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i)
       if (lane + i * 32 < nvec) {
+        float d[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { const float d = v[i][j] - mean; q = fmaf(d, d, q); }
+        for (int j = 0; j < 8; ++j) d[j] = v[i][j] - mean;
+        // short chains: added one by one, the 32 squares of a lane cost a bit of the variance
+        q += ((d[0] * d[0] + d[1] * d[1]) + (d[2] * d[2] + d[3] * d[3])) + ((d[4] * d[4] + d[5] * d[5]) + (d[6] * d[6] + d[7] * d[7]));
       }
-    const float rstd = rsqrtf(warp_sum(q) * inv_cols + eps);
+    const float rstd = rsqrtf(warp_sum(q) / cols + eps);
     if (lane == 0) {
       if (mean_out) mean_out[row] = mean;
       if (rstd_out) rstd_out[row] = rstd;
@@ -574,7 +576,6 @@ layer_norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
   extern __shared__ float fold[];      // [warps][cols]
   constexpr int kWarps = ln_bwd_warps(NV);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = cols >> 3;
-  const float inv_cols = 1.f / cols;
   uint4 gq[NV];
   float acc_g[NV][8], acc_b[NV][8];
 #pragma unroll
@@ -613,8 +614,8 @@ layer_norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
         s2 = fmaf(a, h, s2);
       }
     }
-    s1 = warp_sum(s1) * inv_cols;
-    s2 = warp_sum(s2) * inv_cols;
+    s1 = warp_sum(s1) / cols;
+    s2 = warp_sum(s2) / cols;
     uint4* dxr = reinterpret_cast<uint4*>(dx + base);
 #pragma unroll
     for (int i = 0; i < NV; ++i)
