@@ -373,6 +373,24 @@ def test_xent(vocab):
     close(l2, ref, 1e-3, 1e-3)
 
 
+@pytest.mark.parametrize("rows,cols", [(4096, 1000), (4096, 8192), (296, 8200), (4096, 16392), (4096, 50304)])
+def test_xent_sum_accuracy(rows, cols):
+    """The sum of exponentials of unit-normal logits against 64 bits, for every number of threads a row is given."""
+    err = []
+    for rep in range(max(1, 8192 // rows)):
+        g = torch.Generator(device=DEV).manual_seed(40 + rep)
+        x = torch.randn(rows, cols, device=DEV, generator=g).to(BF)
+        st = K.xent_stats(x, torch.zeros(rows, dtype=torch.long, device=DEV))
+        xd = x.double()
+        err.append(st[:, 1].double() / torch.exp(xd - xd.max(1, keepdim=True).values).sum(1) - 1)
+    err = torch.cat(err)
+    # One rounding to fp32 is 2^-24 / sqrt(3) = 3.4e-8 of the power of two below, 2.5e-8 of the value on average; the threads'
+    # own sums and exponentials average out over 128 threads or more. A sum added in fp32 throughout adds a second rounding of
+    # that size (the last levels of the tree): 3.5e-8 before anything else.
+    assert float(err.pow(2).mean().sqrt()) < 3.5e-8
+    assert abs(float(err.mean())) < 1e-8      # __expf errs by a few units in the last place, not to one side
+
+
 @pytest.mark.parametrize("rows,cols,expanded", [(1, 8, False), (3, 4096, True), (5, 16384 + 8, False), (1200, 2 * 16384 - 8, True)])
 def test_xent_row_scale_and_extremes(rows, cols, expanded):
     """Widths around the 16384 elements a block takes per step, more rows than blocks, incoming gradients per row or one value;
