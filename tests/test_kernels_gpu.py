@@ -314,6 +314,32 @@ def test_column_sum_outputs(rows, cols):
     close(acc, ref + 2.0, 1e-6, 1e-6 * rows ** 0.5 * 4)
 
 
+@pytest.mark.parametrize("rows,cols", [(100000, 64), (25488, 40), (512, 16384), (8192, 256)])
+def test_column_sum_takes_the_kernel_that_suits_the_shape(rows, cols):
+    """Tall or wide matrices: returning the sums costs no more than clearing a buffer and adding them to it (five times as much
+    by the kernel for small matrices), timed in turn as captured graphs."""
+    x = torch.randn(rows, cols, device=DEV, dtype=BF)
+
+    def graph(fn):
+        fn()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(20):
+                fn()
+        return g
+    graphs = [graph(lambda: K.column_sum(x)), graph(lambda: K.column_sum(x, out=torch.zeros(cols, device=DEV)))]
+    best = [1e9, 1e9]
+    for _ in range(5):
+        for i, g in enumerate(graphs):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            g.replay()
+            b.record()
+            torch.cuda.synchronize()
+            best[i] = min(best[i], a.elapsed_time(b))
+    assert best[0] < 1.25 * best[1] + 0.005, best
+
+
 def test_cast_scale_column_sum():
     torch.manual_seed(6)
     x = torch.randn(1000, 776, device=DEV, dtype=BF)
