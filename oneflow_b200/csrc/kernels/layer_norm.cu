@@ -23,6 +23,12 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // Block-wide sum of two values at once; `red` holds 2*32 floats.
 __device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
   a = warp_sum(a);
@@ -505,6 +511,7 @@ layer_norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
                            const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out,
                            float* __restrict__ rstd_out, int rows, int cols, float eps) {
   const int lane = threadIdx.x & 31, nvec = cols >> 3, stride = gridDim.x * 8;
+  const double inv_cols = 1.0 / cols;
   uint4 gq[NV], bq[NV], nxt[NV];
   auto load_row = [&](int row) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<long long>(row) * cols);
@@ -531,7 +538,9 @@ layer_norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloa
       s += ((v[i][0] + v[i][1]) + (v[i][2] + v[i][3])) + ((v[i][4] + v[i][5]) + (v[i][6] + v[i][7]));   // absent vectors are zero
     }
     if (row + stride < rows) load_row(row + stride);   // in flight under this row's math
-    const float mean = warp_sum(s) / cols;
+    // A lane's sum of 8 NV bf16 values is all but exact in 32 bits; added across the lanes in 32 bits too, it lost up to four
+    // roundings (2331 x 1000, values around 1: relative error 4.1e-8, root mean square, against 2.7e-8, which is one rounding).
+    const float mean = static_cast<float>(warp_sum(static_cast<double>(s)) * inv_cols);
     float q = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i)

@@ -215,6 +215,22 @@ def test_layer_norm_narrow_rows(rows, cols):
     close(plain, torch.nn.functional.layer_norm(xd, (cols,)), 2.0 ** -8 * 1.02, 2e-5)
 
 
+@pytest.mark.parametrize("rows,cols", [(2331, 264), (2331, 768), (2331, 1000), (2331, 1280), (2331, 2040)])
+def test_layer_norm_mean_is_rounded_once(rows, cols):
+    """Row means of values around 1, no power of two in a row, against 64 bits."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x = (torch.randn(rows, cols, device=DEV, generator=g) + 1).to(BF)
+    _, mean, rstd = K.layer_norm_fwd(x, None, None, 1e-5)
+    ref = x.double().mean(1)
+    # half a unit in the last place (2^-24 above 1, 2^-25 below). A lane's sum of at most 64 bf16 values rounds away a last bit now
+    # and then: up to 8 % more over such rows in an emulation on the CPU, where 32-bit sums across the lanes are up to 4 times off
+    bound = torch.where(ref >= 1, 2.0 ** -24, 2.0 ** -25) * 1.25
+    assert bool(((mean.double() - ref).abs() <= bound).all())
+    # the square sum of short chains, a division, rsqrtf to two units: 1.5e-7 each at most, 1e-7 root mean square in all
+    r64 = 1 / torch.sqrt(x.double().var(1, unbiased=False) + 1e-5)
+    assert float((rstd.double() / r64 - 1).pow(2).mean().sqrt()) < 1e-7
+
+
 @pytest.mark.parametrize("rows,C,residual", [(1, 8, False), (37, 96, True), (5003, 64, True), (4099, 64, False), (130, 2048, True)])
 def test_batch_norm_sign_mask(rows, C, residual):
     """The backward from the forward's one-bit mask: the same masked gradient as from y (bit for bit), and right against 64 bits.
