@@ -654,27 +654,31 @@ layer_norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
     __syncthreads();
     float* out = (which == 0 ? partial_dgamma : partial_dbeta) + static_cast<long long>(blockIdx.x) * cols;
     for (int c = threadIdx.x; c < cols; c += blockDim.x) {
-      float a = 0.f;
+      float a[4] = {0.f, 0.f, 0.f, 0.f};     // short chains: few rows are summed to the last bit or two
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) a += fold[w * cols + c];
-      out[c] = a;
+      for (int w = 0; w < kWarps; ++w) a[w & 3] += fold[w * cols + c];
+      out[c] = (a[0] + a[1]) + (a[2] + a[3]);
     }
   }
 }
 
-// Folds partial[nparts, cols] into out[cols] (fp32, optionally accumulating, or bf16). Block = 32 columns x 32 part
-// lanes: the lanes of a column stride over the parts, then a shared-memory step adds them. (With 8 lanes a column's 296 parts
-// were a chain of 37 loads: 8 us.)
-__global__ void __launch_bounds__(1024)
+// Folds partial[nparts, cols] into out[cols] (fp32, optionally accumulating, or bf16). Block = 32 columns x LANES part
+// lanes: the lanes of a column stride over the parts, then a shared-memory step adds them. 32 lanes for many parts (with 8 a
+// column's 296 parts are a chain of 37 loads: 8 us). A block of 1024 threads takes 0.3 us longer to start and to meet than one of
+// 256: 8 lanes where each has two loads at most, or where 32 would go round a second time for a few parts (whole backward of 8, 24
+// and 34 rows of 2048: 4.8, 5.4 and 5.2 us with 8 lanes, 5.0, 5.1 and 5.4 with 32).
+template <int LANES>
+__global__ void __launch_bounds__(LANES * 32)
 fold_partials_kernel(const float* __restrict__ pa, const float* __restrict__ pb, void* __restrict__ outa, void* __restrict__ outb,
                      int nparts, int cols, int accumulate, int out_bf16) {
-  __shared__ float sa[32][33], sb[32][33];
+  __shared__ float sa[LANES][33], sb[LANES][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
   float a = 0.f, b = 0.f;
+  constexpr int U = LANES == 8 ? 4 : 5;      // loads in flight: half of what a lane has, and half of the 10 of 296 parts
   if (c < cols) {
-#pragma unroll 5
-    for (int p = ty; p < nparts; p += 32) {
+#pragma unroll U
+    for (int p = ty; p < nparts; p += LANES) {
       a += pa[static_cast<long long>(p) * cols + c];
       b += pb[static_cast<long long>(p) * cols + c];
     }
@@ -682,11 +686,17 @@ fold_partials_kernel(const float* __restrict__ pa, const float* __restrict__ pb,
   sa[ty][tx] = a;
   sb[ty][tx] = b;
   __syncthreads();
-  // warp `ty` adds the 32 partial sums of column `ty` of the block
-  a = warp_sum(sa[tx][ty]);
-  b = warp_sum(sb[tx][ty]);
-  const int co = blockIdx.x * 32 + ty;
-  if (tx == 0 && co < cols) {
+  // LANES threads of a warp add a column's partial sums, 32 / LANES columns a warp
+  const int k = tx % LANES, col = ty * (32 / LANES) + tx / LANES;
+  a = sa[k][col];
+  b = sb[k][col];
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  const int co = blockIdx.x * 32 + col;
+  if (k == 0 && co < cols) {
     if (out_bf16) {
       reinterpret_cast<__nv_bfloat16*>(outa)[co] = __float2bfloat16(a);
       reinterpret_cast<__nv_bfloat16*>(outb)[co] = __float2bfloat16(b);
@@ -696,6 +706,15 @@ fold_partials_kernel(const float* __restrict__ pa, const float* __restrict__ pb,
       ob[co] = accumulate ? ob[co] + b : b;
     }
   }
+}
+
+static void fold_partials(const float* pa, const float* pb, void* outa, void* outb, int nparts, int cols, int accumulate, int out_bf16,
+                          cudaStream_t s) {
+  const unsigned blocks = (cols + 31) / 32;
+  if (nparts <= 16 || (nparts > 32 && nparts <= 48))
+    fold_partials_kernel<8><<<blocks, 256, 0, s>>>(pa, pb, outa, outb, nparts, cols, accumulate, out_bf16);
+  else
+    fold_partials_kernel<32><<<blocks, 1024, 0, s>>>(pa, pb, outa, outb, nparts, cols, accumulate, out_bf16);
 }
 
 static int ln_block_threads(int cols, int& nv) {
@@ -768,7 +787,9 @@ OFB_API int ofb_layer_norm_bwd_to(const void* dy, const void* x, const void* gam
   if (dgamma && !scratch) return fail("layer_norm_bwd: scratch required for parameter gradients");
   int nv;
   const int threads = ln_block_threads(cols, nv);
-  const bool narrow = cols <= 1024;
+  // A warp per row once every SM has a row; with fewer, a whole block a row is faster except for the narrowest (34 x 1024 4.7 against
+  // 5.8 us, 148 x 512 5.5 against 5.6, 296 x 512 6.5 against 5.8; 64 x 256 5.1 against 4.7).
+  const bool narrow = cols <= 1024 && (cols <= 256 || rows > 148);
   int grid = ofb_layer_norm_bwd_parts(rows);      // also the number of partial rows
   const int warps = ln_bwd_warps(cols <= 256 ? 1 : cols <= 512 ? 2 : 4);
   if (narrow) grid = (rows + warps - 1) / warps < 148 ? (rows + warps - 1) / warps : 148;
@@ -808,7 +829,7 @@ OFB_API int ofb_layer_norm_bwd_to(const void* dy, const void* x, const void* gam
   }
   OFB_CUDA_OK(cudaGetLastError());
   if (dgamma) {
-    fold_partials_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(pg, pb, dgamma, dbeta, grid, cols, accumulate_param_grads, param_grads_bf16);
+    fold_partials(pg, pb, dgamma, dbeta, grid, cols, accumulate_param_grads, param_grads_bf16, s);
     OFB_CUDA_OK(cudaGetLastError());
   }
   return 0;
@@ -906,7 +927,7 @@ OFB_API int ofb_layer_norm_bwd_noalloc(const void* dy, const void* x, const void
   }
   OFB_CUDA_OK(cudaGetLastError());
   if (dgamma) {
-    fold_partials_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(pg, pb, dgamma, dbeta, grid, cols, accumulate_param_grads, 0);
+    fold_partials(pg, pb, dgamma, dbeta, grid, cols, accumulate_param_grads, 0, s);
     OFB_CUDA_OK(cudaGetLastError());
   }
   return 0;
