@@ -775,16 +775,11 @@ OFB_API int ofb_layer_norm_fwd(const void* x, const void* gamma, const void* bet
 // Number of partial rows ofb_layer_norm_bwd writes: scratch must hold 2 * this * cols floats.
 OFB_API int ofb_layer_norm_bwd_parts(int rows) { return rows < 296 ? rows : 296; }
 
-// param_grads_bf16: dgamma and dbeta are bf16 (not combined with accumulation), else fp32.
-OFB_API int ofb_layer_norm_bwd_to(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
-                                  const void* add_to_dx, void* dx, void* dgamma, void* dbeta, float* scratch,
-                                  int accumulate_param_grads, int param_grads_bf16, int rows, int cols, void* stream) {
-  if (cols <= 0 || cols % 8 != 0 || cols > 8 * kLnMaxVecPerThread * 1024)
-    return fail("layer_norm_bwd: cols must be a positive multiple of 8 and <= 32768");
-  if ((dgamma == nullptr) != (dbeta == nullptr)) return fail("layer_norm_bwd: dgamma and dbeta must be given together or not at all");
-  if (param_grads_bf16 && accumulate_param_grads) return fail("layer_norm_bwd: bf16 parameter gradients cannot be accumulated");
-  if (rows <= 0) return 0;
-  if (dgamma && !scratch) return fail("layer_norm_bwd: scratch required for parameter gradients");
+// All backward entry points: checked sizes, `scratch` for ofb_layer_norm_bwd_parts(rows) partial rows when dgamma is given.
+// may_allocate = false keeps to kernels without bounded waits: the first look at a device's status word allocates it.
+static int launch_layer_norm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
+                                 const void* add_to_dx, void* dx, void* dgamma, void* dbeta, float* scratch, int accumulate_param_grads,
+                                 int param_grads_bf16, bool may_allocate, int rows, int cols, cudaStream_t s) {
   int nv;
   const int threads = ln_block_threads(cols, nv);
   // A warp per row once every SM has a row; with fewer, a whole block a row is faster except for the narrowest (34 x 1024 4.7 against
@@ -793,7 +788,6 @@ OFB_API int ofb_layer_norm_bwd_to(const void* dy, const void* x, const void* gam
   int grid = ofb_layer_norm_bwd_parts(rows);      // also the number of partial rows
   const int warps = ln_bwd_warps(cols <= 256 ? 1 : cols <= 512 ? 2 : 4);
   if (narrow) grid = (rows + warps - 1) / warps < 148 ? (rows + warps - 1) / warps : 148;
-  auto s = reinterpret_cast<cudaStream_t>(stream);
   float* pg = dgamma ? scratch : nullptr;
   float* pb = dgamma ? scratch + static_cast<long long>(grid) * cols : nullptr;
   auto DY = reinterpret_cast<const __nv_bfloat16*>(dy);
@@ -809,7 +803,7 @@ OFB_API int ofb_layer_norm_bwd_to(const void* dy, const void* x, const void* gam
     if (cols <= 256) layer_norm_bwd_warp_kernel<1><<<grid, warps * 32, smem, s>>>(DY, X, G, mean, rstd, AD, DX, pg, pb, rows, cols);
     else if (cols <= 512) layer_norm_bwd_warp_kernel<2><<<grid, warps * 32, smem, s>>>(DY, X, G, mean, rstd, AD, DX, pg, pb, rows, cols);
     else layer_norm_bwd_warp_kernel<4><<<grid, warps * 32, smem, s>>>(DY, X, G, mean, rstd, AD, DX, pg, pb, rows, cols);
-  } else if (nv <= 2 && aligned16 && !ring_off) {
+  } else if (nv <= 2 && aligned16 && may_allocate && !ring_off) {
     const int smem = kLnRingStages * 3 * cols * 2;
     static bool configured = false;
     if (!configured) {
@@ -833,6 +827,20 @@ OFB_API int ofb_layer_norm_bwd_to(const void* dy, const void* x, const void* gam
     OFB_CUDA_OK(cudaGetLastError());
   }
   return 0;
+}
+
+// param_grads_bf16: dgamma and dbeta are bf16 (not combined with accumulation), else fp32.
+OFB_API int ofb_layer_norm_bwd_to(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
+                                  const void* add_to_dx, void* dx, void* dgamma, void* dbeta, float* scratch,
+                                  int accumulate_param_grads, int param_grads_bf16, int rows, int cols, void* stream) {
+  if (cols <= 0 || cols % 8 != 0 || cols > 8 * kLnMaxVecPerThread * 1024)
+    return fail("layer_norm_bwd: cols must be a positive multiple of 8 and <= 32768");
+  if ((dgamma == nullptr) != (dbeta == nullptr)) return fail("layer_norm_bwd: dgamma and dbeta must be given together or not at all");
+  if (param_grads_bf16 && accumulate_param_grads) return fail("layer_norm_bwd: bf16 parameter gradients cannot be accumulated");
+  if (rows <= 0) return 0;
+  if (dgamma && !scratch) return fail("layer_norm_bwd: scratch required for parameter gradients");
+  return launch_layer_norm_bwd(dy, x, gamma, mean, rstd, add_to_dx, dx, dgamma, dbeta, scratch, accumulate_param_grads, param_grads_bf16,
+                               true, rows, cols, reinterpret_cast<cudaStream_t>(stream));
 }
 
 OFB_API int ofb_layer_norm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
@@ -909,26 +917,6 @@ OFB_API int ofb_layer_norm_bwd_noalloc(const void* dy, const void* x, const void
   if (rows <= 0) return 0;
   float* scratch = nullptr;
   if (noalloc_scratch_ptr(&scratch)) return -1;
-  int nv;
-  const int threads = ln_block_threads(cols, nv);
-  const int grid = rows < kNoAllocMaxParts ? rows : kNoAllocMaxParts;
-  auto s = reinterpret_cast<cudaStream_t>(stream);
-  float* pg = dgamma ? scratch : nullptr;
-  float* pb = dgamma ? scratch + static_cast<long long>(grid) * cols : nullptr;
-  auto DY = reinterpret_cast<const __nv_bfloat16*>(dy);
-  auto X = reinterpret_cast<const __nv_bfloat16*>(x);
-  auto G = reinterpret_cast<const __nv_bfloat16*>(gamma);
-  auto AD = reinterpret_cast<const __nv_bfloat16*>(add_to_dx);
-  auto DX = reinterpret_cast<__nv_bfloat16*>(dx);
-  switch (nv) {
-    case 1: layer_norm_bwd_kernel<1><<<grid, threads, 0, s>>>(DY, X, G, mean, rstd, AD, DX, pg, pb, rows, cols); break;
-    case 2: layer_norm_bwd_kernel<2><<<grid, threads, 0, s>>>(DY, X, G, mean, rstd, AD, DX, pg, pb, rows, cols); break;
-    default: layer_norm_bwd_kernel<4><<<grid, threads, 0, s>>>(DY, X, G, mean, rstd, AD, DX, pg, pb, rows, cols); break;
-  }
-  OFB_CUDA_OK(cudaGetLastError());
-  if (dgamma) {
-    fold_partials(pg, pb, dgamma, dbeta, grid, cols, accumulate_param_grads, 0, s);
-    OFB_CUDA_OK(cudaGetLastError());
-  }
-  return 0;
+  return launch_layer_norm_bwd(dy, x, gamma, mean, rstd, add_to_dx, dx, dgamma, dbeta, scratch, accumulate_param_grads, 0, false, rows, cols,
+                               reinterpret_cast<cudaStream_t>(stream));
 }

@@ -24,7 +24,9 @@
 //   * All calls share the same array, which keeps the previous call's contents. The kernels overwrite
 //     every value they later read, so nothing has to be cleared between calls; but calls that overlap on
 //     the GPU (several streams or threads) race on it. Serialise them on one stream or with events.
-//   * Results are the same as ofb_layer_norm_bwd() for the same inputs.
+//   * Results are the same as ofb_layer_norm_bwd() for the same inputs: bit for bit up to 2048 columns. Wider
+//     rows stream through another kernel there (its waits report to a status word that is allocated at first
+//     use), whose fp32 sums have another order: a bf16 value of dx may be rounded the other way.
 #pragma once
 
 #ifdef __cplusplus

@@ -63,7 +63,7 @@ def test_layer_norm_bwd_noalloc_matches_regular_entry_point_twice():
         rc, dx, dg, db = _noalloc_bwd(lib, dy, x, g, mean, rstd, add)
         assert rc == 0, lib.ofb_last_error()
         torch.cuda.synchronize()
-        # same kernels, same inputs: the two entry points agree to within the tolerance used for the op
+        # another kernel at 4096 columns, the same one at 1024: the two entry points agree to within the tolerance used for the op
         _close(dx, ref_dx, 2e-2)
         _close(dg, ref_dg, 5e-2)
         _close(db, ref_db, 5e-2)
@@ -83,6 +83,22 @@ def test_layer_norm_bwd_noalloc_matches_regular_entry_point_twice():
     _close(dg2, 2 * ref_dg, 5e-2)
     _close(db2, 2 * ref_db, 5e-2)
     assert _native.read_status() == (0, 0)
+
+
+@pytest.mark.parametrize("rows,cols", [(64, 1024), (333, 256), (333, 1024), (5000, 512), (2000, 1536), (77, 2048)])
+def test_layer_norm_bwd_noalloc_is_bitwise_the_regular_entry_point(rows, cols):
+    """Up to 2048 columns the header promises equal bits, whichever kernel the number of rows chooses."""
+    lib = ctypes.CDLL(_native.lib_path("libofb_kernels.so"))
+    lib.ofb_layer_norm_bwd_noalloc.restype = c_int
+    torch.manual_seed(23)
+    x, dy, add = (torch.randn(rows, cols, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    g = torch.randn(cols, device="cuda", dtype=torch.bfloat16)
+    _, mean, rstd = K.layer_norm_fwd(x, g, g, 1e-5)
+    want = K.layer_norm_bwd(dy, x, g, mean, rstd, add_to_dx=add)
+    rc, *got = _noalloc_bwd(lib, dy, x, g, mean, rstd, add)
+    assert rc == 0
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
 
 
 def test_layer_norm_bwd_noalloc_rejects_oversized_problem():
