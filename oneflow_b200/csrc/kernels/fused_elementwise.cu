@@ -348,7 +348,7 @@ OFB_API int ofb_column_sum(const void* x, float* out, int rows, int cols, void* 
 // out = sums, fp32 or bf16 (small matrices: see the kernel)
 OFB_API int ofb_column_sum_store(const void* x, void* out, int rows, int cols, int out_bf16, void* stream) {
   if (cols % 8) return fail("column_sum: cols must be a multiple of 8");
-  if (cols <= 0) return 0;
+  if (cols <= 0) return rows == 0 ? 0 : fail("column_sum: no columns");
   column_sum_store_kernel<<<(unsigned)((cols + 63) / 64 * kColSumCluster), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, out, rows, cols,
                                                                                                           out_bf16);
   OFB_CUDA_OK(cudaGetLastError());

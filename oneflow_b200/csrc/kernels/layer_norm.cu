@@ -735,6 +735,7 @@ OFB_API int ofb_layer_norm_fwd(const void* x, const void* gamma, const void* bet
                                int rows, int cols, float eps, void* stream) {
   if (cols % 8 != 0 || cols > 8 * kLnMaxVecPerThread * 1024) return fail("layer_norm: cols must be a multiple of 8 and <= 32768");
   if (rows <= 0) return 0;
+  if (cols <= 0) return fail("layer_norm: rows without columns have no mean");
   int nv;
   const int threads = ln_block_threads(cols, nv);
   const int grid = rows < 148 * 16 ? rows : 148 * 16;

@@ -218,6 +218,19 @@ def test_layer_norm_narrow_rows(rows, cols):
     close(plain, torch.nn.functional.layer_norm(xd, (cols,)), 2.0 ** -8 * 1.02, 2e-5)
 
 
+def test_rows_without_columns_are_refused():
+    """They have neither a mean nor a column to sum; without rows there is nothing to do."""
+    x = torch.empty(4, 0, device=DEV, dtype=BF)
+    with pytest.raises(_native.NativeLibraryError):
+        K.layer_norm_fwd(x, None, None, 1e-5)
+    for dt in (torch.float32, BF):
+        with pytest.raises(_native.NativeLibraryError):
+            K.column_sum(x, out_dtype=dt)
+    none = torch.empty(0, 64, device=DEV, dtype=BF)
+    assert K.layer_norm_fwd(none, None, None, 1e-5)[0].shape == (0, 64)
+    assert not K.column_sum(none).any() and K.column_sum(none).shape == (64,)
+
+
 @pytest.mark.parametrize("rows,cols", [(2331, 264), (2331, 768), (2331, 1000), (2331, 1280), (2331, 2040)])
 def test_layer_norm_mean_is_rounded_once(rows, cols):
     """Row means of values around 1, no power of two in a row, against 64 bits."""
