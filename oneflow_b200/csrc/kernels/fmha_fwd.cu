@@ -9,9 +9,11 @@
 //   warp 1      tcgen05 issuer: S_t = Q_t K^T, then O_t += P_t V with P_t read from TMEM (it lies over the S_t it came from)
 //   warps 4..7  softmax of stream 0, warps 8..11 of stream 1: one thread owns one whole query row (a TMEM lane), so row
 //               maxima and sums need no exchange, and P goes back to TMEM without touching shared memory
-// The streams are two neighbouring query tiles (SPLIT = false: every K / V tile is loaded once for 256 rows), or, when that
-// would leave SMs without a CTA, the even and the odd key tiles of ONE query tile whose two results are merged at the end
-// (SPLIT = true: twice the CTAs, half the chain).
+// The streams are two neighbouring query tiles (kPairs: every K / V tile is loaded once for 256 rows), or, when that would leave
+// SMs without a CTA, the even and the odd key tiles of ONE query tile whose two results are merged at the end (kSplit: twice the
+// CTAs, half the chain), or the two halves of its only key tile (kOneTile). With dropout the random numbers are most of a stream's
+// work: the last of an odd number of split tiles is halved too. (Without, the branches for that cost more than they gain: 128
+// heads, 1 x 512, D = 128 10.7 against 10.1 us.)
 //
 // What bounds it: the exponentials (16 per clock and SM: 1024 clocks for a 128 x 128 tile) and the two products of a D = 128
 // tile (1024 clocks) alike. Measured on a B200, forward alone, against the one-stream kernel this replaced (P through shared
@@ -62,14 +64,23 @@ struct FmhaFwdCfg {
   static constexpr int SMEM_BYTES = 2 * Q_BYTES + SLOTS * KV_BYTES + BAR_BYTES + XCHG_BYTES;
 };
 
-template <int D, bool DROP, bool SPLIT>
+// How the two streams of a CTA share the work.
+enum FmhaFwdMode {
+  kPairs = 0,      // two neighbouring query tiles
+  kSplit = 1,      // the even and the odd key tiles of one query tile
+  kOneTile = 2,    // no more than 128 keys: their first and second 64
+};
+
+template <int D, bool DROP, int MODE>
 __global__ void __launch_bounds__(384, 1)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, FmhaFwdParams p) {
   using Cfg = FmhaFwdCfg<D>;
   constexpr int BM = 128, BN = 128, DCH = D / 64;  // 64-element chunks along the head dimension
   constexpr int SLOTS = Cfg::SLOTS;
-  constexpr uint32_t IDESC_S = make_idesc_bf16(BM, BN, 0, 0);
+  constexpr bool SPLIT = MODE != kPairs, ONE = MODE == kOneTile;
+  constexpr bool HALVE = ONE || (SPLIT && DROP);   // whether a key tile may be shared by the streams, 64 keys each
+  constexpr uint32_t IDESC_S = make_idesc_bf16(BM, BN, 0, 0), IDESC_S_HALF = make_idesc_bf16(BM, BN / 2, 0, 0);
   constexpr uint32_t IDESC_O = make_idesc_bf16(BM, D, 0, 1);
   constexpr int CH_BYTES = 128 * 128;  // one [128 rows x 64 elements] swizzled chunk
 
@@ -105,6 +116,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   struct Item {
     int q0, bh, h, b, hk, kv_limit;
     int n_it[2];     // key tiles of each stream
+    bool shared;     // HALVE: both streams take half of the last tile
   };
   auto item_of = [&](int item) {
     const int in_chunk_max = p.chunk * p.n_qt;
@@ -125,7 +137,8 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       int kv_end = it.kv_limit;
       if (p.causal) kv_end = min(kv_end, r0 + BM + p.causal_off);
       const int n = (kv_end > 0 && r0 < p.Sq) ? (kv_end + BN - 1) / BN : 0;
-      it.n_it[t] = SPLIT ? (n - t + 1) >> 1 : n;
+      it.shared = HALVE && (n & 1) && kv_end - (n - 1) * BN > BN / 2;    // its second half holds a key that some row sees
+      it.n_it[t] = SPLIT ? (n + (t == 0 || it.shared)) >> 1 : n;
     }
     return it;
   };
@@ -191,7 +204,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       bool ok = true;
       for (int n = 0;; ++n) {
         const Item it = item_of(item);
-        const int tiles = SPLIT ? it.n_it[0] + it.n_it[1] : max(it.n_it[0], it.n_it[1]);
+        const int tiles = ONE ? it.n_it[0] : SPLIT ? it.n_it[0] + it.n_it[1] - it.shared : max(it.n_it[0], it.n_it[1]);
         if (elect_one()) {
           auto load_kv = [&](const CUtensorMap* m, int tile) -> bool {
             const int s = c % SLOTS;
@@ -255,55 +268,69 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       bool ok = true;
       for (int n = 0;; ++n) {
         const Item it = item_of(item);
-        const int tiles = SPLIT ? it.n_it[0] + it.n_it[1] : max(it.n_it[0], it.n_it[1]);
+        const int tiles = ONE ? it.n_it[0] : SPLIT ? it.n_it[0] + it.n_it[1] - it.shared : max(it.n_it[0], it.n_it[1]);
         if (elect_one() && tiles > 0 && ok) {
           const uint32_t kv_base = smem_u32(sKV);
           auto slot_ready = [&](int c) -> bool { return mbar_wait(&kv_full[c % SLOTS], (c / SLOTS) & 1, abort_flag); };
-          auto issue_s = [&](int t, int c) {     // S_t = Q_t K^T with the K tile of load c
+          // S_t = Q_t K^T with the K tile of load c, or (half) with its keys 64 t .. 64 t + 63: eight groups of eight rows further
+          auto issue_s = [&](int t, int c, bool half) {
             const uint32_t q_base = smem_u32(sQ + (SPLIT ? 0 : t) * Cfg::Q_BYTES);
-            const uint32_t k_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES;
+            const uint32_t k_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES + (half ? t * 8192 : 0);
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
               const uint32_t off = (kk >> 2) * CH_BYTES + (kk & 3) * 32;
               umma_bf16_ss(tS + t * BN, make_smem_desc_sw128(q_base + off, 16, 1024), make_smem_desc_sw128(k_base + off, 16, 1024),
-                           IDESC_S, kk != 0 ? 1u : 0u);
+                           half ? IDESC_S_HALF : IDESC_S, kk != 0 ? 1u : 0u);
             }
             umma_commit(&s_full[t]);
           };
-          auto issue_pv = [&](int t, int c, bool first) {   // O_t (+)= P_t V with the V tile of load c
-            const uint32_t v_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES;
+          auto issue_pv = [&](int t, int c, bool first, bool half) {   // O_t (+)= P_t V with the V tile of load c, or with its half
+            const uint32_t v_base = kv_base + (c % SLOTS) * Cfg::KV_BYTES + (half ? t * 8192 : 0);
 #pragma unroll
             for (int kk = 0; kk < BN / 16; ++kk)
-              umma_bf16_ts(tO + t * 128, tS + t * BN + kk * 8, make_smem_desc_sw128(v_base + kk * 2048, CH_BYTES, 1024), IDESC_O,
-                           (first && kk == 0) ? 0u : 1u);
+              if (kk < BN / 32 || !half)
+                umma_bf16_ts(tO + t * 128, tS + t * BN + kk * 8, make_smem_desc_sw128(v_base + kk * 2048, CH_BYTES, 1024), IDESC_O,
+                             (first && kk == 0) ? 0u : 1u);
           };
           auto release = [&](int c) { umma_commit(&kv_empty[c % SLOTS]); };
           if constexpr (SPLIT) {
-            int c = 0;
-            ok = mbar_wait(&q_full[0], 0, abort_flag);
-            for (int t = 0; t < 2 && t < tiles && ok; ++t) {
-              ok = slot_ready(c);
-              if (!ok) break;
+            // loads come in the order K0 K1 V0 K2 V1 K3 ... of the producer; a shared tile's stay until stream 1 has used them too
+            // (for good where there is only one)
+            auto halved = [&](int g) { return ONE || (HALVE && it.shared && g == tiles - 1); };
+            auto next_s = [&](int t, int g) -> bool {
+              const int c = g == 0 ? 0 : 2 * g - 1;
+              if (!slot_ready(c)) return false;
               tc_fence_after();
-              issue_s(t, c);
-              release(c);
-              ++c;
-            }
+              issue_s(t, c, halved(g));
+              if (!ONE && (!halved(g) || t == 1)) release(c);
+              return true;
+            };
+            auto next_pv = [&](int t, int g) -> bool {
+              const int c = g == tiles - 1 ? 2 * tiles - 1 : 2 * g + 2;
+              if (!mbar_wait(&p_full[t], (g >> 1) & 1, abort_flag) || !slot_ready(c)) return false;
+              tc_fence_after();
+              issue_pv(t, c, g < 2, halved(g));
+              if (!ONE && (!halved(g) || t == 1)) release(c);
+              return true;
+            };
+            ok = mbar_wait(&q_full[0], 0, abort_flag) && next_s(0, 0);
+            if (!ONE && tiles > 1) ok = ok && next_s(1, 1);
+            else if (it.shared) ok = ok && next_s(1, 0);
             for (int g = 0; g < tiles && ok; ++g) {
-              const int t = g & 1, i = g >> 1;
-              if (!mbar_wait(&p_full[t], i & 1, abort_flag) || !slot_ready(c)) { ok = false; break; }
-              tc_fence_after();
-              issue_pv(t, c, i == 0);
-              release(c);
-              ++c;
-              if (g + 2 < tiles) {
-                if (!slot_ready(c)) { ok = false; break; }
-                tc_fence_after();
-                issue_s(t, c);
-                release(c);
-                ++c;
+              if (halved(g)) {
+                ok = next_pv(0, g);
+                if (ok) umma_commit(&o_done[0]);
+                if (it.shared) {
+                  ok = ok && next_pv(1, g);
+                  if (ok) umma_commit(&o_done[1]);
+                }
               } else {
-                umma_commit(&o_done[t]);
+                const int t = g & 1;
+                ok = next_pv(t, g);
+                if (!ok) break;
+                if (g + 2 < tiles) ok = next_s(t, g + 2);
+                else if (HALVE && t == 1 && it.shared) ok = next_s(1, tiles - 1);
+                else umma_commit(&o_done[t]);
               }
             }
           } else {
@@ -313,7 +340,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               ok = mbar_wait(&q_full[t], seen[t] & 1, abort_flag);
               if (!ok) break;
               tc_fence_after();
-              issue_s(t, c0);
+              issue_s(t, c0, false);
             }
             if (ok) release(c0);
             for (int i = 0; i < tiles && ok; ++i) {
@@ -324,12 +351,12 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 // O of the item before has left TMEM
                 if (i == 0 && !mbar_wait(&o_free[t], (seen[t] & 1) ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                issue_pv(t, cv, i == 0);
+                issue_pv(t, cv, i == 0, false);
                 if (t == 1 || i >= it.n_it[1]) release(cv);       // the last stream to use the tile
                 if (i + 1 < it.n_it[t]) {
                   if (!slot_ready(ck1)) { ok = false; break; }
                   tc_fence_after();
-                  issue_s(t, ck1);
+                  issue_s(t, ck1, false);
                   if (t == 1 || i + 1 >= it.n_it[1]) release(ck1);
                 } else {
                   umma_commit(&o_done[t]);
@@ -371,15 +398,24 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       float m_ref = -INFINITY, l_run = 0.f;
       const uint64_t scale2 = pack_f32x2(__float_as_uint(p.scale_log2e), __float_as_uint(p.scale_log2e));
       const int col_max = p.causal ? min(row_g + p.causal_off, it.kv_limit - 1) : it.kv_limit - 1;  // last visible column
-      for (int i = 0; i < nt && ok; ++i) {
-        const int col_base = (SPLIT ? 2 * i + t : i) * BN;
+      for (int i = 0; i < nt && ok && (!ONE || i == 0); ++i) {
+        const bool half = ONE || (HALVE && it.shared && i == nt - 1);
+        const int col_base = half ? 2 * i * BN + t * (BN / 2) : (SPLIT ? 2 * i + t : i) * BN;
+        const int nc = half ? 2 : 4, width = nc * 32;      // chunks of 32 key columns
         if (!mbar_wait(&s_full[t], (j0 + i) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const bool need_mask = (p.causal && col_base + BN - 1 > row0 + p.causal_off) || (col_base + BN > it.kv_limit);
+        const bool need_mask = (p.causal && col_base + width - 1 > row0 + p.causal_off) || (col_base + width > it.kv_limit);
         uint32_t sv[4][32];
         __syncwarp();
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld_32x32(tSt + c * 32, sv[c]);
+        for (int c = 0; c < 4; ++c) {
+          if (c < nc) {
+            tmem_ld_32x32(tSt + c * 32, sv[c]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) sv[c][e] = 0xFF800000u;
+          }
+        }
         tmem_wait_ld();
         if (need_mask) {
           const int lim = col_max - col_base;
@@ -408,7 +444,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (__any_sync(0xffffffffu, mx > m_ref + kLazy)) {
           const float m_new = fmaxf(m_ref, mx);
           const float alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m_new);  // m_new is finite here or equals m_ref
-          if (i > 0) {
+          if (!ONE && i > 0) {
 #pragma unroll
             for (int cc = 0; cc < D / 16; ++cc) {
               uint32_t o[16];
@@ -427,6 +463,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         uint64_t rs[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          if (c >= nc) continue;
           uint32_t packed[16];
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
@@ -551,17 +588,17 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
-template <int D, bool DROP, bool SPLIT>
+template <int D, bool DROP, int MODE>
 static int launch_fmha_fwd_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, FmhaFwdParams p,
                               cudaStream_t stream) {
   using Cfg = FmhaFwdCfg<D>;
-  auto kern = fmha_fwd_kernel<D, DROP, SPLIT>;
+  auto kern = fmha_fwd_kernel<D, DROP, MODE>;
   static bool configured = false;
   if (!configured) {
     OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     configured = true;
   }
-  p.n_qt = SPLIT ? (p.Sq + 127) / 128 : (p.Sq + 255) / 256;
+  p.n_qt = MODE == kPairs ? (p.Sq + 255) / 256 : (p.Sq + 127) / 128;
   // heads walked together: as many as keep their keys and values within a third of the L2 cache (the query heads of a group
   // share theirs), but at least one CTA for every SM
   const long long bh = static_cast<long long>(p.B) * p.H;
@@ -578,16 +615,40 @@ static int launch_fmha_fwd_as(const CUtensorMap& tq, const CUtensorMap& tk, cons
 template <int D, bool DROP>
 static int launch_fmha_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FmhaFwdParams& p,
                            cudaStream_t stream) {
+  const long long bh = static_cast<long long>(p.B) * p.H;
+  const long long pairs = bh * ((p.Sq + 255) / 256), tiles = bh * ((p.Sq + 127) / 128);
+  // Up to 128 keys a CTA's whole work is one tile: halved between the streams, by a kernel a third of the size, it takes 4.7 us
+  // instead of 5.8 (8 heads, 1 x 64, D = 64; with dropout 5.9 and 8.6). Pairs do not start a CTA per tile, which pays from two
+  // tiles an SM on (1024 heads, 64 x 64: 27 against 29 us), but not while a second wave of them does one tile of two (96 heads,
+  // 300 x 100: 10.7 against 12.6 us). With dropout the random numbers are most of the work, and halves of tiles balance it best
+  // (1024 heads, 64 x 64: 38 against 49 us; 128 x 128: 45 against 48).
+  if (p.Sk <= 128) {
+    if (DROP || tiles <= 148 || (p.Sq > 128 && pairs > 148 && tiles <= 2 * 148))
+      return launch_fmha_fwd_as<D, DROP, kOneTile>(tq, tk, tv, p, stream);
+    return launch_fmha_fwd_as<D, DROP, kPairs>(tq, tk, tv, p, stream);
+  }
   // Pairs of query tiles load every key once for 256 rows, but give half the CTAs of split key tiles, each with twice the
   // chain. Splitting pays while all its CTAs run at once (batch 1, 8 heads, 2048 keys, D = 64: 20.3 against 33.9 us), and under
   // a causal mask also up to one wave of pairs, as the short tiles of the second wave fill in behind the long ones (16 heads,
   // 2048 keys, D = 128: 29.3 against 37.9 us; 4 heads, 8192 keys: 67 against 125 us) once there are keys enough to split
   // (64 heads, 512 keys: 19.1 against 16.3 us). Otherwise pairs win (16 heads, 2048 keys, D = 128, full: 38.7 against 44.5 us;
   // 16 heads, 4096 keys, causal: 71 against 82 us).
-  const long long bh = static_cast<long long>(p.B) * p.H;
-  const long long pairs = bh * ((p.Sq + 255) / 256), tiles = bh * ((p.Sq + 127) / 128);
-  if (tiles <= 148 || (p.causal && pairs < 148 && p.Sk >= 1024)) return launch_fmha_fwd_as<D, DROP, true>(tq, tk, tv, p, stream);
-  return launch_fmha_fwd_as<D, DROP, false>(tq, tk, tv, p, stream);
+  bool split = tiles <= 148 || (p.causal && pairs < 148 && p.Sk >= 1024);
+  if constexpr (DROP) {
+    // The random numbers bind both forms to a time per step of a stream, so that waves of CTAs decide: a key tile takes a pair one
+    // step of each stream and split tiles half a step; beside the steps a wave costs 0.6 and 0.75 of one. Measured: 80 heads, 494 x
+    // 494, D = 64, causal 39 us in two waves of pairs, 30 us in three of split tiles; 24 heads, 3357 x 3357, D = 128 478 and
+    // 381 us; 512 heads, 512 x 512, D = 64 174 and 208 us; 256 heads, 1 x 2048, D = 128 157 and 95 us.
+    const long long nk = (p.Sk + 127) / 128, wp = (pairs + 147) / 148, wt = (tiles + 147) / 148;
+    split = split || wt * (10 * nk + 15) < wp * (20 * nk + 12);
+  } else {
+    // With one query tile a head a pair has only one, whose stream walks all keys while the other has nothing to do: split from
+    // five key tiles on (256 heads, 1 x 2048, D = 128: 49 against 62 us; 320 heads, 100 x 600: 35.6 against 37.4; but 640 heads,
+    // 128 x 256, D = 64: 30 against 26, 2048 heads, 1 x 512, D = 128: 125 against 116).
+    split = split || (p.Sq <= 128 && p.Sk > 512);
+  }
+  if (split) return launch_fmha_fwd_as<D, DROP, kSplit>(tq, tk, tv, p, stream);
+  return launch_fmha_fwd_as<D, DROP, kPairs>(tq, tk, tv, p, stream);
 }
 
 // 4-D map over a [B, S, H, D] view with a token stride of `row_stride` elements.

@@ -536,6 +536,64 @@ def test_fmha_streams_and_tile_edges(B, H, Hk, Sq, Sk, D, causal, lens):
         close(g, r, 3e-2, 2e-2)
 
 
+def _attention_backward_with_bounds(q, k, v, o, d_o, causal, kv_len, p, keep):
+    """(reference, bound) of dq, dk, dv in fp32 for the forward's own (rounded) output: the kernel rounds P and dS to bf16, half a
+    unit in the last place each (at most 2^-8 of the value, and dS is formed from the rounded P), and every result once; 5 % for
+    the fp32 parts."""
+    B, Sq, H, D = q.shape
+    Sk, Hk = k.shape[1:3]
+    qf, kf, vf, of, df = (t.float().permute(0, 2, 1, 3) for t in (q, k, v, o, d_o))
+    kx, vx = kf.repeat_interleave(H // Hk, 1), vf.repeat_interleave(H // Hk, 1)
+    s = qf @ kx.transpose(-1, -2) / math.sqrt(D)
+    if causal:
+        s = s.masked_fill(~torch.ones(Sq, Sk, dtype=torch.bool, device=q.device).tril(Sk - Sq), float("-inf"))
+    if kv_len is not None:
+        s = s.masked_fill(torch.arange(Sk, device=q.device) >= kv_len[:, None, None, None], float("-inf"))
+    pr = torch.nan_to_num(torch.softmax(s, -1))          # rows that see no key
+    z = 1.0 if keep is None else keep.float() / (1 - p)
+    ds = pr * (df @ vx.transpose(-1, -2) * z - (df * of).sum(-1, keepdim=True)) / math.sqrt(D)
+    pd = pr * z
+
+    def fold(t):        # sum over the query heads of a group
+        return t.view(B, Hk, H // Hk, Sk, D).sum(2)
+    dst, adst, pdt = ds.transpose(-1, -2), ds.abs().transpose(-1, -2), pd.transpose(-1, -2)
+    ref = (ds @ kx, fold(dst @ qf), fold(pdt @ df))
+    terms = (2.0 ** -7 * (ds.abs() @ kx.abs()), 2.0 ** -7 * fold(adst @ qf.abs()), 2.0 ** -8 * fold(pdt @ df.abs()))
+    return [(r.permute(0, 2, 1, 3), (1.05 * (t + r.abs() * 2.0 ** -8) + 1e-5).permute(0, 2, 1, 3)) for r, t in zip(ref, terms)]
+
+
+# Which form of the forward kernel the sizes choose is said beside them.
+@pytest.mark.parametrize("B,H,Hk,Sq,Sk,D,causal,lens,p", [
+    (3, 4, 2, 130, 100, 128, True, None, 0.2),                          # one key tile in halves
+    (2, 8, 8, 200, 64, 64, False, None, 0.2),                           # only its first half
+    (1, 4, 4, 1, 128, 128, False, None, 0.0),
+    (2, 3, 3, 7, 65, 64, False, None, 0.0),                             # one key in the second half
+    (40, 16, 16, 64, 128, 64, False, None, 0.0),                        # one key tile, 640 pairs
+    (3, 4, 4, 100, 300, 64, False, (300, 129, 320), 0.2),               # split, three tiles: the last halved; two tiles
+    (3, 4, 4, 100, 641, 128, True, (641, 577, 576), 0.2),               # split, five tiles and a key, then halves of one key and none
+    (20, 16, 4, 3, 641, 128, False, None, 0.0),                         # split for its length, in three waves
+    (90, 8, 8, 20, 385, 64, False, None, 0.2),                          # split with dropout, five waves
+])
+def test_fmha_halves_and_split_tiles(B, H, Hk, Sq, Sk, D, causal, lens, p):
+    torch.manual_seed(24)
+    q, d_o = torch.randn(B, Sq, H, D, device=DEV, dtype=BF), torch.randn(B, Sq, H, D, device=DEV, dtype=BF)
+    k, v = (torch.randn(B, Sk, Hk, D, device=DEV, dtype=BF) for _ in range(2))
+    kv_len = None if lens is None else torch.tensor([lens[i % len(lens)] for i in range(B)], dtype=torch.int32, device=DEV).clamp(max=Sk)
+    sc, drop = 1 / math.sqrt(D), dict(dropout_p=p, seed=0x1234567890ABCDEF, offset=9)
+    keep = K.fmha_dropout_mask(B, H, Sq, Sk, p, drop["seed"], 9, DEV) if p else None
+    out, lse = K.fmha_fwd(q, k, v, causal=causal, kv_len=kv_len, **drop)
+    ro, rl = K.fmha_reference(q, k, v, causal, sc, kv_len, p, keep)
+    ab, _ = K.fmha_reference(q, k, v.abs(), causal, sc, kv_len, p, keep)
+    # as in the test above: P and both results are rounded to bf16
+    assert bool(((out.float() - ro.float()).abs() <= 1.02 * (ab.float() / 256 + ro.float().abs() / 128) + 1e-6).all())
+    seen = torch.isfinite(rl)
+    assert torch.equal(seen, torch.isfinite(lse))
+    close(lse[seen], rl[seen], 1e-5, 1e-5)       # fp32 on both sides
+    got = K.fmha_bwd(q, k, v, out, d_o, lse, causal=causal, kv_len=kv_len, separate=True, **drop)
+    for g, (r, bound) in zip(got, _attention_backward_with_bounds(q, k, v, out, d_o, causal, kv_len, p, keep)):
+        assert bool(((g.float() - r).abs() <= bound).all())
+
+
 def test_multi_tensor_adamw_sgd_and_norm():
     torch.manual_seed(12)
     sizes = [1000, 65536 + 8, 300000, 16]
