@@ -562,8 +562,14 @@ def _attention_backward_with_bounds(q, k, v, o, d_o, causal, kv_len, p, keep):
     return [(r.permute(0, 2, 1, 3), (1.05 * (t + r.abs() * 2.0 ** -8) + 1e-5).permute(0, 2, 1, 3)) for r, t in zip(ref, terms)]
 
 
-# Which form of the forward kernel the sizes choose is said beside them.
+# Which form of the forward kernel the sizes choose is said beside them; "items" are what a CTA of the 148 works through in turn, so that
+# every slot and phase of its barriers comes round more than once.
 @pytest.mark.parametrize("B,H,Hk,Sq,Sk,D,causal,lens,p", [
+    (50, 16, 16, 200, 200, 64, False, None, 0.2),                       # 800 pairs (5 items), 1600 key tiles (11 items)
+    (50, 16, 4, 256, 320, 128, True, None, 0.2),                        # 800 pairs, 600 key tiles of four heads each
+    (50, 16, 16, 300, 140, 64, True, (0, 140, 65, 0, 129, 64, 140), 0.2),   # 1600 pairs: empty, of one stream only, one or two tiles
+    (50, 16, 16, 300, 140, 128, True, (0, 140, 65, 0, 129, 64, 140), 0.0),
+    (60, 16, 8, 129, 513, 64, False, (513, 0, 128, 385, 1, 257, 512), 0.0),  # 960 pairs of one to five tiles, 2400 key tiles
     (3, 4, 2, 130, 100, 128, True, None, 0.2),                          # one key tile in halves
     (2, 8, 8, 200, 64, 64, False, None, 0.2),                           # only its first half
     (1, 4, 4, 1, 128, 128, False, None, 0.0),
@@ -574,7 +580,7 @@ def _attention_backward_with_bounds(q, k, v, o, d_o, causal, kv_len, p, keep):
     (20, 16, 4, 3, 641, 128, False, None, 0.0),                         # split for its length, in three waves
     (90, 8, 8, 20, 385, 64, False, None, 0.2),                          # split with dropout, five waves
 ])
-def test_fmha_halves_and_split_tiles(B, H, Hk, Sq, Sk, D, causal, lens, p):
+def test_fmha_items_halves_and_dropout(B, H, Hk, Sq, Sk, D, causal, lens, p):
     torch.manual_seed(24)
     q, d_o = torch.randn(B, Sq, H, D, device=DEV, dtype=BF), torch.randn(B, Sq, H, D, device=DEV, dtype=BF)
     k, v = (torch.randn(B, Sk, Hk, D, device=DEV, dtype=BF) for _ in range(2))
