@@ -429,26 +429,27 @@ upsample2_zero_kernel(const bf16* __restrict__ dy, bf16* __restrict__ dx, int N,
 }
 
 // cols[(n, oh, ow)][(r * S + s) * Cin + c] = x[n, stride oh + r - pad, stride ow + s - pad, c] (zero outside and in
-// the padding columns up to ldc). For small Cin (the RGB stem). One CTA per output row (n, oh): the R input rows lie zero-padded
-// in shared memory, where the S Cin values of one filter row are neighbours, and every thread gathers 8 output columns at a time.
-// (A thread that fetched its 8 values from global memory after 64-bit divisions: 996 us for 256 x 224 x 224 x 3, 7 x 7, against
-// 467 us; 976 MB are written, 149 us at the copy rate.)
+// the padding columns up to ldc). For small Cin (the RGB stem). A CTA takes `cpp` neighbouring output columns of one output row
+// (n, oh): the R pieces of input rows that they see lie zero-padded in shared memory, where the S Cin values of one filter row are
+// neighbours, and every thread gathers 8 columns of the matrix at a time. (A thread that fetched its 8 values from global memory
+// after 64-bit divisions: 996 us for 256 x 224 x 224 x 3, 7 x 7, against 463 us; 976 MB are written, 149 us at the copy rate.)
 // CIN_ / R_ / S_ > 0 fix the shape at compile time (constant divisors); 0 takes the runtime values. STAGED = false reads the image
-// directly: rows too wide for shared memory.
+// directly: windows too large for shared memory.
 template <int CIN_, int R_, int S_, bool STAGED>
 __global__ void __launch_bounds__(256)
 im2col_small_kernel(const bf16* __restrict__ x, bf16* __restrict__ cols, int H, int W, int Cin_rt, int R_rt, int S_rt, int stride, int pad,
-                    int OH, int OW, int ldc) {
-  extern __shared__ unsigned short rows_s[];            // [R][(W + 2 pad) Cin]
+                    int OH, int OW, int cpp, int ldc) {
+  extern __shared__ unsigned short rows_s[];            // [R][(stride (cpp - 1) + S) Cin]
   const int Cin = CIN_ > 0 ? CIN_ : Cin_rt, R = R_ > 0 ? R_ : R_rt, S = S_ > 0 ? S_ : S_rt;
+  const int ow0 = blockIdx.y * cpp, n_ow = min(cpp, OW - ow0);
   const int oh = blockIdx.x % OH;
   const long long n = blockIdx.x / OH;
-  const int rlen = (W + 2 * pad) * Cin, lo = pad * Cin, hi = lo + W * Cin;
-  // element i of zero-padded input row r
+  const int from = stride * ow0 * Cin, rlen = (stride * (n_ow - 1) + S) * Cin, lo = pad * Cin, hi = lo + W * Cin;
+  // element i of the piece of zero-padded input row r
   auto fetch = [&](int r, int i) -> unsigned short {
     const int h = stride * oh + r - pad;
-    const bool in = h >= 0 && h < H && i >= lo && i < hi;
-    return in ? reinterpret_cast<const unsigned short*>(x)[(n * H + h) * W * Cin + (i - lo)] : static_cast<unsigned short>(0);
+    const bool in = h >= 0 && h < H && from + i >= lo && from + i < hi;
+    return in ? reinterpret_cast<const unsigned short*>(x)[(n * H + h) * W * Cin + (from + i - lo)] : static_cast<unsigned short>(0);
   };
   if constexpr (STAGED) {
     for (int r = 0; r < R; ++r)
@@ -456,8 +457,8 @@ im2col_small_kernel(const bf16* __restrict__ x, bf16* __restrict__ cols, int H, 
     __syncthreads();
   }
   const int vpr = ldc >> 3, fr = S * Cin, kcols = R * fr;
-  uint4* out = reinterpret_cast<uint4*>(cols) + static_cast<long long>(blockIdx.x) * OW * vpr;
-  for (int i = threadIdx.x; i < OW * vpr; i += blockDim.x) {
+  uint4* out = reinterpret_cast<uint4*>(cols) + (static_cast<long long>(blockIdx.x) * OW + ow0) * vpr;
+  for (int i = threadIdx.x; i < n_ow * vpr; i += blockDim.x) {
     const int ow = i / vpr, col0 = (i - ow * vpr) * 8;
     const int first = stride * ow * Cin;
     uint32_t o[4];
@@ -595,21 +596,24 @@ OFB_API int ofb_im2col_small(const void* x, void* cols, int N, int H, int W, int
                              void* stream) {
   if (ldc % 8 || ldc < R * S * Cin) return fail("im2col: leading dimension must be a multiple of 8 covering R S Cin");
   const int OH = (H + 2 * pad - R) / stride + 1, OW = (W + 2 * pad - S) / stride + 1;
-  if (N <= 0 || OH <= 0 || OW <= 0) return 0;
-  const long long smem = (long long)R * (W + 2 * pad) * Cin * 2;
-  const bool staged = smem <= 200 * 1024;
-  const long long ctas = (long long)N * OH;
-  if (ctas > 0x7FFFFFFFll) return fail("im2col: too many output rows");
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(im2col_small_kernel<3, 7, 7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    OFB_CUDA_OK(cudaFuncSetAttribute(im2col_small_kernel<0, 0, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    configured = true;
-  }
+  if (N <= 0 || OH <= 0 || OW <= 0 || ldc == 0) return 0;
+  const long long rows = (long long)N * OH;
+  if (rows > 0x7FFFFFFFll) return fail("im2col: too many output rows");
+  // Output columns of a CTA: whole rows from two CTAs an SM on, else pieces that make four, down to one round of the threads (1 x
+  // 96 x 96 in whole rows: 6.1 us, in four pieces 3.7; 4 x 224 x 224, 448 rows: 14.5 us, in two pieces 17.2), and never more than
+  // 48 KiB of input, which every device gives without asking.
+  const int round = 256 / (ldc / 8) > 0 ? 256 / (ldc / 8) : 1;
+  int cpp = rows < 2 * 148 ? (int)((OW * rows - 1) / (4 * 148) + 1) : OW;
+  if (cpp < round) cpp = round < OW ? round : OW;
+  const long long fit = (48 * 1024 / (R * Cin > 0 ? 2ll * R * Cin : 1) - S) / stride + 1;      // 0 or less: not one window
+  const bool staged = 2ll * R * S * Cin <= 48 * 1024 && (OW - 1) / (cpp < fit ? cpp : fit) < 65535;
+  if (!staged) cpp = OW;
+  else if (cpp > fit) cpp = (int)fit;
   auto launch = [&](auto kern, long long bytes) {
-    kern<<<(unsigned int)ctas, 256, (size_t)bytes, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)cols, H, W, Cin, R, S, stride, pad, OH, OW,
-                                                                          ldc);
+    kern<<<dim3((unsigned int)rows, (OW - 1) / cpp + 1), 256, (size_t)bytes, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)cols, H, W,
+                                                                                                     Cin, R, S, stride, pad, OH, OW, cpp, ldc);
   };
+  const long long smem = 2ll * R * (stride * (cpp - 1ll) + S) * Cin;
   if (!staged) launch(im2col_small_kernel<0, 0, 0, false>, 0);
   else if (Cin == 3 && R == 7 && S == 7) launch(im2col_small_kernel<3, 7, 7, true>, smem);
   else launch(im2col_small_kernel<0, 0, 0, true>, smem);

@@ -617,7 +617,7 @@ static int launch_fmha_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const C
                            cudaStream_t stream) {
   const long long bh = static_cast<long long>(p.B) * p.H;
   const long long pairs = bh * ((p.Sq + 255) / 256), tiles = bh * ((p.Sq + 127) / 128);
-  // Up to 128 keys a CTA's whole work is one tile: halved between the streams, by a kernel a third of the size, it takes 4.7 us
+  // Up to 128 keys a CTA's whole work is one tile: halved between the streams, by a kernel without ring, loop and rescaling, it takes 4.7 us
   // instead of 5.8 (8 heads, 1 x 64, D = 64; with dropout 5.9 and 8.6). Pairs do not start a CTA per tile, which pays from two
   // tiles an SM on (1024 heads, 64 x 64: 27 against 29 us), but not while a second wave of them does one tile of two (96 heads,
   // 300 x 100: 10.7 against 12.6 us). With dropout the random numbers are most of the work, and halves of tiles balance it best
