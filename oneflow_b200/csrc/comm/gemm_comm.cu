@@ -805,11 +805,7 @@ static int launch_gemm_comm2(const CUtensorMap& tmA, const CUtensorMap& tmAl, co
                              const GemmEpilogue& ep, const GemmCommParams& cp, int grid, cudaStream_t stream) {
   auto kern = gemm_comm2_kernel<B_MN, MODE>;
   constexpr int smem_bytes = MODE == MODE_RS ? 5 * (Gemm2Cfg::A_BYTES + Gemm2Cfg::B_BYTES) + 4 * 32 * 512 + 256 + 1024 : Gemm2Cfg::SMEM_BYTES;
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    configured = true;
-  }
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
   kern<<<grid & ~1, MODE == MODE_AG ? 256 : 192, smem_bytes, stream>>>(tmA, tmAl, tmB, shp, ep, cp);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
@@ -830,12 +826,8 @@ static int launch_gemm_comm(const CUtensorMap& tmA, const CUtensorMap& tmAl, con
                             const GemmEpilogue& ep, const GemmCommParams& cp, int grid, cudaStream_t stream) {
   using Cfg = GemmCfg<BN>;
   auto kern = gemm_comm_kernel<BN, B_MN, MODE>;
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      Cfg::SMEM_BYTES + (MODE == MODE_RS ? 4 * kEpiStageBytesPerWarp : 0)));
-    configured = true;
-  }
   kern<<<grid, MODE == MODE_AG ? 256 : 320, Cfg::SMEM_BYTES + (MODE == MODE_RS ? 4 * kEpiStageBytesPerWarp : 0), stream>>>(tmA, tmAl, tmB, shp, ep, cp);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;

@@ -12,6 +12,8 @@
 #include <string>
 #include <unordered_map>
 
+#include "per_device.h"
+
 #define OFB_API extern "C" __attribute__((visibility("default")))
 
 namespace ofb {
@@ -30,6 +32,15 @@ inline int fail(const std::string& msg) {
     cudaError_t _e = (expr);                                                                   \
     if (_e != cudaSuccess)                                                                     \
       return ::ofb::fail(std::string(#expr) + ": " + cudaGetErrorString(_e));                  \
+  } while (0)
+
+// Runs a CUDA call once for every device that is current here (a static per place and template instance).
+#define OFB_CUDA_OK_ONCE_PER_DEVICE(expr)                     \
+  do {                                                        \
+    static ::ofb::OncePerDevice once_;                        \
+    int dev_ = 0;                                             \
+    OFB_CUDA_OK(cudaGetDevice(&dev_));                        \
+    OFB_CUDA_OK(once_(dev_, [&] { return (expr); }));         \
   } while (0)
 
 // One 64-int status block per device, allocated on first use. Slot 0 holds the first

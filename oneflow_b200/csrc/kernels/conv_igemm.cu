@@ -330,11 +330,7 @@ static int conv_launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const Con
                        cudaStream_t stream) {
   using Cfg = GemmCfg<BN, ST>;
   auto kern = conv_igemm_kernel<MODE, BN, ST, MINB>;
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
-    configured = true;
-  }
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
   static int sm_count = 0;
   if (sm_count == 0) {
     int dev = 0;

@@ -656,11 +656,7 @@ static int launch_fmha_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const C
                            const CUtensorMap& tdq, FmhaBwdParams p, cudaStream_t stream) {
   using Cfg = FmhaBwdCfg<D>;
   auto kern = fmha_bwd_kernel<D, DROP>;
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
-    configured = true;
-  }
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
   p.n_kt = (p.Sk + 127) / 128;
   // heads walked together: as many as keep queries, gradients (bf16) and dQ (fp32) within a third of the L2 cache, but at
   // least one CTA for every SM

@@ -593,11 +593,7 @@ static int launch_fmha_fwd_as(const CUtensorMap& tq, const CUtensorMap& tk, cons
                               cudaStream_t stream) {
   using Cfg = FmhaFwdCfg<D>;
   auto kern = fmha_fwd_kernel<D, DROP, MODE>;
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
-    configured = true;
-  }
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
   p.n_qt = MODE == kPairs ? (p.Sq + 255) / 256 : (p.Sq + 127) / 128;
   // heads walked together: as many as keep their keys and values within a third of the L2 cache (the query heads of a group
   // share theirs), but at least one CTA for every SM

@@ -16,11 +16,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
                        int* status, int max_ctas, cudaStream_t stream) {
   using Cfg = GemmCfg<BN, ST>;
   auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN, ST, MINB>;
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
-    configured = true;
-  }
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
   static int sm_count = 0;
   if (sm_count == 0) {
     int dev = 0;
@@ -39,11 +35,7 @@ template <int A_MN, int B_MN>
 static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmShape& shp, const GemmEpilogue& ep,
                             int* status, int max_ctas, cudaStream_t stream) {
   auto kern = gemm_bf16_2cta_kernel<A_MN, B_MN>;
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Cfg::SMEM8_BYTES));
-    configured = true;
-  }
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Cfg::SMEM8_BYTES));
   static int sm_count = 0;
   if (sm_count == 0) {
     int dev = 0;

@@ -429,11 +429,7 @@ OFB_API int ofb_interaction_tc_fwd(const void* dense, const void* sparse, void* 
   constexpr int STAGES = 3;
   constexpr int SMEM = STAGES * kItTileBytes + 3 * 1024 + 256 + 1024;
   auto kern = interaction_fwd_tc_kernel<STAGES>;
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    configured = true;
-  }
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
   ItParams p{batch, T, out_dim, static_cast<int>((batch + kItSamples - 1) / kItSamples)};
   int grid = 2 * it_sm_count();
   if (grid > p.groups) grid = p.groups;
@@ -452,11 +448,7 @@ OFB_API int ofb_interaction_tc_bwd(const void* dense, const void* sparse, const 
   constexpr int STAGES = 2;
   constexpr int SMEM = 2 * STAGES * kItTileBytes + 8 * kEpiStageBytesPerWarp + 3 * 1024 + 256 + 1024;
   auto kern = interaction_bwd_tc_kernel<STAGES>;
-  static bool configured = false;
-  if (!configured) {
-    OFB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    configured = true;
-  }
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
   ItParams p{batch, T, out_dim, static_cast<int>((batch + kItSamples - 1) / kItSamples)};
   int grid = it_sm_count();
   if (grid > p.groups) grid = p.groups;

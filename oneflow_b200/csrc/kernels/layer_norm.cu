@@ -806,12 +806,8 @@ static int launch_layer_norm_bwd(const void* dy, const void* x, const void* gamm
     else layer_norm_bwd_warp_kernel<4><<<grid, warps * 32, smem, s>>>(DY, X, G, mean, rstd, AD, DX, pg, pb, rows, cols);
   } else if (nv <= 2 && aligned16 && may_allocate && !ring_off) {
     const int smem = kLnRingStages * 3 * cols * 2;
-    static bool configured = false;
-    if (!configured) {
-      OFB_CUDA_OK(cudaFuncSetAttribute(layer_norm_bwd_ring_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLnRingStages * 3 * 4096 * 2));
-      OFB_CUDA_OK(cudaFuncSetAttribute(layer_norm_bwd_ring_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLnRingStages * 3 * 4096 * 2));
-      configured = true;
-    }
+    OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(layer_norm_bwd_ring_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLnRingStages * 3 * 4096 * 2));
+    OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(layer_norm_bwd_ring_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLnRingStages * 3 * 4096 * 2));
     int* status = device_status_ptr();
     if (nv == 1) layer_norm_bwd_ring_kernel<1><<<grid, threads, smem, s>>>(DY, X, G, mean, rstd, AD, DX, pg, pb, rows, cols, status);
     else layer_norm_bwd_ring_kernel<2><<<grid, threads, smem, s>>>(DY, X, G, mean, rstd, AD, DX, pg, pb, rows, cols, status);
