@@ -69,20 +69,22 @@ int gemm_dispatch(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t str
   int bn = a->bn;
   const int mode2 = gemm_mode_2cta();
   bool two = bn == 512 || (mode2 == 1 && bn == 0);
-  // Cost of the three tilings in waves: a wave of the two-SM kernel (74 pairs, 256 x 256) is one unit; measured per wave, a
-  // 128 x 128 tile of the one-SM kernel takes 0.62 of it and a 128 x 256 tile 1.08. So the two-SM kernel wins whenever its tiles
-  // fill the machine, and also where the others would need a second wave (3072 x 1024 x 16384: 48 pairs 88 us, 192 tiles of
-  // 128 x 128 114 us, 96 of 128 x 256 96 us), while few tiles belong to the small tile (2331 x 768 x 3072: 22 against 29 us).
+  // Cost of the three tilings in waves: a wave of the two-SM kernel (74 pairs, 256 x 256) is one unit. Measured over 257 drawn
+  // sizes (K from 128 to 8192, all layouts), a wave of 128 x 128 tiles of the one-SM kernel takes 0.7 of it for short K and 0.85
+  // for long, one of 128 x 256 tiles 1.2; what decides is that two waves of the small tile cost more than one unit and three more
+  // than two (16006 x 304 x 3528: two waves of pairs 53 us, three of 128 x 128 75 us; 3072 x 1024 x 16384: 48 pairs 88 us, 192 tiles
+  // of 128 x 128 114 us), while few tiles belong to the small tile (2331 x 768 x 3072: 22 against 29 us).
   const long long tiles2 = (long long)((a->M + 255) / 256) * ((a->N + 255) / 256);
   const long long tiles256 = (long long)((a->M + 127) / 128) * ((a->N + 255) / 256);
   const long long tiles128 = (long long)((a->M + 127) / 128) * ((a->N + 127) / 128);
   const double cost2 = static_cast<double>((tiles2 + 73) / 74);
-  const double cost256 = 1.08 * static_cast<double>((tiles256 + 147) / 148), cost128 = 0.62 * static_cast<double>((tiles128 + 147) / 148);
+  const double cost256 = 1.16 * static_cast<double>((tiles256 + 147) / 148), cost128 = 0.72 * static_cast<double>((tiles128 + 147) / 148);
   const double cost1 = cost256 < cost128 ? cost256 : cost128;
   if (mode2 == -1 && bn == 0) {
     // Below K = 256 the main loop is shorter than the epilogue, which two one-SM CTAs per SM get through faster (802816 x 256 x 64:
-    // 136 against 156 us; 50176 x 1024 x 256: 56 against 49 us).
-    two = kDefault2Cta && cost2 <= cost1 && a->N >= 256 && a->M >= 256 && a->K >= 256;
+    // 136 against 156 us). Only for a K-major A: with an M-major one (weight gradients) that kernel does not exist, and
+    // 9472 x 3328 x 136 takes 32 us with pairs, 40 us with one-SM tiles.
+    two = kDefault2Cta && cost2 <= cost1 && a->N >= 256 && a->M >= 256 && (a->K >= 256 || a_mn);
   }
   if (mode2 == 0) two = bn == 512;
   // Few K blocks and many tiles: the epilogue is the bottleneck, so run two one-SM CTAs per SM (short ring) instead of one with a
