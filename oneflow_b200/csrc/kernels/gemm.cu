@@ -84,7 +84,8 @@ int gemm_dispatch(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t str
     // Below K = 256 the main loop is shorter than the epilogue, which two one-SM CTAs per SM get through faster (802816 x 256 x 64:
     // 136 against 156 us). Only for a K-major A: with an M-major one (weight gradients) that kernel does not exist, and
     // 9472 x 3328 x 136 takes 32 us with pairs, 40 us with one-SM tiles.
-    two = kDefault2Cta && cost2 <= cost1 && a->N >= 256 && a->M >= 256 && (a->K >= 256 || a_mn);
+    // A caller's limit of one CTA leaves no room for a pair.
+    two = kDefault2Cta && cost2 <= cost1 && a->N >= 256 && a->M >= 256 && (a->K >= 256 || a_mn) && a->max_ctas != 1;
   }
   if (mode2 == 0) two = bn == 512;
   // Few K blocks and many tiles: the epilogue is the bottleneck, so run two one-SM CTAs per SM (short ring) instead of one with a

@@ -115,6 +115,14 @@ def test_gemm_chooses_a_tiling_close_to_the_best(M, N, K, a_layout, b_layout):
     assert chosen < 1.12 * min(forced), (chosen, forced)
 
 
+def test_gemm_keeps_to_the_limit_of_ctas():
+    """48 tiles of 256 x 256 (or 192 of 128 x 128) on two CTAs or one take many times as long as on all, and one longer than two."""
+    a, b = torch.randn(3072, 512, device=DEV, dtype=BF), torch.randn(1024, 512, device=DEV, dtype=BF)
+    free, two, one = timed_in_turn(*(lambda c=c: G.gemm(a, b, max_ctas=c) for c in (0, 2, 1)), n=3)
+    assert two > 10 * free and one > 1.3 * two, (free, two, one)
+    close(G.gemm(a, b, max_ctas=1), G.gemm_reference(a.cpu(), b.cpu()))
+
+
 def test_gemm_default_dispatch_reaches_two_sm_kernel():
     """A problem large enough for the dispatcher's own choice of the two-SM kernel (>= 74 tiles of 256 x 256)."""
     torch.manual_seed(7)
