@@ -748,13 +748,13 @@ OFB_API int ofb_layer_norm_fwd(const void* x, const void* gamma, const void* bet
   // rows belong to the block kernel while a power of two of columns lets it merge without divisions: up to eight rows an SM
   // (8 x 1024 2.1 against 2.7 us, 1600 x 1024 3.9 against 3.6); of the widest, whose eight warps fill an SM's registers, up to
   // five, and where a second wave of warps would be less than half full (64 x 2048 2.2 against 3.7, 1184 x 2048 4.8 against 4.0,
-  // 1185 x 2048 4.9 against 5.3, 2048 x 2048 7.2 against 6.4). With divisions only the widest rows and one an SM (64 x 1280 3.1
-  // against 3.3, 600 x 1280 4.3 against 3.4; 64 x 768 3.1 against 2.7).
+  // 1185 x 2048 4.9 against 5.3, 2048 x 2048 7.2 against 6.4). With divisions only the widest rows, five of them to one an SM
+  // (1 x 1280 3.1 against 2.8, 64 x 1280 3.1 against 3.3, 600 x 1280 4.3 against 3.4; 64 x 768 3.1 against 2.7).
   const bool pow2 = (cols & (cols - 1)) == 0;
   const int per_sm = (rows - 1) / 148 + 1;
   const bool few_rows = cols == 2048 ? per_sm <= 5 || (per_sm > 8 && per_sm <= 12)
                         : pow2       ? cols >= 512 && per_sm <= 8
-                                     : cols > 1024 && per_sm <= 1;
+                                     : cols > 1024 && per_sm <= 1 && rows > 4;
   if (cols <= 2048 && !few_rows) {
     const int warp_grid = (rows + 7) / 8 < 148 * 4 ? (rows + 7) / 8 : 148 * 4;
     if (cols <= 256) layer_norm_fwd_warp_kernel<1><<<warp_grid, 256, 0, s>>>(X, G, B, Y, mean, rstd, rows, cols, eps);

@@ -206,7 +206,7 @@ def test_layer_norm(cols):
 
 
 @pytest.mark.parametrize("rows,cols", [(1, 8), (17, 256), (9, 264), (2500, 512), (130, 520), (1300, 1024), (7, 1032), (1, 2048), (300, 2056),
-                                       (1184, 512), (1185, 512), (1184, 1024), (1185, 1024), (148, 1032), (149, 1032), (740, 2048), (741, 2048), (1185, 2048), (1777, 2048),
+                                       (1184, 512), (1185, 512), (1184, 1024), (1185, 1024), (4, 1536), (5, 1536), (148, 1032), (149, 1032), (740, 2048), (741, 2048), (1185, 2048), (1777, 2048),
                                        (64, 512), (65, 512), (148, 1024), (149, 1024), (1000, 256), (1100, 248)])
 def test_layer_norm_narrow_rows(rows, cols):
     """Widths on both sides of what a warp's lanes hold (256, 512, 1024, 2048), one row to more rows than warps, and the numbers of
