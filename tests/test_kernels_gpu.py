@@ -309,7 +309,7 @@ def test_im2col_small(N, H, W, C, R, stride, pad, ldc):
     assert hw == hw2 and torch.equal(got.cpu(), ref)
 
 
-@pytest.mark.parametrize("N,H,W,C", [(2, 7, 9, 8), (1, 1, 1, 16), (3, 56, 56, 24)])
+@pytest.mark.parametrize("N,H,W,C", [(2, 7, 9, 8), (1, 1, 1, 16), (3, 56, 56, 24), (2, 113, 57, 40), (1, 2, 301, 8), (5, 64, 1, 16)])
 def test_pool_and_stride_index_kernels(N, H, W, C):
     from oneflow_b200.ops import cnn
     x = torch.randn(N, H, W, C, device=DEV, dtype=BF)
@@ -317,15 +317,45 @@ def test_pool_and_stride_index_kernels(N, H, W, C):
     ry, ridx = cnn.maxpool3x3s2_fwd(x.cpu())
     assert torch.equal(y.cpu(), ry)
     dy = torch.randn_like(y)
-    # up to four bf16 gradients meet in fp32 and are rounded once; ties between equal pixels may choose either of them
-    d, rd = cnn.maxpool3x3s2_bwd(dy, idx, (N, H, W, C)).cpu().float(), cnn.maxpool3x3s2_bwd(dy.cpu(), ridx, (N, H, W, C)).float()
-    assert float(((d - rd).abs() > 2.0 ** -8 * rd.abs() + 1e-6).float().mean()) < 5e-3
+    # the taps point at the maxima; ties between equal pixels may choose either of them, so the gradient is checked for these taps
+    OH, OW = y.shape[1:3]
+    tap = idx.long()
+    h = 2 * torch.arange(OH, device=DEV).view(1, -1, 1, 1) - 1 + tap // 3
+    w = 2 * torch.arange(OW, device=DEV).view(1, 1, -1, 1) - 1 + tap % 3
+    assert bool(((h >= 0) & (h < H) & (w >= 0) & (w < W)).all())
+    flat = ((torch.arange(N, device=DEV).view(-1, 1, 1, 1) * H + h) * W + w) * C + torch.arange(C, device=DEV)
+    assert torch.equal(x.flatten()[flat], y)
+    want = torch.zeros(x.numel(), device=DEV, dtype=torch.float64).scatter_add_(0, flat.flatten(), dy.double().flatten())
+    size = torch.zeros_like(want).scatter_add_(0, flat.flatten(), dy.double().abs().flatten())
+    got = cnn.maxpool3x3s2_bwd(dy, idx, (N, H, W, C)).double().flatten()
+    # up to four bf16 gradients meet in fp32 (three roundings of 2^-24 of their size) and are rounded once to bf16
+    assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 3 * 2.0 ** -24 * size).all())
     s = cnn.subsample2(x)
     assert torch.equal(s, x[:, ::2, ::2])
     up = cnn.upsample2_zero(s, (N, H, W, C))
     ref = torch.zeros_like(x)
     ref[:, ::2, ::2] = s
     assert torch.equal(up, ref)
+
+
+def test_index_kernels_beyond_32_bits():
+    """2^31 vectors and a few: the instances of the index kernels that divide in 64 bits (34 GB of results; the pooling and
+    subsampling kernels read four times as much and share the same arithmetic)."""
+    from oneflow_b200.ops import cnn
+    if torch.cuda.mem_get_info()[0] < 60 << 30:
+        pytest.skip("needs 60 GB")
+    N, H, W, C = 1032, 65, 64, 4096          # 2,197,946,368 vectors of 8
+    assert N * H * W * (C // 8) > 1 << 31
+    dy = torch.randn(N, C, device=DEV, dtype=BF)
+    dx = cnn.avgpool_bwd(dy, (N, H, W, C))
+    want = (dy.float() * (1.0 / (H * W))).to(BF)
+    for n in range(N):
+        assert bool((dx[n] == want[n]).all()), n
+    del dx
+    dy = torch.randn(N, (H + 1) // 2, W // 2, C, device=DEV, dtype=BF)
+    dx = cnn.upsample2_zero(dy, (N, H, W, C))
+    for n in range(N):
+        assert torch.equal(dx[n, ::2, ::2], dy[n]) and not dx[n, 1::2].any() and not dx[n, :, 1::2].any(), n
 
 
 @pytest.mark.parametrize("act", [1, 2, 3])
@@ -476,10 +506,13 @@ def test_xent_sum_accuracy(rows, cols):
     assert abs(float(err.mean())) < 1e-8      # __expf errs by a few units in the last place, not to one side
 
 
-@pytest.mark.parametrize("rows,cols,expanded", [(1, 8, False), (3, 4096, True), (5, 16384 + 8, False), (1200, 2 * 16384 - 8, True)])
+@pytest.mark.parametrize("rows,cols,expanded", [(1, 8, False), (3, 4096, True), (5, 16384 + 8, False), (1200, 2 * 16384 - 8, True),
+                                                 (300, 4104, False), (297, 8184, True), (297, 8200, False), (300, 16384, True),
+                                                 (4, 16392, False), (9600, 264, False)])
 def test_xent_row_scale_and_extremes(rows, cols, expanded):
-    """Widths around the 16384 elements a block takes per step, more rows than blocks, incoming gradients per row or one value;
-    entries of -inf, the type's lowest value and a row maximum that comes last."""
+    """Widths around the 4096, 8192 and 16384 elements a block of 128, 256 and 512 threads takes per step and around those at which
+    the number of threads changes, more rows than blocks in the gradient (1184) and in the statistics (9472), incoming gradients per
+    row or one value; entries of -inf, the type's lowest value and a row maximum that comes last."""
     torch.manual_seed(16)
     logits = torch.randn(rows, cols, device=DEV, dtype=BF) * 3
     labels = torch.randint(0, cols, (rows,), device=DEV)
