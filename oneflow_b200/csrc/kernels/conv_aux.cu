@@ -60,8 +60,9 @@ bn_reduce_kernel(const bf16* __restrict__ a, const bf16* __restrict__ x, const b
     // U rows: all loads first (no branch in between: with a bounds check per row the loads were not overlapped)
     auto rows_at = [&](long long r0, long long step, auto n) {
       constexpr int U = decltype(n)::value;
-      uint4 qa[U], qx[MODE == 1 ? U : 1], qy[MODE == 1 ? U : 1];
-      unsigned int bits[MODE == 1 ? U : 1];
+      uint4 qa[U];
+      [[maybe_unused]] uint4 qx[MODE == 1 ? U : 1], qy[MODE == 1 ? U : 1];
+      [[maybe_unused]] unsigned int bits[MODE == 1 ? U : 1];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const long long r = r0 + u * step;
@@ -486,7 +487,7 @@ static inline int aux_grid(long long items) {
 }
 
 // The index kernels split a vector's number into its coordinates; below 2^31 vectors with 32-bit divisions
-// (pooling backward 256 x 112 x 112 x 64: 374 us, with 64-bit divisions 418 us).
+// (a pooling backward with a thread per pixel, 256 x 112 x 112 x 64: 374 us, with 64-bit divisions 418 us).
 #define OFB_AUX_LAUNCH(kern, items, ...)                                                             \
   do {                                                                                               \
     const long long items_ = (items);                                                                \

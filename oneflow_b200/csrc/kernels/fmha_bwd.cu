@@ -22,8 +22,8 @@
 // the copies of Q, dO and dQ move 224 KiB: 4100 clocks, the products themselves 2560), then the fp32 reductions of dQ in L2.
 // The grid has one CTA per key tile, but a running CTA takes over the next one that has not started (cluster launch control), so
 // that barriers, TMEM and the first loads of a tile do not wait for the end of the one before; the order stays the hardware's.
-// Measured on a B200 with delta and the dQ conversion, against the kernel this replaced (one chain S -> P -> dV -> dP -> dS
-// -> dK, dQ -> drain per pair, nothing overlapped), and without the take-over in brackets: batch 4, 32 heads, 2048 x 2048,
+// Measured on a B200 with delta and the dQ conversion, against a kernel with one chain S -> P -> dV -> dP -> dS -> dK, dQ ->
+// drain per pair and nothing overlapped, and without the take-over in brackets: batch 4, 32 heads, 2048 x 2048,
 // D = 128, causal 843 -> 454 us (504); batch 1, 32 / 8 heads, 8192 x 8192, D = 128, causal 2960 -> 1445 us (1490); batch 32,
 // 16 heads, 512 x 512, D = 64 349 -> 215 us (243); batch 8, 16 heads, 500 x 1100, D = 64 179 -> 101 us (118).
 // TMEM: S/P | dP (D = 128: also dQ) | dV | dK | D = 64: dQ.
@@ -601,8 +601,8 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 }
 
 // delta[b,h,s] = sum_d dO[b,s,h,d] * O[b,s,h,d], and the same elements of the fp32 dQ accumulator are cleared. D / 8 lanes
-// share a row, 16 bytes of each operand per lane (one warp per row with 4-byte loads took 49 us where this and the memset
-// it replaces move 134 MB: batch 32, 16 heads, 512 rows, D = 64).
+// share a row, 16 bytes of each operand per lane (one warp per row with 4-byte loads took 49 us where this and a memset of
+// the accumulator move 134 MB: batch 32, 16 heads, 512 rows, D = 64).
 template <int D>
 __global__ void fmha_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta,
                                   float* __restrict__ dq_acc, int B, int S, int H) {

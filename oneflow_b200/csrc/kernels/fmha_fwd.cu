@@ -16,8 +16,8 @@
 // heads, 1 x 512, D = 128 10.7 against 10.1 us.)
 //
 // What bounds it: the exponentials (16 per clock and SM: 1024 clocks for a 128 x 128 tile) and the two products of a D = 128
-// tile (1024 clocks) alike. Measured on a B200, forward alone, against the one-stream kernel this replaced (P through shared
-// memory, two threads a row that met at a barrier on every tile), and in brackets with one CTA per pair: batch 4, 32 heads,
+// tile (1024 clocks) alike. Measured on a B200, forward alone, against a kernel of one stream (P through shared
+// memory, two threads a row that meet at a barrier on every tile), and in brackets with one CTA per pair: batch 4, 32 heads,
 // 2048 x 2048, D = 128, causal 283 -> 163 us (187); batch 1, 32 / 8 heads, 8192 x 8192, D = 128, causal 847 -> 451 us (470);
 // batch 32, 16 heads, 512 x 512, D = 64 143 -> 73 us (88).
 // Pairs: a running CTA takes over the next item that has not started (cluster launch control), so that the first loads of an

@@ -493,11 +493,11 @@ layer_norm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
 }
 
 // ------------------------------------------------------------------------------------------------
-// Narrow rows: one warp owns a row (NV 16-byte vectors per lane, cols <= 256 NV), so a row needs ten shuffles and no barrier.
-// A CTA per row kept 4 to 8 warps waiting on two barriers for 512 to 2048 bytes of work.
-// Bound by memory. Measured on a B200, before and after: forward 16384 x 1024 18.9 -> 14.0 us (10.3 at the copy rate),
-// 2331 x 768 7.4 -> 3.3 us, 8192 x 1536 32 -> 16 us; backward with parameter gradients 16384 x 1024 56 -> 31 us, 2048 x 512
-// 14.3 -> 7 us, 32768 x 256 90 -> 21 us.
+// Narrow rows: one warp owns a row (NV 16-byte vectors per lane, cols <= 256 NV), so a row needs ten shuffles and no barrier, where
+// a CTA per row keeps 4 to 8 warps waiting on two barriers for 512 to 2048 bytes of work.
+// Bound by memory. Measured on a B200 (inputs in L2), a CTA per row and a warp per row: forward 16384 x 1024 16.6 and 12.5 us,
+// 2400 x 768 7.0 and 4.4 us, 16384 x 1536 57 and 26 us; backward with parameter gradients 4096 x 1024 20 and 11 us, 600 x 512 11.8
+// and 5.7 us, 4096 x 256 18.4 and 6.7 us.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void ln_unpack8(const uint4& q, float (&v)[8]) {
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
