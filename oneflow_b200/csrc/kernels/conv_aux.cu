@@ -435,7 +435,7 @@ upsample2_zero_kernel(const bf16* __restrict__ dy, bf16* __restrict__ dx, int N,
 // neighbours, and every thread gathers 8 columns of the matrix at a time. (A thread that fetched its 8 values from global memory
 // after 64-bit divisions: 996 us for 256 x 224 x 224 x 3, 7 x 7, against 463 us; 976 MB are written, 149 us at the copy rate.)
 // CIN_ / R_ / S_ > 0 fix the shape at compile time (constant divisors); 0 takes the runtime values. STAGED = false reads the image
-// directly: windows too large for shared memory.
+// directly: windows too large for shared memory, and small problems.
 template <int CIN_, int R_, int S_, bool STAGED>
 __global__ void __launch_bounds__(256)
 im2col_small_kernel(const bf16* __restrict__ x, bf16* __restrict__ cols, int H, int W, int Cin_rt, int R_rt, int S_rt, int stride, int pad,
@@ -600,24 +600,26 @@ OFB_API int ofb_im2col_small(const void* x, void* cols, int N, int H, int W, int
   if (N <= 0 || OH <= 0 || OW <= 0 || ldc == 0) return 0;
   const long long rows = (long long)N * OH;
   if (rows > 0x7FFFFFFFll) return fail("im2col: too many output rows");
-  // Output columns of a CTA: whole rows from two CTAs an SM on, else pieces that make four, down to one round of the threads (1 x
-  // 96 x 96 in whole rows: 6.1 us, in four pieces 3.7; 4 x 224 x 224, 448 rows: 14.5 us, in two pieces 17.2), and never more than
+  // Output columns of a CTA: one round of its threads for small problems, which read the image through L1 and do without the wait
+  // between staging and gathering (1 x 96 x 96 2.7 against 3.7 us, 4 x 224 x 224 12.8 against 14.1; 32 x 96 x 96 18.2 against 16.4,
+  // 256 x 224 x 224 690 against 466). Staged: whole rows from two CTAs an SM on, else pieces that make four, and never more than
   // 48 KiB of input, which every device gives without asking.
   const int round = 256 / (ldc / 8) > 0 ? 256 / (ldc / 8) : 1;
-  int cpp = rows < 2 * 148 ? (int)((OW * rows - 1) / (4 * 148) + 1) : OW;
-  if (cpp < round) cpp = round < OW ? round : OW;
+  const bool small = rows * OW * (ldc / 8) <= 1 << 20;
+  int cpp = small ? round : rows < 2 * 148 ? (int)((OW * rows - 1) / (4 * 148) + 1) : OW;
+  if (cpp < round || cpp > OW) cpp = round < OW ? round : OW;
   const long long fit = (48 * 1024 / (R * Cin > 0 ? 2ll * R * Cin : 1) - S) / stride + 1;      // 0 or less: not one window
-  const bool staged = 2ll * R * S * Cin <= 48 * 1024 && (OW - 1) / (cpp < fit ? cpp : fit) < 65535;
-  if (!staged) cpp = OW;
-  else if (cpp > fit) cpp = (int)fit;
+  const bool staged = !small && 2ll * R * S * Cin <= 48 * 1024 && (OW - 1) / (cpp < fit ? cpp : fit) < 65535;
+  if (staged && cpp > fit) cpp = (int)fit;
+  if (!staged && (OW - 1) / cpp >= 65535) cpp = OW;
   auto launch = [&](auto kern, long long bytes) {
     kern<<<dim3((unsigned int)rows, (OW - 1) / cpp + 1), 256, (size_t)bytes, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)cols, H, W,
                                                                                                      Cin, R, S, stride, pad, OH, OW, cpp, ldc);
   };
   const long long smem = 2ll * R * (stride * (cpp - 1ll) + S) * Cin;
-  if (!staged) launch(im2col_small_kernel<0, 0, 0, false>, 0);
-  else if (Cin == 3 && R == 7 && S == 7) launch(im2col_small_kernel<3, 7, 7, true>, smem);
-  else launch(im2col_small_kernel<0, 0, 0, true>, smem);
+  const bool stem = Cin == 3 && R == 7 && S == 7;
+  if (!staged) stem ? launch(im2col_small_kernel<3, 7, 7, false>, 0) : launch(im2col_small_kernel<0, 0, 0, false>, 0);
+  else stem ? launch(im2col_small_kernel<3, 7, 7, true>, smem) : launch(im2col_small_kernel<0, 0, 0, true>, smem);
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
 }

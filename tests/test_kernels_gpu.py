@@ -297,11 +297,12 @@ def test_batch_norm_sign_mask(rows, C, residual):
 
 @pytest.mark.parametrize("N,H,W,C,R,stride,pad,ldc", [(2, 224, 224, 3, 7, 2, 3, 152), (1, 9, 11, 3, 7, 2, 3, 152), (3, 5, 7, 4, 3, 1, 1, 40),
                                                       (1, 1, 1, 1, 3, 1, 1, 16), (1, 4, 5000, 8, 3, 2, 1, 72),
-                                                      (1, 97, 95, 3, 7, 2, 3, 152), (700, 9, 11, 3, 7, 2, 3, 160), (600, 3, 1300, 3, 7, 2, 3, 152),
+                                                      (1, 97, 95, 3, 7, 2, 3, 152), (700, 33, 45, 3, 7, 2, 3, 160), (600, 3, 1300, 3, 7, 2, 3, 152),
+                                                      (2, 120, 5000, 3, 7, 2, 3, 152), (3, 150, 701, 4, 3, 1, 1, 40), (40, 64, 65, 4, 3, 1, 1, 40),
                                                       (1, 40, 41, 130, 15, 1, 7, 29256)])
 def test_im2col_small(N, H, W, C, R, stride, pad, ldc):
-    """Odd sizes, padding columns, one pixel, output rows in one piece and in several (few of them; too wide for shared memory),
-    windows too large for it; copies, so bit for bit."""
+    """Odd sizes, padding columns, one pixel; more and less than 2^20 vectors of results (read directly, or staged); output rows in
+    one piece and in several (few of them; too wide for shared memory); windows too large for it; copies, so bit for bit."""
     from oneflow_b200.ops import cnn
     x = torch.randn(N, H, W, C, device=DEV, dtype=BF)
     got, hw = cnn.im2col_small(x, R, R, stride, pad, ldc)
