@@ -81,11 +81,16 @@ int gemm_dispatch(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t str
   const double cost256 = 1.16 * static_cast<double>((tiles256 + 147) / 148), cost128 = 0.72 * static_cast<double>((tiles128 + 147) / 148);
   const double cost1 = cost256 < cost128 ? cost256 : cost128;
   if (mode2 == -1 && bn == 0) {
-    // Below K = 256 the main loop is shorter than the epilogue, which two one-SM CTAs per SM get through faster (802816 x 256 x 64:
-    // 136 against 156 us). Only for a K-major A: with an M-major one (weight gradients) that kernel does not exist, and
-    // 9472 x 3328 x 136 takes 32 us with pairs, 40 us with one-SM tiles.
+    // For short K the epilogue takes longer than the main loop, and two one-SM CTAs per SM (short_k below) get through it faster.
+    // Where there are tiles for them, up to K = 384 if the epilogue does more than store (with bias 8192 x 2048 x 256 22.2 against
+    // 24.3 us, x 384 24.0 against 25.2, x 448 25.0 against 25.9, x 512 25.6 against 26.0), else up to 320 (8192 x 2048 x 256 18.6
+    // against 20.1, x 384 20.6 against 20.9; 50176 x 1024 x 320 48.3 against 48.1, x 384 53.4 against 48.3); below K = 256 always
+    // (802816 x 256 x 64: 136 against 156 us). Only for a K-major A: with an M-major one (weight gradients) that kernel does not
+    // exist, and 9472 x 3328 x 136 takes 32 us with pairs, 40 us with one-SM tiles.
+    const bool bare = !ep.bias && !ep.aux_in && !ep.aux_out && !ep.residual;
+    const bool long_enough = a_mn || a->K > (tiles128 < 2 * 148 ? 255 : bare ? 320 : 384);
     // A caller's limit of one CTA leaves no room for a pair.
-    two = kDefault2Cta && cost2 <= cost1 && a->N >= 256 && a->M >= 256 && (a->K >= 256 || a_mn) && a->max_ctas != 1;
+    two = kDefault2Cta && cost2 <= cost1 && a->N >= 256 && a->M >= 256 && long_enough && a->max_ctas != 1;
   }
   if (mode2 == 0) two = bn == 512;
   // Few K blocks and many tiles: the epilogue is the bottleneck, so run two one-SM CTAs per SM (short ring) instead of one with a

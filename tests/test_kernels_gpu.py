@@ -115,6 +115,20 @@ def test_gemm_chooses_a_tiling_close_to_the_best(M, N, K, a_layout, b_layout):
     assert chosen < 1.12 * min(forced), (chosen, forced)
 
 
+@pytest.mark.parametrize("K", [256, 320, 328, 384, 392])
+def test_gemm_short_k_on_both_sides_of_the_line(K):
+    """Many tiles and few K blocks, ragged rows and columns: the epilogue-bound kernel up to K = 384 (320 without operands in the
+    epilogue), pairs above."""
+    torch.manual_seed(25)
+    a, b = torch.randn(5003, K, device=DEV, dtype=BF), torch.randn(1160, K, device=DEV, dtype=BF)
+    bias = torch.randn(1160, device=DEV, dtype=BF)
+    out, aux = G.gemm(a, b, bias=bias, act="gelu", want_aux=True)
+    ref, raux = G.gemm_reference(a.cpu(), b.cpu(), bias=bias.cpu(), act="gelu", want_aux=True)
+    close(out, ref)
+    close(aux, raux)
+    close(G.gemm(a, b), G.gemm_reference(a.cpu(), b.cpu()))
+
+
 def test_gemm_keeps_to_the_limit_of_ctas():
     """48 tiles of 256 x 256 (or 192 of 128 x 128) on two CTAs or one take many times as long as on all, and one longer than two."""
     a, b = torch.randn(3072, 512, device=DEV, dtype=BF), torch.randn(1024, 512, device=DEV, dtype=BF)
