@@ -87,8 +87,11 @@ int gemm_dispatch(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t str
     // against 20.1, x 384 20.6 against 20.9; 50176 x 1024 x 320 48.3 against 48.1, x 384 53.4 against 48.3); below K = 256 always
     // (802816 x 256 x 64: 136 against 156 us). Only for a K-major A: with an M-major one (weight gradients) that kernel does not
     // exist, and 9472 x 3328 x 136 takes 32 us with pairs, 40 us with one-SM tiles.
-    const bool bare = !ep.bias && !ep.aux_in && !ep.aux_out && !ep.residual;
-    const bool long_enough = a_mn || a->K > (tiles128 < 2 * 148 ? 255 : bare ? 320 : 384);
+    // A product with an activation's gradient keeps to pairs from K = 256 on: alone it is the slower one (55296 x 512 x 256 49.5
+    // against 47.3 us), but pairs leave registers for the blocks of another stream, and backward passes run beside others (the row
+    // update of an embedding beside two such products: 319 against 363 us, the step 3.52 against 3.56 ms).
+    const bool bare = !ep.bias && !ep.aux_out && !ep.residual;
+    const bool long_enough = a_mn || a->K > (tiles128 < 2 * 148 || ep.aux_in ? 255 : bare ? 320 : 384);
     // A caller's limit of one CTA leaves no room for a pair.
     two = kDefault2Cta && cost2 <= cost1 && a->N >= 256 && a->M >= 256 && long_enough && a->max_ctas != 1;
   }
