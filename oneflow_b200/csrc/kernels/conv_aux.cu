@@ -1,7 +1,6 @@
 // Memory-bound companions of the convolution kernels for NHWC bf16 feature maps (C a multiple of 8, 16-byte
 // accesses): batch normalisation (training) fused with the residual add and ReLU, 3x3/s2 max pooling, global
-// average pooling, 2x spatial subsampling and its adjoint (stride-2 convolutions run as stride-1 + subsample or
-// subsample + 1x1), and the im2col of the 7x7/s2 stem whose 3 input channels do not fill a TMA box.
+// average pooling, 2x spatial subsampling and its adjoint (a 1x1 convolution with stride 2 is subsample + 1x1), and the im2col of the 7x7/s2 stem whose 3 input channels do not fill a TMA box.
 //
 // Reference: oneflow/user/kernels/normalization_kernel.cu (cuDNN BN + fused add/relu), pool_gpu_kernel / max_pool
 // kernels, adaptive_avg_pool_gpu_kernel.cu.

@@ -2,8 +2,8 @@
 forward / backward engine over a flat parameter store.
 
 Every convolution runs on the tensor cores: 1x1 filters are plain tcgen05 GEMMs on the [N H W, C] view, 3x3 filters
-the implicit-GEMM kernels of ops/conv.py, the 7x7 RGB stem an im2col + GEMM; stride 2 is expressed as
-(stride-1 conv, subsample) or (subsample, 1x1 conv) so that forward and both gradients stay exact adjoints. Batch
+the implicit-GEMM kernels of ops/conv.py (stride 1 and 2), the 7x7 RGB stem an im2col + GEMM, a 1x1 filter with stride 2 a
+subsampling + GEMM. Batch
 norm uses batch statistics with the residual add and the ReLU fused into its apply kernels. Weight gradients
 accumulate in fp32 directly from the GEMM epilogues; the data-parallel all-reduce of a stage's gradients is issued
 on a side stream as soon as that stage's backward has finished, and one fused SGD-momentum kernel updates the fp32
@@ -79,23 +79,18 @@ class _Conv:
         if self.stride == 2 and self.k == 1:
             x = N.subsample2(x)
         self.x = x
-        y = C.conv_fprop(x, w)
-        if self.stride == 2 and self.k > 1:
-            self.full_shape = tuple(y.shape)
-            y = N.subsample2(y)
-        return y
+        return C.conv_fprop(x, w, self.stride if self.k > 1 else 1)
 
     def bwd(self, dy, need_dx=True, residual=None):
         """``residual`` (shape of the input gradient) is added to the returned gradient."""
         st = self.net.store
         w = st.p[self.name]
-        if self.stride == 2 and self.k > 1:
-            dy = N.upsample2_zero(dy, self.full_shape)
-        C.conv_wgrad(self.x, dy, (self.k, self.k), out=st.g[self.name], accumulate=st.acc_flag(self.name))
+        stride = self.stride if self.k > 1 else 1
+        C.conv_wgrad(self.x, dy, (self.k, self.k), out=st.g[self.name], accumulate=st.acc_flag(self.name), stride=stride)
         dx = None
         if need_dx:
             fuse = residual is not None and not (self.stride == 2 and self.k == 1)
-            dx = C.conv_dgrad(dy, w, residual if fuse else None)
+            dx = C.conv_dgrad(dy, w, residual if fuse else None, stride, self.in_shape[1:3])
             if self.stride == 2 and self.k == 1:
                 dx = N.upsample2_zero(dx, self.in_shape)
             if residual is not None and not fuse:

@@ -868,6 +868,45 @@ def test_conv_implicit_gemm(N, H, W, Cin, Cout, R):
     assert _native.read_status() == (0, 0)
 
 
+@pytest.mark.parametrize("N,H,W,Cin,Cout,R", [(4, 56, 56, 128, 128, 3), (19, 14, 14, 512, 512, 3), (3, 10, 10, 256, 256, 3),
+                                              (2, 19, 13, 64, 128, 3), (2, 9, 16, 128, 64, 5), (1, 1, 1, 64, 64, 3), (70, 56, 56, 128, 64, 3)])
+def test_conv_implicit_gemm_stride2(N, H, W, Cin, Cout, R):
+    """Every other pixel by the tensor map, the input gradient by the parity of its pixel: even and odd maps, all tilings."""
+    from oneflow_b200.ops import conv as C
+    torch.manual_seed(0)
+    x = torch.randn(N, H, W, Cin, device="cuda").bfloat16()
+    w = (torch.randn(Cout, R, R, Cin, device="cuda") / math.sqrt(R * R * Cin)).bfloat16()
+    dy = torch.randn(N, (H + 1) // 2, (W + 1) // 2, Cout, device="cuda").bfloat16()
+    x64, w64 = x.double().requires_grad_(), w.double().requires_grad_()
+    ref = torch.nn.functional.conv2d(x64.permute(0, 3, 1, 2), w64.permute(0, 3, 1, 2), stride=2, padding=(R - 1) // 2).permute(0, 2, 3, 1)
+    ref.backward(dy.double())
+    # results are rounded to bf16 once (2^-9 of their size); the fp32 chain of at most R R C / 16 = 288 sums of size below 43 loses
+    # no more than 288 * 43 * 2^-23
+    y = C.conv_fprop(x, w, 2)
+    torch.testing.assert_close(y.double(), ref.detach(), atol=1.5e-3, rtol=2.0 ** -8)
+    dx = C.conv_dgrad(dy, w, stride=2, in_hw=(H, W))
+    torch.testing.assert_close(dx.double(), x64.grad, atol=1.5e-3, rtol=2.0 ** -8)
+    # fp32 results: a chain of N OH OW / 16 sums at most
+    dw = C.conv_wgrad(x, dy, (R, R), stride=2)
+    size = w64.grad.abs().max().item()
+    tol = max(1e-5, dy[..., 0].numel() / 16 * 2.0 ** -23) * max(size, 1.0)
+    assert (dw - w64.grad).abs().max().item() <= tol
+    dw2 = C.conv_wgrad(x, dy, (R, R), out=dw.clone(), accumulate=True, stride=2)
+    assert (dw2 - 2 * w64.grad).abs().max().item() <= 2 * tol
+    torch.cuda.synchronize()
+    assert _native.read_status() == (0, 0)
+
+
+def test_conv_stride_arguments():
+    from oneflow_b200.ops import conv as C
+    x, w = torch.zeros(1, 6, 6, 64, device="cuda", dtype=BF), torch.zeros(64, 3, 3, 64, device="cuda", dtype=BF)
+    dy = torch.zeros(1, 3, 3, 64, device="cuda", dtype=BF)
+    for call in (lambda: C.conv_fprop(x, w, 3), lambda: C.conv_fprop(x, w[:, :1, :1].contiguous(), 2), lambda: C.conv_dgrad(dy, w, stride=2),
+                 lambda: C.conv_dgrad(dy, w, stride=2, in_hw=(7, 7)), lambda: C.conv_wgrad(x, dy, (3, 3))):
+        with pytest.raises(ValueError):
+            call()
+
+
 def test_flow_conv2d_channels_last_uses_igemm():
     import oneflow_b200 as flow
     torch.manual_seed(0)
