@@ -148,8 +148,11 @@ __global__ void bn_finalize_kernel(const float* __restrict__ sums, float inv_row
 
 // Backward coefficients per channel: dx = a * g + b * x + c with
 //   a = gamma rstd,  b = -a rstd s2 / rows,  c = -a s1 / rows - b mean      (s1 = sum g, s2 = sum g xhat)
+// and the parameter gradients dgamma = s2, dbeta = s1 where wanted (added to what is there with acc_*). A kernel of its own: the
+// element pass with this work at the start of its blocks was slower by more than the launch (802816 x 64: 65 instead of 49 + 2 us).
 __global__ void bn_bwd_coeffs_kernel(const float* __restrict__ sums, const float* __restrict__ mean, const float* __restrict__ rstd,
-                                     const float* __restrict__ gamma, float inv_rows, int C, float* coef) {
+                                     const float* __restrict__ gamma, float inv_rows, int C, float* coef, float* dgamma, int acc_gamma,
+                                     float* dbeta, int acc_beta) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const float a = gamma[c] * rstd[c];
@@ -157,6 +160,8 @@ __global__ void bn_bwd_coeffs_kernel(const float* __restrict__ sums, const float
   coef[c] = a;
   coef[C + c] = b;
   coef[2 * C + c] = -a * sums[c] * inv_rows - b * mean[c];
+  if (dgamma) dgamma[c] = acc_gamma ? dgamma[c] + sums[C + c] : sums[C + c];
+  if (dbeta) dbeta[c] = acc_beta ? dbeta[c] + sums[c] : sums[c];
 }
 
 // Streaming kernels below: when the 8-channel vectors per row divide the block size, a thread keeps the same
@@ -539,13 +544,18 @@ OFB_API int ofb_bn_apply(const void* x, const void* residual, const float* scale
   return 0;
 }
 
-// coef [3 C] is scratch written here. sums = [sum g | sum g xhat] from ofb_bn_reduce(mode 1).
+// coef [3 C] is scratch written here. sums = [sum g | sum g xhat] from ofb_bn_reduce(mode 1). dgamma / dbeta [C] (may be null) receive
+// the parameter gradients, added to what is there with acc_gamma / acc_beta.
 OFB_API int ofb_bn_bwd_apply(const void* dy, const void* x, const void* y, const void* mask, const float* mean, const float* rstd,
-                             const float* gamma, const float* sums, float* coef, long long rows, int C, int relu, void* dx, void* stream) {
+                             const float* gamma, const float* sums, float* coef, long long rows, int C, int relu, float* dgamma, int acc_gamma,
+                             float* dbeta, int acc_beta, void* dx, void* stream) {
   if (C % 8) return fail("bn: channels must be a multiple of 8");
   const long long vecs = rows * (C / 8);
+  if (C == 0 || (vecs == 0 && !dgamma && !dbeta)) return 0;
+  bn_bwd_coeffs_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(sums, mean, rstd, gamma, 1.f / rows, C, coef, dgamma, acc_gamma, dbeta,
+                                                                        acc_beta);
+  OFB_CUDA_OK(cudaGetLastError());
   if (vecs == 0) return 0;
-  bn_bwd_coeffs_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(sums, mean, rstd, gamma, 1.f / rows, C, coef);
   bn_bwd_apply_kernel<<<aux_grid(vecs), 256, 0, (cudaStream_t)stream>>>((const bf16*)dy, (const bf16*)x, (const bf16*)y,
                                                                       (const unsigned char*)mask, coef, vecs, C, relu, (bf16*)dx);
   OFB_CUDA_OK(cudaGetLastError());

@@ -115,19 +115,17 @@ class _BN:
             return N.bn_eval_fwd(x, gamma, beta, rm, rv, residual, relu, net.cfg.bn_eps)
         # on the GPU the backward takes the sign of y from one bit per element instead of y itself
         self.mask = torch.empty(x.numel() // 8, dtype=torch.uint8, device=x.device) if relu and x.is_cuda else None
-        y, self.mean, self.rstd = N.bn_train_fwd(x, gamma, beta, residual, relu, net.cfg.bn_eps, net.cfg.bn_momentum, rm, rv, self.mask)
+        y, self.mean, self.rstd = N.bn_train_fwd(x, gamma, beta, residual, relu, net.cfg.bn_eps, net.cfg.bn_momentum, rm, rv, self.mask,
+                                                 net.bn_sums(self, 0))
         self.x, self.y = x, (y if relu and self.mask is None else None)
         return y
 
     def bwd(self, dy):
         net = self.net
         gamma = net.master(self.name + ".weight")
-        dx, dres, dgamma, dbeta = N.bn_train_bwd(dy, self.x, self.y, self.mean, self.rstd, gamma, self.relu, self.has_res, self.mask)
-        for nm, g in ((self.name + ".weight", dgamma), (self.name + ".bias", dbeta)):
-            if net.store.acc_flag(nm):
-                net.store.g[nm].add_(g)
-            else:
-                net.store.g[nm].copy_(g)
+        names = (self.name + ".weight", self.name + ".bias")
+        dx, dres, _, _ = N.bn_train_bwd(dy, self.x, self.y, self.mean, self.rstd, gamma, self.relu, self.has_res, self.mask,
+                                        net.bn_sums(self, 1), [net.store.g[n] for n in names], [net.store.acc_flag(n) for n in names])
         self.x = self.y = self.mask = None
         return dx, dres
 
@@ -195,7 +193,19 @@ class ResNet:
             self.store.p["fc.weight"][cfg.num_classes:].zero_()
         self.running = {n: (torch.zeros(self._bn_c(n), device=self.device), torch.ones(self._bn_c(n), device=self.device))
                         for n in self.bn_names}
+        self._bn_at, self.bn_channels = {}, 0      # place of each batch norm in the channel sums of a pass
+        for n in self.bn_names:
+            self._bn_at[n] = self.bn_channels
+            self.bn_channels += self._bn_c(n)
+        self._bn_sums = None
         self._master = None   # fp32 master weights (set by the optimizer); batch norm reads its affine parameters there
+
+    def bn_sums(self, bn, backward):
+        """Channel sums [2 C] of one batch norm in a training pass, cleared for all of them at the start of ``forward`` (CUDA only)."""
+        if self._bn_sums is None:
+            return None
+        at = 2 * (self._bn_at[bn.name] + backward * self.bn_channels)
+        return self._bn_sums[at:at + 2 * bn.c]
 
     def _bn_c(self, name):
         return self.store.offsets[name + ".weight"][1]
@@ -231,6 +241,8 @@ class ResNet:
         """images: [N, H, W, 3] bf16 (channels last). Returns logits [N, classes_pad] bf16."""
         cfg = self.cfg
         n = images.shape[0]
+        if self.training and images.is_cuda:
+            self._bn_sums = torch.zeros(4 * self.bn_channels, dtype=torch.float32, device=images.device)
         cols, (oh, ow) = N.im2col_small(images, 7, 7, 2, 3, self.stem_cols)
         self.stem_cols_saved = cols if self.training else None
         y = G.gemm(cols, self.store.p["conv1.weight"]).view(n, oh, ow, cfg.stem)

@@ -20,9 +20,11 @@ def _lib():
 
 
 # ------------------------------------------------------------------------------------------------ batch norm
-def bn_train_fwd(x, gamma, beta, residual=None, relu=False, eps=1e-5, momentum=0.1, running_mean=None, running_var=None, mask=None):
+def bn_train_fwd(x, gamma, beta, residual=None, relu=False, eps=1e-5, momentum=0.1, running_mean=None, running_var=None, mask=None,
+                 sums=None):
     """x [..., C] bf16; gamma / beta fp32 [C]. Returns (y, mean, rstd) with batch statistics over all leading dims. ``mask``
-    (CUDA only): uint8 [x.numel() / 8], receives one bit per element, y > 0, for ``bn_train_bwd``."""
+    (CUDA only): uint8 [x.numel() / 8], receives one bit per element, y > 0, for ``bn_train_bwd``. ``sums`` (CUDA only): fp32 [2 C] of
+    zeros for the channel sums, allocated and cleared here when not given."""
     C = x.shape[-1]
     rows = x.numel() // C
     if not x.is_cuda:
@@ -39,7 +41,8 @@ def bn_train_fwd(x, gamma, beta, residual=None, relu=False, eps=1e-5, momentum=0
             running_mean.mul_(1 - momentum).add_(mean, alpha=momentum)
             running_var.mul_(1 - momentum).add_(var * (rows / max(rows - 1, 1)), alpha=momentum)
         return y.to(x.dtype).view(x.shape), mean, rstd
-    sums = torch.zeros(2 * C, dtype=torch.float32, device=x.device)
+    if sums is None:
+        sums = torch.zeros(2 * C, dtype=torch.float32, device=x.device)
     stats = torch.empty(4, C, dtype=torch.float32, device=x.device)
     mean, rstd, scale, shift = stats[0], stats[1], stats[2], stats[3]
     y = torch.empty_like(x)
@@ -72,9 +75,11 @@ def bn_eval_fwd(x, gamma, beta, running_mean, running_var, residual=None, relu=F
     return y
 
 
-def bn_train_bwd(dy, x, y, mean, rstd, gamma, relu=False, want_residual_grad=False, mask=None):
+def bn_train_bwd(dy, x, y, mean, rstd, gamma, relu=False, want_residual_grad=False, mask=None, sums=None, param_grads=None,
+                 accumulate=(False, False)):
     """Returns (dx, d_residual or None, dgamma, dbeta); y is only read when relu, and not at all when the forward's ``mask`` is
-    given (a sixteenth of its bytes in both passes)."""
+    given (a sixteenth of its bytes in both passes). ``sums`` (CUDA only) as in ``bn_train_fwd``. ``param_grads``: fp32 (dgamma, dbeta)
+    to write, or to add to where ``accumulate`` says so, instead of new ones."""
     C = x.shape[-1]
     rows = x.numel() // C
     if not x.is_cuda:
@@ -84,9 +89,15 @@ def bn_train_bwd(dy, x, y, mean, rstd, gamma, relu=False, want_residual_grad=Fal
         xhat = (x.float().reshape(rows, C) - mean) * rstd
         s1, s2 = g.sum(0), (g * xhat).sum(0)
         dx = gamma * rstd * (g - s1 / rows - xhat * s2 / rows)
+        if param_grads is not None:
+            for dst, new, acc in zip(param_grads, (s2, s1), accumulate):
+                dst.add_(new) if acc else dst.copy_(new)
+            s2, s1 = param_grads
         return dx.to(x.dtype).view(x.shape), (g.to(x.dtype).view(x.shape) if want_residual_grad else None), s2, s1
-    sums = torch.zeros(2 * C, dtype=torch.float32, device=x.device)
+    if sums is None:
+        sums = torch.zeros(2 * C, dtype=torch.float32, device=x.device)
     coef = torch.empty(3 * C, dtype=torch.float32, device=x.device)
+    dgamma, dbeta = param_grads if param_grads is not None else (None, None)
     dx = torch.empty_like(x)
     dres = torch.empty_like(x) if want_residual_grad else None
     lib = _lib()
@@ -96,8 +107,11 @@ def bn_train_bwd(dy, x, y, mean, rstd, gamma, relu=False, want_residual_grad=Fal
     if dres is not None:       # the reduction wrote the masked gradient: the second pass reads that and neither y nor the mask
         dy, y, mask, relu = dres, None, None, False
     check(lib.ofb_bn_bwd_apply(ptr(dy), ptr(x), ptr(y), ptr(mask), ptr(mean), ptr(rstd), ptr(gamma), ptr(sums), ptr(coef), c_longlong(rows),
-                               c_int(C), c_int(int(relu)), ptr(dx), stream_ptr()), "bn_bwd_apply")
+                               c_int(C), c_int(int(relu)), ptr(dgamma), c_int(int(accumulate[0])), ptr(dbeta), c_int(int(accumulate[1])),
+                               ptr(dx), stream_ptr()), "bn_bwd_apply")
     K._count(2)
+    if param_grads is not None:
+        return dx, dres, dgamma, dbeta
     return dx, dres, sums[C:], sums[:C]
 
 

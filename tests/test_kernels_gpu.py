@@ -302,7 +302,13 @@ def test_batch_norm_sign_mask(rows, C, residual):
     xh = (x.double() - mean.double()) * rstd.double()
     s1, s2 = gd.sum(0), (gd * xh).sum(0)
     ref = g.double() * rstd.double() * (gd - s1 / rows - xh * s2 / rows)
-    for d, sg, sb in ((dx, dg, db), (dx2, dg2, db2)):
+    # the sums in a given workspace, the parameter gradients written and added in place
+    work, grads = torch.zeros(4 * C, device=DEV), [torch.full((C,), 7.0, device=DEV), torch.full((C,), -3.0, device=DEV)]
+    y3, mean3, rstd3 = N.bn_train_fwd(x, g, b, res, True, mask=mask, sums=work[:2 * C])
+    close(mean3, x.double().mean(0), 1e-5, 1e-6)
+    dx3, _, dg3, db3 = N.bn_train_bwd(dy, x, None, mean3, rstd3, g, True, residual, mask, work[2 * C:], grads, (False, True))
+    assert dg3 is grads[0] and db3 is grads[1]
+    for d, sg, sb in ((dx, dg, db), (dx2, dg2, db2), (dx3, dg3, db3 + 3.0)):
         # fp32 sums of up to 5003 terms in any order, 2^-24 each against their magnitude; dx rounded to bf16 once
         close(sg, s2, 1e-5, 1e-5 * rows ** 0.5)
         close(sb, s1, 1e-5, 1e-5 * rows ** 0.5)
