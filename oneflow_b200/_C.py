@@ -11,6 +11,7 @@ import torch
 
 from .framework.generator import resolve as _resolve_gen
 
+from .framework import fused_ops
 from .framework.global_tensor import to_global, to_local  # noqa: F401
 from .ops import gemm as G
 from .ops import kernels as K
@@ -163,6 +164,11 @@ def scaled_dot_product_attention(query, key, value, attn_mask=None, dropout_p=0.
     kernel serves bf16 CUDA inputs with head dim 64/128 and no explicit mask, dropout (Philox, regenerated in backward)
     included."""
     D = query.shape[-1]
+    if attn_mask is None and dropout_p == 0.0 and query.is_cuda:
+        ops = fused_ops._native_ops()
+        out = ops.sdpa(query, key, value, bool(is_causal), scale if scale is not None else 1.0 / math.sqrt(D)) if ops is not None else None
+        if out is not None:
+            return out
     H, Hk = query.shape[1], key.shape[1]
     Sq, Sk = query.shape[-2], key.shape[-2]
     if (query.is_cuda and query.dtype == torch.bfloat16 and D in (64, 128) and attn_mask is None and 0.0 <= dropout_p < 1.0

@@ -112,6 +112,27 @@ def build_api(verbose=False):
     return lib
 
 
+def build_torch_ops(verbose=False):
+    """The fused ops on local tensors with their autograd nodes (csrc/torch) as the Python extension module lib/ofb_torch.so."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    srcs = sorted(glob.glob(os.path.join(CSRC, "torch", "*.cpp")))
+    lib = os.path.join(LIB, "ofb_torch.so")
+    kern = os.path.join(LIB, "libofb_kernels.so")
+    if os.path.exists(lib) and not any(_newer(s, lib, [os.path.join(CSRC, "kernels", "ofb_kernels.h")]) for s in srcs):
+        return lib
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    tlib = cpp_extension.library_paths()[0]
+    inc = [f"-isystem{d}" for d in cpp_extension.include_paths() + [os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]]
+    _run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          "-o", lib] + inc + srcs + [kern, f"-L{tlib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+                                     "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}"], os.path.join(OBJ, "torch_ops.log"))
+    print(f"[build] built {os.path.relpath(lib, ROOT)}", flush=True)
+    return lib
+
+
 def build_sanitizers(verbose=False):
     """The host runtime's multi-threaded self-test (csrc/core/selftest) linked with the runtime's sources under ThreadSanitizer
     and under AddressSanitizer + UBSan: lib/ofb_core_selftest_tsan, lib/ofb_core_selftest_asan."""
@@ -172,7 +193,7 @@ def build_api_thread_sanitized(verbose=False):
 
 
 def build_all(verbose=False):
-    return [build_kernels(verbose), build_core(verbose), build_api(verbose)]
+    return [build_kernels(verbose), build_core(verbose), build_api(verbose), build_torch_ops(verbose)]
 
 
 if __name__ == "__main__":

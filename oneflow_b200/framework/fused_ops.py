@@ -34,6 +34,7 @@ import torch
 import torch.distributed as dist
 
 from .. import sbp as S
+from ..ops import _native as _lib
 from ..ops import embedding as E
 from ..ops import gemm as G
 from ..ops import kernels as K
@@ -118,6 +119,18 @@ def _gemm(a, b, **kw):
             y = y + residual.float()
         return y.to(a.dtype), aux
     return G.gemm(a, b, **kw)
+
+
+def _native_ops(*params):
+    """The native module for a call on local tensors, or None where the Python statement has to run: while a plan is recorded, a
+    profiler listens, or the parameters receive their gradients in an optimizer's buffers. The module itself answers None for
+    calls that are not of its form."""
+    if op_trace is not None or _lib._recorder is not None:
+        return None
+    for p in params:
+        if getattr(p, "_main_grad", None) is not None:
+            return None
+    return _lib.torch_ops()
 
 
 # ------------------------------------------------------------------------------------------------ deferred partial sums
@@ -374,8 +387,8 @@ class _Linear(torch.autograd.Function):
         x_nd = None
         if mode == "data":
             dx2 = _gemm(dy2, w2, b_layout="kn", **fuse) if ctx.needs_input_grad[0] else None
-            if fuse and dx2 is not None:
-                cons.fused = True
+            if cons is not None:
+                cons.fused = bool(fuse) and dx2 is not None     # not in a second backward: the values are gone by then
             gw = _wgrad(w, _param_nd(plan, nd_w, None), dy2, x2)
             gb = _bgrad(bias, _param_nd(plan, nd_b, None), dy2)
             x_nd = tuple(plan.out_nd[:]) if g else None
@@ -490,6 +503,11 @@ def mlp(x, w1, b1, w2, b2, *, act="gelu", residual=None, out_sbp=None):
     over the [tokens, ffn] hidden gradient less). SBP handling, fused tensor-parallel products and parameter gradients
     are those of ``linear`` (column-parallel first layer, row-parallel second layer is the Megatron MLP).
     Reference: the fused MLP family (oneflow/user/kernels/cublas_fused_mlp_kernel.cu, cublas_bias_add_relu_matmul_grad)."""
+    if x.is_cuda and not _is_g(x):
+        ops = _native_ops(w1, b1, w2, b2)
+        y = ops.mlp(x, w1, b1, w2, b2, G._act_code(act), residual) if ops is not None else None
+        if y is not None:
+            return y
     link = _ActLink()
     h = linear(x, w1, b1, act=act, _link=(link, None))
     return linear(h, w2, b2, residual=residual, out_sbp=out_sbp, _link=(None, link))
@@ -532,6 +550,11 @@ def linear(x, weight, bias=None, *, act=0, residual=None, out_sbp=None, _link=No
             y = y.reshape(*x.shape[:-1], weight.shape[0], weight.shape[1])
         y = G._act_ref(y, act) if act else y
         return y if residual is None else y + residual
+    if _link is None and x.is_cuda:
+        ops = _native_ops(weight, bias)
+        y = ops.linear(x, weight, bias, act, residual) if ops is not None else None
+        if y is not None:
+            return y
     if x.is_cuda and _native(x, weight) and _aligned(weight) and x.numel() > 0:
         return _Linear.apply(x, weight, bias, residual, act, None, _link)
     w2 = weight if weight.dim() == 2 else weight.reshape(-1, weight.shape[-1])
@@ -634,6 +657,11 @@ def layer_norm(x, normalized_shape, weight=None, bias=None, eps=1e-5, _passthrou
     """LayerNorm over the last axis on the native kernels (rows may be split on any mesh axis; parameters broadcast);
     other forms go to the ATen path."""
     ns = (normalized_shape,) if isinstance(normalized_shape, int) else tuple(normalized_shape)
+    if x.is_cuda and not _passthrough and len(ns) == 1 and ns[0] == x.shape[-1] and weight is not None and bias is not None and not _is_g(x):
+        ops = _native_ops(weight, bias)
+        y = ops.layer_norm(x, weight, bias, eps) if ops is not None else None
+        if y is not None:
+            return y
     ok = len(ns) == 1 and weight is not None and bias is not None and x.shape[-1] % 8 == 0 and x.shape[-1] <= 32768
     if ok and _is_g(x):
         pl = x._placement
@@ -711,6 +739,11 @@ def fused_attention_qkv_packed(qkv, *, seq_len, head_size, causal=True, scale=No
                 qkv = GT.rebox(qkv, tuple(B_ if i == a else t for i, t in enumerate(qkv._nd_sbp)))
                 nd_out.append(B_)
         return _PackedAttention.apply(qkv, seq_len, head_size, causal, sc, pl, tuple(nd_out))
+    if qkv.is_cuda:
+        ops = _native_ops()
+        y = ops.attention_packed(qkv, seq_len, head_size, causal, sc) if ops is not None else None
+        if y is not None:
+            return y
     return _PackedAttention.apply(qkv, seq_len, head_size, causal, sc, None, None)
 
 
@@ -862,6 +895,10 @@ def sparse_softmax_cross_entropy(logits, labels):
                 vocab_start = slice_view(logits.shape, pl.hierarchy, logits._nd_sbp, coords)[1][0]
         return _SparseXent.apply(logits, labels, pl, tuple(nd_rows), vaxis, vocab_start)
     if logits.dim() == 2 and not _is_g(labels) and logits.is_cuda and logits.dtype == torch.bfloat16 and logits.is_contiguous():
+        ops = _native_ops()
+        loss = ops.cross_entropy(logits, labels) if ops is not None else None
+        if loss is not None:
+            return loss
         return _SparseXent.apply(logits, labels, None, None, None, 0)
     return _xent_fallback(logits, labels)
 

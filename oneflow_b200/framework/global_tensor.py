@@ -264,6 +264,19 @@ def _finish(func, args, kwargs, pl, out_nds, local_args=None, local_kwargs=None,
         nd = tuple(out_nds[0]) if out_nds and isinstance(out_nds[0], (tuple, list)) else tuple(out_nds)
         outs = [wrap(t, t.shape, pl, nd) if isinstance(t, torch.Tensor) else t for t in flat]
         return pytree.tree_unflatten(outs, spec)
+    if meta_out is None and pl.size == 1 and _in_placement(pl):
+        # one rank: its shards are the logical tensors, so the result's own shapes are the logical ones
+        if local_args is None:
+            local_args, local_kwargs = pytree.tree_map(_local_of, (args, kwargs))
+        meta_out = func(*local_args, **(local_kwargs or {}))
+        flat, spec = pytree.tree_flatten(meta_out)
+        n_out = sum(isinstance(t, torch.Tensor) for t in flat)
+        if out_nds and not isinstance(out_nds[0], (tuple, list)):
+            out_nds = [tuple(out_nds)] * n_out
+        elif len(out_nds) == 1:
+            out_nds = [tuple(out_nds[0])] * n_out
+        nds = iter(out_nds)
+        return pytree.tree_unflatten([wrap(t, t.shape, pl, next(nds)) if isinstance(t, torch.Tensor) else t for t in flat], spec)
     if meta_out is None:
         meta_out = _infer_meta(func, args, kwargs)
     metas, spec = pytree.tree_flatten(meta_out)
@@ -584,13 +597,24 @@ def squeeze_rule(func, args, kwargs):
     return _remap_dim_rule(func, args, kwargs, lambda d: None if d == q else (d - 1 if d > q else d))
 
 
+def _view_shape(shape, size):
+    """What ``view(size)`` makes of ``shape``: a -1 filled in, a mismatch refused as torch words it."""
+    size = [int(s) for s in size]
+    n, known = math.prod(shape), math.prod(s for s in size if s != -1)
+    if size.count(-1) == 1 and all(s >= -1 for s in size) and known > 0 and n % known == 0:
+        size[size.index(-1)] = n // known
+    elif -1 in size or known != n or any(s < 0 for s in size):
+        return tuple(torch.empty(shape, device="meta").view(size).shape)       # raises, or settles the rare forms
+    return tuple(size)
+
+
 @rule(aten.view.default, aten._unsafe_view.default, aten.reshape.default)
 def view_rule(func, args, kwargs):
     x = args[0]
     pl = x._placement
     in_shape = tuple(x.shape)
-    meta = _infer_meta(func, args, kwargs)
-    out_shape = tuple(meta.shape)
+    meta = None if pl.size == 1 and _in_placement(pl) else _infer_meta(func, args, kwargs)
+    out_shape = _view_shape(in_shape, args[1]) if meta is None else tuple(meta.shape)
     coords = _coords(pl)
     nd_in, nd_out = list(x._nd_sbp), []
     local_out = list(out_shape)
@@ -667,7 +691,8 @@ def _reduce_rule(func, args, kwargs, is_mean=False):
                 nd_out.append(S.split(s.axis if keepdim else s.axis - sum(1 for d in dims if d < s.axis)))
         else:
             nd_out.append(s)
-    meta = _infer_meta(func, args, kwargs)
+    one_rank = pl.size == 1 and _in_placement(pl)
+    meta = None if one_rank else _infer_meta(func, args, kwargs)
     if not _in_placement(pl):
         return _placeholder(meta, pl, tuple(nd_out))
     if is_mean:
@@ -675,7 +700,7 @@ def _reduce_rule(func, args, kwargs, is_mean=False):
         local = torch.sum(x._local, dims, keepdim=keepdim, dtype=kwargs.get("dtype")) / count
     else:
         local = func(x._local, *args[1:], **kwargs)
-    return wrap(local, meta.shape, pl, tuple(nd_out))
+    return wrap(local, local.shape if one_rank else meta.shape, pl, tuple(nd_out))
 
 
 @rule(aten.sum.dim_IntList, aten.sum.default)

@@ -121,6 +121,8 @@ class placement:
 
     def coords(self, rank):
         """Mesh coordinates of a global rank (None if it is outside the placement)."""
+        if len(self.ranks_flat) == 1:
+            return (0,) * len(self.hierarchy) if rank == self.ranks_flat[0] else None
         if rank not in self.ranks_flat:
             return None
         idx = self.ranks_flat.index(rank)

@@ -17,6 +17,7 @@ _LIB_DIR = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__
 _lock = threading.Lock()
 _kernels = None
 _core = None
+_torch_ops = None
 
 
 class NativeLibraryError(RuntimeError):
@@ -89,6 +90,25 @@ def kernels():
                 lib.ofb_gemm_bf16.restype = c_int
                 _kernels = lib
     return _kernels
+
+
+def torch_ops():
+    """The extension module with the fused ops on local tensors (csrc/torch)."""
+    global _torch_ops
+    if _torch_ops is None:
+        with _lock:
+            if _torch_ops is None:
+                path = lib_path("ofb_torch.so")
+                if not os.path.exists(path):
+                    raise NativeLibraryError(f"{path} is missing: run `python -m oneflow_b200.build` (or __graft_entry__.build()) first")
+                import importlib.util
+
+                import torch  # noqa: F401  (its libraries are what the module links against)
+                spec = importlib.util.spec_from_file_location("ofb_torch", path)
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+                _torch_ops = mod
+    return _torch_ops
 
 
 def core():

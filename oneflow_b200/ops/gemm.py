@@ -17,6 +17,7 @@ from . import _native
 
 _count = None     # kernels._count, bound at the first launch (kernels imports this module's siblings)
 ACT_NONE, ACT_GELU, ACT_GELU_TANH, ACT_RELU = 0, 1, 2, 3
+_OUT_TYPES = (torch.bfloat16, torch.float32)
 _ACT_NAMES = {None: 0, "none": 0, "gelu": 1, "gelu_tanh": 2, "relu": 3}
 
 
@@ -88,6 +89,11 @@ def gemm(a, b, *, a_layout="mk", b_layout="nk", bias=None, act=0, residual=None,
     if not a.is_cuda:
         return gemm_reference(a, b, a_layout, b_layout, bias, act, residual, aux_in, want_aux, out, out_dtype,
                               accumulate, alpha)
+    if alpha == 1.0 and bn == 0 and max_ctas == 0 and _native._recorder is None:
+        r = _native.torch_ops().gemm(a, b, a_layout != "mk", b_layout != "nk", bias, act, residual, aux_in, want_aux, out,
+                                     out_dtype == torch.float32, accumulate) if out_dtype in _OUT_TYPES else None
+        if r is not None:
+            return r
     _check_operand(a, "a")
     _check_operand(b, "b")
     M, K = (a.shape if a_layout == "mk" else (a.shape[1], a.shape[0]))

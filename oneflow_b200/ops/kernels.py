@@ -18,7 +18,7 @@ from . import _native
 from ._native import check, ptr, stream_ptr
 
 _DT = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
-launch_count = 0  # number of native kernel-launching calls issued through this module (bench bookkeeping)
+_launch_count = 0  # native kernel-launching calls issued through this module; ``launch_count`` adds those of the native op module
 
 
 def _lib():
@@ -26,8 +26,14 @@ def _lib():
 
 
 def _count(n=1):
-    global launch_count
-    launch_count += n
+    global _launch_count
+    _launch_count += n
+
+
+def __getattr__(name):
+    if name == "launch_count":
+        return _launch_count + (_native._torch_ops.launches() if _native._torch_ops is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def _need_bf16(*ts):
@@ -57,6 +63,10 @@ def layer_norm_fwd(x, gamma, beta, eps=1e-5):
         if beta is not None:
             y = y + beta.float()
         return y.to(x.dtype), mean, rstd
+    if gamma is not None and beta is not None and _native._recorder is None:
+        r = _native.torch_ops().layer_norm_fwd(x, gamma, beta, eps)
+        if r is not None:
+            return r
     _need_bf16(x, gamma, beta)
     y = torch.empty_like(x)
     mean = torch.empty(rows, dtype=torch.float32, device=x.device)
@@ -87,6 +97,10 @@ def layer_norm_bwd(dy, x, gamma, mean, rstd, add_to_dx=None, dgamma=None, dbeta=
             dbeta += db
             return dx.to(x.dtype), dgamma, dbeta
         return dx.to(x.dtype), dg.to(param_dtype), db.to(param_dtype)
+    if dgamma is not None and want_param_grads and gamma is not None and _native._recorder is None:
+        dx = _native.torch_ops().layer_norm_bwd_into(dy, x, gamma, mean, rstd, add_to_dx, dgamma, dbeta)
+        if dx is not None:
+            return dx, dgamma, dbeta
     _need_bf16(dy, x, gamma, add_to_dx)
     dx = torch.empty_like(x)
     accumulate = dgamma is not None
@@ -208,6 +222,8 @@ def column_sum(x, out=None, out_dtype=torch.float32):
             out += r
             return out
         return r.to(out_dtype)
+    if out is not None and _native._recorder is None and _native.torch_ops().column_sum_into(x, out) is not None:
+        return out
     _need_bf16(x)
     if out is not None:
         check(_lib().ofb_column_sum(ptr(x), ptr(out), c_int(rows), c_int(cols), stream_ptr()), "column_sum")
