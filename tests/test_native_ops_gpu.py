@@ -224,6 +224,16 @@ def test_hooks_modes_and_transforms():
                     transform()
                 errors.append(type(e.value))
         assert errors[0] is errors[1]
+    # a node downstream that hands back no gradient counts as zeros
+    class _Nothing(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, t):
+            return t.clone()
+
+        @staticmethod
+        def backward(ctx, d):
+            return None
+    _compare(lambda *_: _Nothing.apply(FO.linear(x, w, b)) + x, [x, w, b])
     # a result may be changed in place, an input that the backward needs may not
     q = _rand(1, 8, 2, 64)
     import oneflow_b200 as flow
