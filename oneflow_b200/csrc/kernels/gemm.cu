@@ -4,12 +4,17 @@
 #include "../common/host_utils.h"
 #include "gemm_tcgen05.cuh"
 #include "gemm_2cta.cuh"
+#include "gemm_few_rows.cuh"
 #include "ofb_kernels.h"
 
 namespace ofb {
 
 // Whether shapes that fill the machine use the two-SM kernel unless told otherwise.
 constexpr bool kDefault2Cta = true;
+// Up to 64 rows the product is a stream of weights (gemm_few_rows.cuh). With 33 rows and more, whose tiles every CTA reads besides, only
+// while the 128-column tiles fit the machine at once: 64 x 32768 x 2048 33.7 against 40.7 us with the tiled kernels, 64 x 40960 x 2048
+// 51.4 against 43.9, 33 x 40960 x 2048 45.4 against 42.3 (17 x 50304 x 2048 44.7 against 60.4).
+static bool few_rows(const OfbGemmArgs* a) { return a->M <= 32 || (a->M <= 64 && a->N <= 32768); }
 
 template <int BN, int A_MN, int B_MN, int ST = 0, int MINB = 1>
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmShape& shp, const GemmEpilogue& ep,
@@ -50,6 +55,57 @@ static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   return 0;
 }
 
+template <int NP, int W_MN>
+static int launch_gemm_few_rows(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmShape& shp, const GemmEpilogue& ep, int* status,
+                                cudaStream_t stream) {
+  using Cfg = FewRowsCfg<NP>;
+  auto kern = gemm_few_rows_kernel<NP, W_MN>;
+  OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(static_cast<unsigned>((shp.N + Cfg::BM - 1) / Cfg::BM * shp.splits));
+  cfg.blockDim = dim3(Cfg::THREADS);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(shp.splits);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  OFB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmW, tmX, shp, ep, status));
+  OFB_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// The K range of a tile is shared by CTAs (a cluster) as far as 256 of them hold the tiles at once (clusters do not fill all 296 places:
+// 8 x 6144 x 2048, 48 tiles: five CTAs each 9.8 us, six 14.9) and each keeps four K blocks, with long K sixteen (8 x 3072 x 1024: four CTAs
+// 6.7 us, eight 7.9; 8 x 4096 x 4096: four 11.0, eight 11.5; 8 x 4096 x 16384: four 30.1, eight 27.9).
+static int gemm_few_rows(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t stream) {
+  const int tiles = (a->N + 127) / 128, kblocks = (a->K + 63) / 64;
+  int parts = kblocks / 16 > 4 ? kblocks / 16 : kblocks / 4 < 4 ? kblocks / 4 : 4;
+  if (parts > 8) parts = 8;
+  if (parts > 256 / tiles) parts = 256 / tiles;
+  if (parts < 1) parts = 1;
+  const int kb_per = (kblocks + parts - 1) / parts;
+  parts = (kblocks + kb_per - 1) / kb_per;          // no part without a K block
+  const int np = a->M <= 16 ? 16 : a->M <= 32 ? 32 : 64;
+  CUtensorMap tmW, tmX;
+  if (!a->b_mn_major) {
+    if (get_tensor_map(&tmW, a->B, 2, 2, a->K, a->N, 0, (uint64_t)a->ldb * 2, 0, 64, 128, 0, 3)) return -1;
+  } else {
+    if (get_tensor_map(&tmW, a->B, 2, 2, a->N, a->K, 0, (uint64_t)a->ldb * 2, 0, 64, 64, 0, 3)) return -1;
+  }
+  if (get_tensor_map(&tmX, a->A, 2, 2, a->K, a->M, 0, (uint64_t)a->lda * 2, 0, 64, np, 0, 3)) return -1;
+  const GemmShape shp{a->M, a->N, a->K, parts};
+  int* status = device_status_ptr();
+#define OFB_FEW_ROWS(NP_)   if (np == NP_) return a->b_mn_major ? launch_gemm_few_rows<NP_, 1>(tmW, tmX, shp, ep, status, stream) : launch_gemm_few_rows<NP_, 0>(tmW, tmX, shp, ep, status, stream);
+  OFB_FEW_ROWS(16)
+  OFB_FEW_ROWS(32)
+  OFB_FEW_ROWS(64)
+#undef OFB_FEW_ROWS
+  return fail("gemm: few rows");
+}
+
 static int gemm_mode_2cta() {
   // OFB_GEMM_2CTA=0 turns the two-SM kernel off, =1 forces it for every shape it supports.
   static int mode = -2;
@@ -64,6 +120,7 @@ int gemm_dispatch(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t str
   if (a->M <= 0 || a->N <= 0 || a->K <= 0) return fail("gemm: empty problem");
   if (a->N % 8 != 0) return fail("gemm: N must be a multiple of 8");
   const int a_mn = a->a_mn_major, b_mn = a->b_mn_major;
+  if (few_rows(a) && !a_mn && a->bn == 0 && a->max_ctas == 0 && gemm_mode_2cta() == -1) return gemm_few_rows(a, ep, stream);
   // K-major: dims {K, rows}, row stride ld*2 bytes. MN-major: dims {rows, K}.
   CUtensorMap tmA, tmB;
   int bn = a->bn;

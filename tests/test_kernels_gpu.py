@@ -913,6 +913,43 @@ def test_conv_stride_arguments():
             call()
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 1032, 72), (15, 128, 64), (16, 136, 1000), (17, 4096, 4096), (33, 264, 136), (64, 50304, 256),
+                                   (64, 120, 16384), (40, 33024, 64), (65, 256, 512)])
+@pytest.mark.parametrize("layout", ["nk", "kn"])
+def test_gemm_few_rows(M, N, K, layout):
+    """Edges of the row classes (16, 32, 64), ragged columns, one K block and K ranges shared by up to eight CTAs; every epilogue."""
+    from oneflow_b200.ops import gemm as G
+    torch.manual_seed(40)
+    x = torch.randn(M, K, device=DEV, dtype=BF)
+    w = torch.randn(N, K, device=DEV, dtype=BF) * K ** -0.5
+    wl = w if layout == "nk" else w.t().contiguous()
+    b, r, h = torch.randn(N, device=DEV, dtype=BF), torch.randn(M, N, device=DEV, dtype=BF), torch.randn(M, N, device=DEV, dtype=BF)
+    p = x.double() @ w.double().t()
+    # fp32 sums of K products of size K^-1/2: at most K / 16 roundings of 2^-23 on partial sums below 8; bf16 results 2^-9 of their size
+    atol = K / 16 * 2.0 ** -20 + 1e-6
+    torch.testing.assert_close(G.gemm(x, wl, b_layout=layout, out_dtype=torch.float32).double(), p, rtol=1e-6, atol=atol)
+    y, aux = G.gemm(x, wl, b_layout=layout, bias=b, act="gelu", want_aux=True, residual=r)
+    pre = p + b.double()
+    torch.testing.assert_close(aux.double(), pre, rtol=2.0 ** -8, atol=atol)
+    # the activation's own approximation is good to 2e-6 (tests of the element-wise kernels)
+    torch.testing.assert_close(y.double(), torch.nn.functional.gelu(pre) + r.double(), rtol=2.0 ** -8, atol=atol + 1e-5)
+    d = G.gemm(x, wl, b_layout=layout, aux_in=h, act="relu")
+    torch.testing.assert_close(d.double(), p * (h > 0), rtol=2.0 ** -8, atol=atol)
+    acc = torch.randn(M, N, device=DEV)
+    out = G.gemm(x, wl, b_layout=layout, out=acc.clone(), accumulate=True)
+    torch.testing.assert_close(out.double(), acc.double() + p, rtol=1e-6, atol=atol)
+    acc = r.clone()
+    G.gemm(x, wl, b_layout=layout, out=acc, accumulate=True)
+    torch.testing.assert_close(acc.double(), p + r.double(), rtol=2.0 ** -7, atol=atol + 2.0 ** -8 * float(p.abs().max()))
+    # a slice of a wider matrix: leading dimensions that are not the row length
+    wide = torch.zeros(M, N + 24, device=DEV, dtype=BF)
+    G.gemm(x, wl, b_layout=layout, out=wide[:, 8:N + 8])
+    torch.testing.assert_close(wide[:, 8:N + 8].double(), p, rtol=2.0 ** -8, atol=atol)
+    assert not wide[:, :8].any() and not wide[:, N + 8:].any()
+    torch.cuda.synchronize()
+    assert _native.read_status() == (0, 0)
+
+
 def test_flow_conv2d_channels_last_uses_igemm():
     import oneflow_b200 as flow
     torch.manual_seed(0)
