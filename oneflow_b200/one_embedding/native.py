@@ -118,23 +118,24 @@ class NativeEmbeddingEngine:
         N, D, dev = self.world, self.dim, self.device
         i32, i64, f32 = torch.int32, torch.int64, torch.float32
         row_bytes = D * 2
-        need = N * self.cap * 8 + 4096 + 2 * (N * self.cap * row_bytes) + (1 << 16)
+        pairs = N * self.cap if N > 1 else 0        # (source, owner) pairs: one rank exchanges nothing
+        need = pairs * 8 + 4096 + 2 * (pairs * row_bytes) + (1 << 16)
         self.arena = SymmetricArena(self.group, self._ranks, dev, need)
         sh = EmbShuffleStruct()
-        sh.keys_off = self.arena.region(N * self.cap * 8)
+        sh.keys_off = self.arena.region(pairs * 8)
         sh.cnt_off = self.arena.region(4096)
-        sh.emb_off = self.arena.region(N * self.cap * row_bytes)
-        sh.grad_off = self.arena.region(N * self.cap * row_bytes)
+        sh.emb_off = self.arena.region(pairs * row_bytes)
+        sh.grad_off = self.arena.region(pairs * row_bytes)
         sh.cap = self.cap
-        self.dcap = _pow2(2 * self.cap)
+        self.dcap = _pow2(2 * self.cap) if N > 1 else 1
         self.dkeys = torch.empty((self.dcap,), dtype=i64, device=dev)
         self.dval = torch.empty((self.dcap,), dtype=i32, device=dev)
         self.cnt = torch.zeros((8,), dtype=i32, device=dev)
         self.inv = torch.empty((self.cap,), dtype=i32, device=dev)
-        self.gsum = torch.zeros((N * self.cap, D), dtype=f32, device=dev)
+        self.gsum = torch.zeros((pairs, D), dtype=f32, device=dev)
         self.slot_tmp = torch.empty((N * self.cap,), dtype=i32, device=dev)
-        self.rowidx = torch.empty((N * self.cap,), dtype=i32, device=dev)
-        self.uoidx = torch.empty((N * self.cap,), dtype=i32, device=dev)
+        self.rowidx = torch.empty((pairs,), dtype=i32, device=dev)
+        self.uoidx = torch.empty((pairs,), dtype=i32, device=dev)
         self.u_row = torch.empty((N * self.cap,), dtype=i32, device=dev)
         self.gacc = torch.zeros((N * self.cap, D), dtype=f32, device=dev)
         self.n_uo = torch.zeros((1,), dtype=i32, device=dev)
@@ -163,7 +164,7 @@ class NativeEmbeddingEngine:
             ctypes.byref(self.arena.ctx), ctypes.byref(self.st), ctypes.byref(self.sh), _native.ptr(ids), _native.ptr(tids),
             c_longlong(n), c_int(columns), c_int(int(insert)), c_uint(self.epoch), _native.ptr(out), c_int(int(self.half)),
             _native.stream_ptr()), "emb_forward")
-        _k._count(5)
+        _k._count(5 if self.world > 1 else 2)
         self._n_last = n
         return out
 
@@ -194,7 +195,7 @@ class NativeEmbeddingEngine:
         _native.check(_native.kernels().ofb_emb_backward(
             ctypes.byref(self.arena.ctx), ctypes.byref(self.st), ctypes.byref(self.sh), _native.ptr(grad), c_longlong(n),
             c_int(int(self.half)), c_uint(self.epoch), ctypes.byref(u), _native.stream_ptr()), "emb_backward")
-        _k._count(4)
+        _k._count(4 if self.world > 1 else 2)
 
     # ------------------------------------------------------------------ inspection / snapshots
     @property

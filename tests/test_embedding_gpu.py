@@ -73,6 +73,40 @@ def test_row_optimizers_match_reference_update(kind, factor):
         torch.testing.assert_close(eng.rows[urows], before, atol=2e-5, rtol=2e-4)
 
 
+@pytest.mark.parametrize("n,distinct,half", [(1, 1, False), (3, 2, True), (37, 5, False), (4099, 40, False), (1025, 1025, True)])
+def test_one_rank_repeated_and_absent_ids(n, distinct, half):
+    """Ragged id counts, many positions on few rows, lookups that do not insert: gradients of repeated ids are summed in fp32."""
+    from oneflow_b200.one_embedding.native import NativeEmbeddingEngine
+
+    def _one_table(e, k):
+        rows = e.find(k).long()
+        assert (rows >= 0).all()
+        return e.rows[rows, :e.dim].double()
+    torch.manual_seed(3)
+    eng = NativeEmbeddingEngine("cuda", 64, 128, 128, INITS[1:2], 1 << 14, seed=3, half=half)
+    dt = torch.float16 if half else torch.bfloat16
+    ids = torch.randint(0, distinct, (n, 1), device="cuda")
+    missing = eng.forward(ids + 10 ** 6, insert=False)
+    assert eng.size == 0 and not missing.any()
+    eng.backward(torch.ones_like(missing), "sgd", {"lr": 1.0}, 1)       # nothing is there to update
+    out = eng.forward(ids)
+    keys, where = torch.unique(ids.flatten(), return_inverse=True)
+    assert eng.size == keys.numel()
+    before = _one_table(eng, keys)
+    assert torch.equal(out.view(n, -1), before[where].to(dt))
+    g = torch.randn(n, eng.dim, device="cuda").to(dt)
+    eng.backward(g.view(out.shape), "sgd", {"lr": 0.5}, 1)
+    total = torch.zeros_like(before).index_add_(0, where, g.double())
+    size = torch.zeros_like(before).index_add_(0, where, g.double().abs())
+    after = _one_table(eng, keys)
+    # fp32 sums of at most n addends in any order, rounded to 16 bits once, and one update in fp32
+    assert bool(((after - (before - 0.5 * total)).abs() <= 0.5 * (n * 2.0 ** -24 * size + 2.0 ** (-11 if half else -8) * total.abs())
+                 + 2.0 ** -23 * (before.abs() + size)).all())
+    assert not eng.gacc.any()
+    again = eng.forward(torch.cat([ids, ids + 10 ** 6]), insert=False)
+    assert torch.equal(again[:n].reshape(n, -1), after[where].to(dt)) and not again[n:].any()
+
+
 def test_snapshot_roundtrip_and_module_path(tmp_path):
     import oneflow_b200 as flow
     from oneflow_b200 import one_embedding as oe
