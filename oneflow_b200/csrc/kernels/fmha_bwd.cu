@@ -18,18 +18,24 @@
 // run in order, so the columns of P are free by then), hence the exponentials of pair i + 1 run while dQ, dK of pair i and
 // dP of pair i + 1 are multiplied and dQ is drained. The chain that remains between two pairs is dS -> dQ -> drain -> dP
 // (at D = 128 dQ has no TMEM columns of its own and takes those of dP).
-// What bounds it: shared-memory bandwidth (per pair at D = 128 the products read 288 KiB of operands, staging dS and dQ and
-// the copies of Q, dO and dQ move 224 KiB: 4100 clocks, the products themselves 2560), then the fp32 reductions of dQ in L2.
+// At D = 64 there is room for the K and V of two key tiles: the scores of the next one are there when this one's gradients have
+// left TMEM.
+// What bounds it: at D = 128 shared-memory bandwidth (per pair the products read 288 KiB of operands, staging dS and dQ and
+// the copies of Q, dO and dQ move 224 KiB: 4100 clocks, the products themselves 2560), the fp32 reductions of dQ in L2, and on long
+// sequences the power limit; at D = 64 the threads that form P and dS (1310 and 1000 clocks of 2700 a pair, products 1280) and, with
+// four pairs a key tile, the 4000 clocks between two key tiles.
 // The grid has one CTA per key tile, but a running CTA takes over the next one that has not started (cluster launch control), so
 // that barriers, TMEM and the first loads of a tile do not wait for the end of the one before; the order stays the hardware's.
-// Measured on a B200 with delta and the dQ conversion, against a kernel with one chain S -> P -> dV -> dP -> dS -> dK, dQ ->
-// drain per pair and nothing overlapped, and without the take-over in brackets: batch 4, 32 heads, 2048 x 2048,
-// D = 128, causal 843 -> 454 us (504); batch 1, 32 / 8 heads, 8192 x 8192, D = 128, causal 2960 -> 1445 us (1490); batch 32,
-// 16 heads, 512 x 512, D = 64 349 -> 215 us (243); batch 8, 16 heads, 500 x 1100, D = 64 179 -> 101 us (118).
+// Measured on a B200, this kernel alone (in brackets with a mask test in every group of four exponentials, dS stored behind the
+// last of them, and dK and dV written a row per thread): batch 4, 32 heads, 2048 x 2048, D = 128, causal 340 us (368); batch 1, 32 / 8
+// heads, 8192 x 8192, D = 128, causal 1377 us (1379); batch 32, 16 heads, 512 x 512, D = 64 126 us (152); batch 8, 16 heads,
+// 500 x 1100, D = 64 70.5 us (86.9); batch 3, 12 heads, 777 x 777, D = 64, causal 20.2 us (24.5).
 // TMEM: S/P | dP (D = 128: also dQ) | dV | dK | D = 64: dQ.
 //
 // Reference counterpart: oneflow/user/kernels/scaled_dot_product_attention_grad_kernel.cu
 // (flash-attention library call).
+#include <type_traits>
+
 #include "../common/host_utils.h"
 #include "../common/philox.cuh"
 #include "../common/ptx.cuh"
@@ -63,12 +69,13 @@ template <int D>
 struct FmhaBwdCfg {
   static constexpr int T_BYTES = 128 * D * 2;            // one [128 x D] tile
   static constexpr int DO_STAGES = D == 128 ? 1 : 2;     // at D = 128 shared memory has room for one dO tile
+  static constexpr int KV_STAGES = D == 128 ? 1 : 2;     // and for the K and V of one key tile
   static constexpr int DS_BYTES = 128 * 128 * 2;
   static constexpr int SLAB_BYTES = 128 * 32 * 4;        // 32 columns of dQ in fp32, two of them in flight
   static constexpr int STAT_BYTES = 2 * 2 * 128 * 4;     // log-sum-exp and delta of two query tiles
   // no slack for aligning by hand: the dynamic shared memory starts the CTA's window (checked by the kernel)
-  static constexpr int BAR_BYTES = 288;                  // 28 mbarriers, TMEM slot, abort flag, two answers of 16 bytes
-  static constexpr int SMEM_BYTES = (4 + DO_STAGES) * T_BYTES + DS_BYTES + 2 * SLAB_BYTES + STAT_BYTES + BAR_BYTES;
+  static constexpr int BAR_BYTES = 288;                  // 30 mbarriers, TMEM slot, abort flag, two answers of 16 bytes
+  static constexpr int SMEM_BYTES = (2 * KV_STAGES + 2 + DO_STAGES) * T_BYTES + DS_BYTES + 2 * SLAB_BYTES + STAT_BYTES + BAR_BYTES;
   static_assert(SMEM_BYTES <= 232448, "shared memory");
 };
 
@@ -86,7 +93,7 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                 const __grid_constant__ CUtensorMap tmdQ, FmhaBwdParams p) {
   using Cfg = FmhaBwdCfg<D>;
-  constexpr int DCH = D / 64, DO_ST = Cfg::DO_STAGES;
+  constexpr int DCH = D / 64, DO_ST = Cfg::DO_STAGES, KV_ST = Cfg::KV_STAGES;
   constexpr int CH_BYTES = 128 * 128;
   constexpr bool kOwnDq = D == 64;                                // dQ has TMEM columns of its own
   constexpr uint32_t IDESC_S = make_idesc_bf16(128, 128, 0, 0);   // S^T, dP^T
@@ -99,36 +106,35 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, (int)kStatusBounds);
     return;
   }
-  uint8_t* sK = smem;
-  uint8_t* sV = sK + Cfg::T_BYTES;
-  uint8_t* sQ = sV + Cfg::T_BYTES;                  // 2 stages
+  uint8_t* sK = smem;                               // KV_ST stages
+  uint8_t* sV = sK + KV_ST * Cfg::T_BYTES;          // KV_ST stages
+  uint8_t* sQ = sV + KV_ST * Cfg::T_BYTES;          // 2 stages
   uint8_t* sdO = sQ + 2 * Cfg::T_BYTES;             // DO_ST stages
   uint8_t* sdS = sdO + DO_ST * Cfg::T_BYTES;        // dS^T: two 64-query chunks of [128 keys x 128 bytes]
   uint8_t* sStage = sdS + Cfg::DS_BYTES;            // two dQ slabs
-  float* sStat = reinterpret_cast<float*>(sStage + 2 * Cfg::SLAB_BYTES);   // [stage][lse | -delta][128]
+  float* sStat = reinterpret_cast<float*>(sStage + 2 * Cfg::SLAB_BYTES);   // [stage][-lse | -delta][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sStat) + Cfg::STAT_BYTES);
-  uint64_t* k_full = bars;
-  uint64_t* v_full = bars + 1;
-  uint64_t* q_full = bars + 2;      // [2]
-  uint64_t* q_empty = bars + 4;     // [2]
-  uint64_t* do_full = bars + 6;     // [2]
-  uint64_t* do_empty = bars + 8;    // [2]
-  uint64_t* stat_full = bars + 10;  // [2] 64 fetching threads
-  uint64_t* stat_empty = bars + 12; // [2] 8 compute warps
-  uint64_t* s_full = bars + 14;
-  uint64_t* p_ready = bars + 15;    // 256
-  uint64_t* dp_full = bars + 16;
-  uint64_t* ds_ready = bars + 17;   // 256
-  uint64_t* ds_free = bars + 18;    // dQ and dK have read dS
-  uint64_t* dq_full = bars + 19;
-  uint64_t* dq_drained = bars + 20; // 128
-  uint64_t* all_done = bars + 21;
-  uint64_t* kv_empty = bars + 22;   // every product of a key tile has finished
-  uint64_t* acc_free = bars + 23;   // 256: dK and dV have left TMEM
-  uint64_t* next_full = bars + 24;  // [2] the answer that names the CTA's next key tile
-  uint64_t* next_empty = bars + 26; // [2] 16 warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
-  uint8_t* answers = reinterpret_cast<uint8_t*>(bars + 30);   // [2] 16 bytes
+  uint64_t* k_full = bars;          // [2]
+  uint64_t* v_full = bars + 2;      // [2]
+  uint64_t* kv_empty = bars + 4;    // [2] every product of a key tile has finished
+  uint64_t* q_full = bars + 6;      // [2]
+  uint64_t* q_empty = bars + 8;     // [2]
+  uint64_t* do_full = bars + 10;    // [2]
+  uint64_t* do_empty = bars + 12;   // [2]
+  uint64_t* stat_full = bars + 14;  // [2] 64 fetching threads
+  uint64_t* stat_empty = bars + 16; // [2] 8 compute warps
+  uint64_t* next_full = bars + 18;  // [2] the answer that names the CTA's next key tile
+  uint64_t* next_empty = bars + 20; // [2] 16 warps
+  uint64_t* s_full = bars + 22;
+  uint64_t* p_ready = bars + 23;    // 256
+  uint64_t* dp_full = bars + 24;
+  uint64_t* ds_ready = bars + 25;   // 256
+  uint64_t* dq_full = bars + 26;
+  uint64_t* dq_drained = bars + 27; // 128
+  uint64_t* all_done = bars + 28;
+  uint64_t* acc_free = bars + 29;   // 256: dK and dV have left TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 30);
+  uint8_t* answers = reinterpret_cast<uint8_t*>(bars + 32);   // [2] 16 bytes
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -167,9 +173,10 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   };
 
   if (threadIdx.x == 0) {
-    mbar_init(k_full, 1);
-    mbar_init(v_full, 1);
     for (int s = 0; s < 2; ++s) {
+      mbar_init(&k_full[s], 1);
+      mbar_init(&v_full[s], 1);
+      mbar_init(&kv_empty[s], 1);
       mbar_init(&q_full[s], 1);
       mbar_init(&q_empty[s], 1);
       mbar_init(&do_full[s], 1);
@@ -181,11 +188,9 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(p_ready, 256);
     mbar_init(dp_full, 1);
     mbar_init(ds_ready, 256);
-    mbar_init(ds_free, 1);
     mbar_init(dq_full, 1);
     mbar_init(dq_drained, 128);
     mbar_init(all_done, 1);
-    mbar_init(kv_empty, 1);
     mbar_init(acc_free, 256);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&next_full[s], 1);
@@ -248,9 +253,10 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               if (!mbar_wait(&q_empty[st], ((g >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
               load(sQ + st * Cfg::T_BYTES, &tmQ, &q_full[st], h, i * 128);
               if (t == 0) {
-                if (!mbar_wait(kv_empty, (act & 1) ^ 1, abort_flag)) { ok = false; break; }
-                load(sK, &tmK, k_full, it.hk, it.k0);
-                load(sV, &tmV, v_full, it.hk, it.k0);
+                const int kv = act % KV_ST;
+                if (!mbar_wait(&kv_empty[kv], ((act / KV_ST) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                load(sK + kv * Cfg::T_BYTES, &tmK, &k_full[kv], it.hk, it.k0);
+                load(sV + kv * Cfg::T_BYTES, &tmV, &v_full[kv], it.hk, it.k0);
               }
               if (!mbar_wait(&do_empty[sd], ((g / DO_ST) & 1) ^ 1, abort_flag)) { ok = false; break; }
               load(sdO + sd * Cfg::T_BYTES, &tmdO, &do_full[sd], h, i * 128);
@@ -261,7 +267,9 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         __syncwarp();
       } else if (warp == 1) {
         if (elect_one() && it.n_iter > 0 && ok) {
-          const uint32_t k_base = smem_u32(sK), v_base = smem_u32(sV), ds_base = smem_u32(sdS);
+          const int kv = act % KV_ST;
+          const uint32_t kv_ph = (act / KV_ST) & 1;
+          const uint32_t k_base = smem_u32(sK + kv * Cfg::T_BYTES), v_base = smem_u32(sV + kv * Cfg::T_BYTES), ds_base = smem_u32(sdS);
           auto kk_off = [](int kk) -> uint32_t { return (kk >> 2) * CH_BYTES + (kk & 3) * 32; };   // K-major step of 16
           auto issue_s = [&](int g) {
             const uint32_t q_base = smem_u32(sQ + (g & 1) * Cfg::T_BYTES);
@@ -285,9 +293,9 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             umma_commit(dp_full);
             return true;
           };
-          ok = mbar_wait(k_full, act & 1, abort_flag) && mbar_wait(&q_full[g0 & 1], (g0 >> 1) & 1, abort_flag);
+          ok = mbar_wait(&k_full[kv], kv_ph, abort_flag) && mbar_wait(&q_full[g0 & 1], (g0 >> 1) & 1, abort_flag);
           if (ok) { tc_fence_after(); issue_s(g0); }
-          ok = ok && mbar_wait(v_full, act & 1, abort_flag);
+          ok = ok && mbar_wait(&v_full[kv], kv_ph, abort_flag);
           ok = ok && issue_dp(g0);
           // the accumulators of the tile before have left TMEM
           ok = ok && mbar_wait(acc_free, (act & 1) ^ 1, abort_flag);
@@ -323,18 +331,17 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             for (int kk = 0; kk < 8; ++kk)
               umma_bf16_ss(tdK, make_smem_desc_sw128(ds_base + kk_off(kk), 16, 1024),
                            make_smem_desc_sw128(q_base + kk * 2048, CH_BYTES, 1024), IDESC_KV, (t | kk) != 0 ? 1u : 0u);
-            umma_commit(ds_free);
             umma_commit(&q_empty[g & 1]);
             if (t + 1 < it.n_iter && !issue_dp(g + 1)) { ok = false; break; }
           }
           if (ok) {
             umma_commit(all_done);
-            umma_commit(kv_empty);
+            umma_commit(&kv_empty[kv]);
           }
         }
         __syncwarp();
       } else if (it.n_iter > 0 && ok) {
-        // warp 2: log-sum-exp in log2 units, +inf where the row does not exist or saw no key (P becomes 0); warp 3: -delta
+        // warp 2: minus log-sum-exp in log2 units, -inf where the row does not exist or saw no key (P becomes 0); warp 3: -delta
         int h = it.hk * group, i = it.i_start;
         for (int t = 0; t < it.n_iter; ++t) {
           const int g = g0 + t, st = g & 1;
@@ -345,7 +352,7 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const long long idx = (static_cast<long long>(it.b) * p.H + h) * p.Sq + row;
             if (warp == 2) {
               const float l = row < p.Sq ? p.lse[idx] : -INFINITY;
-              val[e] = l == -INFINITY ? INFINITY : l * 1.4426950408889634f;
+              val[e] = l == -INFINITY ? -INFINITY : l * -1.4426950408889634f;
             } else {
               val[e] = row < p.Sq ? -p.delta[idx] : 0.f;
             }
@@ -422,8 +429,6 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int n = 0;; ++n) {
       const Item it = item_of(item);
       const int krow = it.k0 + r;
-      __nv_bfloat16* dk_row = p.dk + (static_cast<long long>(it.b) * p.Sk + krow) * p.dkv_row_stride + it.hk * D;
-      __nv_bfloat16* dv_row = p.dv + (static_cast<long long>(it.b) * p.Sk + krow) * p.dkv_row_stride + it.hk * D;
       if (it.n_iter > 0) {
         uint8_t* ds_row = sdS + half * CH_BYTES + r * 128;   // this half's 64 queries = one swizzled chunk
         const uint32_t tSh = tS + lane_addr + half * 64, tdPh = tdP + lane_addr + half * 64;
@@ -434,12 +439,12 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const uint32_t ph = g & 1;
           const int st = g & 1;
           const int q0 = i * 128;
-          const float* lse = sStat + st * 256 + half * 64;
-          const float* ndelta = lse + 128;
+          const float* nlse = sStat + st * 256 + half * 64;
+          const float* ndelta = nlse + 128;
           const bool need_mask = (p.causal && it.k0 + 127 > q0 + p.causal_off) || (it.k0 + 128 > it.kv_limit);
           // first visible query column of this thread's half
           const int c_min = krow >= it.kv_limit ? 64 : (p.causal ? krow - p.causal_off - q0 - half * 64 : 0);
-          uint32_t pk[32];  // P, later dS, as packed bf16 pairs of this key row's 64 queries
+          uint32_t pk[32];  // P as packed bf16 pairs of this key row's 64 queries
           uint32_t keep_bits[DROP ? 2 : 1];  // dropout: bit c of word w = query column 32 * w + c of this half is kept
           if constexpr (DROP) {
             // a Philox draw covers four neighbouring keys of one query: the four lanes that own them draw a quarter each
@@ -466,27 +471,33 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             tmem_ld_32x32(tSh, v[0]);
             tmem_ld_32x32(tSh + 32, v[1]);
             tmem_wait_ld();
+            // one straight piece of code per kind of tile: with the test inside, every four elements were a block of their own and
+            // waited for their own loads and exponentials (1650 clocks a pair instead of 1310; the exponentials alone are 1024)
+            auto form_p = [&](auto masked) {
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+              for (int c = 0; c < 2; ++c) {
 #pragma unroll
-              for (int e = 0; e < 32; e += 4) {
-                const float4 l4 = *reinterpret_cast<const float4*>(lse + c * 32 + e);
-                float x[4];
-                unpack_f32x2(fma_f32x2(pack_f32x2(v[c][e], v[c][e + 1]), scale2,
-                                       pack_f32x2(__float_as_uint(-l4.x), __float_as_uint(-l4.y))), x[0], x[1]);
-                unpack_f32x2(fma_f32x2(pack_f32x2(v[c][e + 2], v[c][e + 3]), scale2,
-                                       pack_f32x2(__float_as_uint(-l4.z), __float_as_uint(-l4.w))), x[2], x[3]);
+                for (int e = 0; e < 32; e += 4) {
+                  const float4 l4 = *reinterpret_cast<const float4*>(nlse + c * 32 + e);
+                  float x[4];
+                  unpack_f32x2(fma_f32x2(pack_f32x2(v[c][e], v[c][e + 1]), scale2, pack_f32x2(__float_as_uint(l4.x), __float_as_uint(l4.y))),
+                               x[0], x[1]);
+                  unpack_f32x2(fma_f32x2(pack_f32x2(v[c][e + 2], v[c][e + 3]), scale2, pack_f32x2(__float_as_uint(l4.z), __float_as_uint(l4.w))),
+                               x[2], x[3]);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) x[k] = fast_exp2(x[k]);
-                if (need_mask) {
+                  for (int k = 0; k < 4; ++k) x[k] = fast_exp2(x[k]);
+                  if constexpr (decltype(masked)::value) {
 #pragma unroll
-                  for (int k = 0; k < 4; ++k)
-                    if (c * 32 + e + k < c_min) x[k] = 0.f;
+                    for (int k = 0; k < 4; ++k)
+                      if (c * 32 + e + k < c_min) x[k] = 0.f;
+                  }
+                  pk[c * 16 + (e >> 1)] = pack_bf16x2(x[0], x[1]);
+                  pk[c * 16 + (e >> 1) + 1] = pack_bf16x2(x[2], x[3]);
                 }
-                pk[c * 16 + (e >> 1)] = pack_bf16x2(x[0], x[1]);
-                pk[c * 16 + (e >> 1) + 1] = pack_bf16x2(x[2], x[3]);
               }
-            }
+            };
+            if (need_mask) form_p(std::true_type());
+            else form_p(std::false_type());
             // Publish P^T (with dropout: only the kept probabilities, which is what multiplied V in the forward; the factor
             // 1 / keep is applied to dV at the end). Only this thread reads these TMEM columns of S, and it has.
 #pragma unroll
@@ -504,7 +515,8 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
           tc_fence_before();
           mbar_arrive(p_ready);
-          // dS = P * (dP - delta); the softmax scale is applied to the finished dK and dQ
+          // dS = P * (dP - delta); the softmax scale is applied to the finished dK and dQ. dP of this pair was issued behind dQ and
+          // dK of the one before: those have read the last dS when it arrives, and every 16 bytes are stored as they are formed
           if (!mbar_wait(dp_full, ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
           {
@@ -516,67 +528,81 @@ fmha_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
             for (int c = 0; c < 2; ++c)
 #pragma unroll
-              for (int e = 0; e < 32; e += 4) {
-                const float4 nd = *reinterpret_cast<const float4*>(ndelta + c * 32 + e);
-                if constexpr (DROP) {   // the gradient reaches P only through the kept entries, scaled by 1 / keep
+              for (int e = 0; e < 32; e += 8) {
+                uint32_t w[4];
 #pragma unroll
-                  for (int k = 0; k < 4; ++k)
-                    v[c][e + k] = (keep_bits[c] >> (e + k)) & 1u ? __float_as_uint(__uint_as_float(v[c][e + k]) * p.drop.inv_keep) : 0u;
+                for (int u = 0; u < 2; ++u) {
+                  const int f = e + 4 * u;
+                  const float4 nd = *reinterpret_cast<const float4*>(ndelta + c * 32 + f);
+                  if constexpr (DROP) {   // the gradient reaches P only through the kept entries, scaled by 1 / keep
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                      v[c][f + k] = (keep_bits[c] >> (f + k)) & 1u ? __float_as_uint(__uint_as_float(v[c][f + k]) * p.drop.inv_keep) : 0u;
+                  }
+                  const uint32_t w0 = pk[c * 16 + (f >> 1)], w1 = pk[c * 16 + (f >> 1) + 1];
+                  float d[4];
+                  unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[c][f], v[c][f + 1]), pack_f32x2(__float_as_uint(nd.x), __float_as_uint(nd.y))),
+                                         pack_f32x2(w0 << 16, w0 & 0xFFFF0000u)), d[0], d[1]);
+                  unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[c][f + 2], v[c][f + 3]), pack_f32x2(__float_as_uint(nd.z), __float_as_uint(nd.w))),
+                                         pack_f32x2(w1 << 16, w1 & 0xFFFF0000u)), d[2], d[3]);
+                  w[2 * u] = pack_bf16x2(d[0], d[1]);
+                  w[2 * u + 1] = pack_bf16x2(d[2], d[3]);
                 }
-                const uint32_t w0 = pk[c * 16 + (e >> 1)], w1 = pk[c * 16 + (e >> 1) + 1];
-                float d[4];
-                unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[c][e], v[c][e + 1]), pack_f32x2(__float_as_uint(nd.x), __float_as_uint(nd.y))),
-                                       pack_f32x2(w0 << 16, w0 & 0xFFFF0000u)), d[0], d[1]);
-                unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[c][e + 2], v[c][e + 3]), pack_f32x2(__float_as_uint(nd.z), __float_as_uint(nd.w))),
-                                       pack_f32x2(w1 << 16, w1 & 0xFFFF0000u)), d[2], d[3]);
-                pk[c * 16 + (e >> 1)] = pack_bf16x2(d[0], d[1]);
-                pk[c * 16 + (e >> 1) + 1] = pack_bf16x2(d[2], d[3]);
+                *reinterpret_cast<uint4*>(ds_row + (((c * 4 + (e >> 3)) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
               }
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(&stat_empty[st]);
-          if (g > 0 && !mbar_wait(ds_free, (g - 1) & 1, abort_flag)) { ok = false; break; }
-#pragma unroll
-          for (int c16 = 0; c16 < 8; ++c16)
-            *reinterpret_cast<uint4*>(ds_row + ((c16 ^ (r & 7)) << 4)) =
-                make_uint4(pk[4 * c16], pk[4 * c16 + 1], pk[4 * c16 + 2], pk[4 * c16 + 3]);
           fence_proxy_async_smem();
           tc_fence_before();
           mbar_arrive(ds_ready);
           if (++i == n_qt) { i = it.i_start; ++h; }
         }
-        // dK, dV of this key tile: TMEM lane = key row; each half writes its half of the D columns
+        // dK (the first half's warps) and dV (the second's) of this key tile: TMEM lane = key row. A warp turns its 32 rows through
+        // its own part of dS, which every product has read by now, so that eight lanes write 128 bytes of a row together. (A thread
+        // writing its own row, 16 bytes in a line of its own per lane and store, kept the next tile waiting for 3500 clocks.)
         if (ok) ok = mbar_wait(all_done, act & 1, abort_flag);
         if (ok) {
           tc_fence_after();
+          const uint32_t src = (half == 0 ? tdK : tdV) + lane_addr;
+          __nv_bfloat16* dst = (half == 0 ? p.dk : p.dv) + (static_cast<long long>(it.b) * p.Sk + it.k0 + quad * 32) * p.dkv_row_stride + it.hk * D;
+          const float osc = half == 0 ? p.scale : (DROP ? p.drop.inv_keep : 1.f);
+          const int rows_here = p.Sk - it.k0 - quad * 32;
 #pragma unroll
-          for (int which = 0; which < 2; ++which) {
-            const uint32_t src = which == 0 ? tdK : tdV;
-            __nv_bfloat16* dst = which == 0 ? dk_row : dv_row;
-            const float osc = which == 0 ? p.scale : (DROP ? p.drop.inv_keep : 1.f);
-#pragma unroll
-            for (int c0 = 0; c0 < D / 64; ++c0) {
-              const int c = half * (D / 64) + c0;
-              uint32_t v[32];
-              __syncwarp();
-              tmem_ld_32x32(src + lane_addr + c * 32, v);
-              tmem_wait_ld();
-              if (krow < p.Sk) {
-#pragma unroll
-                for (int g = 0; g < 4; ++g)
-                  *reinterpret_cast<uint4*>(dst + c * 32 + g * 8) = make_uint4(
-                      pack_bf16x2(__uint_as_float(v[g * 8]) * osc, __uint_as_float(v[g * 8 + 1]) * osc),
-                      pack_bf16x2(__uint_as_float(v[g * 8 + 2]) * osc, __uint_as_float(v[g * 8 + 3]) * osc),
-                      pack_bf16x2(__uint_as_float(v[g * 8 + 4]) * osc, __uint_as_float(v[g * 8 + 5]) * osc),
-                      pack_bf16x2(__uint_as_float(v[g * 8 + 6]) * osc, __uint_as_float(v[g * 8 + 7]) * osc));
-              }
+          for (int c = 0; c < DCH; ++c) {
+            uint32_t v[2][32];
+            __syncwarp();
+            tmem_ld_32x32(src + c * 64, v[0]);
+            tmem_ld_32x32(src + c * 64 + 32, v[1]);
+            tmem_wait_ld();
+            if (c == DCH - 1) {
+              tc_fence_before();
+              mbar_arrive(acc_free);
             }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const uint32_t* x = v[e >> 2] + (e & 3) * 8;
+              *reinterpret_cast<uint4*>(ds_row + ((e ^ (r & 7)) << 4)) =
+                  make_uint4(pack_bf16x2(__uint_as_float(x[0]) * osc, __uint_as_float(x[1]) * osc),
+                             pack_bf16x2(__uint_as_float(x[2]) * osc, __uint_as_float(x[3]) * osc),
+                             pack_bf16x2(__uint_as_float(x[4]) * osc, __uint_as_float(x[5]) * osc),
+                             pack_bf16x2(__uint_as_float(x[6]) * osc, __uint_as_float(x[7]) * osc));
+            }
+            __syncwarp();
+            const uint8_t* warp_rows = sdS + half * CH_BYTES + quad * 32 * 128;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const int row = e * 4 + (lane >> 3), ch = lane & 7;
+              const uint4 q = *reinterpret_cast<const uint4*>(warp_rows + row * 128 + ((ch ^ (row & 7)) << 4));
+              if (row < rows_here) *reinterpret_cast<uint4*>(dst + row * p.dkv_row_stride + c * 64 + ch * 8) = q;
+            }
+            __syncwarp();
           }
-          tc_fence_before();
-          mbar_arrive(acc_free);
         }
       } else if (krow < p.Sk) {
         // Key tile invisible to every query (beyond kv_len, or right of the causal diagonal for all rows): zero gradients.
+        __nv_bfloat16* dk_row = p.dk + (static_cast<long long>(it.b) * p.Sk + krow) * p.dkv_row_stride + it.hk * D;
+        __nv_bfloat16* dv_row = p.dv + (static_cast<long long>(it.b) * p.Sk + krow) * p.dkv_row_stride + it.hk * D;
         for (int i = half * (D / 2); i < (half + 1) * (D / 2); i += 8) {
           *reinterpret_cast<uint4*>(dk_row + i) = make_uint4(0, 0, 0, 0);
           *reinterpret_cast<uint4*>(dv_row + i) = make_uint4(0, 0, 0, 0);
