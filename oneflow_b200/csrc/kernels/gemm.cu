@@ -16,11 +16,11 @@ constexpr bool kDefault2Cta = true;
 // 51.4 against 43.9, 33 x 40960 x 2048 45.4 against 42.3 (17 x 50304 x 2048 44.7 against 60.4).
 static bool few_rows(const OfbGemmArgs* a) { return a->M <= 32 || (a->M <= 64 && a->N <= 32768); }
 
-template <int BN, int A_MN, int B_MN, int ST = 0, int MINB = 1>
-static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmShape& shp, const GemmEpilogue& ep,
+template <int BN, int A_MN, int B_MN, int ST, int MINB, int EPI>
+static int launch_gemm_as(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmShape& shp, const GemmEpilogue& ep,
                        int* status, int max_ctas, cudaStream_t stream) {
   using Cfg = GemmCfg<BN, ST>;
-  auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN, ST, MINB>;
+  auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN, ST, MINB, EPI>;
   OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
   static int sm_count = 0;
   if (sm_count == 0) {
@@ -36,10 +36,30 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
   return 0;
 }
 
-template <int A_MN, int B_MN>
-static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmShape& shp, const GemmEpilogue& ep,
+// The epilogue compiled for itself where there is one: activations of forward products (both operands K-major), gradients of
+// activations in data gradients (B MN-major), fp32 results of weight gradients (A MN-major).
+#define OFB_GEMM_BY_EPILOGUE(launch, ...)                                                                                          \
+  switch (gemm_epilogue_kind(ep)) {                                                                                                \
+    case kEpiLinear: return launch<__VA_ARGS__, kEpiLinear>(tmA, tmB, shp, ep, status, max_ctas, stream);                           \
+    case kEpiGelu: if constexpr (!A_MN && !B_MN) return launch<__VA_ARGS__, kEpiGelu>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
+    case kEpiRelu: if constexpr (!A_MN && !B_MN) return launch<__VA_ARGS__, kEpiRelu>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
+    case kEpiGeluGrad: if constexpr (!A_MN && B_MN) return launch<__VA_ARGS__, kEpiGeluGrad>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
+    case kEpiReluGrad: if constexpr (!A_MN && B_MN) return launch<__VA_ARGS__, kEpiReluGrad>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
+    case kEpiWide: if constexpr (A_MN && B_MN) return launch<__VA_ARGS__, kEpiWide>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
+    default: break;                                                                                                                \
+  }                                                                                                                                \
+  return launch<__VA_ARGS__, kEpiAny>(tmA, tmB, shp, ep, status, max_ctas, stream)
+
+template <int BN, int A_MN, int B_MN, int ST = 0, int MINB = 1>
+static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmShape& shp, const GemmEpilogue& ep,
+                       int* status, int max_ctas, cudaStream_t stream) {
+  OFB_GEMM_BY_EPILOGUE(launch_gemm_as, BN, A_MN, B_MN, ST, MINB);
+}
+
+template <int A_MN, int B_MN, int EPI>
+static int launch_gemm_2cta_as(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmShape& shp, const GemmEpilogue& ep,
                             int* status, int max_ctas, cudaStream_t stream) {
-  auto kern = gemm_bf16_2cta_kernel<A_MN, B_MN>;
+  auto kern = gemm_bf16_2cta_kernel<A_MN, B_MN, EPI>;
   OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Cfg::SMEM8_BYTES));
   static int sm_count = 0;
   if (sm_count == 0) {
@@ -54,6 +74,13 @@ static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   OFB_CUDA_OK(cudaGetLastError());
   return 0;
 }
+
+template <int A_MN, int B_MN>
+static int launch_gemm_2cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmShape& shp, const GemmEpilogue& ep,
+                            int* status, int max_ctas, cudaStream_t stream) {
+  OFB_GEMM_BY_EPILOGUE(launch_gemm_2cta_as, A_MN, B_MN);
+}
+#undef OFB_GEMM_BY_EPILOGUE
 
 template <int NP, int W_MN>
 static int launch_gemm_few_rows(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmShape& shp, const GemmEpilogue& ep, int* status,
@@ -139,16 +166,18 @@ int gemm_dispatch(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t str
   const double cost1 = cost256 < cost128 ? cost256 : cost128;
   if (mode2 == -1 && bn == 0) {
     // For short K the epilogue takes longer than the main loop, and two one-SM CTAs per SM (short_k below) get through it faster.
-    // Where there are tiles for them, up to K = 384 if the epilogue does more than store (with bias 8192 x 2048 x 256 22.2 against
-    // 24.3 us, x 384 24.0 against 25.2, x 448 25.0 against 25.9, x 512 25.6 against 26.0), else up to 320 (8192 x 2048 x 256 18.6
-    // against 20.1, x 384 20.6 against 20.9; 50176 x 1024 x 320 48.3 against 48.1, x 384 53.4 against 48.3); below K = 256 always
-    // (802816 x 256 x 64: 136 against 156 us). Only for a K-major A: with an M-major one (weight gradients) that kernel does not
-    // exist, and 9472 x 3328 x 136 takes 32 us with pairs, 40 us with one-SM tiles.
+    // Where there are tiles for them, up to K = 384 if the epilogue reads or writes more than the result or has GELU in it (with
+    // residual 8773 x 6648 x 272 89 against 114 us with pairs, 43046 x 288 x 312 25.5 against 30.3, with GELU 31909 x 656 x 336 38.5
+    // against 43.9, 302 x 13864 x 352 20.1 against 24.3; with residual 42572 x 1392 x 408 142 against 129), else up to 256 (with bias 21856 x
+    // 1728 x 280 63 against 56 us, with bias and ReLU 25586 x 3896 x 312 124 against 111, 3764 x 6688 x 256 35.8 against 39.7; bare
+    // 3704 x 6520 x 200 31.7 against 32.4). Only for a K-major A: with an M-major one (weight gradients) that kernel does not exist; there
+    // one-SM tiles win up to K = 256 where the result is bf16 (9472 x 3328 x 136 22.4 against 26.7 us, 8480 x 1296 x 256 15.3
+    // against 17.4), pairs where it is fp32 (4248 x 4360 x 168 55.6 against 59).
     // A product with an activation's gradient keeps to pairs from K = 256 on: alone it is the slower one (55296 x 512 x 256 49.5
     // against 47.3 us), but pairs leave registers for the blocks of another stream, and backward passes run beside others (the row
     // update of an embedding beside two such products: 319 against 363 us, the step 3.52 against 3.56 ms).
-    const bool bare = !ep.bias && !ep.aux_out && !ep.residual;
-    const bool long_enough = a_mn || a->K > (tiles128 < 2 * 148 || ep.aux_in ? 255 : bare ? 320 : 384);
+    const bool rich = ep.aux_out || ep.residual || ep.act == kActGeluErf || ep.act == kActGeluTanh;
+    const bool long_enough = a_mn ? ep.out_fp32 || a->K > 256 : a->K > (tiles128 < 2 * 148 || ep.aux_in ? 255 : rich ? 384 : 256);
     // A caller's limit of one CTA leaves no room for a pair.
     two = kDefault2Cta && cost2 <= cost1 && a->N >= 256 && a->M >= 256 && long_enough && a->max_ctas != 1;
   }

@@ -89,7 +89,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
-template <int A_MN, int B_MN>
+template <int A_MN, int B_MN, int EPI = kEpiAny>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Gemm2Cfg::THREADS, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmShape shp,
                       GemmEpilogue ep, int* status) {
@@ -225,10 +225,20 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       int tm, tn;
       tile_coords(t, tiles_m, tiles_n, tm, tn);
       const int m0 = tm * 2 * BM + static_cast<int>(cta) * BM, n0 = tn * BN;
-      if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) break;
-      tc_fence_after();
-      gemm_epilogue_warp<BN>(ep, shp, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN, m0 + quad * 32, n0, lane, stage,
-                             false, half * (BN / 64), (half + 1) * (BN / 64));
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
+      auto finished = [&]() -> bool {
+        if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) return false;
+        tc_fence_after();
+        return true;
+      };
+      if constexpr (EPI == kEpiAny) {
+        if (!finished()) break;
+        gemm_epilogue_warp<BN>(ep, shp, taddr, m0 + quad * 32, n0, lane, stage, false, half * (BN / 64), (half + 1) * (BN / 64));
+      } else {
+        if (!gemm_epilogue_warp_as<EPI, BN>(ep, shp, taddr, m0 + quad * 32, n0, lane, stage, false, half * (BN / 64), (half + 1) * (BN / 64),
+                                             finished))
+          break;
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&tempty[acc]), 0));   // the leader owns the accumulator hand-off

@@ -96,7 +96,7 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   tn = r / gsz;
 }
 
-template <int BN, int A_MN, int B_MN, int ST = 0, int MINB = 1>
+template <int BN, int A_MN, int B_MN, int ST = 0, int MINB = 1, int EPI = kEpiAny>
 __global__ void __launch_bounds__(192, MINB)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          GemmShape shp, GemmEpilogue ep, int* status) {
@@ -229,10 +229,18 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     for (int u = blockIdx.x; u < total_units; u += gridDim.x) {
       int tm, tn;
       tile_coords(u % total_tiles, tiles_m, tiles_n, tm, tn);
-      if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) break;
-      tc_fence_after();
-      gemm_epilogue_warp<BN>(ep, shp, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN, tm * BM + quad * 32, tn * BN,
-                             lane, stage, splits > 1);
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
+      auto finished = [&]() -> bool {
+        if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) return false;
+        tc_fence_after();
+        return true;
+      };
+      if constexpr (EPI == kEpiAny) {
+        if (!finished()) break;
+        gemm_epilogue_warp<BN>(ep, shp, taddr, tm * BM + quad * 32, tn * BN, lane, stage, splits > 1);
+      } else {
+        if (!gemm_epilogue_warp_as<EPI, BN>(ep, shp, taddr, tm * BM + quad * 32, tn * BN, lane, stage, splits > 1, 0, BN / 32, finished)) break;
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
