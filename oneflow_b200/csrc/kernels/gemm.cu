@@ -45,6 +45,7 @@ static int launch_gemm_as(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
     case kEpiRelu: if constexpr (!A_MN && !B_MN) return launch<__VA_ARGS__, kEpiRelu>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
     case kEpiGeluGrad: if constexpr (!A_MN && B_MN) return launch<__VA_ARGS__, kEpiGeluGrad>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
     case kEpiReluGrad: if constexpr (!A_MN && B_MN) return launch<__VA_ARGS__, kEpiReluGrad>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
+    case kEpiMasked: if constexpr (!A_MN && B_MN) return launch<__VA_ARGS__, kEpiMasked>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
     case kEpiWide: if constexpr (A_MN && B_MN) return launch<__VA_ARGS__, kEpiWide>(tmA, tmB, shp, ep, status, max_ctas, stream); break; \
     default: break;                                                                                                                \
   }                                                                                                                                \
@@ -281,6 +282,8 @@ OFB_API int ofb_gemm_bf16(const OfbGemmArgs* a, void* stream) {
   ep.act = a->act;
   ep.out_fp32 = a->out_fp32;
   ep.accumulate = a->accumulate;
+  ep.residual_mask = a->residual ? reinterpret_cast<const unsigned char*>(a->residual_mask) : nullptr;
+  if (reinterpret_cast<uintptr_t>(ep.residual_mask) & 3) return fail("gemm: the residual's mask must be 4-byte aligned");
   return gemm_dispatch(a, ep, reinterpret_cast<cudaStream_t>(stream));
 }
 

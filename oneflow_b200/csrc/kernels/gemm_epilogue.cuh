@@ -215,6 +215,17 @@ __device__ __forceinline__ void epi_store_f32(uint32_t stage, int lane, const fl
   __syncwarp();
 }
 
+// The mask bits of 32 columns of a row of the residual: bit j for column col0 + j (col0 a multiple of 32).
+__device__ __forceinline__ uint32_t epi_mask_bits(const unsigned char* mask, long long row, int col0, int n_cols) {
+  const unsigned char* p = mask + row * (n_cols >> 3) + (col0 >> 3);
+  if ((n_cols & 31) == 0) return __ldg(reinterpret_cast<const unsigned int*>(p));
+  uint32_t bits = 0;
+#pragma unroll
+  for (int g = 0; g < 4; ++g)
+    if (col0 + g * 8 < n_cols) bits |= static_cast<uint32_t>(p[g]) << (8 * g);
+  return bits;
+}
+
 // Elementwise part and stores of one 32-column chunk whose accumulator values are already in `r`.
 __device__ __forceinline__ void gemm_epilogue_chunk(const GemmEpilogue& ep, const uint32_t (&r)[32], int row0, int col0, int rows_valid,
                                                     int cols_valid, int lane, uint32_t stage, bool atomic_out) {
@@ -278,6 +289,11 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmEpilogue& ep, cons
   if (ep.residual) {
     float h[32];
     epi_load_bf16(stage, lane, ep.residual + static_cast<long long>(row0) * ep.ldr + col0, ep.ldr, rows_valid, cols_valid, h);
+    if (ep.residual_mask) {
+      const uint32_t keep = lane < rows_valid ? epi_mask_bits(ep.residual_mask, row0 + lane, col0, col0 + cols_valid) : 0u;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) h[j] = (keep >> j) & 1u ? h[j] : 0.f;
+    }
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] += h[j];
   }
@@ -325,10 +341,12 @@ enum GemmEpiKind : int {
   kEpiRelu = 4,      // bias, ReLU, bf16
   kEpiReluGrad = 5,  // gradient of ReLU at aux_in, bf16
   kEpiWide = 6,      // fp32: stored, added, or added atomically
+  kEpiMasked = 7,    // residual where its mask has a one, bf16
 };
 static inline int gemm_epilogue_kind(const GemmEpilogue& ep) {
   if (ep.out_fp32) return !ep.bias && !ep.residual && !ep.aux_in && !ep.aux_out && ep.act == kActNone ? kEpiWide : kEpiAny;
   if (ep.accumulate) return kEpiAny;
+  if (ep.residual_mask) return ep.act == kActNone && !ep.aux_in && !ep.aux_out && !ep.bias ? kEpiMasked : kEpiAny;
   if (ep.act == kActNone && !ep.aux_in && !ep.aux_out) return kEpiLinear;
   if (ep.act == kActGeluErf && !ep.aux_in && ep.bias && !ep.residual) return kEpiGelu;
   if (ep.act == kActRelu && !ep.aux_in && ep.bias && !ep.residual && !ep.aux_out) return kEpiRelu;
@@ -372,12 +390,15 @@ __device__ __forceinline__ bool gemm_epilogue_warp_as(const GemmEpilogue& ep, co
   const int rows_valid = shp.M - row0;
   int nchunks = (shp.N - n0 + 31) / 32;
   if (nchunks > c_end) nchunks = c_end;
-  constexpr bool kReads = KIND == kEpiLinear || KIND == kEpiGeluGrad || KIND == kEpiReluGrad;
-  const __nv_bfloat16* src = KIND == kEpiLinear ? ep.residual : ep.aux_in;
-  const long long ld = KIND == kEpiLinear ? ep.ldr : ep.ld_aux;
+  constexpr bool kReads = KIND == kEpiLinear || KIND == kEpiMasked || KIND == kEpiGeluGrad || KIND == kEpiReluGrad;
+  constexpr bool kAdds = KIND == kEpiLinear || KIND == kEpiMasked;
+  const __nv_bfloat16* src = kAdds ? ep.residual : ep.aux_in;
+  const long long ld = kAdds ? ep.ldr : ep.ld_aux;
   if (kReads && src) src += static_cast<long long>(row0) * ld + n0;
   uint4 q[4];
+  uint32_t keep = 0;
   if (kReads && src && c_begin < nchunks) epi_fetch_bf16(src + c_begin * 32, ld, rows_valid, shp.N - n0 - c_begin * 32, lane, q);
+  if (KIND == kEpiMasked && c_begin < nchunks && lane < rows_valid) keep = epi_mask_bits(ep.residual_mask, row0 + lane, n0 + c_begin * 32, shp.N);
   if (!wait()) return false;
 #pragma unroll 1
   for (int c = c_begin; c < nchunks; ++c) {
@@ -419,9 +440,12 @@ __device__ __forceinline__ bool gemm_epilogue_warp_as(const GemmEpilogue& ep, co
       float h[32];
       epi_spread_bf16(stage, lane, q, h);
       if (c + 1 < nchunks) epi_fetch_bf16(src + (c + 1) * 32, ld, rows_valid, cols_valid - 32, lane, q);
+      const uint32_t keep_now = keep;
+      if (KIND == kEpiMasked && c + 1 < nchunks && lane < rows_valid) keep = epi_mask_bits(ep.residual_mask, row0 + lane, col0 + 32, shp.N);
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         if constexpr (KIND == kEpiLinear) v[j] += h[j];
+        else if constexpr (KIND == kEpiMasked) v[j] += (keep_now >> j) & 1u ? h[j] : 0.f;
         else if constexpr (KIND == kEpiGeluGrad) v[j] *= gelu_erf_grad(h[j]);
         else v[j] = h[j] > 0.f ? v[j] : 0.f;
       }

@@ -52,7 +52,7 @@ __device__ __forceinline__ uint4 few_rows_pack(const float (&v)[8]) {
 }
 
 // The order of operations of gemm_epilogue_chunk, for 8 columns of one row.
-__device__ __forceinline__ void few_rows_epilogue(const GemmEpilogue& ep, float (&v)[8], long long row, int col) {
+__device__ __forceinline__ void few_rows_epilogue(const GemmEpilogue& ep, float (&v)[8], long long row, int col, int n_cols) {
   float h[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) v[j] *= ep.alpha;
@@ -72,8 +72,9 @@ __device__ __forceinline__ void few_rows_epilogue(const GemmEpilogue& ep, float 
   }
   if (ep.residual) {
     few_rows_unpack(*reinterpret_cast<const uint4*>(ep.residual + row * ep.ldr + col), h);
+    const unsigned int keep = ep.residual_mask ? ep.residual_mask[row * (n_cols >> 3) + (col >> 3)] : 0xffu;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] += h[j];
+    for (int j = 0; j < 8; ++j) v[j] += (keep >> j) & 1u ? h[j] : 0.f;
   }
   if (ep.out_fp32) {
     float4* p = reinterpret_cast<float4*>(reinterpret_cast<float*>(ep.C) + row * ep.ldc + col);
@@ -234,7 +235,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
           v[4] += hi[p].x; v[5] += hi[p].y; v[6] += hi[p].z; v[7] += hi[p].w;
         }
       }
-      few_rows_epilogue(ep, v, m, n0 + c);
+      few_rows_epilogue(ep, v, m, n0 + c, shp.N);
     }
   }
   cluster_sync_all();      // nobody leaves while a peer may read its sums

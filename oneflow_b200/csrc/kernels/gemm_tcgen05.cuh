@@ -40,6 +40,7 @@ struct GemmEpilogue {
   int act;                        // GemmAct applied to (alpha*acc + bias)
   int out_fp32;                   // C is fp32
   int accumulate;                 // C += result
+  const unsigned char* residual_mask;   // [M, N / 8] or null: bit j of a byte is 0 where the residual of column j counts as 0
 };
 
 struct GemmShape {

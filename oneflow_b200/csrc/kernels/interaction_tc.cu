@@ -174,32 +174,36 @@ interaction_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_
 }
 
 // ------------------------------------------------------------------------------------------------ backward
-template <int STAGES>
+template <int X_STAGES, int A_STAGES>
 __global__ void __launch_bounds__(448, 1)
 interaction_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmD,
                           const __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ d_dense,
                           __nv_bfloat16* __restrict__ d_sparse, ItParams p, int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* xt = smem;                              // [STAGES] X tiles
-  uint8_t* at = smem + STAGES * kItTileBytes;      // [STAGES] A tiles
-  uint8_t* epi = at + STAGES * kItTileBytes;       // [8] epilogue staging, 4 KB each
+  uint8_t* xt = smem;                              // [X_STAGES] X tiles
+  uint8_t* at = smem + X_STAGES * kItTileBytes;    // [A_STAGES] A tiles
+  uint8_t* epi = at + A_STAGES * kItTileBytes;     // [8] epilogue staging, 4 KB each
   __nv_bfloat16* gbuf = reinterpret_cast<__nv_bfloat16*>(epi + 8 * kEpiStageBytesPerWarp);  // [3][512]
   uint64_t* x_full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(gbuf) + 3 * 1024);
-  uint64_t* a_full = x_full + STAGES;
-  uint64_t* empty = a_full + STAGES;
-  uint64_t* tfull = empty + STAGES;
+  uint64_t* x_empty = x_full + X_STAGES;
+  uint64_t* a_full = x_empty + X_STAGES;
+  uint64_t* a_empty = a_full + A_STAGES;
+  uint64_t* tfull = a_empty + A_STAGES;
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  for (int i = threadIdx.x; i < 2 * STAGES * kItTileBytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < (X_STAGES + A_STAGES) * kItTileBytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < X_STAGES; ++s) {
       mbar_init(&x_full[s], 1);
+      mbar_init(&x_empty[s], 1);
+    }
+    for (int s = 0; s < A_STAGES; ++s) {
       mbar_init(&a_full[s], kItSamples);
-      mbar_init(&empty[s], 1);
+      mbar_init(&a_empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
@@ -228,7 +232,7 @@ interaction_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_
       int stage = 0;
       uint32_t phase = 0;
       for (int g = blockIdx.x; g < p.groups; g += gridDim.x) {
-        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) break;
+        if (!mbar_wait(&x_empty[stage], phase ^ 1, abort_flag)) break;
         mbar_arrive_expect_tx(&x_full[stage], tx_bytes);
         uint8_t* tile = xt + stage * kItTileBytes;
         for (int h = 0; h < 2; ++h) {
@@ -236,20 +240,20 @@ interaction_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_
             tma_load_2d(tile + h * kItHalfBytes + s * 32 * 128, &tmS, &x_full[stage], h * 64, (g * kItSamples + s) * T);
           tma_load_2d(tile + h * kItHalfBytes + 96 * 128, &tmD, &x_full[stage], h * 64, g * kItSamples);
         }
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        if (++stage == X_STAGES) { stage = 0; phase ^= 1; }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     if (elect_one()) {
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
+      int stage = 0, a_stage = 0, acc = 0;
+      uint32_t phase = 0, a_phase = 0, acc_phase = 0;
       for (int g = blockIdx.x; g < p.groups; g += gridDim.x) {
         if (!mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag)) break;
         if (!mbar_wait(&x_full[stage], phase, abort_flag)) break;
-        if (!mbar_wait(&a_full[stage], phase, abort_flag)) break;
+        if (!mbar_wait(&a_full[a_stage], a_phase, abort_flag)) break;
         tc_fence_after();
-        const uint32_t a_base = smem_u32(at + stage * kItTileBytes);
+        const uint32_t a_base = smem_u32(at + a_stage * kItTileBytes);
         const uint32_t b_base = smem_u32(xt + stage * kItTileBytes);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {  // K = the 128 tile rows, 16 per instruction
@@ -257,9 +261,11 @@ interaction_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_
           const uint64_t db = make_smem_desc_sw128(b_base + k * 2048, kItHalfBytes, 1024);
           umma_bf16_ss(tmem_base + acc * 128, da, db, IDESC, k != 0 ? 1u : 0u);
         }
-        umma_commit(&empty[stage]);
+        umma_commit(&x_empty[stage]);
+        umma_commit(&a_empty[a_stage]);
         umma_commit(&tfull[acc]);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        if (++stage == X_STAGES) { stage = 0; phase ^= 1; }
+        if (++a_stage == A_STAGES) { a_stage = 0; a_phase ^= 1; }
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }
@@ -273,18 +279,23 @@ interaction_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_
       const int npairs = T * (T + 1) / 2;
       int stage = 0;
       uint32_t phase = 0;
-      for (int g = blockIdx.x; g < p.groups; g += gridDim.x) {
-        const long long b = static_cast<long long>(g) * kItSamples + q;
-        // pair gradients of this sample, fetched before the wait so that the load latency overlaps it
-        uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
+      uint4 v0, v1;
+      // pair gradients of this warp's sample of group g
+      auto fetch = [&](long long g) {
+        const long long b = g * kItSamples + q;
+        v0 = v1 = make_uint4(0, 0, 0, 0);
         if (b < p.batch) {
           const uint4* src = reinterpret_cast<const uint4*>(dout + b * p.out_dim + kItD);
           if (lane * 8 < npairs) v0 = __ldg(src + lane);
           if ((lane + 32) * 8 < npairs) v1 = __ldg(src + lane + 32);
         }
-        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) break;
+      };
+      fetch(blockIdx.x);
+      for (int g = blockIdx.x; g < p.groups; g += gridDim.x) {
+        if (!mbar_wait(&a_empty[stage], phase ^ 1, abort_flag)) break;
         reinterpret_cast<uint4*>(gb)[lane] = v0;
         reinterpret_cast<uint4*>(gb)[lane + 32] = v1;
+        fetch(static_cast<long long>(g) + gridDim.x);      // arrives while this group's operand is put together
         __syncwarp();
         const uint32_t a_tile = smem_u32(at + stage * kItTileBytes);
         const int t = lane;
@@ -336,7 +347,7 @@ interaction_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_
         fence_proxy_async_smem();  // generic-proxy stores above -> tensor-core (async proxy) reads
         __syncwarp();
         if (lane == 0) mbar_arrive(&a_full[stage]);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        if (++stage == A_STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else {
@@ -347,37 +358,67 @@ interaction_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_
     const uint32_t stage_sm = smem_u32(epi + (warp - 6) * kEpiStageBytesPerWarp);
     int acc = 0;
     uint32_t acc_phase = 0;
+    auto dense_rows = [&](long long g) {      // dense vectors of group g: 0..3
+      const long long left = p.batch - g * kItSamples;
+      return left >= kItSamples ? kItSamples : (left > 0 ? static_cast<int>(left) : 0);
+    };
+    // the part of dout that the dense gradients add, asked for one group ahead: lane 4 r + i holds columns 8 i.. of row r
+    uint4 add0 = make_uint4(0, 0, 0, 0), add1 = add0;
+    auto fetch = [&](long long g) {
+      const __nv_bfloat16* src = dout + (g * kItSamples + (lane >> 2)) * p.out_dim + half * 64 + (lane & 3) * 8;
+      add0 = add1 = make_uint4(0, 0, 0, 0);
+      if ((lane >> 2) < dense_rows(g)) {
+        add0 = __ldg(reinterpret_cast<const uint4*>(src));
+        add1 = __ldg(reinterpret_cast<const uint4*>(src + 32));
+      }
+    };
+    if (q == kItSamples) fetch(blockIdx.x);
     for (int g = blockIdx.x; g < p.groups; g += gridDim.x) {
       if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) break;
       tc_fence_after();
-      const long long b0 = static_cast<long long>(g) * kItSamples;
-#pragma unroll 1
-      for (int c = half * 2; c < half * 2 + 2; ++c) {
-        uint32_t r[32];
-        __syncwarp();
-        tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * 128 + c * 32, r);
-        tmem_wait_ld();
-        float v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-        if (q < kItSamples) {
-          const long long b = b0 + q;
-          epi_store_bf16(stage_sm, lane, v, d_sparse + b * T * kItD + c * 32, kItD, b < p.batch ? T : 0, 32, false);
-        } else {
-          long long left = p.batch - b0;
-          const int rv = left >= kItSamples ? kItSamples : (left > 0 ? static_cast<int>(left) : 0);
-          float h[32];
-          epi_load_bf16(stage_sm, lane, dout + b0 * p.out_dim + c * 32, p.out_dim, rv, 32, h);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] += h[j];
-          epi_store_bf16(stage_sm, lane, v, d_dense + b0 * kItD + c * 32, kItD, rv, 32, false);
-        }
-      }
+      uint32_t r[2][32];
+      __syncwarp();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * 128 + half * 64;
+      tmem_ld_32x32(taddr, r[0]);
+      tmem_ld_32x32(taddr + 32, r[1]);
+      tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
+      const long long b0 = static_cast<long long>(g) * kItSamples;
+      const uint4 now0 = add0, now1 = add1;
+      if (q == kItSamples) fetch(static_cast<long long>(g) + gridDim.x);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int col = half * 64 + i * 32;
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[i][j]);
+        if (q < kItSamples) {
+          const long long b = b0 + q;
+          epi_store_bf16(stage_sm, lane, v, d_sparse + b * T * kItD + col, kItD, b < p.batch ? T : 0, 32, false);
+        } else {
+          epi_sts(epi_addr64(stage_sm, lane >> 2, lane & 3), i ? now1 : now0);
+          __syncwarp();
+          if (lane < 8) {
+#pragma unroll
+            for (int ch = 0; ch < 4; ++ch) {
+              const uint4 x = epi_lds(epi_addr64(stage_sm, lane, ch));
+              const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 f = unpack_bf16x2(w[j]);
+                v[ch * 8 + 2 * j] += f.x;
+                v[ch * 8 + 2 * j + 1] += f.y;
+              }
+            }
+          }
+          __syncwarp();
+          epi_store_bf16(stage_sm, lane, v, d_dense + b0 * kItD + col, kItD, dense_rows(g), 32, false);
+        }
+      }
     }
   }
 
@@ -445,9 +486,9 @@ OFB_API int ofb_interaction_tc_bwd(const void* dense, const void* sparse, const 
   if (batch == 0) return 0;
   CUtensorMap tmS, tmD;
   if (it_maps(&tmS, &tmD, dense, sparse, batch, T)) return -1;
-  constexpr int STAGES = 2;
-  constexpr int SMEM = 2 * STAGES * kItTileBytes + 8 * kEpiStageBytesPerWarp + 3 * 1024 + 256 + 1024;
-  auto kern = interaction_bwd_tc_kernel<STAGES>;
+  constexpr int X_STAGES = 3, A_STAGES = 2;
+  constexpr int SMEM = (X_STAGES + A_STAGES) * kItTileBytes + 8 * kEpiStageBytesPerWarp + 3 * 1024 + 256 + 1024;
+  auto kern = interaction_bwd_tc_kernel<X_STAGES, A_STAGES>;
   OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
   ItParams p{batch, T, out_dim, static_cast<int>((batch + kItSamples - 1) / kItSamples)};
   int grid = it_sm_count();

@@ -26,6 +26,7 @@ typedef struct OfbGemmArgs {
   int bn;          // tile width override: 0 auto, 128 or 256
   int max_ctas;    // 0 = one CTA per SM
   float alpha;
+  const void* residual_mask;  // one bit per element of the residual, [M, N / 8] bytes: 0 adds nothing (null: all are added)
 } OfbGemmArgs;
 
 // Set-associative LRU cache of fp32 rows (lru_cache.cu): 32 ways per set, storage provided by the caller.

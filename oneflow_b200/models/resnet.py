@@ -81,8 +81,9 @@ class _Conv:
         self.x = x
         return C.conv_fprop(x, w, self.stride if self.k > 1 else 1)
 
-    def bwd(self, dy, need_dx=True, residual=None):
-        """``residual`` (shape of the input gradient) is added to the returned gradient."""
+    def bwd(self, dy, need_dx=True, residual=None, residual_mask=None):
+        """``residual`` (shape of the input gradient) is added to the returned gradient, ``residual_mask``: where its bits are set
+        (1 x 1 filters of stride 1)."""
         st = self.net.store
         w = st.p[self.name]
         stride = self.stride if self.k > 1 else 1
@@ -90,7 +91,7 @@ class _Conv:
         dx = None
         if need_dx:
             fuse = residual is not None and not (self.stride == 2 and self.k == 1)
-            dx = C.conv_dgrad(dy, w, residual if fuse else None, stride, self.in_shape[1:3])
+            dx = C.conv_dgrad(dy, w, residual if fuse else None, stride, self.in_shape[1:3], residual_mask)
             if self.stride == 2 and self.k == 1:
                 dx = N.upsample2_zero(dx, self.in_shape)
             if residual is not None and not fuse:
@@ -120,14 +121,19 @@ class _BN:
         self.x, self.y = x, (y if relu and self.mask is None else None)
         return y
 
-    def bwd(self, dy):
+    def bwd(self, dy, dy_mask=None):
+        """(gradient of x, that of the residual, its mask or None). With the forward's mask the residual's gradient is dy where the bits
+        are set: its consumers read the two, and nothing is written for it. ``dy_mask``: such a mask for dy itself (no ReLU here)."""
         net = self.net
         gamma = net.master(self.name + ".weight")
         names = (self.name + ".weight", self.name + ".bias")
-        dx, dres, _, _ = N.bn_train_bwd(dy, self.x, self.y, self.mean, self.rstd, gamma, self.relu, self.has_res, self.mask,
+        dy = dy.contiguous()
+        mask = self.mask if dy_mask is None else dy_mask
+        dx, dres, _, _ = N.bn_train_bwd(dy, self.x, self.y, self.mean, self.rstd, gamma, self.relu or dy_mask is not None,
+                                        self.has_res and mask is None, mask,
                                         net.bn_sums(self, 1), [net.store.g[n] for n in names], [net.store.acc_flag(n) for n in names])
         self.x = self.y = self.mask = None
-        return dx, dres
+        return (dx, dy, mask) if self.has_res and mask is not None else (dx, dres, None)
 
 
 class _Bottleneck:
@@ -152,15 +158,14 @@ class _Bottleneck:
         return self.bn3.fwd(self.conv3.fwd(y), residual=idn, relu=True)
 
     def bwd(self, dy):
-        d3, dres = self.bn3.bwd(dy)
+        d3, dres, dmask = self.bn3.bwd(dy)
         d = self.conv3.bwd(d3)
-        d, _ = self.bn2.bwd(d)
+        d = self.bn2.bwd(d)[0]
         d = self.conv2.bwd(d)
-        d, _ = self.bn1.bwd(d)
+        d = self.bn1.bwd(d)[0]
         if self.down is not None:
-            dd, _ = self.down[1].bwd(dres)
-            dres = self.down[0].bwd(dd)
-        return self.conv1.bwd(d, residual=dres)     # identity-branch gradient added in the dgrad GEMM epilogue
+            dres, dmask = self.down[0].bwd(self.down[1].bwd(dres, dmask)[0]), None
+        return self.conv1.bwd(d, residual=dres, residual_mask=dmask)     # identity-branch gradient added in the dgrad GEMM epilogue
 
 
 class ResNet:
@@ -274,7 +279,7 @@ class ResNet:
             if stage_done is not None and i < len(self.stages) - 1:
                 stage_done(i)
         d = N.maxpool3x3s2_bwd(d, self.pool_idx, self.pool_in_shape)
-        d, _ = self.bn1.bwd(d)
+        d = self.bn1.bwd(d)[0]
         G.gemm(d.view(-1, self.cfg.stem), self.stem_cols_saved, a_layout="km", b_layout="kn", out=st.g["conv1.weight"],
                out_dtype=torch.float32, accumulate=st.acc_flag("conv1.weight"))
         self.stem_cols_saved = None

@@ -32,7 +32,7 @@ class GemmArgs(Structure):
         ("M", c_int), ("N", c_int), ("K", c_int),
         ("a_mn_major", c_int), ("b_mn_major", c_int),
         ("act", c_int), ("out_fp32", c_int), ("accumulate", c_int), ("bn", c_int), ("max_ctas", c_int),
-        ("alpha", c_float),
+        ("alpha", c_float), ("residual_mask", c_void_p),
     ]
 
 

@@ -56,9 +56,9 @@ def conv_fprop(x, w, stride=1):
     return y
 
 
-def conv_dgrad(dy, w, residual=None, stride=1, in_hw=None):
-    """Gradient of conv_fprop wrt x (+ ``residual`` of the same shape, added in the GEMM epilogue for 1x1 filters). ``in_hw`` is the
-    size of x's map, needed with stride 2."""
+def conv_dgrad(dy, w, residual=None, stride=1, in_hw=None, residual_mask=None):
+    """Gradient of conv_fprop wrt x (+ ``residual`` of the same shape, added in the GEMM epilogue for 1x1 filters, and there only where
+    the bits of ``residual_mask`` are set). ``in_hw`` is the size of x's map, needed with stride 2."""
     N, H, W, Cout = dy.shape
     _, R, S, Cin = w.shape
     _check_stride(R, S, stride)
@@ -68,7 +68,10 @@ def conv_dgrad(dy, w, residual=None, stride=1, in_hw=None):
         H, W = in_hw
     if R == 1 and S == 1:
         res2d = residual.reshape(-1, Cin) if residual is not None else None
-        return G.gemm(dy.reshape(-1, Cout), w.reshape(Cout, Cin), b_layout="kn", residual=res2d).view(N, H, W, Cin)
+        return G.gemm(dy.reshape(-1, Cout), w.reshape(Cout, Cin), b_layout="kn", residual=res2d,
+                      residual_mask=residual_mask).view(N, H, W, Cin)
+    if residual_mask is not None:
+        raise ValueError("conv_dgrad: masked residuals come with 1 x 1 filters")
     if residual is not None:
         return K.bias_mask_scale(conv_dgrad(dy, w, None, stride, in_hw), None, None, 1.0, addend=residual)
     if not _igemm_ok(dy, w):

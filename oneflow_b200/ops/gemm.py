@@ -44,7 +44,7 @@ def _act_grad_ref(h, act):
 
 
 def gemm_reference(a, b, a_layout="mk", b_layout="nk", bias=None, act=0, residual=None, aux_in=None,
-                   want_aux=False, out=None, out_dtype=torch.bfloat16, accumulate=False, alpha=1.0):
+                   want_aux=False, out=None, out_dtype=torch.bfloat16, accumulate=False, alpha=1.0, residual_mask=None):
     """fp32 PyTorch statement of what the kernel computes (oracle for tests, CPU path)."""
     act = _act_code(act)
     A = a.float() if a_layout == "mk" else a.float().t()
@@ -58,7 +58,11 @@ def gemm_reference(a, b, a_layout="mk", b_layout="nk", bias=None, act=0, residua
     elif act:
         v = _act_ref(v, act)
     if residual is not None:
-        v = v + residual.float()
+        r = residual.float()
+        if residual_mask is not None:
+            bits = residual_mask.view(r.shape[0], -1, 1) >> torch.arange(8, dtype=torch.uint8, device=r.device) & 1
+            r = torch.where(bits.view(r.shape) != 0, r, 0.)
+        v = v + r
     if accumulate and out is not None:
         v = v + out.float()
     res = v.to(out_dtype)
@@ -78,18 +82,19 @@ def _check_operand(t, name):
 
 
 def gemm(a, b, *, a_layout="mk", b_layout="nk", bias=None, act=0, residual=None, aux_in=None, want_aux=False,
-         out=None, out_dtype=torch.bfloat16, accumulate=False, alpha=1.0, bn=0, max_ctas=0):
+         out=None, out_dtype=torch.bfloat16, accumulate=False, alpha=1.0, bn=0, max_ctas=0, residual_mask=None):
     """``out = epilogue(alpha * A @ B^T)`` with A logical [M,K] and B logical [N,K].
 
     a_layout: "mk" (a is [M,K]) or "km" (a is [K,M]);  b_layout: "nk" (b is [N,K]) or "kn" (b is [K,N]).
     Epilogue order: +bias -> (aux_out = pre-activation) -> act  (or  *act'(aux_in))  -> +residual -> (+out).
-    Returns ``out`` or ``(out, aux)`` when ``want_aux``.
+    ``residual_mask``: contiguous uint8 [M, N / 8], bit j of byte i of a row says whether column 8 i + j of the residual counts (the
+    masks of ``cnn.bn_train_fwd``). Returns ``out`` or ``(out, aux)`` when ``want_aux``.
     """
     act = _act_code(act)
     if not a.is_cuda:
         return gemm_reference(a, b, a_layout, b_layout, bias, act, residual, aux_in, want_aux, out, out_dtype,
-                              accumulate, alpha)
-    if alpha == 1.0 and bn == 0 and max_ctas == 0 and _native._recorder is None:
+                              accumulate, alpha, residual_mask)
+    if alpha == 1.0 and residual_mask is None and bn == 0 and max_ctas == 0 and _native._recorder is None:
         r = _native.torch_ops().gemm(a, b, a_layout != "mk", b_layout != "nk", bias, act, residual, aux_in, want_aux, out,
                                      out_dtype == torch.float32, accumulate) if out_dtype in _OUT_TYPES else None
         if r is not None:
@@ -116,6 +121,10 @@ def gemm(a, b, *, a_layout="mk", b_layout="nk", bias=None, act=0, residual=None,
     for t, nm in ((bias, "bias"), (residual, "residual"), (aux_in, "aux_in")):
         if t is not None and (t.dtype != torch.bfloat16 or t.data_ptr() % 16 != 0):
             raise TypeError(f"gemm: {nm} must be 16-byte aligned bfloat16")
+    if residual_mask is not None:
+        if residual is None or residual_mask.dtype != torch.uint8 or residual_mask.numel() != M * N // 8 or \
+                not residual_mask.is_contiguous() or residual_mask.device != residual.device:
+            raise ValueError("gemm: a residual mask is M * N / 8 contiguous bytes beside a residual")
     # positional, in the order of GemmArgs._fields_: one call instead of an attribute store per field
     args = _native.GemmArgs(
         a.data_ptr(), b.data_ptr(), out.data_ptr(),
@@ -124,7 +133,8 @@ def gemm(a, b, *, a_layout="mk", b_layout="nk", bias=None, act=0, residual=None,
         a.stride(0), b.stride(0), out.stride(0), 0 if residual is None else residual.stride(0),
         aux_in.stride(0) if aux_in is not None else (aux.stride(0) if aux is not None else 0),
         M, N, K, 0 if a_layout == "mk" else 1, 0 if b_layout == "nk" else 1,
-        act, out_dtype == torch.float32, bool(accumulate), bn, max_ctas, alpha)
+        act, out_dtype == torch.float32, bool(accumulate), bn, max_ctas, alpha,
+        None if residual_mask is None else residual_mask.data_ptr())
     lib = _native.kernels()
     if _native._recorder is not None:
         for t in (a, b, out, bias, residual, aux_in, aux):

@@ -950,6 +950,30 @@ def test_gemm_few_rows(M, N, K, layout):
     assert _native.read_status() == (0, 0)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (64, 136, 72), (129, 72, 64), (300, 264, 256), (257, 1032, 512), (4096, 512, 640), (2000, 64, 1024)])
+@pytest.mark.parametrize("layout", ["nk", "kn"])
+@pytest.mark.parametrize("bias", [False, True])
+def test_gemm_masked_residual(M, N, K, layout, bias):
+    """One and two SMs a tile, up to 64 rows, rows of the mask that are and are not whole words; what the mask hides may be NaN."""
+    from oneflow_b200.ops import gemm as G
+    torch.manual_seed(41)
+    x = torch.randn(M, K, device=DEV, dtype=BF)
+    w = torch.randn(N, K, device=DEV, dtype=BF) * K ** -0.5
+    r = torch.randn(M, N, device=DEV, dtype=BF)
+    b = torch.randn(N, device=DEV, dtype=BF) if bias else None
+    mask = torch.randint(0, 256, (M, N // 8), device=DEV, dtype=torch.uint8)
+    keep = ((mask.view(M, N // 8, 1) >> torch.arange(8, device=DEV, dtype=torch.uint8)) & 1).view(M, N) != 0
+    r = torch.where(keep, r, float("nan"))
+    y = G.gemm(x, w if layout == "nk" else w.t().contiguous(), b_layout=layout, bias=b, residual=r, residual_mask=mask)
+    ref = x.double() @ w.double().t() + torch.where(keep, r, 0.).double()
+    # fp32 sums of K products of size K^-1/2: at most K / 16 roundings of 2^-23 on partial sums below 8; bf16 results 2^-9 of their size
+    torch.testing.assert_close(y.double(), ref if b is None else ref + b.double(), rtol=2.0 ** -8, atol=K / 16 * 2.0 ** -20 + 1e-6)
+    with pytest.raises(ValueError):
+        G.gemm(x, w, residual=r, residual_mask=mask.view(-1)[1:])
+    with pytest.raises(ValueError):
+        G.gemm(x, w, residual_mask=mask)
+
+
 def test_flow_conv2d_channels_last_uses_igemm():
     import oneflow_b200 as flow
     torch.manual_seed(0)
