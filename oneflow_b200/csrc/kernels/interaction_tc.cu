@@ -11,8 +11,13 @@
 // Backward: dX = A X with the same X tile as the (MN-major) B operand and A = the symmetric gradient matrix of the
 //           three samples laid out block-diagonally (plus row/column 96 + s for the dense vector), which three
 //           builder warps assemble in shared memory from dout while the previous tile runs.
-// Roles per CTA: warp 0 TMA producer, warp 1 MMA issuer, then builder (backward only: 4) and epilogue warps (backward: 8); the
+// Roles per CTA: warp 0 TMA producer, warp 1 MMA issuer, then builder (backward only: 6) and epilogue warps (backward: 8); the
 // tiles flow through a multi-stage shared-memory ring and two TMEM accumulators, every wait is bounded.
+//
+// Bound: memory (55296 samples of 26 features read 0.42 GB and write 0.38 GB in the backward, 122 us at 6547 GB/s). One CTA a SM has
+// under 2000 clocks a tile, so no role may stand in front of a load on each one: the builders and the dense rows' epilogue ask for
+// dout a tile ahead, X has three stages and A two (the ring is what keeps reads in flight), and two sets of builders take tiles in turn.
+// With one set, two stages of both and loads where they are used 270 us; loads ahead and the third stage 225; the second set 173.
 //
 // Reference: oneflow/user/kernels/fused_dot_feature_interaction_kernel.cu (wmma, one CTA per sample).
 #include "../common/host_utils.h"
@@ -26,6 +31,7 @@ constexpr int kItD = 128;
 constexpr int kItHalfBytes = 128 * 128;          // [128 rows][64 columns] bf16
 constexpr int kItTileBytes = 2 * kItHalfBytes;   // 32 KB
 constexpr int kItSamples = 3;
+constexpr int kItBuilderSets = 2;                // backward: A tiles in the making
 
 struct ItParams {
   long long batch;
@@ -174,18 +180,19 @@ interaction_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_
 }
 
 // ------------------------------------------------------------------------------------------------ backward
-template <int X_STAGES, int A_STAGES>
-__global__ void __launch_bounds__(448, 1)
+template <int X_STAGES>
+__global__ void __launch_bounds__(512, 1)
 interaction_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmD,
                           const __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ d_dense,
                           __nv_bfloat16* __restrict__ d_sparse, ItParams p, int* status) {
+  constexpr int A_STAGES = kItBuilderSets;         // a set of builder warps fills its own A tile
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* xt = smem;                              // [X_STAGES] X tiles
   uint8_t* at = smem + X_STAGES * kItTileBytes;    // [A_STAGES] A tiles
   uint8_t* epi = at + A_STAGES * kItTileBytes;     // [8] epilogue staging, 4 KB each
-  __nv_bfloat16* gbuf = reinterpret_cast<__nv_bfloat16*>(epi + 8 * kEpiStageBytesPerWarp);  // [3][512]
-  uint64_t* x_full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(gbuf) + 3 * 1024);
+  __nv_bfloat16* gbuf = reinterpret_cast<__nv_bfloat16*>(epi + 8 * kEpiStageBytesPerWarp);  // [2][3][512]
+  uint64_t* x_full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(gbuf) + kItBuilderSets * kItSamples * 1024);
   uint64_t* x_empty = x_full + X_STAGES;
   uint64_t* a_full = x_empty + X_STAGES;
   uint64_t* a_empty = a_full + A_STAGES;
@@ -271,91 +278,90 @@ interaction_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmS, const __grid_
       }
     }
     __syncwarp();
-  } else if (warp < 6) {
-    // ---------------------------------------------------------------- builders of the gradient operand
-    const int q = warp & 3;
-    if (q < kItSamples) {
-      __nv_bfloat16* gb = gbuf + q * 512;
-      const int npairs = T * (T + 1) / 2;
-      int stage = 0;
-      uint32_t phase = 0;
-      uint4 v0, v1;
-      // pair gradients of this warp's sample of group g
-      auto fetch = [&](long long g) {
-        const long long b = g * kItSamples + q;
-        v0 = v1 = make_uint4(0, 0, 0, 0);
-        if (b < p.batch) {
-          const uint4* src = reinterpret_cast<const uint4*>(dout + b * p.out_dim + kItD);
-          if (lane * 8 < npairs) v0 = __ldg(src + lane);
-          if ((lane + 32) * 8 < npairs) v1 = __ldg(src + lane + 32);
-        }
-      };
-      fetch(blockIdx.x);
-      for (int g = blockIdx.x; g < p.groups; g += gridDim.x) {
-        if (!mbar_wait(&a_empty[stage], phase ^ 1, abort_flag)) break;
-        reinterpret_cast<uint4*>(gb)[lane] = v0;
-        reinterpret_cast<uint4*>(gb)[lane + 32] = v1;
-        fetch(static_cast<long long>(g) + gridDim.x);      // arrives while this group's operand is put together
-        __syncwarp();
-        const uint32_t a_tile = smem_u32(at + stage * kItTileBytes);
-        const int t = lane;
-        const int row = 32 * q + t;
-        const __nv_bfloat16 zero = __float2bfloat16(0.f);
-        // row (q, t): columns (q, u) of the diagonal block, feature order dense = 0, sparse u = u + 1
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          __nv_bfloat16 e[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int u = 8 * j + i;
-            const int hi = (t > u ? t : u) + 1, lo = (t > u ? u : t) + 1;
-            const int idx = hi * (hi - 1) / 2 + lo;
-            e[i] = (t < T && u < T && u != t && idx < npairs) ? gb[idx] : zero;
-          }
-          uint4 qv;
-          qv.x = (uint32_t)__bfloat16_as_ushort(e[0]) | ((uint32_t)__bfloat16_as_ushort(e[1]) << 16);
-          qv.y = (uint32_t)__bfloat16_as_ushort(e[2]) | ((uint32_t)__bfloat16_as_ushort(e[3]) << 16);
-          qv.z = (uint32_t)__bfloat16_as_ushort(e[4]) | ((uint32_t)__bfloat16_as_ushort(e[5]) << 16);
-          qv.w = (uint32_t)__bfloat16_as_ushort(e[6]) | ((uint32_t)__bfloat16_as_ushort(e[7]) << 16);
-          epi_sts(it_swz(a_tile + (q >> 1) * kItHalfBytes, row, (q & 1) * 4 + j), qv);
-        }
-        // row (q, t), column 96 + q: the pair with the dense vector
-        {
-          const __nv_bfloat16 gd = t < T ? gb[t * (t + 1) / 2] : zero;
-          const uint32_t hv = __bfloat16_as_ushort(gd);
-          uint4 qv = make_uint4(0, 0, 0, 0);
-          if (q == 0) qv.x = hv;
-          if (q == 1) qv.x = hv << 16;
-          if (q == 2) qv.y = hv;
-          epi_sts(it_swz(a_tile + kItHalfBytes, row, 4), qv);
-        }
-        // row 96 + q: the same pair gradients along the columns (q, u)
-        if (lane < 4) {
-          __nv_bfloat16 e[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int u = 8 * lane + i;
-            e[i] = u < T ? gb[u * (u + 1) / 2] : zero;
-          }
-          uint4 qv;
-          qv.x = (uint32_t)__bfloat16_as_ushort(e[0]) | ((uint32_t)__bfloat16_as_ushort(e[1]) << 16);
-          qv.y = (uint32_t)__bfloat16_as_ushort(e[2]) | ((uint32_t)__bfloat16_as_ushort(e[3]) << 16);
-          qv.z = (uint32_t)__bfloat16_as_ushort(e[4]) | ((uint32_t)__bfloat16_as_ushort(e[5]) << 16);
-          qv.w = (uint32_t)__bfloat16_as_ushort(e[6]) | ((uint32_t)__bfloat16_as_ushort(e[7]) << 16);
-          epi_sts(it_swz(a_tile + (q >> 1) * kItHalfBytes, 96 + q, (q & 1) * 4 + lane), qv);
-        }
-        fence_proxy_async_smem();  // generic-proxy stores above -> tensor-core (async proxy) reads
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&a_full[stage]);
-        if (++stage == A_STAGES) { stage = 0; phase ^= 1; }
+  } else if (warp < 2 + kItBuilderSets * kItSamples) {
+    // ---------------------------------------------------------------- builders of the gradient operand: a warp per sample, the two
+    // sets in turn
+    const int q = (warp - 2) % kItSamples, stage = (warp - 2) / kItSamples;
+    __nv_bfloat16* gb = gbuf + (warp - 2) * 512;
+    const int npairs = T * (T + 1) / 2;
+    const int step = kItBuilderSets * gridDim.x, first = blockIdx.x + stage * gridDim.x;
+    uint32_t phase = 0;
+    uint4 v0, v1;
+    // pair gradients of this warp's sample of group g
+    auto fetch = [&](long long g) {
+      const long long b = g * kItSamples + q;
+      v0 = v1 = make_uint4(0, 0, 0, 0);
+      if (b < p.batch) {
+        const uint4* src = reinterpret_cast<const uint4*>(dout + b * p.out_dim + kItD);
+        if (lane * 8 < npairs) v0 = __ldg(src + lane);
+        if ((lane + 32) * 8 < npairs) v1 = __ldg(src + lane + 32);
       }
+    };
+    fetch(first);
+    for (int g = first; g < p.groups; g += step) {
+      if (!mbar_wait(&a_empty[stage], phase ^ 1, abort_flag)) break;
+      reinterpret_cast<uint4*>(gb)[lane] = v0;
+      reinterpret_cast<uint4*>(gb)[lane + 32] = v1;
+      fetch(static_cast<long long>(g) + step);           // arrives while this group's operand is put together
+      __syncwarp();
+      const uint32_t a_tile = smem_u32(at + stage * kItTileBytes);
+      const int t = lane;
+      const int row = 32 * q + t;
+      const __nv_bfloat16 zero = __float2bfloat16(0.f);
+      // row (q, t): columns (q, u) of the diagonal block, feature order dense = 0, sparse u = u + 1
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        __nv_bfloat16 e[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int u = 8 * j + i;
+          const int hi = (t > u ? t : u) + 1, lo = (t > u ? u : t) + 1;
+          const int idx = hi * (hi - 1) / 2 + lo;
+          e[i] = (t < T && u < T && u != t && idx < npairs) ? gb[idx] : zero;
+        }
+        uint4 qv;
+        qv.x = (uint32_t)__bfloat16_as_ushort(e[0]) | ((uint32_t)__bfloat16_as_ushort(e[1]) << 16);
+        qv.y = (uint32_t)__bfloat16_as_ushort(e[2]) | ((uint32_t)__bfloat16_as_ushort(e[3]) << 16);
+        qv.z = (uint32_t)__bfloat16_as_ushort(e[4]) | ((uint32_t)__bfloat16_as_ushort(e[5]) << 16);
+        qv.w = (uint32_t)__bfloat16_as_ushort(e[6]) | ((uint32_t)__bfloat16_as_ushort(e[7]) << 16);
+        epi_sts(it_swz(a_tile + (q >> 1) * kItHalfBytes, row, (q & 1) * 4 + j), qv);
+      }
+      // row (q, t), column 96 + q: the pair with the dense vector
+      {
+        const __nv_bfloat16 gd = t < T ? gb[t * (t + 1) / 2] : zero;
+        const uint32_t hv = __bfloat16_as_ushort(gd);
+        uint4 qv = make_uint4(0, 0, 0, 0);
+        if (q == 0) qv.x = hv;
+        if (q == 1) qv.x = hv << 16;
+        if (q == 2) qv.y = hv;
+        epi_sts(it_swz(a_tile + kItHalfBytes, row, 4), qv);
+      }
+      // row 96 + q: the same pair gradients along the columns (q, u)
+      if (lane < 4) {
+        __nv_bfloat16 e[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int u = 8 * lane + i;
+          e[i] = u < T ? gb[u * (u + 1) / 2] : zero;
+        }
+        uint4 qv;
+        qv.x = (uint32_t)__bfloat16_as_ushort(e[0]) | ((uint32_t)__bfloat16_as_ushort(e[1]) << 16);
+        qv.y = (uint32_t)__bfloat16_as_ushort(e[2]) | ((uint32_t)__bfloat16_as_ushort(e[3]) << 16);
+        qv.z = (uint32_t)__bfloat16_as_ushort(e[4]) | ((uint32_t)__bfloat16_as_ushort(e[5]) << 16);
+        qv.w = (uint32_t)__bfloat16_as_ushort(e[6]) | ((uint32_t)__bfloat16_as_ushort(e[7]) << 16);
+        epi_sts(it_swz(a_tile + (q >> 1) * kItHalfBytes, 96 + q, (q & 1) * 4 + lane), qv);
+      }
+      fence_proxy_async_smem();  // generic-proxy stores above -> tensor-core (async proxy) reads
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&a_full[stage]);
+      phase ^= 1;
     }
   } else {
-    // ---------------------------------------------------------------- epilogue (warps 6..13): two warps per TMEM lane
+    // ---------------------------------------------------------------- epilogue (warps 8..15): two warps per TMEM lane
     // quadrant, each draining two of the four 32-column chunks (one warp per scheduler alone cannot keep up)
     const int q = warp & 3;
-    const int half = (warp - 6) >> 2;
-    const uint32_t stage_sm = smem_u32(epi + (warp - 6) * kEpiStageBytesPerWarp);
+    const int half = (warp - 8) >> 2;
+    const uint32_t stage_sm = smem_u32(epi + (warp - 8) * kEpiStageBytesPerWarp);
     int acc = 0;
     uint32_t acc_phase = 0;
     auto dense_rows = [&](long long g) {      // dense vectors of group g: 0..3
@@ -486,14 +492,14 @@ OFB_API int ofb_interaction_tc_bwd(const void* dense, const void* sparse, const 
   if (batch == 0) return 0;
   CUtensorMap tmS, tmD;
   if (it_maps(&tmS, &tmD, dense, sparse, batch, T)) return -1;
-  constexpr int X_STAGES = 3, A_STAGES = 2;
-  constexpr int SMEM = (X_STAGES + A_STAGES) * kItTileBytes + 8 * kEpiStageBytesPerWarp + 3 * 1024 + 256 + 1024;
-  auto kern = interaction_bwd_tc_kernel<X_STAGES, A_STAGES>;
+  constexpr int X_STAGES = 3;
+  constexpr int SMEM = (X_STAGES + kItBuilderSets) * kItTileBytes + 8 * kEpiStageBytesPerWarp + kItBuilderSets * kItSamples * 1024 + 256 + 1024;
+  auto kern = interaction_bwd_tc_kernel<X_STAGES>;
   OFB_CUDA_OK_ONCE_PER_DEVICE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
   ItParams p{batch, T, out_dim, static_cast<int>((batch + kItSamples - 1) / kItSamples)};
   int grid = it_sm_count();
   if (grid > p.groups) grid = p.groups;
-  kern<<<grid, 448, SMEM, reinterpret_cast<cudaStream_t>(stream)>>>(
+  kern<<<grid, 512, SMEM, reinterpret_cast<cudaStream_t>(stream)>>>(
       tmS, tmD, reinterpret_cast<const __nv_bfloat16*>(dout), reinterpret_cast<__nv_bfloat16*>(d_dense),
       reinterpret_cast<__nv_bfloat16*>(d_sparse), p, device_status_ptr());
   OFB_CUDA_OK(cudaGetLastError());

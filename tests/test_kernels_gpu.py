@@ -849,6 +849,27 @@ def test_dot_feature_interaction(self_inter, T, D):
     torch.testing.assert_close(sparse.grad.float(), s32.grad, atol=0.15, rtol=0.03)
 
 
+@pytest.mark.parametrize("B", [1, 3, 445, 1333, 6000])
+@pytest.mark.parametrize("T", [1, 26, 31])
+def test_dot_feature_interaction_backward_tiles(B, T):
+    """Three samples a tile, tiles in turn over the SMs and two sets of builder warps: one tile, a tile of one sample, a second tile for
+    one SM, a third, several rounds."""
+    from oneflow_b200.ops.interaction import dot_feature_interaction, dot_feature_interaction_reference
+    torch.manual_seed(5)
+    dense = (torch.randn(B, 128, device=DEV) * 0.5).to(BF).requires_grad_()
+    sparse = (torch.randn(B, T, 128, device=DEV) * 0.5).to(BF).requires_grad_()
+    pad = -(T * (T + 1) // 2) % 8
+    out = dot_feature_interaction([dense, sparse], output_concat=dense, output_padding=pad)
+    d64, s64 = dense.detach().double().requires_grad_(), sparse.detach().double().requires_grad_()
+    ref = dot_feature_interaction_reference([d64, s64], output_concat=d64, output_padding=pad)
+    g = torch.randn(out.shape, device=DEV).to(BF)
+    out.backward(g)
+    ref.backward(g.double())
+    # fp32 sums of up to 33 products below 16, at most 33 roundings of 2^-24 on partial sums below 64, then one rounding to bf16
+    torch.testing.assert_close(dense.grad.double(), d64.grad.double(), rtol=2.0 ** -8, atol=33 * 2.0 ** -18)
+    torch.testing.assert_close(sparse.grad.double(), s64.grad.double(), rtol=2.0 ** -8, atol=33 * 2.0 ** -18)
+
+
 @pytest.mark.parametrize("N,H,W,Cin,Cout,R", [(4, 56, 56, 64, 64, 3), (3, 28, 28, 128, 128, 3), (5, 14, 14, 256, 256, 3),
                                               (6, 7, 7, 512, 512, 3), (2, 19, 13, 64, 128, 3), (2, 16, 16, 64, 64, 5)])
 def test_conv_implicit_gemm(N, H, W, Cin, Cout, R):
