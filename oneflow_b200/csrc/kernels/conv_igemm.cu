@@ -156,38 +156,62 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         const int kb0 = (u / total_tiles) * kb_per, kb1 = PARITY ? tile_kblocks(t) : min(kblocks, kb0 + kb_per);
         const ConvParity q(g, PARITY ? t / class_tiles : 0);
         int n0 = 0, h0 = 0, w0 = 0;
-        if (MODE != kConvWgrad) conv_tile_origin(g, tm, 128, n0, h0, w0);
+        // a 64-column box of dW: channel, and where its tap reads x
+        [[maybe_unused]] int col_c[BN / 64], col_w[BN / 64], col_h[BN / 64];
+        if constexpr (MODE == kConvWgrad) {
+          conv_tile_origin(g, kb0, 64, n0, h0, w0);
+#pragma unroll
+          for (int c = 0; c < BN / 64; ++c) {
+            const int col = tn * BN + c * 64, tap = col / g.CA;
+            col_c[c] = col % g.CA;
+            col_w[c] = tap % g.S - pad_w;
+            col_h[c] = tap / g.S - pad_h;
+          }
+        } else {
+          conv_tile_origin(g, tm, 128, n0, h0, w0);
+        }
+        // Boxes of 64 channels past the last one are left out: what stays in their place in shared memory only reaches rows or
+        // columns of the accumulator that nobody stores. (Boxes outside the tensor are slow: with half of each weight tile outside,
+        // 3 x 3 on 256 x 56 x 56 x 64 took 246 us forward, where the gradient of x, whose boxes all lay inside, took 120.)
+        const int a_boxes = MODE == kConvWgrad ? min(BM, g.CO - tm * BM) / 64 : BM / 64;
+        const int b_boxes = min(BN, (MODE == kConvWgrad ? g.R * g.S * g.CA : g.CO) - tn * BN) / 64;
+        const uint32_t tx_bytes = (a_boxes + b_boxes) * (64 * 128);
+        // Tap and channel chunk of the K block are carried along, as the origin of a box of pixels below: one thread feeds the ring, and
+        // with divisions on each K block it came too late (256 images, 3 x 3: w's gradient 28 x 28 x 128 74.5 -> 61.1 us, 56 x 56 x 64
+        // 175 -> 128; forward 28 x 28 x 128 67.9 -> 62.7, gradient of x 67.1 -> 62.3).
+        int c0 = 0, r = PARITY ? q.r0 : 0, s = PARITY ? q.s0 : 0;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
-          mbar_arrive_expect_tx(&full[stage], A_BYTES + B_BYTES);
+          mbar_arrive_expect_tx(&full[stage], tx_bytes);
           uint8_t* a_dst = sA + stage * A_BYTES;
           uint8_t* b_dst = sB + stage * B_BYTES;
           if (MODE == kConvFprop) {
-            const int tap = kb / cpb, c0 = (kb % cpb) * BK;
-            const int r = tap / g.S, s = tap % g.S;
             tma_load_4d(a_dst, &tmA, &full[stage], c0, g.stride * w0 + s - pad_w, g.stride * h0 + r - pad_h, n0);
-            tma_load_2d(b_dst, &tmB, &full[stage], kb * BK, tn * BN);                      // W[k rows][tap * C + c]
+#pragma unroll
+            for (int c = 0; c < BN / 64; ++c)                                              // W[k rows][tap * C + c]
+              if (c < b_boxes) tma_load_2d(b_dst + c * (BK * 128), &tmB, &full[stage], kb * BK, tn * BN + c * 64);
           } else if (MODE == kConvDgrad) {
-            const int tap = kb / cpb, c0 = (kb % cpb) * BK;                                // c0: chunk of dY channels (= Cout)
-            const int r = PARITY ? q.r0 + 2 * (tap / q.n_s) : tap / g.S, s = PARITY ? q.s0 + 2 * (tap % q.n_s) : tap % g.S;
             const int dw = PARITY ? (q.a_w + pad_w - s) / 2 : pad_w - s, dh = PARITY ? (q.a_h + pad_h - r) / 2 : pad_h - r;
             tma_load_4d(a_dst, &tmA, &full[stage], c0, w0 + dw, h0 + dh, n0);
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)                                              // W[k0.. rows][tap * Cin + cin chunk]
-              tma_load_2d(b_dst + c * (BK * 128), &tmB, &full[stage], (r * g.S + s) * g.CO + tn * BN + c * 64, c0);
+              if (c < b_boxes) tma_load_2d(b_dst + c * (BK * 128), &tmB, &full[stage], (r * g.S + s) * g.CO + tn * BN + c * 64, c0);
           } else {
-            conv_tile_origin(g, kb, 64, n0, h0, w0);
 #pragma unroll
-            for (int c = 0; c < BM / 64; ++c) tma_load_4d(a_dst + c * (BK * 128), &tmA, &full[stage], tm * BM + c * 64, w0, h0, n0);
+            for (int c = 0; c < BM / 64; ++c)
+              if (c < a_boxes) tma_load_4d(a_dst + c * (BK * 128), &tmA, &full[stage], tm * BM + c * 64, w0, h0, n0);
 #pragma unroll
-            for (int c = 0; c < BN / 64; ++c) {
-              const int col = tn * BN + c * 64;  // column of dW: tap * Cin + channel
-              const int tap = col / g.CA, c0 = col % g.CA;
-              const int r = tap / g.S, s = tap % g.S;
-              // columns past the last tap read out of bounds (tap >= R S): shifted far outside so that they come back as zeros
-              tma_load_4d(b_dst + c * (BK * 128), &tmB, &full[stage], c0,
-                          tap < g.R * g.S ? g.stride * w0 + s - pad_w : -(1 << 20), g.stride * h0 + r - pad_h, n0);
+            for (int c = 0; c < BN / 64; ++c)
+              if (c < b_boxes) tma_load_4d(b_dst + c * (BK * 128), &tmB, &full[stage], col_c[c], g.stride * w0 + col_w[c], g.stride * h0 + col_h[c], n0);
+            if ((w0 += 1 << g.lbw) >= g.tiles_w << g.lbw) {                                // the next box of pixels
+              w0 = 0;
+              if ((h0 += 1 << g.lbh) >= g.tiles_h << g.lbh) { h0 = 0; n0 += 64 >> (g.lbw + g.lbh); }
             }
+          }
+          if (MODE != kConvWgrad && (c0 += BK) == g.CA) {                                  // the next tap
+            c0 = 0;
+            s += PARITY ? 2 : 1;
+            if (s >= g.S) { s = PARITY ? q.s0 : 0; r += PARITY ? 2 : 1; }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -403,13 +427,18 @@ OFB_API int ofb_conv_fprop(const void* x, const void* w, void* y, int N, int H, 
   g.tiles_w = (g.W + bw - 1) / bw; g.tiles_h = (g.H + bh - 1) / bh; g.tiles_n = (N + bn - 1) / bn;
   CUtensorMap tmA, tmB;
   if (conv_tensor_map(&tmA, x, N, H, W, Cin, bw, bh, bn, stride)) return -1;
-  const int bnt = Cout >= 256 ? 256 : 128;
-  if (get_tensor_map(&tmB, w, 2, 2, static_cast<uint64_t>(R) * S * Cin, Cout, 0, static_cast<uint64_t>(R) * S * Cin * 2, 0, 64, bnt, 0, 3))
+  const int bnt = Cout >= 256 ? 256 : (Cout > 64 ? 128 : 64);
+  if (get_tensor_map(&tmB, w, 2, 2, static_cast<uint64_t>(R) * S * Cin, Cout, 0, static_cast<uint64_t>(R) * S * Cin * 2, 0, 64, 64, 0, 3))
     return -1;
   GemmEpilogue ep;
   std::memset(&ep, 0, sizeof(ep));
   ep.C = y; ep.ldc = Cout; ep.alpha = 1.f;
   const int units = g.tiles_w * g.tiles_h * g.tiles_n * ((Cout + bnt - 1) / bnt);
+  // 64 output channels: tiles of their width (three quarters of the shared-memory traffic per K block); 256 x 56 x 56 x 64, 3 x 3, 86 us
+  // forward, 86 for the gradient of x (tiles of 128: 246 and 120)
+  if (bnt == 64) {
+    return units >= 4 * 148 ? conv_launch<kConvFprop, 64, 3, 2>(tmA, tmB, g, ep, units, stream) : conv_launch<kConvFprop, 64>(tmA, tmB, g, ep, units, stream);
+  }
   // few K blocks: the accumulator drain bounds the tile rate, two CTAs per SM (short ring) double it
   if (bnt == 128 && R * S * (Cin / 64) <= 18 && units >= 4 * 148) return conv_launch<kConvFprop, 128, 2, 2>(tmA, tmB, g, ep, units, stream);
   return bnt == 256 ? conv_launch<kConvFprop, 256>(tmA, tmB, g, ep, units, stream) : conv_launch<kConvFprop, 128>(tmA, tmB, g, ep, units, stream);
@@ -434,8 +463,14 @@ OFB_API int ofb_conv_dgrad(const void* dy, const void* w, void* dx, int N, int H
   GemmEpilogue ep;
   std::memset(&ep, 0, sizeof(ep));
   ep.C = dx; ep.ldc = Cin; ep.alpha = 1.f;
-  const int bnt = Cin >= 256 ? 256 : 128;
+  const int bnt = Cin >= 256 ? 256 : (Cin > 64 ? 128 : 64);
   const int units = stride * stride * g.tiles_w * g.tiles_h * g.tiles_n * ((Cin + bnt - 1) / bnt);
+  if (bnt == 64) {
+    if (stride == 2)
+      return units >= 4 * 148 ? conv_launch<kConvDgrad, 64, 3, 2, true>(tmA, tmB, g, ep, units, stream)
+                              : conv_launch<kConvDgrad, 64, 0, 1, true>(tmA, tmB, g, ep, units, stream);
+    return units >= 4 * 148 ? conv_launch<kConvDgrad, 64, 3, 2>(tmA, tmB, g, ep, units, stream) : conv_launch<kConvDgrad, 64>(tmA, tmB, g, ep, units, stream);
+  }
   if (stride == 2) {
     // at most four taps a tile (3 x 3): short K loops, as below
     if (bnt == 128 && units >= 4 * 148) return conv_launch<kConvDgrad, 128, 2, 2, true>(tmA, tmB, g, ep, units, stream);

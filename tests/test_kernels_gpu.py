@@ -924,6 +924,30 @@ def test_conv_implicit_gemm_stride2(N, H, W, Cin, Cout, R):
     assert _native.read_status() == (0, 0)
 
 
+@pytest.mark.parametrize("N,H,W,Cin,Cout,R,stride", [(3, 30, 28, 64, 192, 3, 1), (3, 31, 29, 192, 64, 3, 2), (8, 96, 100, 64, 64, 3, 1),
+                                                     (10, 90, 100, 64, 64, 3, 2), (2, 9, 7, 64, 64, 3, 2), (1, 8, 8, 320, 320, 3, 1),
+                                                     (2, 12, 20, 192, 64, 5, 1), (1, 3, 5, 64, 128, 7, 1)])
+def test_conv_channel_boxes(N, H, W, Cin, Cout, R, stride):
+    """Tiles of 64 channels, alone and as the last part of wider ones; a few tiles and more than four per SM; taps in every order."""
+    from oneflow_b200.ops import conv as C
+    torch.manual_seed(42)
+    x = torch.randn(N, H, W, Cin, device=DEV).to(BF)
+    w = (torch.randn(Cout, R, R, Cin, device=DEV) / math.sqrt(R * R * Cin)).to(BF)
+    x64, w64 = x.double().requires_grad_(), w.double().requires_grad_()
+    ref = torch.nn.functional.conv2d(x64.permute(0, 3, 1, 2), w64.permute(0, 3, 1, 2), stride=stride, padding=R // 2).permute(0, 2, 3, 1)
+    dy = torch.randn(ref.shape, device=DEV).to(BF)
+    ref.backward(dy.double())
+    # fp32 sums of n terms: at most n / 16 (16 terms an instruction) roundings of 2^-23 on partial sums below 8 (32 for the gradient of x,
+    # whose terms are not normalised, 8 sqrt(n) for that of w); results in bf16 another 2^-9 of their size
+    n = R * R * max(Cin, Cout)
+    torch.testing.assert_close(C.conv_fprop(x, w, stride).double(), ref.detach(), rtol=2.0 ** -8, atol=n / 16 * 2.0 ** -20 + 1e-6)
+    torch.testing.assert_close(C.conv_dgrad(dy, w, None, stride, (H, W)).double(), x64.grad, rtol=2.0 ** -8, atol=n / 16 * 2.0 ** -18 + 1e-6)
+    px = N * ref.shape[1] * ref.shape[2]
+    torch.testing.assert_close(C.conv_wgrad(x, dy, (R, R), stride=stride).double(), w64.grad, rtol=1e-5, atol=px / 16 * 2.0 ** -20 * px ** 0.5)
+    torch.cuda.synchronize()
+    assert _native.read_status() == (0, 0)
+
+
 def test_conv_stride_arguments():
     from oneflow_b200.ops import conv as C
     x, w = torch.zeros(1, 6, 6, 64, device="cuda", dtype=BF), torch.zeros(64, 3, 3, 64, device="cuda", dtype=BF)
