@@ -212,7 +212,7 @@ int gemm_dispatch(const OfbGemmArgs* a, const GemmEpilogue& ep, cudaStream_t str
     if (get_tensor_map(&tmA, a->A, 2, 2, a->M, a->K, 0, (uint64_t)a->lda * 2, 0, 64, 64, 0, 3)) return -1;
   }
   if (!b_mn) {
-    if (get_tensor_map(&tmB, a->B, 2, 2, a->K, a->N, 0, (uint64_t)a->ldb * 2, 0, 64, gemm_b_rows(a->N, bn), 0, 3)) return -1;
+    if (get_tensor_map(&tmB, a->B, 2, 2, a->K, a->N, 0, (uint64_t)a->ldb * 2, 0, 64, a_mn ? bn : gemm_b_rows(a->N, bn), 0, 3)) return -1;
   } else {
     if (get_tensor_map(&tmB, a->B, 2, 2, a->N, a->K, 0, (uint64_t)a->ldb * 2, 0, 64, 64, 0, 3)) return -1;
   }
