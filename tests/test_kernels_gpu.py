@@ -1019,6 +1019,25 @@ def test_gemm_masked_residual(M, N, K, layout, bias):
         G.gemm(x, w, residual_mask=mask)
 
 
+@pytest.mark.parametrize("N", [8, 56, 64, 72, 128, 184, 192, 200])
+@pytest.mark.parametrize("bn", [0, 128, 256])
+def test_gemm_narrow_tile(N, bn):
+    """All of N in one tile, from a part of one 64-row box of weights to the whole tile; all layouts, a last K block that is not full."""
+    from oneflow_b200.ops import gemm as G
+    torch.manual_seed(43)
+    M, K = 328, 200
+    x, w = torch.randn(M, K, device=DEV, dtype=BF), torch.randn(N, K, device=DEV, dtype=BF) * K ** -0.5
+    ref = x.double() @ w.double().t()
+    for al in ("mk", "km"):
+        for bl in ("nk", "kn"):
+            y = G.gemm(x if al == "mk" else x.t().contiguous(), w if bl == "nk" else w.t().contiguous(), a_layout=al, b_layout=bl, bn=bn,
+                       out_dtype=torch.float32)
+            # fp32 sums of K products of size K^-1/2: at most K / 16 roundings of 2^-23 on partial sums below 8
+            torch.testing.assert_close(y.double(), ref, rtol=1e-6, atol=K / 16 * 2.0 ** -20)
+    torch.cuda.synchronize()
+    assert _native.read_status() == (0, 0)
+
+
 def test_flow_conv2d_channels_last_uses_igemm():
     import oneflow_b200 as flow
     torch.manual_seed(0)
